@@ -232,15 +232,21 @@ struct flite_ctx {
 
     // ---- single-grid building blocks ------------------------------------
     LevelView &V(int l) { return lv[l].v; }
-    // small levels gather with a warp per node (the lanes load and evaluate
-    // the incidences in parallel, the sums keep their order): there a
-    // thread per node leaves most SMs idle and each thread waits on a long
-    // chain of dependent loads
-    // lanes per node of each level's gathers (1, 4, 8, 16 or 32)
+    // lanes per node of each level's gathers (1, 4, 8, 16 or 32).  By
+    // default the widest group that keeps the level's threads within
+    // kLaneThreads: below that a thread per node leaves SMs idle and each
+    // thread waits on a long chain of dependent loads, above it the extra
+    // lanes only add instructions.  Sums of one relaxation step's kernels on
+    // bump-channel levels (us, lanes 1/4/8/32): 788 nodes 192/118/98/84,
+    // 1,707 147/103/91/82, 8,731 199/137/110/129, 23,549 156/135/134/209,
+    // 80,640 144/202/245/527.  A case group's cases share the launch.
     int lanes[kMaxLevels] = {0};
     int lanes_of(int l) const {
         if (l < kMaxLevels && lanes[l] > 0) return lanes[l];
-        return lv[l].v.N < kSmallLevelNodes ? 32 : 1;
+        const size_t n = (size_t)lv[l].v.N * std::max(group, 1);
+        for (int u = 32; u > 2; u /= 2)
+            if (u * n <= kLaneThreads) return u;
+        return 1;
     }
     unsigned gblk(int l, int g) const { return (unsigned)((g * (size_t)lv[l].v.N + nb - 1) / nb); }
     // levels whose gathers that walk the same incidence list share one walk

@@ -32,31 +32,68 @@ namespace flite {
 static __device__ __forceinline__ int tid() { return blockIdx.x * blockDim.x + threadIdx.x; }
 
 // Group-per-node gathers (small levels): U lanes (a power of two up to 32)
-// serve one node.  Lane l of a group evaluates the terms of incidence k0 + l;
-// the group then applies them to the node's accumulators in incidence order,
-// every lane doing the same additions on broadcast terms, so the sums are
-// those of the serial loop bit for bit.  Groups past the last node stay in
-// the loop (the shuffles need every lane) but apply nothing.
-template <int U, int K, class T, class Terms, class Add>
-__device__ __forceinline__ void group_gather(int beg, int end, bool active, int gl, Terms &&terms, Add &&add) {
+// serve one node, M sums of the node take R terms each from every incidence.
+// Lane l of the group evaluates the M*R terms of incidence k0 + l and leaves
+// them in the warp's shared slab gs[term][lane] (rows of 33 values: the lanes
+// that read different terms of one incidence hit different banks); lane m of
+// the group then adds sum m's terms in incidence order, so the sums are those
+// of the serial loop bit for bit (lanes past the last incidence leave zeros,
+// and x + 0 is x).  `out` holds the sums so far on entry and the new ones, in
+// every lane, on return.  Groups past the last node stay in the loop (the
+// warp's barriers need every lane) but add nothing.
+// What bounds it: the latency of one node's chain.  The serial part is one
+// add per term on M lanes at once; broadcasting every term to every lane
+// instead takes 2 M R shuffles and M R adds per incidence of the warp.
+constexpr int kSlabRow = 33;
+template <int U, int M, int R, class T, class Terms>
+__device__ __forceinline__ void group_sum(T *gs, int beg, int end, bool active, int gl, Terms &&terms, T *out) {
+    constexpr int C = (M + U - 1) / U;  // sums per lane
+    constexpr int S = U < 8 ? U : 8;    // incidences added per step
+    const int lane = (int)(threadIdx.x & 31), g0 = lane - gl;
+    T acc[C];
+#pragma unroll
+    for (int c = 0; c < C; ++c) acc[c] = T(0);
+#pragma unroll
+    for (int m = 0; m < M; ++m)
+        if (m % U == gl) acc[m / U] = out[m];
     const int span = active ? end - beg : 0;
-    const unsigned trips = (unsigned)((span + U - 1) / U);
-    const unsigned maxtrips = __reduce_max_sync(0xffffffffu, trips);
-    for (unsigned t = 0; t < maxtrips; ++t) {
-        const int k0 = beg + (int)t * U;
-        T v[K];
+    const int longest = (int)__reduce_max_sync(0xffffffffu, (unsigned)span);
+    for (int t = 0; t < longest; t += U) {
+        T v[M * R];
 #pragma unroll
-        for (int c = 0; c < K; ++c) v[c] = T(0);
-        if (active && k0 + gl < end) terms(k0 + gl, v);
-        const int n = active ? min(U, end - k0) : 0;
-        for (int q = 0; q < U; ++q) {
-            T x[K];
+        for (int c = 0; c < M * R; ++c) v[c] = T(0);
+        if (t + gl < span) terms(beg + t + gl, v);
 #pragma unroll
-            for (int c = 0; c < K; ++c) x[c] = __shfl_sync(0xffffffffu, v[c], q, U);
-            if (q < n) add(x);
+        for (int c = 0; c < M * R; ++c) gs[c * kSlabRow + lane] = v[c];
+        __syncwarp();
+        const int n = min(U, longest - t);
+        for (int q = 0; q < n; q += S) {
+            T x[C][S][R];
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                const int m = gl + c * U < M ? gl + c * U : 0;
+#pragma unroll
+                for (int k = 0; k < S; ++k)
+#pragma unroll
+                    for (int r = 0; r < R; ++r) x[c][k][r] = gs[(m * R + r) * kSlabRow + g0 + q + k];
+            }
+#pragma unroll
+            for (int k = 0; k < S; ++k)
+#pragma unroll
+                for (int r = 0; r < R; ++r)
+#pragma unroll
+                    for (int c = 0; c < C; ++c) acc[c] = acc[c] + x[c][k][r];
         }
+        __syncwarp();
     }
+#pragma unroll
+    for (int m = 0; m < M; ++m) out[m] = __shfl_sync(0xffffffffu, acc[m / U], m % U, U);
 }
+// the calling warp's slab of K terms out of the block's (blocks of at most
+// 256 threads)
+#define FLITE_GROUP_SLAB(T, K)                                   \
+    __shared__ T gslab_[U > 1 ? 8 * (K)*kSlabRow : 1];           \
+    T *gs = gslab_ + (U > 1 ? (threadIdx.x >> 5) * (K)*kSlabRow : 0)
 
 // ---- makePressureField (def_par:13612-13630) ------------------------------
 template <bool B>
@@ -161,38 +198,34 @@ __global__ void k_timestep(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_) {
     const double ri = L.u[i], ro = 1. / ri;
     const double m1 = L.u[N + i], m2 = L.u[2 * N + i], m3 = L.u[3 * N + i];
     const double cc = dmax(c1 * L.p[i] * ro, 0.001);
-    double acc = 0.0, h = 0.0;
     if constexpr (U > 1) {
-        const int beg = L.inc_ptr[i], end = L.inc_ptr[i + 1];
-        group_gather<U, 3, double>(
-            beg, end, active, gl,
+        FLITE_GROUP_SLAB(double, 8);
+        // sum 0: the convective and acoustic terms; sum 1: the viscous ones
+        double x[2] = {0.0, 0.0};
+        group_sum<U, 2, 2, double>(
+            gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl,
             [&](int k, double *v) {
-            const int2 t = L.inc[k];
-            const int e = t.x >= 0 ? t.x : ~t.x;
-            const double wx = L.wx[e], wy = L.wy[e], wz = L.wz[e];
-            const double al = (wx * wx + wy * wy) + wz * wz;
-            const double vn = ((wx * m1 + wy * m2) + wz * m3) * ro;
-            v[0] = fabs(vn);
-            v[1] = sqrt(cc * al);
-            if (P.viscous) {
-                const int j = t.y;
-                const double vis = dmax(P.am, P.sa ? L.mu[j] + L.u[5 * N + j] / P.Re : L.mu[j]);
-                v[2] = 2.0 * vis * al / L.u[j];
-            }
+                const int2 t = L.inc[k];
+                const int e = t.x >= 0 ? t.x : ~t.x;
+                const double wx = L.wx[e], wy = L.wy[e], wz = L.wz[e];
+                const double al = (wx * wx + wy * wy) + wz * wz;
+                const double vn = ((wx * m1 + wy * m2) + wz * m3) * ro;
+                v[0] = fabs(vn);
+                v[1] = sqrt(cc * al);
+                if (P.viscous) {
+                    const int j = t.y;
+                    const double vis = dmax(P.am, P.sa ? L.mu[j] + L.u[5 * N + j] / P.Re : L.mu[j]);
+                    v[2] = 2.0 * vis * al / L.u[j];
+                }
             },
-            [&](const double *x) {
-            acc = (acc + x[0]) + x[1];
-            if (P.viscous) h = h + x[2];
-            });
-    } else
-    for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) ts_inc(P, L, L.inc[k], m1, m2, m3, ro, cc, acc, h);
-    auto bterms = [&](int k, double *v) { ts_bterms(P, L, k, v); };
-    auto badd = [&](const double *x) { ts_badd(P, x, acc, h); };
-    if constexpr (U > 1) {
-        group_gather<U, 6, double>(L.binc_ptr[i], L.binc_ptr[i + 1], active, gl, bterms, badd);
+            x);
+        group_sum<U, 2, 4, double>(
+            gs, L.binc_ptr[i], L.binc_ptr[i + 1], active, gl, [&](int k, double *v) { ts_bterms(P, L, k, v); }, x);
         if (!active || gl) return;
-        ts_store(L, i, acc, h);
+        ts_store(L, i, x[0], x[1]);
     } else {
+        double acc = 0.0, h = 0.0;
+        for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) ts_inc(P, L, L.inc[k], m1, m2, m3, ro, cc, acc, h);
         ts_finish(P, L, i, acc, h);
     }
 }
@@ -245,46 +278,43 @@ __global__ void k_jst_lap(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_) {
     const bool active = i_raw < L.N;
     const int i = active ? i_raw : L.N - 1;  // idle groups read a valid node
     const int N = L.N;
-    double l0 = 0, l1 = 0, l2 = 0, l3 = 0, l4 = 0, s7 = 0, s8 = 0;
-    const double ui0 = L.u[i], ui1 = L.u[N + i], ui2 = L.u[2 * N + i], ui3 = L.u[3 * N + i], ui4 = L.u[4 * N + i];
+    const double ui[5] = {L.u[i], L.u[N + i], L.u[2 * N + i], L.u[3 * N + i], L.u[4 * N + i]};
     const double pi = L.p[i];
     if constexpr (U > 1) {
-        const int beg = L.inc_ptr[i], end = L.inc_ptr[i + 1];
-        group_gather<U, 7, double>(
-            beg, end, active, gl,
+        FLITE_GROUP_SLAB(double, 7);
+        double x[7] = {0, 0, 0, 0, 0, 0, 0};
+        group_sum<U, 7, 1, double>(
+            gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl,
             [&](int k, double *v) {
-            const int2 t = L.inc[k];
-            const int j = t.y;
-            double df = 1.0;
-            if (P.useDissW) df = 1. / L.slen[t.x >= 0 ? t.x : ~t.x];
-            const double uj0 = L.u[j], uj1 = L.u[N + j], uj2 = L.u[2 * N + j], uj3 = L.u[3 * N + j];
-            const double uj4 = L.u[4 * N + j], pj = L.p[j];
-            // x - y is x + (-y): the subtractions of the serial loop become
-            // additions of negated terms
-            if (t.x >= 0) {
-                v[0] = -((ui0 - uj0) * df); v[1] = -((ui1 - uj1) * df); v[2] = -((ui2 - uj2) * df);
-                v[3] = -((ui3 - uj3) * df); v[4] = -((((ui4 - uj4) + pi) - pj) * df);
-                v[5] = -(pi - pj); v[6] = pi + pj;
-            } else {
-                v[0] = (uj0 - ui0) * df; v[1] = (uj1 - ui1) * df; v[2] = (uj2 - ui2) * df;
-                v[3] = (uj3 - ui3) * df; v[4] = (((uj4 - ui4) + pj) - pi) * df;
-                v[5] = pj - pi; v[6] = pj + pi;
-            }
+                const int2 t = L.inc[k];
+                const int j = t.y;
+                double df = 1.0;
+                if (P.useDissW) df = 1. / L.slen[t.x >= 0 ? t.x : ~t.x];
+                const double uj[5] = {L.u[j], L.u[N + j], L.u[2 * N + j], L.u[3 * N + j], L.u[4 * N + j]};
+                const double pj = L.p[j];
+                // x - y is x + (-y): the subtractions of the serial loop become
+                // additions of negated terms
+                if (t.x >= 0) {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) v[c] = -((ui[c] - uj[c]) * df);
+                    v[4] = -((((ui[4] - uj[4]) + pi) - pj) * df);
+                    v[5] = -(pi - pj); v[6] = pi + pj;
+                } else {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) v[c] = (uj[c] - ui[c]) * df;
+                    v[4] = (((uj[4] - ui[4]) + pj) - pi) * df;
+                    v[5] = pj - pi; v[6] = pj + pi;
+                }
             },
-            [&](const double *x) {
-            l0 = l0 + x[0]; l1 = l1 + x[1]; l2 = l2 + x[2]; l3 = l3 + x[3]; l4 = l4 + x[4];
-            s7 = s7 + x[5]; s8 = s8 + x[6];
-            });
+            x);
         if (!active || gl) return;
+        const LapAcc a = {{x[0], x[1], x[2], x[3], x[4]}, x[5], x[6]};
+        lap_store(L, i, a);
     } else {
         LapAcc a = {{0, 0, 0, 0, 0}, 0, 0};
-        const double ui[5] = {ui0, ui1, ui2, ui3, ui4};
         for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) lap_inc(P, L, L.inc[k], ui, pi, a);
         lap_store(L, i, a);
-        return;
     }
-    LapAcc a = {{l0, l1, l2, l3, l4}, s7, s8};
-    lap_store(L, i, a);
 }
 
 // ---- makeArtificialDissipation2, pass 3 (def_par:11770-11906), scalar -----
@@ -332,9 +362,9 @@ __global__ void __launch_bounds__(256, U == 1 ? 4 : 1) k_jst_flux(CaseArg<B, Par
     for (int c = 0; c < 5; ++c) { Li[c] = L.lap[c * N + i]; Ui[c] = L.u[c * N + i]; }
     const double vdi = L.vdt[i], coni = L.conn[i], si = L.sens[i];
     if constexpr (U > 1) {
-        const int beg = L.inc_ptr[i], end = L.inc_ptr[i + 1];
-        group_gather<U, 10, double>(
-            beg, end, active, gl,
+        FLITE_GROUP_SLAB(double, 10);
+        group_sum<U, 5, 2, double>(
+            gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl,
             [&](int k, double *v) {
             const int2 t = L.inc[k];
             const int j = t.y;
@@ -357,9 +387,7 @@ __global__ void __launch_bounds__(256, U == 1 ? 4 : 1) k_jst_flux(CaseArg<B, Par
                 }
             }
             },
-            [&](const double *x) {
-            for (int c = 0; c < 5; ++c) acc[c] = (acc[c] + x[2 * c]) + x[2 * c + 1];
-            });
+            acc);
         if (!active || gl) return;
     } else
     for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) jflux_inc(P, L, L.inc[k], k4, vdi, coni, si, Li, Ui, acc);
@@ -717,8 +745,9 @@ __global__ void __launch_bounds__(256, U == 1 ? 3 : 1) k_visc_grad(CaseArg<B, Pa
         for (int c = 0; c < 12; ++c) g[c] = g[c] + d[c];
     };
     if constexpr (U > 1) {
-        group_gather<U, 12, double>(L.inc_ptr[i], L.inc_ptr[i + 1], active, gl, iterms, add);
-        group_gather<U, 12, double>(L.binc_ptr[i], L.binc_ptr[i + 1], active, gl, bterms, add);
+        FLITE_GROUP_SLAB(double, 12);
+        group_sum<U, 12, 1, double>(gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl, iterms, g);
+        group_sum<U, 12, 1, double>(gs, L.binc_ptr[i], L.binc_ptr[i + 1], active, gl, bterms, g);
         if (!active || gl) return;
     } else {
         for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) vgrad_inc(L, L.inc[k], qi, g);
@@ -827,8 +856,19 @@ __global__ void __launch_bounds__(256, U == 1 ? 3 : 1) k_visc_flux(CaseArg<B, Pa
         for (int c = 0; c < 4; ++c) acc[c] = (acc[c] + g[c]) + g[4 + c];
     };
     if constexpr (U > 1) {
-        group_gather<U, 4, double>(L.inc_ptr[i], L.inc_ptr[i + 1], active, gl, iterms, iadd);
-        group_gather<U, 9, double>(L.binc_ptr[i], L.binc_ptr[i + 1], active, gl, bterms, badd);
+        FLITE_GROUP_SLAB(double, 8);
+        group_sum<U, 4, 1, double>(gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl, iterms, acc);
+        // a face that does not count leaves zeros
+        group_sum<U, 4, 2, double>(
+            gs, L.binc_ptr[i], L.binc_ptr[i + 1], active, gl,
+            [&](int k, double *v) {
+                double t[9];
+                bterms(k, t);
+                if (t[8] == 0.0) return;
+#pragma unroll
+                for (int c = 0; c < 4; ++c) { v[2 * c] = t[c]; v[2 * c + 1] = t[4 + c]; }
+            },
+            acc);
         if (!active || gl) return;
     } else {
         for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) {
@@ -1010,8 +1050,9 @@ __global__ void __launch_bounds__(256, U == 1 ? 3 : 1) k_visc2_grad(CaseArg<B, P
         for (int c = 0; c < 12; ++c) g[c] = g[c] + d[c];
     };
     if constexpr (U > 1) {
-        group_gather<U, 12, double>(L.inc_ptr[i], L.inc_ptr[i + 1], active, gl, iterms, add);
-        group_gather<U, 12, double>(L.binc_ptr[i], L.binc_ptr[i + 1], active, gl, bterms, add);
+        FLITE_GROUP_SLAB(double, 12);
+        group_sum<U, 12, 1, double>(gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl, iterms, g);
+        group_sum<U, 12, 1, double>(gs, L.binc_ptr[i], L.binc_ptr[i + 1], active, gl, bterms, g);
         if (!active || gl) return;
     } else {
         for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) {
@@ -1138,8 +1179,18 @@ __global__ void __launch_bounds__(256, U == 1 ? 2 : 1) k_visc2_flux(CaseArg<B, P
         for (int c = 0; c < 4; ++c) acc[c] = acc[c] + g[c];
     };
     if constexpr (U > 1) {
-        group_gather<U, 4, double>(L.inc_ptr[i], L.inc_ptr[i + 1], active, gl, iterms, iadd);
-        group_gather<U, 5, double>(L.binc_ptr[i], L.binc_ptr[i + 1], active, gl, bterms, badd);
+        FLITE_GROUP_SLAB(double, 4);
+        group_sum<U, 4, 1, double>(gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl, iterms, acc);
+        group_sum<U, 4, 1, double>(
+            gs, L.binc_ptr[i], L.binc_ptr[i + 1], active, gl,
+            [&](int k, double *v) {
+                double t[5];
+                bterms(k, t);
+                if (t[4] == 0.0) return;
+#pragma unroll
+                for (int c = 0; c < 4; ++c) v[c] = t[c];
+            },
+            acc);
         if (!active || gl) return;
     } else {
         for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) {
@@ -1477,8 +1528,8 @@ __device__ __forceinline__ void delta_flux(const DeltaRec &n, float wx, float wy
 // interior residual of node i as the anchor's FP64 sum plus the FP32 sum of
 // the flux increments of its edges
 template <int U>
-__device__ __forceinline__ void gather_interior_delta(const LevelView &L, int i, double *r, bool active = true,
-                                         int gl = 0) {
+__device__ __forceinline__ void gather_interior_delta(const LevelView &L, int i, double *r, bool active, int gl,
+                                                      double *gs) {
     float acc[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
     const DeltaRec me = load_delta(L.dq, i);
     auto terms = [&](int k, float *s5, bool &first) {
@@ -1491,18 +1542,15 @@ __device__ __forceinline__ void gather_interior_delta(const LevelView &L, int i,
         for (int c = 0; c < 5; ++c) s5[c] = g1[c] + g2[c];
     };
     if constexpr (U > 1) {
-        // the terms carry the node's sign of the edge as a sixth value
-        group_gather<U, 6, float>(
-            L.inc_ptr[i], L.inc_ptr[i + 1], active, gl,
+        group_sum<U, 5, 1, float>(
+            reinterpret_cast<float *>(gs), L.inc_ptr[i], L.inc_ptr[i + 1], active, gl,
             [&](int k, float *v) {
                 bool first;
                 terms(k, v, first);
-                v[5] = first ? 1.f : 0.f;
+                if (!first)
+                    for (int c = 0; c < 5; ++c) v[c] = -v[c];  // x - y is x + (-y)
             },
-            [&](const float *x) {
-                const bool f = x[5] != 0.f;
-                for (int c = 0; c < 5; ++c) acc[c] = f ? acc[c] + x[c] : acc[c] - x[c];
-            });
+            acc);
     } else {
         for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) {
             float v[5];
@@ -1556,8 +1604,8 @@ __device__ __forceinline__ void gather_interior_central2(const LevelView &L, int
 // each incident edge, summed in edge order: the same numbers, in the same
 // order, as the edge kernel followed by the buffer gather
 template <int U>
-__device__ __forceinline__ void gather_interior_central(const LevelView &L, int i, double *r, bool active = true,
-                                         int gl = 0) {
+__device__ __forceinline__ void gather_interior_central(const LevelView &L, int i, double *r, bool active, int gl,
+                                                        double *gs) {
     r[0] = r[1] = r[2] = r[3] = r[4] = 0.0;
     const NodeRec si = load_node(L.q, i);
     // the flux of incidence k with this node's sign (x - y is x + (-y))
@@ -1579,7 +1627,7 @@ __device__ __forceinline__ void gather_interior_central(const LevelView &L, int 
         r[0] = r[0] + g[0]; r[1] = r[1] + g[1]; r[2] = r[2] + g[2]; r[3] = r[3] + g[3]; r[4] = r[4] + g[4];
     };
     if constexpr (U > 1) {
-        group_gather<U, 5, double>(L.inc_ptr[i], L.inc_ptr[i + 1], active, gl, terms, add);
+        group_sum<U, 5, 1, double>(gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl, terms, r);
     } else {
         for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) {
             double v[5];
@@ -1591,8 +1639,8 @@ __device__ __forceinline__ void gather_interior_central(const LevelView &L, int 
 
 // interior edges of node i from the FP64 edge buffer, in edge order
 template <int U>
-__device__ __forceinline__ void gather_interior(const LevelView &L, int i, double *r, bool active = true,
-                                         int gl = 0) {
+__device__ __forceinline__ void gather_interior(const LevelView &L, int i, double *r, bool active, int gl,
+                                                double *gs) {
     r[0] = r[1] = r[2] = r[3] = r[4] = 0.0;
     auto terms = [&](int k, double *g) {
         const int s = L.inc[k].x;
@@ -1603,7 +1651,7 @@ __device__ __forceinline__ void gather_interior(const LevelView &L, int i, doubl
         r[0] = r[0] + g[0]; r[1] = r[1] + g[1]; r[2] = r[2] + g[2]; r[3] = r[3] + g[3]; r[4] = r[4] + g[4];
     };
     if constexpr (U > 1) {
-        group_gather<U, 5, double>(L.inc_ptr[i], L.inc_ptr[i + 1], active, gl, terms, add);
+        group_sum<U, 5, 1, double>(gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl, terms, r);
     } else {
         for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) {
             double v[5];
@@ -1620,7 +1668,7 @@ __device__ __forceinline__ void gather_interior(const LevelView &L, int i, doubl
 // entry following its first in the node's list
 template <int U>
 __device__ __forceinline__ void gather_boundary(const LevelView &L, int i, double *r, bool active = true,
-                                         int gl = 0) {
+                                                int gl = 0, double *gs = nullptr) {
     auto terms = [&](int k, double *g) {
         const int v = L.binc[k];
         const double *b = L.bflux + (size_t)(v >> 1) * 10 + (v & 1) * 5;
@@ -1649,8 +1697,28 @@ __device__ __forceinline__ void gather_boundary(const LevelView &L, int i, doubl
         }
     };
     if constexpr (U > 1) {
-        if (L.bgterm) group_gather<U, 11, double>(L.binc_ptr[i], L.binc_ptr[i + 1], active, gl, terms_gcl, add_gcl);
-        else group_gather<U, 5, double>(L.binc_ptr[i], L.binc_ptr[i + 1], active, gl, terms, add);
+        if (L.bgterm) {
+            // two terms per entry: -t, +g; a self-edge's entries, which follow
+            // one another, give -t1, -t2 and +g1, +g2
+            group_sum<U, 5, 2, double>(
+                gs, L.binc_ptr[i], L.binc_ptr[i + 1], active, gl,
+                [&](int k, double *g) {
+                    const int v = L.binc[k];
+                    const size_t o = (size_t)(v >> 1) * 10, own = o + (v & 1) * 5;
+                    const int2 nd = L.bedge[v >> 1];
+                    const bool self = nd.x == nd.y;
+                    const double *t = self ? ((v & 1) ? L.bflux + o : L.bgterm + o) : L.bgterm + own;
+                    const double *f = self ? t + 5 : L.bflux + own;
+                    const bool plus0 = self && (v & 1), minus1 = self && !(v & 1);
+                    for (int c = 0; c < 5; ++c) {
+                        g[2 * c] = plus0 ? t[c] : -t[c];
+                        g[2 * c + 1] = minus1 ? -f[c] : f[c];
+                    }
+                },
+                r);
+        } else {
+            group_sum<U, 5, 1, double>(gs, L.binc_ptr[i], L.binc_ptr[i + 1], active, gl, terms, r);
+        }
     } else if (L.bgterm) {
         for (int k = L.binc_ptr[i]; k < L.binc_ptr[i + 1]; ++k) {
             double v[11];
@@ -1691,9 +1759,23 @@ __device__ __forceinline__ void store_anchor(const LevelView &L, int i, const do
 // one-step forms (modes as in k_node_update)
 // LEAN: a run without engine conditions and without explicit time stepping
 // (the branches for those are left out of the code)
+struct TailIn {  // what the tail reads of its node, loaded ahead by the group gathers
+    double diss[5], up[5], dt, V, p;
+    unsigned char cls;
+};
+__device__ __forceinline__ TailIn load_tail(const LevelView &L, int i) {
+    const int N = L.N;
+    TailIn t;
+    t.dt = L.dt[i];
+    t.V = L.V[i];
+    t.p = L.p[i];
+    t.cls = L.bc[i];
+    for (int c = 0; c < 5; ++c) { t.diss[c] = L.diss[c * N + i]; t.up[c] = L.uprev[c * N + i]; }
+    return t;
+}
 template <bool LEAN = false>
 __device__ __forceinline__ void node_tail(const Params &P, const LevelView &L, int i, double *r, int mode,
-                                          int stage) {
+                                          int stage, const TailIn *in = nullptr) {
     const int N = L.N;
     if (mode == MODE_RESID) {
         for (int c = 0; c < 5; ++c) L.rhs[c * N + i] = r[c];
@@ -1701,13 +1783,13 @@ __device__ __forceinline__ void node_tail(const Params &P, const LevelView &L, i
     }
     if (P.addts && mode == MODE_STAGE)  // addTimeDifferences (def_par:1184-1241)
         for (int c = 0; c < 5; ++c) r[c] = r[c] + time_difference(P, L, i, c);
-    for (int c = 0; c < 5; ++c) r[c] = r[c] + L.diss[c * N + i];
-    double dt = L.dt[i];
-    const double V = L.V[i];
+    for (int c = 0; c < 5; ++c) r[c] = r[c] + (in ? in->diss[c] : L.diss[c * N + i]);
+    double dt = in ? in->dt : L.dt[i];
+    const double V = in ? in->V : L.V[i];
     // solveSystem's dual-time step, or the explicit global step (def_par:1427-1442)
     if (P.unsteady) dt = (!LEAN && P.explicit_) ? *L.ptsg : dt / (1.0 + 1.5 * dt / P.dtp);
     for (int c = 0; c < 5; ++c) r[c] = dt * r[c] / V;  // solveSystem
-    const unsigned char cls = L.bc[i];
+    const unsigned char cls = in ? in->cls : L.bc[i];
     double n0 = 0, n1 = 0, n2 = 0;
     if (cls != BC_NONE) { n0 = L.nx[i]; n1 = L.ny[i]; n2 = L.nz[i]; }
     bc_increment<!LEAN>(P, cls, n0, n1, n2, r);
@@ -1716,7 +1798,7 @@ __device__ __forceinline__ void node_tail(const Params &P, const LevelView &L, i
     if (P.sa && L.grid > 1 && (cls == BC_FAR3 || (!LEAN && is_engine(cls)))) r[0] = r[1] = r[2] = r[3] = r[4] = 0.0;
     const double dtJ = stage > 0 ? P.CFL * P.RK[stage - 1] : P.CFL;
     double d[5], up[5], un[5];
-    for (int c = 0; c < 5; ++c) { d[c] = dtJ * r[c]; up[c] = L.uprev[c * N + i]; }
+    for (int c = 0; c < 5; ++c) { d[c] = dtJ * r[c]; up[c] = in ? in->up[c] : L.uprev[c * N + i]; }
     clipped_update(P, up, d, un);
     if (mode == MODE_RFINE) {
         // the density floor of updateSolutionVector acts on grp%u, which is
@@ -1781,24 +1863,28 @@ __global__ void __launch_bounds__(256, PREC == GATHER_CENTRAL2 ? 2 : (U == 1 ? 3
     const bool active = i_raw < L.N;
     const int i = active ? i_raw : L.N - 1;  // idle groups read a valid node
     double r[5];
+    FLITE_GROUP_SLAB(double, 10);
+    // a node's own operands are read before the chain of its gather starts
+    TailIn in;
+    if constexpr (U > 1) in = load_tail(L, i);
     if constexpr (PREC == GATHER_DELTA) {
-        gather_interior_delta<U>(L, i, r, active, gl);
+        gather_interior_delta<U>(L, i, r, active, gl, gs);
     } else if constexpr (PREC == GATHER_BUFFER) {
-        gather_interior<U>(L, i, r, active, gl);
+        gather_interior<U>(L, i, r, active, gl, gs);
     } else if constexpr (PREC == GATHER_CENTRAL2) {
         gather_interior_central2(L, i, r);
     } else {
-        gather_interior_central<U>(L, i, r, active, gl);
+        gather_interior_central<U>(L, i, r, active, gl, gs);
     }
     double rint[5];
     if constexpr (PREC == GATHER_ANCHOR)
         for (int c = 0; c < 5; ++c) rint[c] = r[c];
-    gather_boundary<U>(L, i, r, active, gl);
+    gather_boundary<U>(L, i, r, active, gl, gs);
     // with a group per node every lane holds the same sums; one lane goes on
     if constexpr (U > 1)
         if (!active || gl) return;
     if constexpr (PREC == GATHER_ANCHOR) store_anchor(L, i, rint);
-    node_tail<PREC == GATHER_LEAN>(P, L, i, r, mode, stage);
+    node_tail<PREC == GATHER_LEAN>(P, L, i, r, mode, stage, U > 1 ? &in : nullptr);
 }
 // ---- the same node update with the central fluxes gathered from a
 // shared-memory stage of the node block (GATHER_CENTRAL, a thread per node).

@@ -53,9 +53,9 @@ __global__ void k_bnd_flux(CaseArg<B, Params> P, CaseArg<B, LevelView> L);
 enum { GATHER_BUFFER = 0, GATHER_CENTRAL = 1, GATHER_ANCHOR = 2, GATHER_DELTA = 3, GATHER_CENTRAL2 = 4, GATHER_LEAN = 5 };
 template <int PREC, int U, bool B = false>
 __global__ void k_node_update(CaseArg<B, Params> P, CaseArg<B, LevelView> L, int mode, int stage);
-// gathers: U lanes per node (1 = a thread per node); by default levels
-// below kSmallLevelNodes nodes use a warp per node
-constexpr int kSmallLevelNodes = 8192;
+// gathers: U lanes per node (1 = a thread per node); by default the widest
+// group with at most this many threads on the level (flite_ctx::lanes_of)
+constexpr size_t kLaneThreads = 98304;
 constexpr int kMaxLevels = 16;
 template <bool B = false>
 __global__ void k_delta_state(CaseArg<B, LevelView> L);

@@ -414,8 +414,8 @@ int flite_set_kernel_options(flite_ctx *ctx, int32_t edge_block, int32_t node_bl
  * numbering; edges keep their numbers.                                      */
 int flite_set_node_order(int32_t order);
 /* Lanes per node of the node gathers of a level (no effect on any result):
- * 1 (a thread per node), 4, 8, 16 or 32, or 0 for the default (32 below 8192
- * nodes, else 1).  Drops the captured cycle graph.                         */
+ * 1 (a thread per node), 4, 8, 16 or 32, or 0 for the default (the widest group
+ * that keeps the level within 98,304 threads).  Drops the captured cycle graph. */
 int flite_set_gather_lanes(flite_ctx *ctx, int32_t level, int32_t lanes);
 /* How a level's fused central gather with a thread per node (fluxType 1,
  * FP64) reads its incidences: 0 (the default) through the node's incidence

@@ -1,0 +1,53 @@
+"""Every gather shape gives the state of a thread per node bit for bit: groups
+of 4, 8, 16 and 32 lanes (one node's terms added by one lane per sum), on a
+mesh whose node counts leave a partly filled last warp on each level, and the
+default choice on levels on both sides of its threshold.
+"""
+import numpy as np
+import pytest
+
+from flite3d_b200 import Mesh, Solver, default_controls, initial_state
+
+pytestmark = pytest.mark.gpu
+
+CASES = {
+    "euler": dict(),
+    "weighted": dict(useDissipationWeighting=1),
+    "hllc2": dict(fluxType=4, HLLCFluxOrder=2, Automaticlipping=1, CFLNumber=1.0),
+    "laminar": dict(ReynoldsNumber=500.0, CFLNumber=1.0, wallsAreIsentropic=1),
+    "laminar_compact": dict(ReynoldsNumber=500.0, CFLNumber=1.0, viscosityScheme=2),
+    "mixed": dict(precision=1),
+}
+
+
+def states(mesh, ctl, lanes, cycles=2):
+    c = default_controls(**{**dict(ReynoldsNumber=0.0, fluxType=1, CFLNumber=2.0, multigridScheme=3,
+                                   numberOfGridsToUse=mesh.nlevels), **ctl})
+    s = Solver(c, mesh)
+    for level in range(1, mesh.nlevels + 1):
+        s.set_gather_lanes(level, lanes)
+    s.set_state(initial_state(c, mesh, perturb_seed=5, amplitude=0.03))
+    s.start()
+    for it in range(1, cycles + 1):
+        s.cycle(it)
+    out = [s.get_state(level) for level in range(1, mesh.nlevels + 1)]
+    s.close()
+    return out
+
+
+@pytest.mark.parametrize("name", list(CASES))
+def test_group_shapes_match_a_thread_per_node(name):
+    mesh = Mesh.bump_channel(17, 7, 6, 0.05, nlevels=3)
+    want = states(mesh, CASES[name], 1)
+    assert all(np.all(np.isfinite(u)) for u in want)
+    # FLITE_MIXED sums FP32 increments in the same order in every shape
+    for lanes in (4, 8, 16, 32, 0):
+        for level, (a, b) in enumerate(zip(want, states(mesh, CASES[name], lanes)), 1):
+            assert np.array_equal(a, b), (lanes, level)
+
+
+@pytest.mark.parametrize("size", [(17, 7, 6), (40, 13, 13), (61, 19, 20), (75, 24, 25)])
+def test_default_shape_matches_a_thread_per_node(size):
+    mesh = Mesh.bump_channel(*size, 0.05, nlevels=3)
+    for a, b in zip(states(mesh, CASES["laminar"], 1, 1), states(mesh, CASES["laminar"], 0, 1)):
+        assert np.array_equal(a, b)
