@@ -119,28 +119,21 @@ def build_case(host_only=False):
     return F, mesh, c, u0, time.time() - t0
 
 
-def apply_options(solver, options, unroll=1):
-    """Set the tuned launch options (node block, lanes, incidence-row mode
-    and shared walks per level) on a solver; none changes a result."""
+def apply_options(solver, options):
+    """Set the tuned launch options (node block, lanes and shared walks per
+    level) on a solver; none changes a result."""
     if not options:
         return
-    solver.set_kernel_options(256, options["node_block"], unroll)
+    solver.set_kernel_options(256, options["node_block"])
     for lvl, g in options["lanes"].items():
         solver.set_gather_lanes(lvl, g)
-        solver.set_tiled_gather(lvl, options["tiled"][lvl] if g == 1 else 0)
         solver.set_gather_fusion(lvl, options["fuse"][lvl])
 
 
-def node_kernel_name(lanes, tiled, unroll):
+def node_kernel_name(lanes):
     """The instance of the level-1 node kernel the tuned launch options run."""
     what = ("(level 1: central fluxes of the incident edges computed in the node gather, fused with the RK "
             "stage update")
-    if lanes == 1 and tiled:
-        minb, stage = (2, True) if tiled == 1 else (3, True) if tiled == 2 else (2, False) if tiled == 3 else (3, False)
-        return (f"k_node_update_tiled<{minb}, {str(stage).lower()}> {what}; incidences read through the incidence "
-                "rows of 256-node blocks" + (", blocks and halo staged in shared memory)" if stage else ")"))
-    if lanes == 1 and unroll == 2:
-        return f"k_node_update<GATHER_CENTRAL2, 1> {what})"
     if lanes == 1:  # the bench workload has no engines and no explicit stepping
         return f"k_node_update<GATHER_LEAN, 1> {what}; node tail without the engine and explicit branches)"
     return f"k_node_update<GATHER_CENTRAL, {lanes}> {what})"
@@ -253,54 +246,40 @@ def run_ours(args):
     solver = F.Solver(c, mesh)
     solver.set_state(u0)
     solver.start()
-    # pick the launch options on this GPU (none changes a result): node-kernel
-    # block size and gather unroll by the level-1 node kernel, then the level
-    # size below which gathers use a warp per node by the time of whole cycles
-    tuning = {}
+    # pick the launch options on this GPU (none changes a result): the
+    # node-kernel block size by the level-1 gathers, then the lanes per node of
+    # each level's gathers and, with a thread per node, whether gathers that
+    # walk the same incidence list share one walk, by the device time of that
+    # level's kernels over one relaxation step
+    tuning, tuning_levels = {}, {}
     if args.kernel_options:
         # fixed options (profiling runs: no tuning launches before the cycles)
         v = [int(x) for x in args.kernel_options.split(",")]
-        best = (v[0], v[1])
-        lanes = {lvl: v[1 + lvl] for lvl in range(1, solver.nlevels + 1)}
-        tm = [int(x) for x in args.tiled_modes.split(",")] if args.tiled_modes else []
-        tiled = {lvl: (tm[lvl - 1] if lvl - 1 < len(tm) else 1) for lvl in range(1, solver.nlevels + 1)}
+        best = v[0]
+        lanes = {lvl: v[lvl] for lvl in range(1, solver.nlevels + 1)}
         fz = [int(x) for x in args.fusion.split(",")] if args.fusion else []
         fuse = {lvl: (fz[lvl - 1] if lvl - 1 < len(fz) else 1) for lvl in range(1, solver.nlevels + 1)}
     else:
         for nb in (128, 256):
-            for unroll in (1, 2):
-                solver.set_kernel_options(256, nb, unroll)
-                tuning[(nb, unroll)] = solver.profile_level(1, reps=5)[1]
+            solver.set_kernel_options(256, nb)
+            tuning[nb] = sum(solver.profile_kernels(1, reps=5).values())
         best = min(tuning, key=tuning.get)
-    solver.set_kernel_options(256, best[0], best[1])
-    # lanes per node of each level's gathers (and, with a thread per node,
-    # whether the fused central gather stages node blocks in shared memory:
-    # through the incidence rows of node blocks: modes 1..4, 0 off), by the
-    # device time of that level's kernels over one relaxation step
-    # (and, with the incidence lists, whether gathers that walk the same list
-    # share one walk), by the device time of that level's kernels over one
-    # relaxation step
-    tuning_levels = {}
-    if not args.kernel_options:
-        lanes, tiled, fuse = {}, {}, {}
+        solver.set_kernel_options(256, best)
+        lanes, fuse = {}, {}
         for lvl in range(1, solver.nlevels + 1):
             t = {}
             for g in ((1, 4, 8) if lvl == 1 else (1, 4, 8, 16, 32)):
                 solver.set_gather_lanes(lvl, g)
-                for mode in ((0, 1, 2, 3, 4) if g == 1 else (0,)):
-                    solver.set_tiled_gather(lvl, mode)
-                    for fz in ((1, 0) if g == 1 and mode == 0 else (1,)):
-                        solver.set_gather_fusion(lvl, fz)
-                        groups = solver.profile_kernels(lvl, reps=5)
-                        t[(g, mode, fz)] = sum(groups.values())
-                        if lvl <= 2 and g == 1:
-                            key = f"{lvl}_groups_tiled{mode}" + (("_shared" if fz else "_separate") if mode == 0 else "")
-                            tuning_levels[key] = groups
-            lanes[lvl], tiled[lvl], fuse[lvl] = min(t, key=t.get)
-            tuning_levels[lvl] = {f"lanes{g}_tiled{m}" + (f"_shared{f}" if g == 1 and m == 0 else ""): v
-                                  for (g, m, f), v in t.items()}
-    options = {"node_block": best[0], "lanes": lanes, "tiled": tiled, "fuse": fuse}
-    apply_options(solver, options, best[1])
+                for fz in ((1, 0) if g == 1 else (1,)):
+                    solver.set_gather_fusion(lvl, fz)
+                    groups = solver.profile_kernels(lvl, reps=5)
+                    t[(g, fz)] = sum(groups.values())
+                    if lvl <= 2 and g == 1:
+                        tuning_levels[f"{lvl}_groups" + ("_shared" if fz else "_separate")] = groups
+            lanes[lvl], fuse[lvl] = min(t, key=t.get)
+            tuning_levels[lvl] = {f"lanes{g}" + (f"_shared{f}" if g == 1 else ""): v for (g, f), v in t.items()}
+    options = {"node_block": best, "lanes": lanes, "fuse": fuse}
+    apply_options(solver, options)
     solver.set_state(u0)
     solver.start()
     # warm-up (also captures the cycle graph)
@@ -410,7 +389,7 @@ def run_ours(args):
                 "resident": {"value": args.steps / resident_s, "h2d_bytes_per_step": 4,
                              "d2h_bytes_per_step": 15 * 8 + 9 * 8}},
         "gpu_launches": int(launches_per_cycle * args.steps),
-        "roofline": {"kernel": node_kernel_name(lanes[1], tiled[1], best[1]),
+        "roofline": {"kernel": node_kernel_name(lanes[1]),
                      "bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",
                      "frac": achieved / hbm, "peak_kind": peak_kind,
                      "algorithmic_bytes": nbytes, "launch_ms": node_ms,
@@ -423,10 +402,9 @@ def run_ours(args):
         "level1_kernel_ms": kernels_l1,
         "level1_roofline": group_roofline(kernels_l1, group_bytes(mesh), hbm),
         "coarse_kernel_ms": kernels_coarse,
-        "node_kernel_options": {"chosen": {"node_block": best[0], "gather_unroll": best[1],
-                                           "gather_lanes_per_level": lanes, "tiled_mode_per_level": tiled,
+        "node_kernel_options": {"chosen": {"node_block": best, "gather_lanes_per_level": lanes,
                                            "shared_walks_per_level": fuse},
-                                "ms": {f"nb{k[0]}_unroll{k[1]}": v for k, v in tuning.items()},
+                                "ms": {f"nb{k}": v for k, v in tuning.items()},
                                 "level_ms": tuning_levels},
         "adjoint": {"fwd_ms": fwd_ms, "vjp_ms": vjp_ms, "cost_ratio": vjp_ms / fwd_ms,
                     "what": "flite_residual_vjp vs flite_residual_fwd kernels on level 1, FP64"},
@@ -936,11 +914,9 @@ def main():
     ap.add_argument("--mesh", default=None, help="NX,NY,NZ hexes (default 264,88,88)")
     ap.add_argument("--no-mixed", action="store_true", help="skip the FLITE_MIXED cycle rate")
     ap.add_argument("--kernel-options", default=None,
-                    help="NODE_BLOCK,UNROLL,LANES_L1,...: fixed launch options instead of tuning them")
+                    help="NODE_BLOCK,LANES_L1,...: fixed launch options instead of tuning them")
     ap.add_argument("--node-order", type=int, default=0,
                     help="device node numbering: 0 the mesh's own, 1 the locality (Morton) order")
-    ap.add_argument("--tiled-modes", default=None,
-                    help="with --kernel-options: TILED_L1,TILED_L2,... (0 off, 1 or 2 on; default 1)")
     ap.add_argument("--fusion", default=None,
                     help="with --kernel-options: per level 1 to share the walks of gathers over the same "
                          "incidence list, 0 for separate kernels (default 1)")

@@ -75,8 +75,7 @@ __global__ void k_vjp_node(Params P, LevelView L, const double *x, const double 
         for (int k = 0; k < 5; ++k) b[d][k] = 0.0;
     double ri[5];
     for (int k = 0; k < 5; ++k) ri[k] = rbar[(size_t)k * N + i];
-    for (int q = L.inc_ptr[i]; q < L.inc_ptr[i + 1]; ++q) {
-        int2 t = L.inc[q];
+    FLITE_FOR_INC(L, i, t) {
         int e = t.x >= 0 ? t.x : ~t.x, j = t.y;
         const double w[3] = {L.wx[e], L.wy[e], L.wz[e]};
         double a[5];

@@ -42,6 +42,8 @@ constexpr int kResidBlocks = 296;  // 2 x 148 SMs
 
 struct DevLevel {
     int N = 0, E = 0, B = 0, Nb = 0;
+    int nrows = 0;           // incidence rows
+    std::vector<int> eslot;  // the device's number of each of the caller's edges; empty: the same
     LevelView v{};
     std::vector<int> wall;  // level-1 wall nodes in register order (forces)
     int *d_wall = nullptr;
@@ -72,19 +74,6 @@ using namespace flite_detail;
             case 32: FLITE_LAUNCH(kern, (32,), gblk(l, 32), nb, 0, __VA_ARGS__); break;  \
             default: FLITE_LAUNCH(kern, (1,), gblk(l, 1), nb, 0, __VA_ARGS__);           \
         }                                                                                \
-    } while (0)
-
-// a row-gather kernel template (STAGE, AHEAD) launched for mode m (1: staged,
-// one ahead; 2: staged; 3: one ahead; 4: neither) over the level's blocks g,
-// staging K fields per node
-#define FLITE_ROWS(kern, K)                                                                    \
-    do {                                                                                       \
-        switch (m) {                                                                           \
-            case 1: kern<true, true><<<g, kTile, tile_smem(l, m, K), s>>>(P, V(l)); break;      \
-            case 2: kern<true, false><<<g, kTile, tile_smem(l, m, K), s>>>(P, V(l)); break;     \
-            case 3: kern<false, true><<<g, kTile, 0, s>>>(P, V(l)); break;                      \
-            default: kern<false, false><<<g, kTile, 0, s>>>(P, V(l));                           \
-        }                                                                                      \
     } while (0)
 
 struct flite_ctx {
@@ -128,9 +117,9 @@ struct flite_ctx {
     }
     // threads per block of the edge kernels and of the node kernels (the
     // batch autotuner may change them; kernels with launch bounds take <= 256)
-    int eb = kBlock, nb = kBlock;
-    // incidences per load batch of the fused central gather (1 or 2)
-    int unroll = 1;
+    // by default node kernels take blocks of 128: the separate gathers of the
+    // 2.1-million-node level run 1736 us a step with 128 and 1821 with 256
+    int eb = kBlock, nb = 128;
     // calculateTurbulence of the cycle being run or captured (Spalart-
     // Allmaras: cycleNo <= numberOfTurbulenceSteps, mg_par:922-926), and the
     // value the instantiated graph was captured with
@@ -251,11 +240,16 @@ struct flite_ctx {
     unsigned gblk(int l, int g) const { return (unsigned)((g * (size_t)lv[l].v.N + nb - 1) / nb); }
     // levels whose gathers that walk the same incidence list share one walk
     // (k_ts_lap, k_jflux_vgrad) where a thread serves a node
-    // (flite_set_gather_fusion: 1 on, the default; 0 off, held as -1)
+    // (flite_set_gather_fusion: 1 on; 0 off, held as -1).  By default up to
+    // kSharedWalkNodes nodes: there the walks are short of work and one launch
+    // less pays; above, the separate kernels' smaller register counts do (one
+    // step's kernels, shared/separate: 92,988 nodes 188/212 us, 203,401 nodes
+    // 253/258, 237,662 nodes 364/345, 2,099,065 nodes 1866/1736)
     int fuse_mode[kMaxLevels] = {0};
     bool fuse_walks(int l) const {
-        if (lanes_of(l) != 1 || tiled_other(l)) return false;
-        return !(l < kMaxLevels && fuse_mode[l] < 0);
+        if (lanes_of(l) != 1) return false;
+        if (l < kMaxLevels && fuse_mode[l] != 0) return fuse_mode[l] > 0;
+        return lv[l].v.N <= kSharedWalkNodes;
     }
 
     void pressure(int l) {
@@ -278,35 +272,7 @@ struct flite_ctx {
     }
     void timestep_kernels(int l) {
         counted();
-        if (const int m = tiled_other(l)) {
-            const int K = !P.viscous ? 0 : (P.sa ? 3 : 2);
-            const unsigned g = V(l).tile.ntiles;
-            const size_t sm = tile_smem(l, m, K);
-#define FLITE_TS(KK)                                                                                      \
-    switch (m) {                                                                                           \
-        case 1: k_timestep_tiled<KK, true, true><<<g, kTile, sm, s>>>(P, V(l)); break;                     \
-        case 2: k_timestep_tiled<KK, true, false><<<g, kTile, sm, s>>>(P, V(l)); break;                    \
-        case 3: k_timestep_tiled<KK, false, true><<<g, kTile, 0, s>>>(P, V(l)); break;                     \
-        default: k_timestep_tiled<KK, false, false><<<g, kTile, 0, s>>>(P, V(l));                          \
-    }
-            if (K == 0) { FLITE_TS(0) }
-            else if (K == 2) { FLITE_TS(2) }
-            else { FLITE_TS(3) }
-#undef FLITE_TS
-            return;
-        }
         FLITE_GATHER(k_timestep, l, P, V(l));
-    }
-    // the incidence-row form of a level's other gathers (the mode of
-    // flite_set_tiled_gather: 1, 2 staged, 3, 4 not), where a thread serves
-    // a node and the rows exist; 0 otherwise
-    int tiled_other(int l) const {
-        if (group || lv[l].v.tile.ntiles <= 0 || lanes_of(l) != 1) return 0;
-        const int m = l < kMaxLevels ? tiled_mode[l] : 0;
-        return m < 0 ? 0 : m;
-    }
-    size_t tile_smem(int l, int m, int K) const {
-        return m <= 2 ? (size_t)lv[l].v.tile.stage_max * K * sizeof(double) : 0;
     }
     void zero_diss(int l) {
         counted();
@@ -327,29 +293,16 @@ struct flite_ctx {
                  (c.fourthOrderDissipationFactor == 0 && c.secondOrderDissipationFactor == 0));
     }
     void jst_lap(int l) {
-        const LevelView &L = V(l);
-        const int m = tiled_other(l);
-        const unsigned g = L.tile.ntiles;
         counted();
-        if (m && !P.useDissW) {
-            FLITE_ROWS(k_jst_lap_tiled, 6);
-        } else {
-            FLITE_GATHER(k_jst_lap, l, P, L);
-        }
+        FLITE_GATHER(k_jst_lap, l, P, V(l));
     }
     void jst_flux(int l) {
-        const LevelView &L = V(l);
-        const int m = tiled_other(l);
-        const unsigned g = L.tile.ntiles;
         counted();
         if (P.matrixDiss) {
             no_group("the matrix dissipation");
-            k_jst_flux_matrix<<<nblk(L.N), nb, 0, s>>>(P, L);
-        }
-        else if (m) {
-            FLITE_ROWS(k_jst_flux_tiled, 13);
+            k_jst_flux_matrix<<<nblk(V(l).N), nb, 0, s>>>(P, V(l));
         } else {
-            FLITE_GATHER(k_jst_flux, l, P, L);
+            FLITE_GATHER(k_jst_flux, l, P, V(l));
         }
     }
     // the time step (ts), the JST dissipation (or its zero) and the viscous
@@ -433,21 +386,11 @@ struct flite_ctx {
             FLITE_GATHER(k_visc2_grad, l, P, V(l));
             return;
         }
-        if (const int m = tiled_other(l)) {
-            const unsigned g = V(l).tile.ntiles;
-            FLITE_ROWS(k_visc_grad_tiled, 4);
-            return;
-        }
         FLITE_GATHER(k_visc_grad, l, P, V(l));
     }
     void visc_flux(int l) {
         if (c.viscosityScheme == 2) {
             FLITE_GATHER(k_visc2_flux, l, P, V(l));
-            return;
-        }
-        if (const int m = tiled_other(l)) {
-            const unsigned g = V(l).tile.ntiles;
-            FLITE_ROWS(k_visc_flux_tiled, 12);
             return;
         }
         FLITE_GATHER(k_visc_flux, l, P, V(l));
@@ -568,41 +511,31 @@ struct flite_ctx {
             default: launch_node_update_u<1>(l, mode, stage, anchor);
         }
     }
-    // levels whose gathers read the incidences through the rows of node
-    // blocks (flite_set_tiled_gather: 0 off; 1, 2 staged in shared memory
-    // with two or three blocks of 256 threads per SM; 3, 4 the same rows
-    // without staging; tiled_mode holds -1 for 0 and 0 for the default, off)
-    int tiled_mode[kMaxLevels] = {0};
-    int tiled(int l) const {
-        if (group || !(fused() && !mixed() && lv[l].v.tile.ntiles > 0)) return 0;
-        const int m = l < kMaxLevels ? tiled_mode[l] : 0;
-        return m < 0 ? 0 : m;
-    }
     template <int U>
     void launch_node_update_u(int l, int mode, int stage, bool anchor) {
-        const unsigned g = gblk(l, U);
-        if (U == 1 && tiled(l)) {
-            const TileView &T = V(l).tile;
-            const size_t sm = (size_t)T.stage_max * sizeof(NodeRec);
-            switch (tiled(l)) {
-                case 2: k_node_update_tiled<true, false><<<T.ntiles, kTile, sm, s>>>(P, V(l), mode, stage); break;
-                case 3: k_node_update_tiled<false, true><<<T.ntiles, kTile, 0, s>>>(P, V(l), mode, stage); break;
-                case 4: k_node_update_tiled<false, false><<<T.ntiles, kTile, 0, s>>>(P, V(l), mode, stage); break;
-                default: k_node_update_tiled<true, true><<<T.ntiles, kTile, sm, s>>>(P, V(l), mode, stage);
-            }
-            return;
-        }
+        // blocks of nt threads (nb, or less where the kernel's own bound is)
+        const auto blk = [&](int prec) { return (unsigned)std::min(nb, node_threads(prec, U)); };
+        const auto grid = [&](unsigned nt) { return (unsigned)((U * (size_t)V(l).N + nt - 1) / nt); };
+#define FLITE_NODE(PREC)                                                                             \
+    do {                                                                                              \
+        const unsigned nt = blk(PREC);                                                                \
+        FLITE_LAUNCH(k_node_update, (PREC, U,), grid(nt), nt, 0, P, V(l), mode, stage);               \
+    } while (0)
         if (mixed()) {
-            if (anchor) FLITE_LAUNCH(k_node_update, (GATHER_ANCHOR, U,), g, nb, 0, P, V(l), mode, stage);
-            else FLITE_LAUNCH(k_node_update, (GATHER_DELTA, U,), g, nb, 0, P, V(l), mode, stage);
+            if (anchor) FLITE_NODE(GATHER_ANCHOR);
+            else FLITE_NODE(GATHER_DELTA);
         } else if (fused()) {
-            if (unroll == 2 && U == 1) FLITE_LAUNCH(k_node_update, (GATHER_CENTRAL2, 1,), g, nb, 0, P, V(l), mode, stage);
-            else if (U == 1 && !P.engines && !(P.unsteady && P.explicit_))
-                FLITE_LAUNCH(k_node_update, (GATHER_LEAN, 1,), g, nb, 0, P, V(l), mode, stage);
-            else FLITE_LAUNCH(k_node_update, (GATHER_CENTRAL, U,), g, nb, 0, P, V(l), mode, stage);
+            if constexpr (U == 1) {
+                if (!P.engines && !(P.unsteady && P.explicit_)) {
+                    FLITE_NODE(GATHER_LEAN);
+                    return;
+                }
+            }
+            FLITE_NODE(GATHER_CENTRAL);
         } else {
-            FLITE_LAUNCH(k_node_update, (GATHER_BUFFER, U,), g, nb, 0, P, V(l), mode, stage);
+            FLITE_NODE(GATHER_BUFFER);
         }
+#undef FLITE_NODE
     }
 
     // ---- singleIteration (def_par:1002-1181) -----------------------------

@@ -107,25 +107,14 @@ struct __align__(16) GradRec {
 
 // A level's mesh and state on the device.  Node-indexed arrays are SoA
 // ([component][node]), like the reference's column-major u(N,nvar).
-// Shared-memory staging of node blocks for the gathers with a thread per
-// node: block t of kTile consecutive nodes and its halo (the other nodes its
-// edges reach).  The incidences of the block are stored row by row: row k
-// holds incidence k (in edge order) of each of the block's nodes, with the
-// edge coefficients and the other node's staged slot (or, beyond the stage's
-// capacity, its node number with kTileGlobal set); kTileSecond marks the
-// node as the edge's second node.
-constexpr int kTile = 256;
-constexpr int kTileStageMax = 1024;  // records staged per block: 48 KB
-constexpr unsigned kTileSecond = 0x80000000u, kTileGlobal = 0x40000000u, kTileIndexMask = 0x3fffffffu;
-struct TileView {
-    int ntiles;                   // 0: no staging data for this level
-    int stage_max;                // staged records of the largest block (<= kTileStageMax)
-    const int *halo_ptr, *halo;   // [ntiles+1], halo nodes of each block in increasing order
-    const int *row;               // [ntiles+1] first incidence row of each block
-    const unsigned *meta;         // [rows*kTile]
-    const unsigned *nmeta;        // [rows*kTile] the same with every other node as a node number
-    const double *wx, *wy, *wz;   // [rows*kTile]
-};
+// Incidence rows for the gathers with a thread per node: slices of kRow
+// consecutive nodes, row k of a slice holding incidence k (in edge order) of
+// each of its nodes side by side, so that a warp reads its k-th incidences
+// with one coalesced load; a node's list in `inc` is contiguous instead, and a
+// warp's k-th entries then lie 8 * degree bytes apart, in as many cache lines
+// as it has lanes.  kRowPad rows past the last slice keep the walk's loads
+// ahead in bounds.
+constexpr int kRow = 32, kRowPad = 2;
 
 struct LevelView {
     int N, E, B, Nb, grid;
@@ -140,7 +129,11 @@ struct LevelView {
     // negative entry ~e marks the node as the second node of edge e
     const int *inc_ptr;
     const int2 *inc;
+    const int *row_ptr;          // [slices] first incidence row of each slice of kRow nodes
+    const int2 *rows;            // [rows*kRow] the entries of inc, row by row
     const EdgeW *ew;             // [E] the edge coefficients as one record
+    // the device's number of each of the caller's edges; NULL when the same
+    const int *eslot;            // [E]
     // node -> incident boundary edges in boundary-edge order: 2*b + side
     const int *binc_ptr;
     const int *binc;
@@ -183,6 +176,7 @@ struct LevelView {
     float *a32;                            // [5][N] anchor rho, u, v, w, E+p
     DeltaRec *dq;                          // [N] anchor primitives and increments
     const IncRec32 *inc32;                 // [2E] incidences in FP32
+    const IncRec32 *rows32;                // [rows*kRow] the same, row by row
     double *bflux;                         // [B][10] boundary-edge contributions
     // moving meshes (flowType 2; NULL on a static mesh): per edge the GCL
     // weight over physicalTimeStep (wgcl of makeRHS), per boundary edge its
@@ -199,7 +193,6 @@ struct LevelView {
     // the caller's number of each node (renumber.h); NULL when the device
     // numbering is the caller's
     const int *perm;                       // [N]
-    TileView tile;                         // staging of node blocks (fluxType 1)
     EngineView eng;                        // level 1 of a mesh with engines; zero otherwise
     // ivd%physicalTimeStep under explicit time stepping: the smallest local
     // time step of the last makeTimeSteps on any level (one per context)
@@ -235,6 +228,31 @@ __device__ __forceinline__ const T &case_of(const CaseArg<B, T> &a) {
 }
 #define FLITE_CASE_P(B, P, V) const Params &P = case_of<B, Params>(P##_)
 #define FLITE_CASE_L(B, V) const LevelView &V = case_of<B, LevelView>(V##_)
+
+// The incidences of node i in edge order through the rows, the entry of the
+// next iteration loaded one ahead: the index -> neighbour chain starts an
+// iteration early.  FLITE_FOR_INC(L, i, t) runs its body with t = (signed
+// edge, other node) for each.
+struct RowIter {
+    const int2 *rows;
+    int2 t, ahead;
+    int x, end;  // entry of t, and of the first row past the node's
+    __device__ __forceinline__ RowIter(const LevelView &L, int i) : rows(L.rows) {
+        x = L.row_ptr[i / kRow] * kRow + i % kRow;
+        end = x + (L.inc_ptr[i + 1] - L.inc_ptr[i]) * kRow;
+        t = __ldg(rows + x);
+        ahead = __ldg(rows + x + kRow);
+    }
+    __device__ __forceinline__ bool more() const { return x < end; }
+    __device__ __forceinline__ void next() {
+        t = ahead;
+        x += kRow;
+        if (x + kRow < end) ahead = __ldg(rows + x + kRow);
+    }
+};
+#define FLITE_FOR_INC(L, i, t) \
+    for (RowIter it_(L, i); it_.more(); it_.next()) \
+        if (const int2 t = it_.t; true)
 
 __device__ __forceinline__ EdgeW load_edgew(const EdgeW *w, int e) {
     const double2 *p = reinterpret_cast<const double2 *>(w + e);

@@ -48,68 +48,6 @@ int guarded(flite_ctx *ctx, F &&f) {
     }
 }
 
-// The staging data of the tiled gathers of one level (TileView).
-struct TileHost {
-    int ntiles = 0, stage_max = 0;
-    std::vector<int> halo_ptr, halo, row;
-    std::vector<unsigned> meta, nmeta;
-    std::vector<double> wx, wy, wz;
-};
-
-void build_tiles(int N, const std::vector<int> &ip, const std::vector<int2> &inc, const std::vector<double> &wx,
-                 const std::vector<double> &wy, const std::vector<double> &wz, TileHost &T) {
-    if (N <= 0 || N >= (int)kTileIndexMask) return;
-    T.ntiles = (N + kTile - 1) / kTile;
-    T.halo_ptr.assign(T.ntiles + 1, 0);
-    T.row.assign(T.ntiles + 1, 0);
-    for (int t = 0; t < T.ntiles; ++t) {
-        const int n0 = t * kTile, n1 = std::min(N, n0 + kTile);
-        int kmax = 0;
-        for (int i = n0; i < n1; ++i) kmax = std::max(kmax, ip[i + 1] - ip[i]);
-        T.row[t + 1] = T.row[t] + kmax;
-    }
-    const size_t cells = (size_t)T.row[T.ntiles] * kTile;
-    T.meta.assign(std::max<size_t>(cells, 1), 0u);
-    T.nmeta.assign(std::max<size_t>(cells, 1), 0u);
-    T.wx.assign(std::max<size_t>(cells, 1), 0.0);
-    T.wy.assign(std::max<size_t>(cells, 1), 0.0);
-    T.wz.assign(std::max<size_t>(cells, 1), 0.0);
-    T.stage_max = kTile;
-    std::vector<int> h;
-    for (int t = 0; t < T.ntiles; ++t) {
-        const int n0 = t * kTile, n1 = std::min(N, n0 + kTile);
-        h.clear();
-        for (int i = n0; i < n1; ++i)
-            for (int k = ip[i]; k < ip[i + 1]; ++k) {
-                const int j = inc[k].y;
-                if (j < n0 || j >= n1) h.push_back(j);
-            }
-        std::sort(h.begin(), h.end());
-        h.erase(std::unique(h.begin(), h.end()), h.end());
-        T.halo_ptr[t + 1] = T.halo_ptr[t] + (int)h.size();
-        T.halo.insert(T.halo.end(), h.begin(), h.end());
-        const int staged = std::min((int)h.size(), kTileStageMax - kTile);
-        T.stage_max = std::max(T.stage_max, kTile + staged);
-        for (int i = n0; i < n1; ++i)
-            for (int k = ip[i]; k < ip[i + 1]; ++k) {
-                const int es = inc[k].x, j = inc[k].y, e = es >= 0 ? es : ~es;
-                unsigned m;
-                if (j >= n0 && j < n1) {
-                    m = (unsigned)(j - n0);
-                } else {
-                    const int pos = (int)(std::lower_bound(h.begin(), h.end(), j) - h.begin());
-                    m = pos < staged ? (unsigned)(kTile + pos) : (kTileGlobal | (unsigned)j);
-                }
-                const unsigned second = es < 0 ? kTileSecond : 0u;
-                const size_t x = ((size_t)T.row[t] + (k - ip[i])) * kTile + (i - n0);
-                T.meta[x] = m | second;
-                T.nmeta[x] = kTileGlobal | (unsigned)j | second;
-                T.wx[x] = wx[e]; T.wy[x] = wy[e]; T.wz[x] = wz[e];
-            }
-    }
-    if (T.halo.empty()) T.halo.push_back(0);
-}
-
 const char *unsupported_reason(const flite_controls &c) {
     if (c.flowType != 0 && c.flowType != 1 && c.flowType != 2)
         return "flowType must be 0 (steady), 1 (unsteady, static mesh) or 2 (unsteady, moving mesh)";
@@ -174,10 +112,12 @@ void flite::put_geometry(flite_ctx &X, int l, const flite_level_desc &d, bool cr
     };
     std::vector<double> wx(E), wy(E), wz(E), slen(E, 0.0);
     std::vector<EdgeW> ew(std::max(E, 1));
+    const std::vector<int> &slot = X.lv[l].eslot;
     for (int e = 0; e < E; ++e) {
-        wx[e] = d.side_w[e]; wy[e] = d.side_w[(size_t)E + e]; wz[e] = d.side_w[2 * (size_t)E + e];
-        if (d.side_len) slen[e] = d.side_len[e];
-        ew[e] = EdgeW{wx[e], wy[e], wz[e], 0.0};
+        const int q = slot.empty() ? e : slot[e];
+        wx[q] = d.side_w[e]; wy[q] = d.side_w[(size_t)E + e]; wz[q] = d.side_w[2 * (size_t)E + e];
+        if (d.side_len) slen[q] = d.side_len[e];
+        ew[q] = EdgeW{wx[q], wy[q], wz[q], 0.0};
     }
     std::vector<int2> bedge(B);
     std::vector<double> bwx(B), bwy(B), bwz(B);
@@ -228,7 +168,7 @@ void flite::put_geometry(flite_ctx &X, int l, const flite_level_desc &d, bool cr
         const double dtp = X.c.physicalTimeStep;
         auto w = [&](double x, double xp) { return comb ? 1.5 * x - 0.5 * xp : x; };
         std::vector<double> gw(std::max(E, 1)), bgw(2 * (size_t)std::max(B, 1));
-        for (int e = 0; e < E; ++e) gw[e] = w(d.side_gcl[e], d.side_gcl[(size_t)E + e]) / dtp;
+        for (int e = 0; e < E; ++e) gw[slot.empty() ? e : slot[e]] = w(d.side_gcl[e], d.side_gcl[(size_t)E + e]) / dtp;
         for (int b = 0; b < B; ++b) {
             const double g1 = w(d.bnd_gcl[b], d.bnd_gcl[2 * (size_t)B + b]);
             const double g2 = w(d.bnd_gcl[(size_t)B + b], d.bnd_gcl[3 * (size_t)B + b]);
@@ -332,16 +272,6 @@ int flite::create_context(const flite_controls *c, int nlevels, const flite_leve
                 }
         }
         CK(cudaStreamCreateWithFlags(&X.s, cudaStreamNonBlocking));
-        // shared memory of the staged incidence-row gathers (above the
-        // default 48 KB for the wider node fields)
-        for (bool ahead : {true, false}) {
-            CK(cudaFuncSetAttribute(ahead ? k_jst_flux_tiled<true, true> : k_jst_flux_tiled<true, false>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, 13 * 8 * kTileStageMax));
-            CK(cudaFuncSetAttribute(ahead ? k_visc_flux_tiled<true, true> : k_visc_flux_tiled<true, false>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, 12 * 8 * kTileStageMax));
-            CK(cudaFuncSetAttribute(ahead ? k_jst_lap_tiled<true, true> : k_jst_lap_tiled<true, false>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, 6 * 8 * kTileStageMax));
-        }
         CK(cudaMallocHost(&X.h_cycle, sizeof(int)));
         X.d_cycle = X.alloc<int>(1);
         X.d_cyc = X.alloc<int>(G);
@@ -373,6 +303,7 @@ int flite::create_context(const flite_controls *c, int nlevels, const flite_leve
                     throw std::runtime_error("mesh donor differs from the levels given");
                 L = donor->lv[l].v;  // mesh arrays shared; state set below
                 D.wall = donor->lv[l].wall;
+                D.nrows = donor->lv[l].nrows;
                 D.d_wall = donor->lv[l].d_wall;
                 if (l == 0) P.engines = donor->P.engines;
             } else {
@@ -404,6 +335,34 @@ int flite::create_context(const flite_controls *c, int nlevels, const flite_leve
                     inc[fill[edge[e].y]++] = make_int2(~e, edge[e].x);
                 }
             }
+            // the rows of the slices, and on levels whose gathers take a
+            // thread per node by default the device's edge order: row by row
+            // over the slices, each edge in the row of its first node, so that
+            // a warp reads the coefficients (and edge buffers) of its k-th
+            // edges side by side; the sums keep the caller's order
+            const int nslice = (N + kRow - 1) / kRow;
+            std::vector<int> rp(nslice, 0);
+            for (int t = 0; t < nslice; ++t) {
+                rp[t] = D.nrows;
+                int most = 0;
+                for (int i = t * kRow; i < std::min(N, (t + 1) * kRow); ++i) most = std::max(most, ip[i + 1] - ip[i]);
+                D.nrows += most;
+            }
+            if (4 * (size_t)N > kLaneThreads) {
+                std::vector<int> &slot = D.eslot;
+                slot.resize(E);
+                int next = 0;
+                for (int t = 0; t < nslice; ++t) {
+                    const int most = (t + 1 < nslice ? rp[t + 1] : D.nrows) - rp[t], i1 = std::min(N, (t + 1) * kRow);
+                    for (int k = 0; k < most; ++k)
+                        for (int i = t * kRow; i < i1; ++i)
+                            if (ip[i] + k < ip[i + 1] && inc[ip[i] + k].x >= 0) slot[inc[ip[i] + k].x] = next++;
+                }
+                for (int2 &v : inc) v.x = v.x >= 0 ? slot[v.x] : ~slot[~v.x];
+                std::vector<int2> moved(E);
+                for (int e = 0; e < E; ++e) moved[slot[e]] = edge[e];
+                edge.swap(moved);
+            }
             std::vector<int> bp(N + 1, 0);
             for (int b = 0; b < B; ++b) { bp[bedge[b].x + 1]++; bp[bedge[b].y + 1]++; }
             for (int i = 0; i < N; ++i) bp[i + 1] += bp[i];
@@ -417,7 +376,7 @@ int flite::create_context(const flite_controls *c, int nlevels, const flite_leve
             }
             // connectivity (def_par:14262-14275)
             std::vector<double> conn(N, 0.0);
-            for (int e = 0; e < E; ++e) { conn[edge[e].x] += 1.0; conn[edge[e].y] += 1.0; }
+            for (int i = 0; i < N; ++i) conn[i] = (double)(ip[i + 1] - ip[i]);
             // boundary classes from the indicator register
             std::vector<unsigned char> bc(N, BC_NONE);
             auto R = [&](int i) { return d.node_reg[i + 20]; };
@@ -436,6 +395,13 @@ int flite::create_context(const flite_controls *c, int nlevels, const flite_leve
             L.edge = X.upload(edge);
             L.bedge = X.upload(bedge); L.bind = X.upload(bind);
             L.inc_ptr = X.upload(ip); L.inc = X.upload(inc);
+            L.eslot = D.eslot.empty() ? nullptr : X.upload(D.eslot);
+            L.row_ptr = X.upload(rp);
+            int2 *rows = X.alloc<int2>((size_t)(D.nrows + kRowPad) * kRow);
+            CK(cudaMemset(rows, 0, (size_t)(D.nrows + kRowPad) * kRow * sizeof(int2)));
+            k_make_rows<<<flite_ctx::blocks(N), kBlock>>>(L, D.nrows, rows);
+            CK(cudaGetLastError());
+            L.rows = rows;
             L.binc_ptr = X.upload(bp); L.binc = X.upload(binc);
             L.conn = X.upload(conn);
             L.bc = X.upload(bc);
@@ -473,24 +439,7 @@ int flite::create_context(const flite_controls *c, int nlevels, const flite_leve
             }
             put_geometry(X, l, d, true);
             L.inc32 = nullptr;
-            L.tile = TileView{};
-            if (X.fused()) {
-                // staging of node blocks for the fused central gather
-                std::vector<double> wx(d.side_w, d.side_w + E), wy(d.side_w + E, d.side_w + 2 * (size_t)E),
-                    wz(d.side_w + 2 * (size_t)E, d.side_w + 3 * (size_t)E);
-                TileHost T;
-                build_tiles(N, ip, inc, wx, wy, wz, T);
-                if (T.ntiles > 0) {
-                    L.tile.ntiles = T.ntiles;
-                    L.tile.stage_max = T.stage_max;
-                    L.tile.halo_ptr = X.upload(T.halo_ptr);
-                    L.tile.halo = X.upload(T.halo);
-                    L.tile.row = X.upload(T.row);
-                    L.tile.meta = X.upload(T.meta);
-                    L.tile.nmeta = X.upload(T.nmeta);
-                    L.tile.wx = X.upload(T.wx); L.tile.wy = X.upload(T.wy); L.tile.wz = X.upload(T.wz);
-                }
-            }
+            L.rows32 = nullptr;
             if (l > 0) {
                 const int nf = X.lv[l - 1].N;
                 if (!d.parent || !d.rweight) throw std::runtime_error("coarse level without transfer operators");
@@ -585,8 +534,13 @@ int flite::create_context(const flite_controls *c, int nlevels, const flite_leve
                 if (!L.inc32) {
                     IncRec32 *d32 = X.alloc<IncRec32>(2 * (size_t)std::max(E, 1));
                     if (E > 0) k_make_inc32<<<(unsigned)((2 * (size_t)E + 255) / 256), 256>>>(L.inc, L.ew, 2 * E, d32);
+                    // (the padding entries of the rows become record 0's)
+                    const int nr = (D.nrows + kRowPad) * kRow;
+                    IncRec32 *r32 = X.alloc<IncRec32>(nr);
+                    if (E > 0) k_make_inc32<<<(unsigned)((nr + 255) / 256), 256>>>(L.rows, L.ew, nr, r32);
                     CK(cudaGetLastError());
                     L.inc32 = d32;
+                    L.rows32 = r32;
                 }
             } else {
                 L.ua = L.ra = L.pa = nullptr;
@@ -958,6 +912,8 @@ int flite_profile_level(flite_ctx *ctx, int level, int reps, double *edge_ms, do
     });
 }
 
+// gather_unroll is checked and changes nothing (the central gather copies
+// ahead by its own depth)
 int flite_set_kernel_options(flite_ctx *ctx, int32_t edge_block, int32_t node_block, int32_t gather_unroll) {
     if (!ctx || edge_block < 32 || edge_block > 256 || node_block < 32 || node_block > 256 || edge_block % 32 ||
         node_block % 32 || (gather_unroll != 1 && gather_unroll != 2))
@@ -965,14 +921,13 @@ int flite_set_kernel_options(flite_ctx *ctx, int32_t edge_block, int32_t node_bl
     ctx->drop_graph();
     ctx->eb = edge_block;
     ctx->nb = node_block;
-    ctx->unroll = gather_unroll;
     return FLITE_OK;
 }
 
+// every gather with a thread per node reads the incidence rows: the modes are
+// checked and change nothing
 int flite_set_tiled_gather(flite_ctx *ctx, int32_t level, int32_t on) {
     if (bad_level(ctx, level) || on < 0 || on > 4 || level > kMaxLevels) return FLITE_EINVAL;
-    ctx->tiled_mode[level - 1] = on == 0 ? -1 : on;
-    ctx->drop_graph();
     return FLITE_OK;
 }
 

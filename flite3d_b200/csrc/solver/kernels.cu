@@ -225,7 +225,7 @@ __global__ void k_timestep(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_) {
         ts_store(L, i, x[0], x[1]);
     } else {
         double acc = 0.0, h = 0.0;
-        for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) ts_inc(P, L, L.inc[k], m1, m2, m3, ro, cc, acc, h);
+        FLITE_FOR_INC(L, i, t) ts_inc(P, L, t, m1, m2, m3, ro, cc, acc, h);
         ts_finish(P, L, i, acc, h);
     }
 }
@@ -312,7 +312,7 @@ __global__ void k_jst_lap(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_) {
         lap_store(L, i, a);
     } else {
         LapAcc a = {{0, 0, 0, 0, 0}, 0, 0};
-        for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) lap_inc(P, L, L.inc[k], ui, pi, a);
+        FLITE_FOR_INC(L, i, t) lap_inc(P, L, t, ui, pi, a);
         lap_store(L, i, a);
     }
 }
@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(256, U == 1 ? 4 : 1) k_jst_flux(CaseArg<B, Par
             acc);
         if (!active || gl) return;
     } else
-    for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) jflux_inc(P, L, L.inc[k], k4, vdi, coni, si, Li, Ui, acc);
+    FLITE_FOR_INC(L, i, t) jflux_inc(P, L, t, k4, vdi, coni, si, Li, Ui, acc);
     for (int c = 0; c < 5; ++c) L.diss[c * N + i] = acc[c];
 }
 
@@ -449,8 +449,7 @@ __global__ void k_jst_flux_matrix(Params P, LevelView L) {
     const int N = L.N;
     const double k4 = L.grid == 1 ? P.k4 : P.cgdf;
     double acc[5] = {0, 0, 0, 0, 0};
-    for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) {
-        const int2 t = L.inc[k];
+    FLITE_FOR_INC(L, i, t) {
         const bool first = t.x >= 0;
         const int e = first ? t.x : ~t.x;
         const int i1 = first ? i : t.y, i2 = first ? t.y : i;
@@ -482,8 +481,7 @@ __global__ void k_lp_sums(Params P, LevelView L) {
     double g[15], l[5], lx[3] = {0.0, 0.0, 0.0}, s21 = 0.0, pd = 0.0, ps = 0.0;
     for (int c = 0; c < 15; ++c) g[c] = 0.0;
     for (int c = 0; c < 5; ++c) l[c] = 0.0;
-    for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) {
-        const int2 t = L.inc[k];
+    FLITE_FOR_INC(L, i, t) {
         const bool first = t.x >= 0;
         const int e = first ? t.x : ~t.x;
         const int i1 = first ? i : t.y, i2 = first ? t.y : i;
@@ -538,8 +536,7 @@ __global__ void k_lp_flux(Params P, LevelView L) {
     if (i >= L.N) return;
     const int N = L.N;
     double acc[5] = {0, 0, 0, 0, 0};
-    for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) {
-        const int2 t = L.inc[k];
+    FLITE_FOR_INC(L, i, t) {
         const bool first = t.x >= 0;
         const int e = first ? t.x : ~t.x;
         const int i1 = first ? i : t.y, i2 = first ? t.y : i;
@@ -577,8 +574,7 @@ __global__ void k_first_order_diss(Params P, LevelView L) {
     const int N = L.N;
     double acc[5] = {0, 0, 0, 0, 0};
     const double vdi = L.vdt[i], coni = L.conn[i];
-    for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) {
-        int2 t = L.inc[k];
+    FLITE_FOR_INC(L, i, t) {
         int j = t.y;
         double vdj = L.vdt[j];
         const bool first = t.x >= 0;
@@ -728,8 +724,7 @@ __global__ void __launch_bounds__(256, U == 1 ? 3 : 1) k_visc_grad(CaseArg<B, Pa
     };
     double qi[4];
     prim(i, qi);
-    auto iterms = [&](int k, double *d) {
-        int2 t = L.inc[k];
+    auto iterms = [&](const int2 t, double *d) {
         int e = t.x >= 0 ? t.x : ~t.x;
         double qj[4];
         prim(t.y, qj);
@@ -746,11 +741,12 @@ __global__ void __launch_bounds__(256, U == 1 ? 3 : 1) k_visc_grad(CaseArg<B, Pa
     };
     if constexpr (U > 1) {
         FLITE_GROUP_SLAB(double, 12);
-        group_sum<U, 12, 1, double>(gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl, iterms, g);
+        group_sum<U, 12, 1, double>(gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl,
+                                         [&](int k, double *v) { iterms(L.inc[k], v); }, g);
         group_sum<U, 12, 1, double>(gs, L.binc_ptr[i], L.binc_ptr[i + 1], active, gl, bterms, g);
         if (!active || gl) return;
     } else {
-        for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) vgrad_inc(L, L.inc[k], qi, g);
+        FLITE_FOR_INC(L, i, t) vgrad_inc(L, t, qi, g);
         visc_grad_boundary(L, i, g);
     }
     visc_grad_finish(P, L, i, g);
@@ -834,8 +830,7 @@ __global__ void __launch_bounds__(256, U == 1 ? 3 : 1) k_visc_flux(CaseArg<B, Pa
     ui[0] = L.prim[i]; ui[1] = L.prim[N + i]; ui[2] = L.prim[2 * N + i];
     double acc[4] = {0, 0, 0, 0};
     // interior edge: the edge flux with the sign of this node (x - y is x + (-y))
-    auto iterms = [&](int k, double *g) {
-        int2 t = L.inc[k];
+    auto iterms = [&](const int2 t, double *g) {
         int e = t.x >= 0 ? t.x : ~t.x, j = t.y;
         double tj[9], uj[3];
         for (int c = 0; c < 9; ++c) tj[c] = L.tau[c * N + j];
@@ -857,7 +852,8 @@ __global__ void __launch_bounds__(256, U == 1 ? 3 : 1) k_visc_flux(CaseArg<B, Pa
     };
     if constexpr (U > 1) {
         FLITE_GROUP_SLAB(double, 8);
-        group_sum<U, 4, 1, double>(gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl, iterms, acc);
+        group_sum<U, 4, 1, double>(gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl,
+                                        [&](int k, double *v) { iterms(L.inc[k], v); }, acc);
         // a face that does not count leaves zeros
         group_sum<U, 4, 2, double>(
             gs, L.binc_ptr[i], L.binc_ptr[i + 1], active, gl,
@@ -871,9 +867,9 @@ __global__ void __launch_bounds__(256, U == 1 ? 3 : 1) k_visc_flux(CaseArg<B, Pa
             acc);
         if (!active || gl) return;
     } else {
-        for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) {
+        FLITE_FOR_INC(L, i, t) {
             double v[4];
-            iterms(k, v);
+            iterms(t, v);
             iadd(v);
         }
         for (int k = L.binc_ptr[i]; k < L.binc_ptr[i + 1]; ++k) {
@@ -908,8 +904,7 @@ __global__ void __launch_bounds__(256, 3) k_ts_lap(CaseArg<B, Params> P_, CaseAr
     const double cc = dmax(P.gamma * pi * ro, 0.001);
     double acc = 0.0, h = 0.0;
     LapAcc a = {{0, 0, 0, 0, 0}, 0, 0};
-    for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) {
-        const int2 t = L.inc[k];
+    FLITE_FOR_INC(L, i, t) {
         ts_inc(P, L, t, ui[1], ui[2], ui[3], ro, cc, acc, h);
         lap_inc(P, L, t, ui, pi, a);
     }
@@ -936,8 +931,7 @@ __global__ void __launch_bounds__(256, 2) k_jflux_vgrad(CaseArg<B, Params> P_, C
     const double qi[4] = {L.prim[i], L.prim[N + i], L.prim[2 * N + i], L.prim[3 * N + i]};
     double g[12];
     for (int c = 0; c < 12; ++c) g[c] = 0.0;
-    for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) {
-        const int2 t = L.inc[k];
+    FLITE_FOR_INC(L, i, t) {
         jflux_inc(P, L, t, k4, vdi, coni, si, Li, Ui, acc);
         vgrad_inc(L, t, qi, g);
     }
@@ -1019,8 +1013,7 @@ __global__ void __launch_bounds__(256, U == 1 ? 3 : 1) k_visc2_grad(CaseArg<B, P
     };
     double qi[4];
     prim(i, qi);
-    auto iterms = [&](int k, double *d) {
-        int2 t = L.inc[k];
+    auto iterms = [&](const int2 t, double *d) {
         int e = t.x >= 0 ? t.x : ~t.x;
         double qj[4];
         prim(t.y, qj);
@@ -1051,13 +1044,14 @@ __global__ void __launch_bounds__(256, U == 1 ? 3 : 1) k_visc2_grad(CaseArg<B, P
     };
     if constexpr (U > 1) {
         FLITE_GROUP_SLAB(double, 12);
-        group_sum<U, 12, 1, double>(gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl, iterms, g);
+        group_sum<U, 12, 1, double>(gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl,
+                                         [&](int k, double *v) { iterms(L.inc[k], v); }, g);
         group_sum<U, 12, 1, double>(gs, L.binc_ptr[i], L.binc_ptr[i + 1], active, gl, bterms, g);
         if (!active || gl) return;
     } else {
-        for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) {
+        FLITE_FOR_INC(L, i, t) {
             double v[12];
-            iterms(k, v);
+            iterms(t, v);
             add(v);
         }
         for (int k = L.binc_ptr[i]; k < L.binc_ptr[i + 1]; ++k) {
@@ -1137,8 +1131,7 @@ __global__ void __launch_bounds__(256, U == 1 ? 2 : 1) k_visc2_flux(CaseArg<B, P
     Visc2Node me;
     load_visc2(P, L, i, me);
     double acc[4] = {0, 0, 0, 0};
-    auto iterms = [&](int k, double *g) {
-        const int2 t = L.inc[k];
+    auto iterms = [&](const int2 t, double *g) {
         const int e = t.x >= 0 ? t.x : ~t.x;
         Visc2Node nb;
         load_visc2(P, L, t.y, nb);
@@ -1180,7 +1173,8 @@ __global__ void __launch_bounds__(256, U == 1 ? 2 : 1) k_visc2_flux(CaseArg<B, P
     };
     if constexpr (U > 1) {
         FLITE_GROUP_SLAB(double, 4);
-        group_sum<U, 4, 1, double>(gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl, iterms, acc);
+        group_sum<U, 4, 1, double>(gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl,
+                                        [&](int k, double *v) { iterms(L.inc[k], v); }, acc);
         group_sum<U, 4, 1, double>(
             gs, L.binc_ptr[i], L.binc_ptr[i + 1], active, gl,
             [&](int k, double *v) {
@@ -1193,9 +1187,9 @@ __global__ void __launch_bounds__(256, U == 1 ? 2 : 1) k_visc2_flux(CaseArg<B, P
             acc);
         if (!active || gl) return;
     } else {
-        for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) {
+        FLITE_FOR_INC(L, i, t) {
             double v[4];
-            iterms(k, v);
+            iterms(t, v);
             iadd(v);
         }
         for (int k = L.binc_ptr[i]; k < L.binc_ptr[i + 1]; ++k) {
@@ -1221,8 +1215,7 @@ __global__ void k_gradient(Params P, LevelView L) {
     for (int c = 0; c < 15; ++c) g[c] = 0.0;
     const double ri = L.u[i];
     const double qi[5] = {ri, L.u[N + i] / ri, L.u[2 * N + i] / ri, L.u[3 * N + i] / ri, L.u[4 * N + i]};
-    for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) {
-        int2 t = L.inc[k];
+    FLITE_FOR_INC(L, i, t) {
         int e = t.x >= 0 ? t.x : ~t.x, j = t.y;
         const double rj = L.u[j];
         const double qj[5] = {rj, L.u[N + j] / rj, L.u[2 * N + j] / rj, L.u[3 * N + j] / rj, L.u[4 * N + j]};
@@ -1275,8 +1268,7 @@ __global__ void k_gradient_rec(LevelView L) {
     for (int c = 0; c < 15; ++c) g[c] = 0.0;
     const PrimRec Qi = load_prim(L.qp, i);
     const double qi[5] = {Qi.r, Qi.u, Qi.v, Qi.w, Qi.E};
-    for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) {
-        const int2 t = L.inc[k];
+    FLITE_FOR_INC(L, i, t) {
         const int e = t.x >= 0 ? t.x : ~t.x;
         const PrimRec Qj = load_prim(L.qp, t.y);
         const double qj[5] = {Qj.r, Qj.u, Qj.v, Qj.w, Qj.E};
@@ -1327,8 +1319,7 @@ __global__ void k_ls_gradient(Params P, LevelView L) {
     for (int sc = 0; sc < 5; ++sc) b[sc][0] = b[sc][1] = b[sc][2] = 0.0;
     const double ri = L.u[i];
     const double qi[5] = {ri, L.u[N + i] / ri, L.u[2 * N + i] / ri, L.u[3 * N + i] / ri, L.u[4 * N + i]};
-    for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) {
-        int2 t = L.inc[k];
+    FLITE_FOR_INC(L, i, t) {
         int j = t.y;
         const bool first = t.x >= 0;
         const int i1 = first ? i : j, i2 = first ? j : i;
@@ -1370,8 +1361,7 @@ __global__ void k_minmax(Params P, LevelView L) {
     for (int c = 0; c < 5; ++c) { mn[c] = 1.0e15; mx[c] = 1.0e15; }
     const double ri = L.u[i];
     const double qi[5] = {ri, L.u[N + i] / ri, L.u[2 * N + i] / ri, L.u[3 * N + i] / ri, L.u[4 * N + i]};
-    for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) {
-        int2 t = L.inc[k];
+    FLITE_FOR_INC(L, i, t) {
         int j = t.y;
         const double rj = L.u[j];
         const double qj[5] = {rj, L.u[N + j] / rj, L.u[2 * N + j] / rj, L.u[3 * N + j] / rj, L.u[4 * N + j]};
@@ -1493,6 +1483,17 @@ __global__ void k_delta_state(CaseArg<B, LevelView> L_) {
     p[0] = d[0]; p[1] = d[1]; p[2] = d[2];
 }
 
+// the rows of a level from its incidence lists; entries past a node's
+// degree are the node itself with edge 0 (never used)
+__global__ void k_make_rows(LevelView L, int nrows, int2 *rows) {
+    const int i = tid();
+    if (i >= L.N) return;
+    const int beg = L.inc_ptr[i], deg = L.inc_ptr[i + 1] - beg, s = i / kRow;
+    const int first = L.row_ptr[s], last = (s + 1) * kRow < L.N ? L.row_ptr[s + 1] : nrows;
+    for (int k = 0; k < last - first; ++k)
+        rows[(size_t)(first + k) * kRow + i % kRow] = k < deg ? L.inc[beg + k] : make_int2(0, i);
+}
+
 // FP32 incidences of the increments (w rounded once; j is ~j when the node
 // is the edge's second node)
 __global__ void k_make_inc32(const int2 *inc, const EdgeW *ew, int n, IncRec32 *o) {
@@ -1532,8 +1533,7 @@ __device__ __forceinline__ void gather_interior_delta(const LevelView &L, int i,
                                                       double *gs) {
     float acc[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
     const DeltaRec me = load_delta(L.dq, i);
-    auto terms = [&](int k, float *s5, bool &first) {
-        const IncRec32 t = load_inc32(L.inc32, k);
+    auto terms = [&](const IncRec32 &t, float *s5, bool &first) {
         first = t.j >= 0;
         const DeltaRec nb = load_delta(L.dq, first ? t.j : ~t.j);
         float g1[5], g2[5];
@@ -1546,16 +1546,18 @@ __device__ __forceinline__ void gather_interior_delta(const LevelView &L, int i,
             reinterpret_cast<float *>(gs), L.inc_ptr[i], L.inc_ptr[i + 1], active, gl,
             [&](int k, float *v) {
                 bool first;
-                terms(k, v, first);
+                terms(load_inc32(L.inc32, k), v, first);
                 if (!first)
                     for (int c = 0; c < 5; ++c) v[c] = -v[c];  // x - y is x + (-y)
             },
             acc);
     } else {
-        for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) {
+        const int deg = L.inc_ptr[i + 1] - L.inc_ptr[i];
+        const IncRec32 *row = L.rows32 + ((size_t)L.row_ptr[i / kRow] * kRow + i % kRow);
+        for (int k = 0; k < deg; ++k, row += kRow) {
             float v[5];
             bool first;
-            terms(k, v, first);
+            terms(load_inc32(row, 0), v, first);
             if (first) {
                 for (int c = 0; c < 5; ++c) acc[c] += v[c];
             } else {
@@ -1567,74 +1569,109 @@ __device__ __forceinline__ void gather_interior_delta(const LevelView &L, int i,
     for (int c = 0; c < 5; ++c) r[c] = L.ra[c * N + i] + (double)acc[c];
 }
 
-// the same sum with the loads of two incidences issued before either flux
-// is computed (more loads in flight per thread); the additions stay in edge
-// order, so the result is the same bit for bit
-__device__ __forceinline__ void gather_interior_central2(const LevelView &L, int i, double *r) {
+// Interior central fluxes of node i with a thread per node, summed in edge
+// order: the other nodes' records and the edges' coefficients of the next
+// kPipe - 1 incidences are copied ahead into the thread's own slots of shared
+// memory (asynchronous copies hold no registers, and each thread waits for
+// its own only).
+// What bounds it: the latency of the loads, not their bytes.  On the
+// 815,425-node level one launch takes 131 us with the copies ahead, 154 us
+// with plain loads from the incidence lists and 172 us with plain loads from
+// the rows; kPipe 2, 3 and 4 take 154, 139 and 140 us without the prefetch
+// below, 5 blocks of 128 threads per SM fit without spills, 4 and 6 take 152
+// and 163 us.
+constexpr int kPipe = 3, kPipeThreads = 128;
+__device__ __forceinline__ void copy_ahead16(void *d, const void *g) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(d)), "l"(g)
+                 : "memory");
+}
+__device__ __forceinline__ void copy_ahead8(void *d, const void *g) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(d)), "l"(g)
+                 : "memory");
+}
+__device__ __forceinline__ void gather_central_ahead(const LevelView &L, int i, double *r) {
+    __shared__ double2 sq[kPipe][3][kPipeThreads];
+    __shared__ double sw[kPipe][3][kPipeThreads];
+    const int tx = threadIdx.x;
     r[0] = r[1] = r[2] = r[3] = r[4] = 0.0;
+    const int deg = L.inc_ptr[i + 1] - L.inc_ptr[i];
+    const int2 *row = L.rows + ((size_t)L.row_ptr[i / kRow] * kRow + i % kRow);
     const NodeRec si = load_node(L.q, i);
-    const int end = L.inc_ptr[i + 1];
-    int k = L.inc_ptr[i];
-    auto add = [&](const int2 t, const EdgeW &w, const NodeRec &n) {
-        const NodeRec &sj = n;
-        double f[5];
-        if (t.x >= 0) {
-            central_flux_rec(si, sj, w.wx, w.wy, w.wz, f);
-            r[0] = r[0] + f[0]; r[1] = r[1] + f[1]; r[2] = r[2] + f[2]; r[3] = r[3] + f[3]; r[4] = r[4] + f[4];
-        } else {
-            central_flux_rec(sj, si, w.wx, w.wy, w.wz, f);
-            r[0] = r[0] - f[0]; r[1] = r[1] - f[1]; r[2] = r[2] - f[2]; r[3] = r[3] - f[3]; r[4] = r[4] - f[4];
-        }
+    int side[kPipe];
+    auto issue = [&](const int2 t, int d) {
+        const int e = t.x >= 0 ? t.x : ~t.x;
+        const double2 *q = reinterpret_cast<const double2 *>(L.q + t.y);
+        copy_ahead16(&sq[d][0][tx], q);
+        copy_ahead16(&sq[d][1][tx], q + 1);
+        copy_ahead16(&sq[d][2][tx], q + 2);
+        copy_ahead8(&sw[d][0][tx], L.wx + e);
+        copy_ahead8(&sw[d][1][tx], L.wy + e);
+        copy_ahead8(&sw[d][2][tx], L.wz + e);
+        side[d] = t.x;
     };
-    for (; k + 1 < end; k += 2) {
-        const int2 t0 = L.inc[k], t1 = L.inc[k + 1];
-        const EdgeW w0 = load_edgew(L.ew, t0.x >= 0 ? t0.x : ~t0.x);
-        const EdgeW w1 = load_edgew(L.ew, t1.x >= 0 ? t1.x : ~t1.x);
-        const NodeRec n0 = load_node(L.q, t0.y), n1 = load_node(L.q, t1.y);
-        add(t0, w0, n0);
-        add(t1, w1, n1);
+#pragma unroll
+    for (int d = 0; d < kPipe - 1; ++d) {
+        if (d < deg) issue(__ldg(row + d * kRow), d);
+        asm volatile("cp.async.commit_group;");
     }
-    if (k < end) {
-        const int2 t0 = L.inc[k];
-        add(t0, load_edgew(L.ew, t0.x >= 0 ? t0.x : ~t0.x), load_node(L.q, t0.y));
+    int2 t = make_int2(0, 0);
+    if (kPipe - 1 < deg) t = __ldg(row + (kPipe - 1) * kRow);
+    for (int k0 = 0; k0 < deg; k0 += kPipe) {
+#pragma unroll
+        for (int d = 0; d < kPipe; ++d) {
+            const int k = k0 + d, kn = k + kPipe - 1;
+            if (k >= deg) break;
+            if (kn < deg) issue(t, (d + kPipe - 1) % kPipe);
+            asm volatile("cp.async.commit_group;");
+            if (kn + 1 < deg) t = __ldg(row + (size_t)(kn + 1) * kRow);
+            asm volatile("cp.async.wait_group %0;" ::"n"(kPipe - 1) : "memory");
+            const double2 a = sq[d][0][tx], b = sq[d][1][tx], c = sq[d][2][tx];
+            const NodeRec n = {a.x, a.y, b.x, b.y, c.x, c.y};
+            const double wx = sw[d][0][tx], wy = sw[d][1][tx], wz = sw[d][2][tx];
+            double f[5];
+            if (side[d] >= 0) {
+                central_flux_rec(si, n, wx, wy, wz, f);
+                r[0] = r[0] + f[0]; r[1] = r[1] + f[1]; r[2] = r[2] + f[2]; r[3] = r[3] + f[3]; r[4] = r[4] + f[4];
+            } else {
+                central_flux_rec(n, si, wx, wy, wz, f);
+                r[0] = r[0] - f[0]; r[1] = r[1] - f[1]; r[2] = r[2] - f[2]; r[3] = r[3] - f[3]; r[4] = r[4] - f[4];
+            }
+        }
     }
 }
+// The block's incidence rows (one contiguous run) on their way to L2 before
+// the walk asks for them row by row: 16-byte aligned, whole rows of 256 bytes.
+__device__ __forceinline__ void prefetch_rows(const LevelView &L) {
+    if (threadIdx.x) return;
+    const int i0 = blockIdx.x * blockDim.x;
+    const int s0 = i0 / kRow, s1 = min(i0 + (int)blockDim.x, L.N) / kRow;
+    const int r0 = L.row_ptr[s0], r1 = s1 * kRow < L.N ? L.row_ptr[s1] : r0;
+    if (r1 > r0)
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(L.rows + (size_t)r0 * kRow),
+                     "r"((unsigned)(r1 - r0) * (unsigned)(kRow * sizeof(int2))));
+}
 
-// interior central fluxes of node i computed from the two node records of
-// each incident edge, summed in edge order: the same numbers, in the same
-// order, as the edge kernel followed by the buffer gather
+// the same sums with a group of lanes per node
 template <int U>
 __device__ __forceinline__ void gather_interior_central(const LevelView &L, int i, double *r, bool active, int gl,
                                                         double *gs) {
     r[0] = r[1] = r[2] = r[3] = r[4] = 0.0;
     const NodeRec si = load_node(L.q, i);
-    // the flux of incidence k with this node's sign (x - y is x + (-y))
-    auto terms = [&](int k, double *g) {
-        const int2 t = L.inc[k];
-        const int e = t.x >= 0 ? t.x : ~t.x;
-        const EdgeW w = load_edgew(L.ew, e);
-        const NodeRec n = load_node(L.q, t.y);
-        double f[5];
-        if (t.x >= 0) {
-            central_flux_rec(si, n, w.wx, w.wy, w.wz, f);
-            for (int c = 0; c < 5; ++c) g[c] = f[c];
-        } else {
-            central_flux_rec(n, si, w.wx, w.wy, w.wz, f);
-            for (int c = 0; c < 5; ++c) g[c] = -f[c];
-        }
-    };
-    auto add = [&](const double *g) {
-        r[0] = r[0] + g[0]; r[1] = r[1] + g[1]; r[2] = r[2] + g[2]; r[3] = r[3] + g[3]; r[4] = r[4] + g[4];
-    };
-    if constexpr (U > 1) {
-        group_sum<U, 5, 1, double>(gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl, terms, r);
-    } else {
-        for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) {
-            double v[5];
-            terms(k, v);
-            add(v);
-        }
-    }
+    group_sum<U, 5, 1, double>(
+        gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl,
+        [&](int k, double *g) {
+            const int2 t = L.inc[k];
+            const EdgeW w = load_edgew(L.ew, t.x >= 0 ? t.x : ~t.x);
+            const NodeRec n = load_node(L.q, t.y);
+            if (t.x >= 0) {
+                central_flux_rec(si, n, w.wx, w.wy, w.wz, g);
+            } else {  // this node's sign: x - y is x + (-y)
+                double f[5];
+                central_flux_rec(n, si, w.wx, w.wy, w.wz, f);
+                for (int c = 0; c < 5; ++c) g[c] = -f[c];
+            }
+        },
+        r);
 }
 
 // interior edges of node i from the FP64 edge buffer, in edge order
@@ -1642,8 +1679,8 @@ template <int U>
 __device__ __forceinline__ void gather_interior(const LevelView &L, int i, double *r, bool active, int gl,
                                                 double *gs) {
     r[0] = r[1] = r[2] = r[3] = r[4] = 0.0;
-    auto terms = [&](int k, double *g) {
-        const int s = L.inc[k].x;
+    auto terms = [&](const int2 t, double *g) {
+        const int s = t.x;
         const double *f = L.flux + (size_t)(s >= 0 ? s : ~s) * 5;
         for (int c = 0; c < 5; ++c) g[c] = s >= 0 ? f[c] : -f[c];  // x - y is x + (-y)
     };
@@ -1651,11 +1688,12 @@ __device__ __forceinline__ void gather_interior(const LevelView &L, int i, doubl
         r[0] = r[0] + g[0]; r[1] = r[1] + g[1]; r[2] = r[2] + g[2]; r[3] = r[3] + g[3]; r[4] = r[4] + g[4];
     };
     if constexpr (U > 1) {
-        group_sum<U, 5, 1, double>(gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl, terms, r);
+        group_sum<U, 5, 1, double>(gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl,
+                                        [&](int k, double *v) { terms(L.inc[k], v); }, r);
     } else {
-        for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) {
+        FLITE_FOR_INC(L, i, t) {
             double v[5];
-            terms(k, v);
+            terms(t, v);
             add(v);
         }
     }
@@ -1853,7 +1891,7 @@ __device__ __forceinline__ void node_tail(const Params &P, const LevelView &L, i
 // same, stored as the new mixed-precision anchor), GATHER_DELTA (anchor +
 // FP32 increments)
 template <int PREC, int U, bool B>
-__global__ void __launch_bounds__(256, PREC == GATHER_CENTRAL2 ? 2 : (U == 1 ? 3 : 1))
+__global__ void __launch_bounds__(node_threads(PREC, U), U > 1 ? 1 : (central_ahead(PREC) ? 5 : 3))
     k_node_update(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_, int mode, int stage) {
     FLITE_CASE_P(B, P, L);
     FLITE_CASE_L(B, L);
@@ -1862,6 +1900,7 @@ __global__ void __launch_bounds__(256, PREC == GATHER_CENTRAL2 ? 2 : (U == 1 ? 3
     if (U == 1 && i_raw >= L.N) return;
     const bool active = i_raw < L.N;
     const int i = active ? i_raw : L.N - 1;  // idle groups read a valid node
+    if constexpr (U == 1 && central_ahead(PREC)) prefetch_rows(L);
     double r[5];
     FLITE_GROUP_SLAB(double, 10);
     // a node's own operands are read before the chain of its gather starts
@@ -1871,8 +1910,8 @@ __global__ void __launch_bounds__(256, PREC == GATHER_CENTRAL2 ? 2 : (U == 1 ? 3
         gather_interior_delta<U>(L, i, r, active, gl, gs);
     } else if constexpr (PREC == GATHER_BUFFER) {
         gather_interior<U>(L, i, r, active, gl, gs);
-    } else if constexpr (PREC == GATHER_CENTRAL2) {
-        gather_interior_central2(L, i, r);
+    } else if constexpr (U == 1) {
+        gather_central_ahead(L, i, r);
     } else {
         gather_interior_central<U>(L, i, r, active, gl, gs);
     }
@@ -1886,378 +1925,6 @@ __global__ void __launch_bounds__(256, PREC == GATHER_CENTRAL2 ? 2 : (U == 1 ? 3
     if constexpr (PREC == GATHER_ANCHOR) store_anchor(L, i, rint);
     node_tail<PREC == GATHER_LEAN>(P, L, i, r, mode, stage, U > 1 ? &in : nullptr);
 }
-// ---- the same node update with the central fluxes gathered from a
-// shared-memory stage of the node block (GATHER_CENTRAL, a thread per node).
-// Block t handles the kTile nodes t*kTile.. of the level; it first copies
-// their 48-byte records and those of the block's halo (the other nodes its
-// edges reach, in increasing node order) into shared memory with coalesced
-// or independent loads, then every thread walks its node's incidences in
-// edge order through the block's incidence rows (row k holds incidence k of
-// every node of the block: the coefficients and the staged slot of the
-// other node, read with coalesced loads).  A neighbour beyond the stage's
-// capacity is read from the global records.  The flux of each incidence and
-// the order of the additions are those of k_node_update, so the results are
-// identical bit for bit.
-__device__ __forceinline__ NodeRec load_node_shared(const NodeRec *rec, int slot) {
-    const float4 *p = reinterpret_cast<const float4 *>(rec + slot);
-    NodeRec o;
-    float4 *d = reinterpret_cast<float4 *>(&o);
-    d[0] = p[0]; d[1] = p[1]; d[2] = p[2];
-    return o;
-}
-
-template <bool STAGE, bool AHEAD>
-__global__ void __launch_bounds__(kTile, AHEAD ? 2 : 3) k_node_update_tiled(Params P, LevelView L, int mode,
-                                                                            int stage) {
-    extern __shared__ float4 stage_mem[];
-    NodeRec *rec = reinterpret_cast<NodeRec *>(stage_mem);
-    const TileView &T = L.tile;
-    const int t = blockIdx.x, n0 = t * kTile;
-    const int cnt = min(kTile, L.N - n0);
-    if (STAGE) {
-        const int h0 = T.halo_ptr[t];
-        const int nh = min(T.halo_ptr[t + 1] - h0, kTileStageMax - kTile);
-        const float4 *q = reinterpret_cast<const float4 *>(L.q);
-        // 16-byte pieces: 3 per record, own records then the halo's
-        for (int s = threadIdx.x; s < 3 * (cnt + nh); s += blockDim.x) {
-            const int r = s / 3, part = s - 3 * r;
-            const int j = r < cnt ? n0 + r : T.halo[h0 + (r - cnt)];
-            const int slot = r < cnt ? r : kTile + (r - cnt);
-            stage_mem[3 * slot + part] = __ldg(q + 3 * (size_t)j + part);
-        }
-        __syncthreads();
-    }
-    if ((int)threadIdx.x >= cnt) return;
-    const int i = n0 + threadIdx.x;
-    const NodeRec si = STAGE ? load_node_shared(rec, threadIdx.x) : load_node(L.q, i);
-    const int deg = L.inc_ptr[i + 1] - L.inc_ptr[i];
-    const size_t base = (size_t)T.row[t] * kTile + threadIdx.x;
-    const unsigned *meta = STAGE ? T.meta : T.nmeta;
-    auto fetch = [&](unsigned m) -> NodeRec {
-        const int v = (int)(m & kTileIndexMask);
-        if (!STAGE || (m & kTileGlobal)) return load_node(L.q, v);
-        return load_node_shared(rec, v);
-    };
-    double r[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    if (!AHEAD) {
-        for (int k = 0; k < deg; ++k) {
-            const size_t x = base + (size_t)k * kTile;
-            const unsigned m = __ldg(meta + x);
-            const double wx = __ldg(T.wx + x), wy = __ldg(T.wy + x), wz = __ldg(T.wz + x);
-            const NodeRec n = fetch(m);
-            double f[5];
-            if (!(m & kTileSecond)) {
-                central_flux_rec(si, n, wx, wy, wz, f);
-                r[0] = r[0] + f[0]; r[1] = r[1] + f[1]; r[2] = r[2] + f[2]; r[3] = r[3] + f[3]; r[4] = r[4] + f[4];
-            } else {
-                central_flux_rec(n, si, wx, wy, wz, f);
-                r[0] = r[0] + (-f[0]); r[1] = r[1] + (-f[1]); r[2] = r[2] + (-f[2]); r[3] = r[3] + (-f[3]);
-                r[4] = r[4] + (-f[4]);
-            }
-        }
-        gather_boundary<1>(L, i, r);
-        node_tail(P, L, i, r, mode, stage);
-        return;
-    }
-    // the loads of incidence k+1 are issued before incidence k is evaluated
-    unsigned m0 = 0;
-    double wx0 = 0, wy0 = 0, wz0 = 0;
-    NodeRec n0r{};
-    if (deg > 0) {
-        m0 = __ldg(meta + base);
-        wx0 = __ldg(T.wx + base); wy0 = __ldg(T.wy + base); wz0 = __ldg(T.wz + base);
-        n0r = fetch(m0);
-    }
-    for (int k = 0; k < deg; ++k) {
-        unsigned m1 = 0;
-        double wx1 = 0, wy1 = 0, wz1 = 0;
-        NodeRec n1r{};
-        if (k + 1 < deg) {
-            const size_t x = base + (size_t)(k + 1) * kTile;
-            m1 = __ldg(meta + x);
-            wx1 = __ldg(T.wx + x); wy1 = __ldg(T.wy + x); wz1 = __ldg(T.wz + x);
-            n1r = fetch(m1);
-        }
-        double f[5];
-        if (!(m0 & kTileSecond)) {
-            central_flux_rec(si, n0r, wx0, wy0, wz0, f);
-            r[0] = r[0] + f[0]; r[1] = r[1] + f[1]; r[2] = r[2] + f[2]; r[3] = r[3] + f[3]; r[4] = r[4] + f[4];
-        } else {
-            central_flux_rec(n0r, si, wx0, wy0, wz0, f);
-            r[0] = r[0] + (-f[0]); r[1] = r[1] + (-f[1]); r[2] = r[2] + (-f[2]); r[3] = r[3] + (-f[3]);
-            r[4] = r[4] + (-f[4]);
-        }
-        m0 = m1; wx0 = wx1; wy0 = wy1; wz0 = wz1; n0r = n1r;
-    }
-    gather_boundary<1>(L, i, r);
-    node_tail(P, L, i, r, mode, stage);
-}
-
-// ---- the other gathers of a level through the incidence rows of node blocks
-// Each kernel walks its node's incidences in edge order through the block's
-// incidence rows (row k holds incidence k of each node of the block), with
-// the loads of incidence k+1 issued before incidence k is evaluated.  With
-// STAGE the K node fields (SoA arrays) it reads at the other node are first
-// copied for the block and its halo into shared memory as sm[slot*K + c];
-// without, they are read from the global arrays.  The per-incidence
-// arithmetic and the order of the additions are those of the kernels'
-// thread-per-node forms above, so the results are identical bit for bit.
-template <int K>
-__device__ __forceinline__ void stage_fields(double *sm, const TileView &T, const double *const *f, int n0, int cnt,
-                                             int h0, int nh) {
-#pragma unroll 1
-    for (int c = 0; c < K; ++c)
-        for (int s = threadIdx.x; s < cnt + nh; s += blockDim.x) {
-            const int j = s < cnt ? n0 + s : T.halo[h0 + (s - cnt)];
-            const int slot = s < cnt ? s : kTile + (s - cnt);
-            sm[slot * K + c] = __ldg(f[c] + j);
-        }
-}
-
-// the block of the calling thread and its halo (staged part), with the
-// fields staged when STAGE; returns the node, or -1 for the block's idle
-// threads
-template <int K, bool STAGE>
-__device__ __forceinline__ int tile_begin(double *sm, const LevelView &L, const double *const *f) {
-    const int n0 = blockIdx.x * kTile;
-    const int cnt = min(kTile, L.N - n0);
-    if (STAGE && K > 0) {
-        const int h0 = L.tile.halo_ptr[blockIdx.x];
-        const int nh = min(L.tile.halo_ptr[blockIdx.x + 1] - h0, kTileStageMax - kTile);
-        stage_fields<K>(sm, L.tile, f, n0, cnt, h0, nh);
-        __syncthreads();
-    }
-    return (int)threadIdx.x < cnt ? n0 + (int)threadIdx.x : -1;
-}
-
-// one incidence of the row walk: the other node's K fields, the flags and
-// (when W) the edge coefficients
-template <int K, bool STAGE, bool W>
-struct Inc {
-    unsigned m;
-    double w[3];
-    double v[K > 0 ? K : 1];
-    __device__ __forceinline__ void load(const LevelView &L, const double *sm, const double *const *f, size_t x) {
-        m = __ldg((STAGE ? L.tile.meta : L.tile.nmeta) + x);
-        if (W) { w[0] = __ldg(L.tile.wx + x); w[1] = __ldg(L.tile.wy + x); w[2] = __ldg(L.tile.wz + x); }
-        const int idx = (int)(m & kTileIndexMask);
-        if (!STAGE || (m & kTileGlobal)) {
-#pragma unroll
-            for (int c = 0; c < K; ++c) v[c] = __ldg(f[c] + idx);
-        } else {
-#pragma unroll
-            for (int c = 0; c < K; ++c) v[c] = sm[idx * K + c];
-        }
-    }
-    __device__ __forceinline__ bool first() const { return !(m & kTileSecond); }
-};
-
-// walk node i's incidence rows calling fn(inc) in edge order (AHEAD: the
-// loads of incidence k+1 issued before fn sees incidence k)
-template <int K, bool STAGE, bool W, bool AHEAD, class Fn>
-__device__ __forceinline__ void row_walk(const LevelView &L, const double *sm, const double *const *f, int i,
-                                         Fn &&fn) {
-    const int deg = L.inc_ptr[i + 1] - L.inc_ptr[i];
-    const size_t base = (size_t)L.tile.row[blockIdx.x] * kTile + threadIdx.x;
-    if (deg <= 0) return;
-    if (!AHEAD) {
-        for (int k = 0; k < deg; ++k) {
-            Inc<K, STAGE, W> a;
-            a.load(L, sm, f, base + (size_t)k * kTile);
-            fn(a);
-        }
-        return;
-    }
-    Inc<K, STAGE, W> a, b;
-    a.load(L, sm, f, base);
-    for (int k = 0; k < deg; ++k) {
-        if (k + 1 < deg) b.load(L, sm, f, base + (size_t)(k + 1) * kTile);
-        fn(a);
-        a = b;
-    }
-}
-
-// makeTimeSteps: K = 0 (inviscid: the other node is not read), 2 (mu, rho),
-// 3 (with the SA nu~)
-template <int K, bool STAGE, bool AHEAD>
-__global__ void __launch_bounds__(kTile, 3) k_timestep_tiled(Params P, LevelView L) {
-    extern __shared__ double sm[];
-    const int N = L.N;
-    const double *f[3] = {L.mu, L.u, L.u + 5 * (size_t)N};
-    const int i = tile_begin<K, STAGE>(sm, L, f);
-    if (i < 0) return;
-    const double c1 = P.gamma;
-    const double ri = L.u[i], ro = 1. / ri;
-    const double m1 = L.u[N + i], m2 = L.u[2 * N + i], m3 = L.u[3 * N + i];
-    const double cc = dmax(c1 * L.p[i] * ro, 0.001);
-    double acc = 0.0, h = 0.0;
-    row_walk<K, STAGE, true, AHEAD>(L, sm, f, i, [&](const Inc<K, STAGE, true> &t) {
-        const double wx = t.w[0], wy = t.w[1], wz = t.w[2];
-        double al = (wx * wx + wy * wy) + wz * wz;
-        double vn = ((wx * m1 + wy * m2) + wz * m3) * ro;
-        acc = (acc + fabs(vn)) + sqrt(cc * al);
-        if (K > 0) {
-            double vis = dmax(P.am, K == 3 ? t.v[0] + t.v[K == 3 ? 2 : 0] / P.Re : t.v[0]);
-            double dv = 2.0 * vis * al / t.v[K > 1 ? 1 : 0];
-            h = h + dv;
-        }
-    });
-    ts_finish(P, L, i, acc, h);
-}
-
-// makeArtificialDissipation2 passes 1-2 (no dissipation weighting): the
-// other node's u and p
-template <bool STAGE, bool AHEAD>
-__global__ void __launch_bounds__(kTile, 3) k_jst_lap_tiled(Params P, LevelView L) {
-    extern __shared__ double sm[];
-    const int N = L.N;
-    const double *f[6] = {L.u, L.u + N, L.u + 2 * (size_t)N, L.u + 3 * (size_t)N, L.u + 4 * (size_t)N, L.p};
-    const int i = tile_begin<6, STAGE>(sm, L, f);
-    if (i < 0) return;
-    double l0 = 0, l1 = 0, l2 = 0, l3 = 0, l4 = 0, s7 = 0, s8 = 0;
-    const double ui0 = L.u[i], ui1 = L.u[N + i], ui2 = L.u[2 * N + i], ui3 = L.u[3 * N + i], ui4 = L.u[4 * N + i];
-    const double pi = L.p[i];
-    const double df = 1.0;
-    row_walk<6, STAGE, false, AHEAD>(L, sm, f, i, [&](const Inc<6, STAGE, false> &t) {
-        const double uj0 = t.v[0], uj1 = t.v[1], uj2 = t.v[2], uj3 = t.v[3], uj4 = t.v[4], pj = t.v[5];
-        if (t.first()) {
-            double d0 = ui0 - uj0, d1 = ui1 - uj1, d2 = ui2 - uj2, d3 = ui3 - uj3;
-            double d4 = ((ui4 - uj4) + pi) - pj;
-            l0 = l0 - d0 * df; l1 = l1 - d1 * df; l2 = l2 - d2 * df; l3 = l3 - d3 * df; l4 = l4 - d4 * df;
-            double dp = pi - pj, sp = pi + pj;
-            s7 = s7 - dp; s8 = s8 + sp;
-        } else {
-            double d0 = uj0 - ui0, d1 = uj1 - ui1, d2 = uj2 - ui2, d3 = uj3 - ui3;
-            double d4 = ((uj4 - ui4) + pj) - pi;
-            l0 = l0 + d0 * df; l1 = l1 + d1 * df; l2 = l2 + d2 * df; l3 = l3 + d3 * df; l4 = l4 + d4 * df;
-            double dp = pj - pi, sp = pj + pi;
-            s7 = s7 + dp; s8 = s8 + sp;
-        }
-    });
-    double fact = 1. / L.conn[i];
-    L.sens[i] = 12. * fabs(s7 / s8);
-    L.lap[i] = fact * l0;
-    L.lap[N + i] = fact * l1;
-    L.lap[2 * N + i] = fact * l2;
-    L.lap[3 * N + i] = fact * l3;
-    L.lap[4 * N + i] = fact * l4;
-}
-
-// makeArtificialDissipation2 pass 3, scalar: the other node's V/dt,
-// connectivity, sensor, Laplacian and u
-template <bool STAGE, bool AHEAD>
-__global__ void __launch_bounds__(kTile, AHEAD ? 2 : 3) k_jst_flux_tiled(Params P, LevelView L) {
-    extern __shared__ double sm[];
-    const int N = L.N;
-    const double *f[13] = {L.vdt, L.conn, L.sens,
-                           L.lap, L.lap + N, L.lap + 2 * (size_t)N, L.lap + 3 * (size_t)N, L.lap + 4 * (size_t)N,
-                           L.u, L.u + N, L.u + 2 * (size_t)N, L.u + 3 * (size_t)N, L.u + 4 * (size_t)N};
-    const int i = tile_begin<13, STAGE>(sm, L, f);
-    if (i < 0) return;
-    const double k4 = L.grid == 1 ? P.k4 : P.cgdf;
-    double acc[5] = {0, 0, 0, 0, 0};
-    double Li[5], Ui[5];
-    for (int c = 0; c < 5; ++c) { Li[c] = L.lap[c * N + i]; Ui[c] = L.u[c * N + i]; }
-    const double vdi = L.vdt[i], coni = L.conn[i], si = L.sens[i];
-    row_walk<13, STAGE, false, AHEAD>(L, sm, f, i, [&](const Inc<13, STAGE, false> &t) {
-        const bool first = t.first();
-        const double vdj = t.v[0], conj = t.v[1];
-        double d0 = first ? dmin(vdi, vdj) : dmin(vdj, vdi);
-        d0 = d0 / (first ? (coni + conj) : (conj + coni));
-        const double sj = t.v[2];
-        double d2 = d0 * P.k2 * (first ? dmax(si, sj) : dmax(sj, si));
-        double d4 = d0 * k4;
-        d4 = d4 > d2 ? d4 - d2 : 0.0;
-#pragma unroll
-        for (int c = 0; c < 5; ++c) {
-            const double Lj = t.v[3 + c], Uj = t.v[8 + c];
-            if (first) {
-                double d4v = Li[c] - Lj, d2v = Ui[c] - Uj;
-                acc[c] = (acc[c] - d4v * d4) + d2v * d2;
-            } else {
-                double d4v = Lj - Li[c], d2v = Uj - Ui[c];
-                acc[c] = (acc[c] + d4v * d4) - d2v * d2;
-            }
-        }
-    });
-    for (int c = 0; c < 5; ++c) L.diss[c * N + i] = acc[c];
-}
-
-// makeViscosityTerm pass 1 (gradients, then the node's stress and heat
-// flux as in k_visc_grad): the other node's (u, v, w, T)
-template <bool STAGE, bool AHEAD>
-__global__ void __launch_bounds__(kTile, 3) k_visc_grad_tiled(Params P, LevelView L) {
-    extern __shared__ double sm[];
-    const int N = L.N;
-    const double *f[4] = {L.prim, L.prim + N, L.prim + 2 * (size_t)N, L.prim + 3 * (size_t)N};
-    const int i = tile_begin<4, STAGE>(sm, L, f);
-    if (i < 0) return;
-    double g[12];
-    for (int c = 0; c < 12; ++c) g[c] = 0.0;
-    const double qi[4] = {L.prim[i], L.prim[N + i], L.prim[2 * N + i], L.prim[3 * N + i]};
-    row_walk<4, STAGE, true, AHEAD>(L, sm, f, i, [&](const Inc<4, STAGE, true> &t) {
-        const bool first = t.first();
-#pragma unroll
-        for (int a = 0; a < 3; ++a)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                double v = (first ? qi[c] + t.v[c] : t.v[c] + qi[c]) * t.w[a];
-                g[a * 4 + c] = g[a * 4 + c] + (first ? v : -v);
-            }
-    });
-    for (int k = L.binc_ptr[i]; k < L.binc_ptr[i + 1]; ++k) {
-        double v[12];
-        visc_grad_bterms(L, k, v);
-        for (int c = 0; c < 12; ++c) g[c] = g[c] + v[c];
-    }
-    visc_grad_finish(P, L, i, g);
-}
-
-// makeViscosityTerm pass 2 (as k_visc_flux): the other node's stress, heat
-// flux and velocity
-template <bool STAGE, bool AHEAD>
-__global__ void __launch_bounds__(kTile, AHEAD ? 2 : 3) k_visc_flux_tiled(Params P, LevelView L) {
-    extern __shared__ double sm[];
-    const int N = L.N;
-    const double *f[12] = {L.tau, L.tau + N, L.tau + 2 * (size_t)N, L.tau + 3 * (size_t)N, L.tau + 4 * (size_t)N,
-                           L.tau + 5 * (size_t)N, L.tau + 6 * (size_t)N, L.tau + 7 * (size_t)N,
-                           L.tau + 8 * (size_t)N, L.prim, L.prim + N, L.prim + 2 * (size_t)N};
-    const int i = tile_begin<12, STAGE>(sm, L, f);
-    if (i < 0) return;
-    double ti[9], ui[3];
-    for (int c = 0; c < 9; ++c) ti[c] = L.tau[c * N + i];
-    ui[0] = L.prim[i]; ui[1] = L.prim[N + i]; ui[2] = L.prim[2 * N + i];
-    double acc[4] = {0, 0, 0, 0};
-    row_walk<12, STAGE, true, AHEAD>(L, sm, f, i, [&](const Inc<12, STAGE, true> &t) {
-        const bool first = t.first();
-        const double *tj = t.v, *uj = t.v + 9;
-        double fl[4];
-        visc_edge_flux(first ? ti : tj, first ? tj : ti, first ? ui : uj, first ? uj : ui, t.w[0], t.w[1], t.w[2],
-                       fl);
-        for (int c = 0; c < 4; ++c) acc[c] = acc[c] + (first ? fl[c] : -fl[c]);
-    });
-    visc_flux_boundary(L, i, acc);
-    for (int c = 0; c < 4; ++c) L.diss[(1 + c) * N + i] = L.diss[(1 + c) * N + i] - acc[c];
-}
-
-#define FLITE_TILED_INST(STAGE, AHEAD)                                                     \
-    template __global__ void k_timestep_tiled<0, STAGE, AHEAD>(Params, LevelView);         \
-    template __global__ void k_timestep_tiled<2, STAGE, AHEAD>(Params, LevelView);         \
-    template __global__ void k_timestep_tiled<3, STAGE, AHEAD>(Params, LevelView);         \
-    template __global__ void k_jst_lap_tiled<STAGE, AHEAD>(Params, LevelView);            \
-    template __global__ void k_jst_flux_tiled<STAGE, AHEAD>(Params, LevelView);           \
-    template __global__ void k_visc_grad_tiled<STAGE, AHEAD>(Params, LevelView);          \
-    template __global__ void k_visc_flux_tiled<STAGE, AHEAD>(Params, LevelView);
-FLITE_TILED_INST(true, true)
-FLITE_TILED_INST(true, false)
-FLITE_TILED_INST(false, true)
-FLITE_TILED_INST(false, false)
-#undef FLITE_TILED_INST
-
-template __global__ void k_node_update_tiled<true, true>(Params, LevelView, int, int);
-template __global__ void k_node_update_tiled<true, false>(Params, LevelView, int, int);
-template __global__ void k_node_update_tiled<false, true>(Params, LevelView, int, int);
-template __global__ void k_node_update_tiled<false, false>(Params, LevelView, int, int);
 template __global__ void k_node_update<GATHER_BUFFER, 1, false>(Params, LevelView, int, int);
 template __global__ void k_node_update<GATHER_BUFFER, 1, true>(CaseTab<Params>, CaseTab<LevelView>, int, int);
 template __global__ void k_node_update<GATHER_BUFFER, 4, false>(Params, LevelView, int, int);
@@ -2300,8 +1967,6 @@ template __global__ void k_node_update<GATHER_DELTA, 16, false>(Params, LevelVie
 template __global__ void k_node_update<GATHER_DELTA, 16, true>(CaseTab<Params>, CaseTab<LevelView>, int, int);
 template __global__ void k_node_update<GATHER_DELTA, 32, false>(Params, LevelView, int, int);
 template __global__ void k_node_update<GATHER_DELTA, 32, true>(CaseTab<Params>, CaseTab<LevelView>, int, int);
-template __global__ void k_node_update<GATHER_CENTRAL2, 1, false>(Params, LevelView, int, int);
-template __global__ void k_node_update<GATHER_CENTRAL2, 1, true>(CaseTab<Params>, CaseTab<LevelView>, int, int);
 template __global__ void k_timestep<1, false>(Params, LevelView);
 template __global__ void k_timestep<1, true>(CaseTab<Params>, CaseTab<LevelView>);
 template __global__ void k_timestep<4, false>(Params, LevelView);

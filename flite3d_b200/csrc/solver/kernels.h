@@ -50,12 +50,17 @@ __global__ void k_bnd_flux(CaseArg<B, Params> P, CaseArg<B, LevelView> L);
 // GATHER_LEAN: GATHER_CENTRAL for runs without engine conditions and
 // without explicit time stepping, whose node tail leaves those branches out
 // (they cost the thread-per-node form its last free registers)
-enum { GATHER_BUFFER = 0, GATHER_CENTRAL = 1, GATHER_ANCHOR = 2, GATHER_DELTA = 3, GATHER_CENTRAL2 = 4, GATHER_LEAN = 5 };
+enum { GATHER_BUFFER = 0, GATHER_CENTRAL = 1, GATHER_ANCHOR = 2, GATHER_DELTA = 3, GATHER_LEAN = 5 };
+// the gathers that copy ahead with a thread per node run blocks of at most
+// 128 threads
+constexpr bool central_ahead(int prec) { return prec == GATHER_CENTRAL || prec == GATHER_ANCHOR || prec == GATHER_LEAN; }
+constexpr int node_threads(int prec, int u) { return u == 1 && central_ahead(prec) ? 128 : 256; }
 template <int PREC, int U, bool B = false>
 __global__ void k_node_update(CaseArg<B, Params> P, CaseArg<B, LevelView> L, int mode, int stage);
 // gathers: U lanes per node (1 = a thread per node); by default the widest
 // group with at most this many threads on the level (flite_ctx::lanes_of)
 constexpr size_t kLaneThreads = 98304;
+constexpr int kSharedWalkNodes = 220000;
 constexpr int kMaxLevels = 16;
 template <bool B = false>
 __global__ void k_delta_state(CaseArg<B, LevelView> L);
@@ -64,6 +69,7 @@ __global__ void k_sa_grad(Params P, LevelView L);
 __global__ void k_sa_diff(Params P, LevelView L);
 __global__ void k_sa_conv(Params P, LevelView L, int td);
 __global__ void k_sa_stage(Params P, LevelView L, int mode, int stage, int turb);
+__global__ void k_make_rows(LevelView L, int nrows, int2 *rows);
 __global__ void k_make_inc32(const int2 *inc, const EdgeW *ew, int n, IncRec32 *o);
 __global__ void k_copy(const double *a, double *b, size_t n);
 template <bool B = false>
@@ -99,18 +105,6 @@ __global__ void k_resid_partial(LevelView L, double *part, int nblk);
 __global__ void k_resid_final(const double *part, int nblk, double *out);
 __global__ void k_forces(Params P, LevelView L, const int *wall, int nwall, double alphaR, double betaR,
                          double ground, double d0, double d1, double d2, double *part);
-template <bool STAGE, bool AHEAD>
-__global__ void k_node_update_tiled(Params P, LevelView L, int mode, int stage);
-template <int K, bool STAGE, bool AHEAD>
-__global__ void k_timestep_tiled(Params P, LevelView L);
-template <bool STAGE, bool AHEAD>
-__global__ void k_jst_lap_tiled(Params P, LevelView L);
-template <bool STAGE, bool AHEAD>
-__global__ void k_jst_flux_tiled(Params P, LevelView L);
-template <bool STAGE, bool AHEAD>
-__global__ void k_visc_grad_tiled(Params P, LevelView L);
-template <bool STAGE, bool AHEAD>
-__global__ void k_visc_flux_tiled(Params P, LevelView L);
 // dst[c*N + i] = src[c*N + map[i]] for c < ncomp (node arrays between the
 // caller's numbering and the device's)
 __global__ void k_permute_nodes(double *dst, const double *src, const int *map, int N, int ncomp);

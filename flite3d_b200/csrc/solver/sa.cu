@@ -47,8 +47,7 @@ __global__ void k_sa_timestep(Params P, LevelView L) {
     const double ro = 1. / L.u[i];
     const double m1 = L.u[N + i], m2 = L.u[2 * N + i], m3 = L.u[3 * N + i];
     double acc = 0.0, h = 0.0;
-    for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) {
-        const int2 t = L.inc[k];
+    FLITE_FOR_INC(L, i, t) {
         const int e = t.x >= 0 ? t.x : ~t.x, j = t.y;
         const double wx = L.wx[e], wy = L.wy[e], wz = L.wz[e];
         const double al = (wx * wx + wy * wy) + wz * wz;
@@ -96,8 +95,7 @@ __global__ void k_sa_grad(Params P, LevelView L) {
     const double* __restrict__ nt = L.u + 5 * (size_t)N;
     const double ti = nt[i];
     double g0 = 0.0, g1 = 0.0, g2 = 0.0;
-    for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) {
-        const int2 t = L.inc[k];
+    FLITE_FOR_INC(L, i, t) {
         const int e = t.x >= 0 ? t.x : ~t.x;
         const double tj = nt[t.y];
         const double s = t.x >= 0 ? ti + tj : tj + ti;  // (nu1 + nu2) in the edge's order
@@ -141,8 +139,7 @@ __global__ void k_sa_diff(Params P, LevelView L) {
         return visc(n) * ((wx * L.sag[n] + wy * L.sag[N + n]) + wz * L.sag[2 * N + n]);
     };
     double acc = 0.0;
-    for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) {
-        const int2 t = L.inc[k];
+    FLITE_FOR_INC(L, i, t) {
         const int e = t.x >= 0 ? t.x : ~t.x;
         const int n1 = t.x >= 0 ? i : t.y, n2 = t.x >= 0 ? t.y : i;
         const double wx = L.wx[e], wy = L.wy[e], wz = L.wz[e];
@@ -174,8 +171,7 @@ __global__ void k_sa_conv(Params P, LevelView L, int td) {
     prim(i, qi);
     // an unsteady stage's time difference comes first (def_par:1073)
     double acc = td ? time_difference(P, L, i, 5) : 0.0;
-    for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) {
-        const int2 t = L.inc[k];
+    FLITE_FOR_INC(L, i, t) {
         const int e = t.x >= 0 ? t.x : ~t.x;
         double qj[4];
         prim(t.y, qj);

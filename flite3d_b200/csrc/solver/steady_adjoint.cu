@@ -127,8 +127,7 @@ __global__ void k_adj_sensor_parts(LevelView L, const double *p, double *nh6, do
     if (i >= L.N) return;
     double s6 = 0.0, s7 = 0.0;
     const double pi = p[i];
-    for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) {
-        const int2 t = L.inc[k];
+    FLITE_FOR_INC(L, i, t) {
         const double pj = p[t.y];
         if (t.x >= 0) s6 -= pi - pj;
         else s6 += pj - pi;
@@ -288,8 +287,7 @@ __global__ void k_adj_jst_edges(Params P, LevelView L, const double *u0, const d
         li[c] = lap[(size_t)c * N + i];
         Dbi[c] = Dbar[(size_t)c * N + i];
     }
-    for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) {
-        const int2 t = L.inc[k];
+    FLITE_FOR_INC(L, i, t) {
         const int j = t.y;
         const bool first = t.x >= 0;  // this node is the edge's i1
         const double rj = L.V[j] / dt[j], cj = L.conn[j], sj = sens[j];
@@ -356,8 +354,8 @@ __global__ void k_adj_jst_lap(LevelView L, const double *nhbar, const double *nh
     for (int c = 0; c < 5; ++c) nbi[c] = nhbar[(size_t)c * N + i];
     const double b6i = nh6bar[i], b7i = nh7bar[i];
     double ub[5] = {0, 0, 0, 0, 0}, pb = 0.0;
-    for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) {
-        const int j = L.inc[k].y;
+    FLITE_FOR_INC(L, i, t) {
+        const int j = t.y;
         for (int c = 0; c < 5; ++c) ub[c] += nhbar[(size_t)c * N + j] - nbi[c];
         pb += nhbar[(size_t)4 * N + j] - nbi[4];
         pb += nh6bar[j] - b6i;
@@ -440,14 +438,14 @@ __global__ void k_adj_timestep(Params P, LevelView L, const double *u0, const do
     const double pi = p0[i];
     double ub[5] = {0, 0, 0, 0, 0}, pb = 0.0;
     double fu[5], fp;
-    for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) {
-        const int e = L.inc[k].x >= 0 ? L.inc[k].x : ~L.inc[k].x;
+    FLITE_FOR_INC(L, i, t) {
+        const int e = t.x >= 0 ? t.x : ~t.x;
         const double w[3] = {L.wx[e], L.wy[e], L.wz[e]};
         ts_term_grad(P, ui, pi, w, fu, &fp, nullptr);
         for (int c = 0; c < 5; ++c) ub[c] += sbi * fu[c];
         pb += sbi * fp;
         if (visc) {
-            const int j = L.inc[k].y;
+            const int j = t.y;
             const double al = (w[0] * w[0] + w[1] * w[1]) + w[2] * w[2];
             double dr, dm, da;
             h += visc_ts_term(P, mu[j], u0[j], al, &dr, &dm, &da);  // the other end's term
@@ -633,8 +631,7 @@ __global__ void k_adj_visc_sums(LevelView L, const double *prim, double *G) {
     for (int c = 0; c < 12; ++c) g[c] = 0.0;
     double qi[4];
     for (int c = 0; c < 4; ++c) qi[c] = prim[(size_t)c * N + i];
-    for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) {
-        const int2 t = L.inc[k];
+    FLITE_FOR_INC(L, i, t) {
         const int e = t.x >= 0 ? t.x : ~t.x;
         const double w[3] = {L.wx[e], L.wy[e], L.wz[e]};
         for (int c = 0; c < 4; ++c) {
@@ -705,8 +702,7 @@ __global__ void k_adj_visc_flux(LevelView L, const double *Dbar, const double *t
     for (int c = 0; c < 9; ++c) ti[c] = tau[(size_t)c * N + i];
     for (int c = 0; c < 3; ++c) vi[c] = prim[(size_t)c * N + i];
     for (int c = 0; c < 4; ++c) Wi[c] = -Dbar[(size_t)(1 + c) * N + i];
-    for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) {
-        const int2 t = L.inc[k];
+    FLITE_FOR_INC(L, i, t) {
         const int e = t.x >= 0 ? t.x : ~t.x;
         const double w[3] = {L.wx[e], L.wy[e], L.wz[e]};
         double W[4];
@@ -814,8 +810,7 @@ __global__ void k_adj_visc_prim(Params P, LevelView L, const double *u0, const d
     const int N = L.N;
     double gi[12], qb[4] = {0, 0, 0, 0};
     for (int c = 0; c < 12; ++c) gi[c] = Gbar[(size_t)c * N + i];
-    for (int k = L.inc_ptr[i]; k < L.inc_ptr[i + 1]; ++k) {
-        const int2 t = L.inc[k];
+    FLITE_FOR_INC(L, i, t) {
         const int e = t.x >= 0 ? t.x : ~t.x;
         const double w[3] = {L.wx[e], L.wy[e], L.wz[e]};
         for (int c = 0; c < 4; ++c)
@@ -1457,7 +1452,17 @@ static void geometry_sweep(flite_ctx &X, SteadyAdjoint &A, const double *lam, co
 
 static void download_geometry(flite_ctx &X, SteadyAdjoint &A, double *swb, double *bwb, double *vb) {
     LevelView &L = X.V(0);
-    if (swb) CK(cudaMemcpyAsync(swb, A.swbar, 3 * (size_t)L.E * sizeof(double), cudaMemcpyDeviceToHost, X.s));
+    if (swb) {
+        const size_t n = 3 * (size_t)L.E;
+        const double *src = A.swbar;
+        if (L.eslot && n) {  // in the caller's edge order
+            double *t = X.io_buffer(n);
+            k_permute_nodes<<<X.blocks(n), kBlock, 0, X.s>>>(t, A.swbar, L.eslot, L.E, 3);
+            CK(cudaGetLastError());
+            src = t;
+        }
+        CK(cudaMemcpyAsync(swb, src, n * sizeof(double), cudaMemcpyDeviceToHost, X.s));
+    }
     if (bwb && L.B > 0)
         CK(cudaMemcpyAsync(bwb, A.bwbar, 3 * (size_t)L.B * sizeof(double), cudaMemcpyDeviceToHost, X.s));
     if (vb) X.get_nodes(0, vb, A.Vbar, 1);

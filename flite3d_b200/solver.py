@@ -317,17 +317,15 @@ class Solver:
         self._ck(self.be.set_kernel_options(self._h, edge_block, node_block, gather_unroll), "set_kernel_options")
 
     def set_tiled_gather(self, level, mode=1):
-        """How the fused central gather of a level reads its incidences: 0
-        through the node's incidence list; 1..4 through the incidence rows of
-        256-node blocks, with the block and its halo staged in shared memory
-        (1, 2) or not (3, 4).  No effect on any result."""
+        """Earlier forms of the thread-per-node gathers (0..4): checked, and
+        without effect (every such gather reads the incidence rows)."""
         self._ck(self.be.set_tiled_gather(self._h, level, mode), "set_tiled_gather")
 
     def set_gather_fusion(self, level, on=1):
         """Whether a level's gathers that walk the same incidence list share
         one walk (time step with Laplacian, JST flux with viscous gradients)
-        where a thread serves a node: 1 (default) or 0.  No effect on any
-        result."""
+        where a thread serves a node: 1 or 0; without this call levels of at
+        most 220,000 nodes do.  No effect on any result."""
         self._ck(self.be.set_gather_fusion(self._h, level, on), "set_gather_fusion")
 
     def set_gather_lanes(self, level, lanes):

@@ -401,9 +401,9 @@ int flite_cycle_launches(flite_ctx *ctx, int64_t *n);
 int flite_profile_level(flite_ctx *ctx, int level, int reps, double *edge_ms,
                         double *node_ms);
 /* Launch options of a context (no effect on any result): threads per block
- * of the edge kernels and of the node kernels (32..256, multiples of 32) and
- * the incidences whose loads the fused central gather issues together (1 or
- * 2).  Drops the captured cycle graph.                                     */
+ * of the edge kernels and of the node kernels (32..256, multiples of 32; the
+ * central gather with a thread per node takes at most 128).  gather_unroll is
+ * 1 or 2 and changes nothing.  Drops the captured cycle graph.              */
 int flite_set_kernel_options(flite_ctx *ctx, int32_t edge_block, int32_t node_block, int32_t gather_unroll);
 /* Node numbering of the contexts created after this call (no effect on any
  * result; no reference counterpart): 1 renumbers the nodes of every level
@@ -417,20 +417,14 @@ int flite_set_node_order(int32_t order);
  * 1 (a thread per node), 4, 8, 16 or 32, or 0 for the default (the widest group
  * that keeps the level within 98,304 threads).  Drops the captured cycle graph. */
 int flite_set_gather_lanes(flite_ctx *ctx, int32_t level, int32_t lanes);
-/* How a level's fused central gather with a thread per node (fluxType 1,
- * FP64) reads its incidences: 0 (the default) through the node's incidence
- * list; 1..4 through incidence rows of blocks of 256 nodes (row k holds
- * incidence k of every node of the block with its edge coefficients, read
- * with coalesced loads a step ahead), with the block's nodes and the other
- * nodes its edges reach staged in shared memory (1: compiled for two blocks
- * per SM, 2: three) or read from global memory (3: two, 4: three).  No
- * effect on any result.  Drops the captured cycle graph.                   */
+/* Earlier forms of the gathers with a thread per node (0..4); they all read
+ * the incidence rows now, and the modes are checked and change nothing.     */
 int flite_set_tiled_gather(flite_ctx *ctx, int32_t level, int32_t on);
 /* Whether a level's node gathers that walk the same incidence list share one
- * walk where a thread serves a node and the list form is used: the time step
- * with the JST Laplacian, and the JST flux with the viscous gradients.  1 (the
- * default) shares, 0 runs them as separate kernels.  No effect on any result.
- * Drops the captured cycle graph.                                           */
+ * walk where a thread serves a node: the time step with the JST Laplacian,
+ * and the JST flux with the viscous gradients.  1 shares, 0 runs them as
+ * separate kernels; without this call levels of at most 220,000 nodes share.
+ * No effect on any result.  Drops the captured cycle graph.                 */
 int flite_set_gather_fusion(flite_ctx *ctx, int32_t level, int32_t on);
 /* Average device ms of the kernel groups of one relaxation step of a level,
  * in order: pressure, time steps, dissipation, viscous primitives, viscous
