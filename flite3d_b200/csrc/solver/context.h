@@ -43,7 +43,7 @@ constexpr int kResidBlocks = 296;  // 2 x 148 SMs
 struct DevLevel {
     int N = 0, E = 0, B = 0, Nb = 0;
     int nrows = 0;           // incidence rows
-    std::vector<int> eslot;  // the device's number of each of the caller's edges; empty: the same
+    bool orphans = false;    // coarse level: some finer node has no parent here
     LevelView v{};
     std::vector<int> wall;  // level-1 wall nodes in register order (forces)
     int *d_wall = nullptr;
@@ -82,6 +82,10 @@ struct flite_ctx {
     std::vector<DevLevel> lv;
     std::vector<void *> allocs;
     cudaStream_t s = nullptr;
+    // a second stream for the part of restrictGrid that does not depend on the
+    // other (in a captured cycle: a branch of the graph)
+    cudaStream_t side = nullptr;
+    cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
     int *d_cycle = nullptr;
     int *d_cyc = nullptr;  // per-level cycle numbers
     double *d_part = nullptr, *d_out = nullptr;
@@ -196,6 +200,10 @@ struct flite_ctx {
         allocs.push_back(p);
         return (T *)p;
     }
+    void release(void *p) {
+        allocs.erase(std::find(allocs.begin(), allocs.end(), p));
+        CK(cudaFree(p));
+    }
     template <class T>
     T *upload(const std::vector<T> &h) {
         T *d = alloc<T>(h.size());
@@ -209,6 +217,9 @@ struct flite_ctx {
         if (d_io) cudaFree(d_io);
         for (void *p : allocs) cudaFree(p);
         if (h_cycle) cudaFreeHost(h_cycle);
+        for (cudaEvent_t e : ev)
+            if (e) cudaEventDestroy(e);
+        if (side) cudaStreamDestroy(side);
         if (s) cudaStreamDestroy(s);
     }
 
@@ -252,10 +263,30 @@ struct flite_ctx {
         return lv[l].v.N <= kSharedWalkNodes;
     }
 
-    void pressure(int l) {
+    // pass over the state of level l (STATE_*), with the boundary edges' fluxes
+    // where `bnd`
+    void state_pass(int l, int what, bool bnd = false) {
+        const LevelView &L = V(l);
+        if (fused()) what |= STATE_REC;  // only the central gathers read the records
         counted();
-        FLITE_LAUNCH(k_pressure, (), nblk(V(l).N), nb, 0, P, V(l));
+        if (bnd)
+            FLITE_LAUNCH(k_state_pass, (true,), nblk((size_t)L.N + L.B), nb, 0, P, L, what, (const int *)d_cycle);
+        else
+            FLITE_LAUNCH(k_state_pass, (false,), nblk(L.N), nb, 0, P, L, what, (const int *)d_cycle);
     }
+    void pressure(int l) { state_pass(l, 0); }
+    bool visc() const { return c.ReynoldsNumber > 0.0; }
+    // passes of a level with lanes per node take their boundary fluxes from
+    // the state pass or evaluate them in the node pass: the launch of the
+    // boundary kernel costs these levels more than its work
+    bool group_level(int l) const { return lanes_of(l) > 1; }
+    // the node pass leaves the pressure (and records) of the next stage; with
+    // engines the pass of the inlet nodes ends later (k_engine_finish)
+    bool emits() const { return !P.engines; }
+    // the node pass evaluates the boundary edges: lanes per node, the FP64
+    // central flux of a static mesh without engines; the Spalart-Allmaras
+    // kernels between the stages read the state in u
+    bool inline_bnd(int l) const { return group_level(l) && fused() && !mixed() && !sa() && emits(); }
     // makeTimeSteps's ivd%physicalTimeStep under explicit time stepping
     // (unsteady runs read it; steady ones never do)
     void explicit_step(int l) {
@@ -318,39 +349,43 @@ struct flite_ctx {
         if (!fuse_walks(l) || !jst_gathers(l)) return 0;
         return (c.ReynoldsNumber > 0.0 && !P.matrixDiss && c.viscosityScheme == 1) ? 2 : 1;
     }
-    void ts_jst_viscous(int l, bool ts) {
-        const bool visc = c.ReynoldsNumber > 0.0;
-        if (!fuse_walks(l) || !jst_gathers(l)) {
+    // `prim`: the viscous primitives are there already.  With lanes per node
+    // the shared walks are always taken, and with `fold` the last part may be
+    // left to the node pass that follows (the PRE_* returned).
+    int ts_jst_viscous(int l, bool ts, bool prim, bool fold) {
+        const bool grp = group_level(l);
+        if ((!grp && !fuse_walks(l)) || !jst_gathers(l)) {
             if (ts) timesteps(l);
             jst(l);
-            viscous(l);
-            return;
+            viscous(l, prim);
+            return PRE_NONE;
         }
         if (ts) {
             counted();
-            FLITE_LAUNCH(k_ts_lap, (), nblk(V(l).N), nb, 0, P, V(l));
+            FLITE_GATHER(k_ts_lap, l, P, V(l));
             explicit_step(l);
         } else {
             jst_lap(l);
         }
-        if (visc) {
+        if (visc() && !prim) viscous_prim(l);
+        fold = fold && inline_bnd(l);  // (the pass must not write the state it reads)
+        if (visc() && !P.matrixDiss && c.viscosityScheme == 1) {
             counted();
-            FLITE_LAUNCH(k_visc_prim, (), nblk(V(l).N), nb, 0, P, V(l));
-        }
-        if (visc && !P.matrixDiss && c.viscosityScheme == 1) {
-            counted();
-            FLITE_LAUNCH(k_jflux_vgrad, (), nblk(V(l).N), nb, 0, P, V(l));
+            FLITE_GATHER(k_jflux_vgrad, l, P, V(l));
+            if (fold) return PRE_VISC;
         } else {
+            if (fold && !visc() && !P.matrixDiss) return PRE_JST;
             jst_flux(l);
-            if (visc) {
+            if (visc()) {
                 counted();
                 visc_grad(l);
             }
         }
-        if (visc) {
+        if (visc()) {
             counted();
             visc_flux(l);
         }
+        return PRE_NONE;
     }
     void first_order_diss(int l) {
         no_group("dissipation scheme 3");
@@ -371,11 +406,11 @@ struct flite_ctx {
         counted();
         k_lp_flux<<<nblk(V(l).N), nb, 0, s>>>(P, V(l));
     }
+    void viscous_prim(int l) { state_pass(l, STATE_PRIM); }
     // makeViscosityTerm (def_par:5198-5893), subtracted from the dissipation
-    void viscous(int l) {
-        if (!(c.ReynoldsNumber > 0.0)) return;
-        counted();
-        FLITE_LAUNCH(k_visc_prim, (), nblk(V(l).N), nb, 0, P, V(l));
+    void viscous(int l, bool prim = false) {
+        if (!visc()) return;
+        if (!prim) viscous_prim(l);
         counted();
         visc_grad(l);
         counted();
@@ -423,7 +458,9 @@ struct flite_ctx {
     // makeRHS up to the node gather (def_par:1587-1607 and the edge loops);
     // with FLITE_MIXED, `anchor` selects the FP64 evaluation that refreshes
     // the anchor state, otherwise the FP32 increments over it
-    void rhs_terms(int l, bool anchor = true) {
+    // `delta`: the increments' records are there already, `bnd`: so are the
+    // boundary fluxes, or the node pass evaluates them
+    void rhs_terms(int l, bool anchor = true, bool delta = false, bool bnd = false) {
         const LevelView &L = V(l);
         if (c.reconstruction == FLITE_RECON_VAN_ALBADA && L.grid == 1) {
             // the extension reconstructs from the Galerkin gradients, through
@@ -444,7 +481,8 @@ struct flite_ctx {
             }
         }
         if (L.E > 0) {
-            if (mixed() && !anchor) {
+            if (mixed() && !anchor && delta) {
+            } else if (mixed() && !anchor) {
                 // FP32 records of the increments over the anchor
                 counted();
                 FLITE_LAUNCH(k_delta_state, (), nblk(L.N), nb, 0, L);
@@ -454,7 +492,7 @@ struct flite_ctx {
                 edge_flux_launch(L);
             }
         }
-        if (L.B > 0) {
+        if (L.B > 0 && !bnd) {
             counted();
             FLITE_LAUNCH(k_bnd_flux, (), eblk(L.B), eb, 0, P, L);
         }
@@ -484,9 +522,9 @@ struct flite_ctx {
             default: k_edge_flux<1, false><<<ng, eb, 0, s>>>(P, L);
         }
     }
-    void node_update(int l, int mode, int stage, bool anchor = true) {
+    void node_update(int l, int mode, int stage, bool anchor = true, int pre = PRE_NONE, int io = 0) {
         counted();
-        launch_node_update(l, mode, stage, anchor);
+        launch_node_update(l, mode, stage, anchor, pre, io);
     }
     // the level-1 engine inlet terms after a node pass of `mode` (engine.cu)
     void engine_pass(int l, int mode) {
@@ -502,123 +540,190 @@ struct flite_ctx {
             k_engine_finish<<<nblk(n), nb, 0, s>>>(P, L, mode, all ? 1 : 0);
         }
     }
-    void launch_node_update(int l, int mode, int stage, bool anchor) {
+    void launch_node_update(int l, int mode, int stage, bool anchor, int pre = PRE_NONE, int io = 0) {
         switch (lanes_of(l)) {
-            case 4: launch_node_update_u<4>(l, mode, stage, anchor); break;
-            case 8: launch_node_update_u<8>(l, mode, stage, anchor); break;
-            case 16: launch_node_update_u<16>(l, mode, stage, anchor); break;
-            case 32: launch_node_update_u<32>(l, mode, stage, anchor); break;
-            default: launch_node_update_u<1>(l, mode, stage, anchor);
+            case 4: launch_node_update_u<4>(l, mode, stage, anchor, pre, io); break;
+            case 8: launch_node_update_u<8>(l, mode, stage, anchor, pre, io); break;
+            case 16: launch_node_update_u<16>(l, mode, stage, anchor, pre, io); break;
+            case 32: launch_node_update_u<32>(l, mode, stage, anchor, pre, io); break;
+            default: launch_node_update_u<1>(l, mode, stage, anchor, pre, io);
         }
     }
     template <int U>
-    void launch_node_update_u(int l, int mode, int stage, bool anchor) {
+    void launch_node_update_u(int l, int mode, int stage, bool anchor, int pre, int io) {
         // blocks of nt threads (nb, or less where the kernel's own bound is)
         const auto blk = [&](int prec) { return (unsigned)std::min(nb, node_threads(prec, U)); };
         const auto grid = [&](unsigned nt) { return (unsigned)((U * (size_t)V(l).N + nt - 1) / nt); };
-#define FLITE_NODE(PREC)                                                                             \
+#define FLITE_NODE(PREC, PRE)                                                                        \
     do {                                                                                              \
         const unsigned nt = blk(PREC);                                                                \
-        FLITE_LAUNCH(k_node_update, (PREC, U,), grid(nt), nt, 0, P, V(l), mode, stage);               \
+        FLITE_LAUNCH(k_node_update, (PREC, U, PRE,), grid(nt), nt, 0, P, V(l), mode, stage, io);      \
     } while (0)
         if (mixed()) {
-            if (anchor) FLITE_NODE(GATHER_ANCHOR);
-            else FLITE_NODE(GATHER_DELTA);
+            if (anchor) FLITE_NODE(GATHER_ANCHOR, PRE_NONE);
+            else FLITE_NODE(GATHER_DELTA, PRE_NONE);
         } else if (fused()) {
             if constexpr (U == 1) {
                 if (!P.engines && !(P.unsteady && P.explicit_)) {
-                    FLITE_NODE(GATHER_LEAN);
+                    FLITE_NODE(GATHER_LEAN, PRE_NONE);
                     return;
                 }
             }
-            FLITE_NODE(GATHER_CENTRAL);
+            if constexpr (U > 1) {
+                if (pre == PRE_JST) {
+                    FLITE_NODE(GATHER_CENTRAL, PRE_JST);
+                    return;
+                }
+                if (pre == PRE_VISC) {
+                    FLITE_NODE(GATHER_CENTRAL, PRE_VISC);
+                    return;
+                }
+            }
+            FLITE_NODE(GATHER_CENTRAL, PRE_NONE);
         } else {
-            FLITE_NODE(GATHER_BUFFER);
+            FLITE_NODE(GATHER_BUFFER, PRE_NONE);
         }
 #undef FLITE_NODE
     }
 
     // ---- singleIteration (def_par:1002-1181) -----------------------------
-    void singleIteration(int l, bool calcDiss) {
+    // after the step's state pass (pressure, records, primitives and, with
+    // `bnd`, boundary fluxes of stage 1)
+    void singleIteration(int l, bool calcDiss, bool bnd) {
+        int pre = PRE_NONE;
         if (calcDiss) {
-            pressure(l);  // p = |p| is the identity after the 0.1 floor
             if ((c.dissipationScheme == 1 && V(l).grid == 1) || c.dissipationScheme == 3) {
                 timesteps(l);
                 dissipation(l);
-                viscous(l);
+                viscous(l, true);
             } else {
-                ts_jst_viscous(l, true);
+                pre = ts_jst_viscous(l, true, true, true);
             }
             if (turb()) {
                 sa_timesteps(l);
                 sa_diffusion(l);
             }
         }
+        const bool own = inline_bnd(l), emit = emits();
         for (int st = 1; st <= P.nstage; ++st) {
             // u == uprev at stage 1: the FP64 evaluation there is the anchor
-            // of the mixed-precision increments of the later stages.  The
-            // pressure and flux records of stage 1 are those of the step's
-            // own pressure pass when it ran (nothing has changed u since)
-            if (st > 1 || !calcDiss) pressure(l);
-            rhs_terms(l, st == 1);
+            // of the mixed-precision increments of the later stages
+            if (st > 1 && !emit) pressure(l);
+            rhs_terms(l, st == 1, st > 1 && emit, own || (st == 1 && bnd));
             sa_stage(l, MODE_STAGE, st);
-            node_update(l, MODE_STAGE, st, st == 1);
+            node_update(l, MODE_STAGE, st, st == 1, st == 1 ? pre : PRE_NONE, stage_io(st, P.nstage, own, emit));
             engine_pass(l, MODE_STAGE);
         }
     }
     // ---- doTimeIterations (def_par:966-1000) -----------------------------
     void doTimeIterations(int l, int nsteps, bool calcDiss) {
-        counted();
-        FLITE_LAUNCH(k_case_cycle, (), 1, 1, 0, V(l), d_cycle);
-        for (int i = 0; i < nsteps; ++i) {
+        if (nsteps <= 0) {
             counted();
-            FLITE_LAUNCH(k_case_save_u, (), nblk(nvar() * (size_t)V(l).N), nb, 0, V(l), nvar() * (size_t)V(l).N);
-            singleIteration(l, calcDiss);
+            FLITE_LAUNCH(k_case_cycle, (), 1, 1, 0, V(l), d_cycle);
+        }
+        for (int i = 0; i < nsteps; ++i) {
+            const bool bnd = group_level(l) && !inline_bnd(l) && c.flowType != 2;
+            state_pass(l, STATE_STEP | (calcDiss && visc() ? STATE_PRIM : 0), bnd);
+            singleIteration(l, calcDiss, bnd);
         }
     }
     // ---- restrictGrid (def_par:12141-12430) ------------------------------
+    // the coarse level's one-step update and the fine level's increment do not
+    // depend on each other: the coarse part runs on the side stream (a branch
+    // of the captured graph), where the small level's chain of launches hides
+    // behind the fine level's.  The fine part waits for the coarse state
+    // before it writes what that was restricted from.  Under explicit time
+    // stepping the fine part reads the coarse level's step: no branch.
     void restrictGrid(int fl) {
         const int cl = fl + 1;
-        counted();
-        FLITE_LAUNCH(k_restrict_state, (), nblk(V(cl).N), nb, 0, P, V(cl), V(fl));
-        if (c.coarseGridDissipationScheme == 2) {
-            ts_jst_viscous(cl, true);
+        const bool branch = !(P.explicit_ && P.unsteady);
+        auto coarse_state = [&] {
+            counted();
+            FLITE_LAUNCH(k_restrict_state, (), nblk(kChildLanes * (size_t)V(cl).N), nb, 0, P, V(cl), V(fl));
+        };
+        auto coarse = [&] {
+            int pre = PRE_NONE;
+            if (c.coarseGridDissipationScheme == 2) {
+                pre = ts_jst_viscous(cl, true, true, true);
+            } else {
+                timesteps(cl);
+                if (c.coarseGridDissipationScheme == 3) first_order_diss(cl);
+                viscous(cl, true);
+            }
+            const bool own = inline_bnd(cl);
+            rhs_terms(cl, true, false, own);
+            if (turb()) {
+                sa_timesteps(cl);
+                sa_diffusion(cl);
+            }
+            sa_stage(cl, MODE_RCOARSE, 0);
+            node_update(cl, MODE_RCOARSE, 0, true, pre, own ? IO_BND : 0);
+        };
+        // with lanes per node the fine pass reads its neighbours' state (the
+        // folded JST flux, the boundary edges), so the density floor it would
+        // write there waits for k_restrict_incr, which visits the nodes with a
+        // parent
+        const bool own = inline_bnd(fl) && !lv[cl].orphans;
+        const bool bnd = group_level(fl) && !own && c.flowType != 2;
+        auto fine_head = [&] {
+            state_pass(fl, visc() ? STATE_PRIM : 0, bnd);
+        };
+        auto fine = [&] {
+            int pre = PRE_NONE;
+            // the fine part uses scheme 1 on level 1 under dissipationScheme 1,
+            // scheme 2 otherwise (def_par:12269-12273)
+            if (c.dissipationScheme == 1 && V(fl).grid == 1) {
+                lp_diss(fl);
+                viscous(fl, true);
+            } else {
+                pre = ts_jst_viscous(fl, false, true, own);
+            }
+            rhs_terms(fl, false, false, bnd || own);
+            if (turb()) sa_diffusion(fl);  // the fine level keeps its turbulent time steps
+            sa_stage(fl, MODE_RFINE, 0);
+            node_update(fl, MODE_RFINE, 0, false, pre, own ? IO_BND | IO_LATER : 0);
+            engine_pass(fl, MODE_RFINE);
+        };
+        if (branch) {
+            struct Side {  // launches go to the side stream in its scope
+                flite_ctx &x;
+                explicit Side(flite_ctx &c) : x(c) { std::swap(x.s, x.side); }
+                ~Side() { std::swap(x.s, x.side); }
+            };
+            CK(cudaEventRecord(ev[0], s));
+            CK(cudaStreamWaitEvent(side, ev[0], 0));
+            {
+                Side on(*this);
+                coarse_state();
+                CK(cudaEventRecord(ev[1], s));
+                coarse();
+                CK(cudaEventRecord(ev[2], s));
+            }
+            fine_head();
+            CK(cudaStreamWaitEvent(s, ev[1], 0));
+            fine();
+            CK(cudaStreamWaitEvent(s, ev[2], 0));
         } else {
-            timesteps(cl);
-            if (c.coarseGridDissipationScheme == 3) first_order_diss(cl);
-            viscous(cl);
+            coarse_state();
+            coarse();
+            fine_head();
+            fine();
         }
-        rhs_terms(cl);
-        if (turb()) {
-            sa_timesteps(cl);
-            sa_diffusion(cl);
-        }
-        sa_stage(cl, MODE_RCOARSE, 0);
-        node_update(cl, MODE_RCOARSE, 0);
-        pressure(fl);
-        // the fine part uses scheme 1 on level 1 under dissipationScheme 1,
-        // scheme 2 otherwise (def_par:12269-12273)
-        if (c.dissipationScheme == 1 && V(fl).grid == 1) {
-            lp_diss(fl);
-            viscous(fl);
-        } else {
-            ts_jst_viscous(fl, false);
-        }
-        rhs_terms(fl, false);
-        if (turb()) sa_diffusion(fl);  // the fine level keeps its turbulent time steps
-        sa_stage(fl, MODE_RFINE, 0);
-        node_update(fl, MODE_RFINE, 0, false);
-        engine_pass(fl, MODE_RFINE);
         counted();
-        FLITE_LAUNCH(k_restrict_incr, (), nblk(V(cl).N), nb, 0, P, V(cl), V(fl));
+        FLITE_LAUNCH(k_restrict_incr, (), nblk(kChildLanes * (size_t)V(cl).N), nb, 0, P, V(cl), V(fl), own ? 1 : 0);
     }
     // ---- prolongateGrid (def_par:12432-12570) ----------------------------
     void prolongateGrid(int cl) {
         const int fl = cl - 1;
+        const unsigned g = nblk(kChildLanes * (size_t)V(cl).N);
         counted();
-        FLITE_LAUNCH(k_prolong_coarse, (), nblk(V(cl).N), nb, 0, P, V(cl), V(fl));
-        counted();
-        FLITE_LAUNCH(k_prolong_fine, (), nblk(V(fl).N), nb, 0, P, V(cl), V(fl));
+        if (!lv[cl].orphans) {
+            FLITE_LAUNCH(k_prolong, (), g, nb, 0, P, V(cl), V(fl));
+        } else {
+            FLITE_LAUNCH(k_prolong_coarse, (), g, nb, 0, P, V(cl), V(fl));
+            counted();
+            FLITE_LAUNCH(k_prolong_fine, (), nblk(V(fl).N), nb, 0, P, V(cl), V(fl));
+        }
         engine_pass(fl, MODE_PROLONG);
     }
     // the head of a physical time step (mg_par:586-602): laminar viscosity
@@ -637,7 +742,7 @@ struct flite_ctx {
     }
     void mapFineToCoarse(int fl) {
         counted();
-        FLITE_LAUNCH(k_restrict_u, (), nblk(V(fl + 1).N), nb, 0, V(fl + 1), V(fl));
+        FLITE_LAUNCH(k_restrict_u, (), nblk(kChildLanes * (size_t)V(fl + 1).N), nb, 0, V(fl + 1), V(fl));
     }
     // ---- oneCycle (mg_par:907-1196) --------------------------------------
     void oneCycle() {
@@ -748,6 +853,7 @@ struct flite_ctx {
             cudaStreamEndCapture(s, g);
             if (*g) cudaGraphDestroy(*g);
             *g = nullptr;
+            cudaGetLastError();  // an unfinished branch's
             throw;
         }
         counting = false;
@@ -770,6 +876,7 @@ struct flite_ctx {
             counting = false;
             cudaStreamEndCapture(s, &g);
             if (g) cudaGraphDestroy(g);
+            cudaGetLastError();  // an unfinished branch's
             throw;
         }
         counting = false;

@@ -150,6 +150,11 @@ struct LevelView {
     const int *child;                // [N_fine]
     // state
     double *u, *uprev, *rhs, *src, *diss;  // [5][N]
+    // the state and records between the stages of a step: a stage that reads
+    // its neighbours' values writes the other copy (StageIO, kernels.h)
+    double *ub;                            // [5][N] (levels with group gathers)
+    NodeRec *qb;                           // [N] (central flux)
+    DeltaRec *dqb;                         // [N] (FLITE_MIXED)
     double *p, *dt, *mu;                   // [N]
     double *hvis;                          // [N]  viscous time-step term
     double *lap;                           // [5][N] undivided Laplacian
@@ -311,14 +316,14 @@ __device__ __forceinline__ double pressure(const Params &P, double r, double m1,
 // second-order backward difference on level 1 with timeScheme 2 (with the
 // previous volumes of a moving mesh; a static mesh's are the volumes), first
 // order elsewhere
-__device__ __forceinline__ double time_difference(const Params &P, const LevelView &L, int i, int c) {
+__device__ __forceinline__ double time_difference(const Params &P, const LevelView &L, const double *u, int i, int c) {
     const size_t k = (size_t)c * L.N + i;
     const double Vi = L.V[i];
     if (L.grid == 1 && P.bdf2) {
         const double Vp = L.Vp ? L.Vp[i] : Vi, Vp2 = L.Vp2 ? L.Vp2[i] : Vi;
-        return (((1.5 * Vi) * L.u[k] - (2.0 * Vp) * L.uold[k]) + (0.5 * Vp2) * L.uold2[k]) / P.dtp;
+        return (((1.5 * Vi) * u[k] - (2.0 * Vp) * L.uold[k]) + (0.5 * Vp2) * L.uold2[k]) / P.dtp;
     }
-    return Vi * (L.u[k] - L.uold[k]) / P.dtp;
+    return Vi * (u[k] - L.uold[k]) / P.dtp;
 }
 
 // tangential projection used by every slip condition (def_par:4448-4451,

@@ -110,14 +110,28 @@ void flite::put_geometry(flite_ctx &X, int l, const flite_level_desc &d, bool cr
         else if (!h.empty())
             CK(cudaMemcpy(const_cast<T *>(field), h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice));
     };
-    std::vector<double> wx(E), wy(E), wz(E), slen(E, 0.0);
-    std::vector<EdgeW> ew(std::max(E, 1));
-    const std::vector<int> &slot = X.lv[l].eslot;
-    for (int e = 0; e < E; ++e) {
-        const int q = slot.empty() ? e : slot[e];
-        wx[q] = d.side_w[e]; wy[q] = d.side_w[(size_t)E + e]; wz[q] = d.side_w[2 * (size_t)E + e];
-        if (d.side_len) slen[q] = d.side_len[e];
-        ew[q] = EdgeW{wx[q], wy[q], wz[q], 0.0};
+    // edge arrays: from the caller's own memory, put into the device's edge
+    // order there
+    double *edges_in = nullptr;  // staging: side_w (3E), then the GCL weights
+    auto free_staging = [](double *p) { cudaFree(p); };
+    if (E > 0) CK(cudaMalloc(&edges_in, 3 * (size_t)E * sizeof(double)));
+    std::unique_ptr<double, decltype(free_staging)> staging(edges_in, free_staging);
+    const unsigned ge = (unsigned)((E + 255) / 256);
+    if (create) {
+        double *w = X.alloc<double>(3 * (size_t)E);
+        L.wx = w; L.wy = w + E; L.wz = w + 2 * (size_t)E;
+        L.slen = X.alloc<double>(E);
+        L.ew = X.alloc<EdgeW>(E);
+    }
+    if (E > 0) {
+        CK(cudaMemcpy(edges_in, d.side_w, 3 * (size_t)E * sizeof(double), cudaMemcpyHostToDevice));
+        k_put_edges<<<ge, 256>>>(E, L.eslot, edges_in, const_cast<double *>(L.wx), const_cast<double *>(L.wy),
+                                 const_cast<double *>(L.wz), const_cast<EdgeW *>(L.ew));
+        CK(cudaGetLastError());
+        if (d.side_len) CK(cudaMemcpy(edges_in, d.side_len, (size_t)E * sizeof(double), cudaMemcpyHostToDevice));
+        else CK(cudaMemset(edges_in, 0, (size_t)E * sizeof(double)));
+        k_put_edge_values<<<ge, 256>>>(E, L.eslot, edges_in, const_cast<double *>(L.slen));
+        CK(cudaGetLastError());
     }
     std::vector<int2> bedge(B);
     std::vector<double> bwx(B), bwy(B), bwz(B);
@@ -147,7 +161,6 @@ void flite::put_geometry(flite_ctx &X, int l, const flite_level_desc &d, bool cr
     std::vector<double> coords(3 * (size_t)N, 0.0), cm(3 * (size_t)N, 0.0);
     if (l == 0 && d.coords) std::memcpy(coords.data(), d.coords, 3 * (size_t)N * sizeof(double));
     if (l == 0 && d.coord_move) std::memcpy(cm.data(), d.coord_move, 3 * (size_t)N * sizeof(double));
-    put(L.wx, wx); put(L.wy, wy); put(L.wz, wz); put(L.slen, slen); put(L.ew, ew);
     put(L.bwx, bwx); put(L.bwy, bwy); put(L.bwz, bwz);
     put(L.V, std::vector<double>(d.volume, d.volume + N));
     put(L.wdist, d.wall_dist ? std::vector<double>(d.wall_dist, d.wall_dist + N) : std::vector<double>(N, 0.0));
@@ -168,20 +181,26 @@ void flite::put_geometry(flite_ctx &X, int l, const flite_level_desc &d, bool cr
         const double dtp = X.c.physicalTimeStep;
         auto w = [&](double x, double xp) { return comb ? 1.5 * x - 0.5 * xp : x; };
         std::vector<double> gw(std::max(E, 1)), bgw(2 * (size_t)std::max(B, 1));
-        for (int e = 0; e < E; ++e) gw[slot.empty() ? e : slot[e]] = w(d.side_gcl[e], d.side_gcl[(size_t)E + e]) / dtp;
+        for (int e = 0; e < E; ++e) gw[e] = w(d.side_gcl[e], d.side_gcl[(size_t)E + e]) / dtp;
         for (int b = 0; b < B; ++b) {
             const double g1 = w(d.bnd_gcl[b], d.bnd_gcl[2 * (size_t)B + b]);
             const double g2 = w(d.bnd_gcl[(size_t)B + b], d.bnd_gcl[3 * (size_t)B + b]);
             bgw[b] = X.c.boundaryTerm == 1 ? g1 / dtp : 4.0 * g1 / dtp;
             bgw[(size_t)B + b] = X.c.boundaryTerm == 1 ? g2 / dtp : 4.0 * g2 / dtp;
         }
-        put(L.gclw, gw);
+        if (create) L.gclw = X.alloc<double>(E);
+        if (E > 0) {
+            CK(cudaMemcpy(edges_in, gw.data(), (size_t)E * sizeof(double), cudaMemcpyHostToDevice));
+            k_put_edge_values<<<ge, 256>>>(E, L.eslot, edges_in, const_cast<double *>(L.gclw));
+            CK(cudaGetLastError());
+        }
         put(L.bgclw, bgw);
         if (l == 0) {
             put(L.Vp, std::vector<double>(d.volume_prev, d.volume_prev + N));
             put(L.Vp2, std::vector<double>(d.volume_prev2, d.volume_prev2 + N));
         }
     }
+    CK(cudaStreamSynchronize(nullptr));  // the context's own stream does not wait for these kernels
 }
 
 extern "C" {
@@ -272,6 +291,8 @@ int flite::create_context(const flite_controls *c, int nlevels, const flite_leve
                 }
         }
         CK(cudaStreamCreateWithFlags(&X.s, cudaStreamNonBlocking));
+        CK(cudaStreamCreateWithFlags(&X.side, cudaStreamNonBlocking));
+        for (cudaEvent_t &e : X.ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         CK(cudaMallocHost(&X.h_cycle, sizeof(int)));
         X.d_cycle = X.alloc<int>(1);
         X.d_cyc = X.alloc<int>(G);
@@ -304,6 +325,7 @@ int flite::create_context(const flite_controls *c, int nlevels, const flite_leve
                 L = donor->lv[l].v;  // mesh arrays shared; state set below
                 D.wall = donor->lv[l].wall;
                 D.nrows = donor->lv[l].nrows;
+                D.orphans = donor->lv[l].orphans;
                 D.d_wall = donor->lv[l].d_wall;
                 if (l == 0) P.engines = donor->P.engines;
             } else {
@@ -335,11 +357,7 @@ int flite::create_context(const flite_controls *c, int nlevels, const flite_leve
                     inc[fill[edge[e].y]++] = make_int2(~e, edge[e].x);
                 }
             }
-            // the rows of the slices, and on levels whose gathers take a
-            // thread per node by default the device's edge order: row by row
-            // over the slices, each edge in the row of its first node, so that
-            // a warp reads the coefficients (and edge buffers) of its k-th
-            // edges side by side; the sums keep the caller's order
+            // the first row of each slice of kRow nodes (LevelView::rows)
             const int nslice = (N + kRow - 1) / kRow;
             std::vector<int> rp(nslice, 0);
             for (int t = 0; t < nslice; ++t) {
@@ -347,21 +365,6 @@ int flite::create_context(const flite_controls *c, int nlevels, const flite_leve
                 int most = 0;
                 for (int i = t * kRow; i < std::min(N, (t + 1) * kRow); ++i) most = std::max(most, ip[i + 1] - ip[i]);
                 D.nrows += most;
-            }
-            if (4 * (size_t)N > kLaneThreads) {
-                std::vector<int> &slot = D.eslot;
-                slot.resize(E);
-                int next = 0;
-                for (int t = 0; t < nslice; ++t) {
-                    const int most = (t + 1 < nslice ? rp[t + 1] : D.nrows) - rp[t], i1 = std::min(N, (t + 1) * kRow);
-                    for (int k = 0; k < most; ++k)
-                        for (int i = t * kRow; i < i1; ++i)
-                            if (ip[i] + k < ip[i + 1] && inc[ip[i] + k].x >= 0) slot[inc[ip[i] + k].x] = next++;
-                }
-                for (int2 &v : inc) v.x = v.x >= 0 ? slot[v.x] : ~slot[~v.x];
-                std::vector<int2> moved(E);
-                for (int e = 0; e < E; ++e) moved[slot[e]] = edge[e];
-                edge.swap(moved);
             }
             std::vector<int> bp(N + 1, 0);
             for (int b = 0; b < B; ++b) { bp[bedge[b].x + 1]++; bp[bedge[b].y + 1]++; }
@@ -392,15 +395,39 @@ int flite::create_context(const flite_controls *c, int nlevels, const flite_leve
                 }
             }
             // upload
-            L.edge = X.upload(edge);
+            int2 *dedge = X.upload(edge);
+            L.edge = dedge;
             L.bedge = X.upload(bedge); L.bind = X.upload(bind);
-            L.inc_ptr = X.upload(ip); L.inc = X.upload(inc);
-            L.eslot = D.eslot.empty() ? nullptr : X.upload(D.eslot);
+            int2 *dinc = X.upload(inc);
+            L.inc_ptr = X.upload(ip); L.inc = dinc;
             L.row_ptr = X.upload(rp);
             int2 *rows = X.alloc<int2>((size_t)(D.nrows + kRowPad) * kRow);
-            CK(cudaMemset(rows, 0, (size_t)(D.nrows + kRowPad) * kRow * sizeof(int2)));
+            // entries of no node: second node (of edge 0), so no edge's first
+            CK(cudaMemset(rows, 0xff, (size_t)(D.nrows + kRowPad) * kRow * sizeof(int2)));
             k_make_rows<<<flite_ctx::blocks(N), kBlock>>>(L, D.nrows, rows);
             CK(cudaGetLastError());
+            // on levels whose gathers take a thread per node by default the
+            // device numbers the edges row by row over the slices, each edge
+            // in the row of its first node, so that a warp reads the
+            // coefficients (and edge buffers) of its k-th edges side by side;
+            // the sums keep the caller's order
+            L.eslot = nullptr;
+            if (4 * (size_t)N > kLaneThreads && E > 0) {
+                int *slot = X.alloc<int>(E), *first = X.alloc<int>(D.nrows);
+                const unsigned gr = flite_ctx::blocks((size_t)D.nrows * kRow);
+                k_row_firsts<<<gr, kBlock>>>(rows, D.nrows, first);
+                k_scan_rows<<<1, 1024>>>(first, D.nrows);
+                k_edge_slots<<<gr, kBlock>>>(rows, D.nrows, first, slot);
+                k_renumber_edges<<<gr, kBlock>>>(rows, D.nrows * kRow, slot);
+                k_renumber_edges<<<flite_ctx::blocks(2 * (size_t)E), kBlock>>>(dinc, 2 * E, slot);
+                int2 *moved = X.alloc<int2>(E);
+                k_move_edges<<<flite_ctx::blocks(E), kBlock>>>(E, slot, dedge, moved);
+                CK(cudaGetLastError());
+                L.edge = moved;
+                L.eslot = slot;
+                X.release(dedge);
+                X.release(first);
+            }
             L.rows = rows;
             L.binc_ptr = X.upload(bp); L.binc = X.upload(binc);
             L.conn = X.upload(conn);
@@ -449,6 +476,7 @@ int flite::create_context(const flite_controls *c, int nlevels, const flite_leve
                     par[f] = d.parent[f] - 1;
                     if (par[f] >= N) throw std::runtime_error("parent out of range");
                     if (par[f] >= 0) cp[par[f] + 1]++;
+                    else D.orphans = true;
                 }
                 for (int i = 0; i < N; ++i) cp[i + 1] += cp[i];
                 // children in the order of the caller's fine numbering, the
@@ -503,6 +531,11 @@ int flite::create_context(const flite_controls *c, int nlevels, const flite_leve
             const bool visc = c->ReynoldsNumber > 0.0;
             L.q = X.alloc<NodeRec>(N);
             CK(cudaMemset(L.q, 0, (size_t)N * sizeof(NodeRec)));
+            // the other copies of the records and of the state that the stages
+            // alternate (any level may be given lanes per node later)
+            L.qb = X.fused() && !X.mixed() ? X.alloc<NodeRec>(N) : nullptr;
+            L.ub = X.fused() && !X.mixed() ? X.alloc<double>(5 * (size_t)N) : nullptr;
+            L.dqb = nullptr;
             // stress and heat flux (scheme 1), or the scaled gradients with mu
             // and k (scheme 2)
             L.tau = visc ? X.alloc<double>((c->viscosityScheme == 2 ? 14 : 9) * (size_t)N) : nullptr;
@@ -526,6 +559,7 @@ int flite::create_context(const flite_controls *c, int nlevels, const flite_leve
                 L.pa = X.alloc<double>(N);
                 L.a32 = X.alloc<float>(5 * (size_t)N);
                 L.dq = X.alloc<DeltaRec>(N);
+                L.dqb = X.alloc<DeltaRec>(N);
                 // a zero anchor makes the increments the full FP32 fluxes
                 // until the first FP64 evaluation
                 for (double *a : {L.ua, L.ra}) CK(cudaMemset(a, 0, 5 * (size_t)N * sizeof(double)));
@@ -968,13 +1002,13 @@ int flite_profile_kernels(flite_ctx *ctx, int level, int reps, double *ms, int32
             else if (fz == 1) X.jst_flux(l);
             return fz != 2;
         });
-        k.push_back([&] { if (visc) k_visc_prim<<<X.nblk(L.N), X.nb, 0, X.s>>>(X.P, L); return visc; });
+        k.push_back([&] { if (visc) X.viscous_prim(l); return visc; });
         k.push_back([&] { if (visc && fz != 2) X.visc_grad(l); return visc && fz != 2; });
         k.push_back([&] { if (visc) X.visc_flux(l); return visc; });
         k.push_back([&] { X.rhs_terms(l, true); return true; });
         k.push_back([&] { X.launch_node_update(l, MODE_RFINE, 0, true); return true; });
-        k.push_back([&] { if (fz) k_ts_lap<<<X.nblk(L.N), X.nb, 0, X.s>>>(X.P, L); return fz != 0; });
-        k.push_back([&] { if (fz == 2) k_jflux_vgrad<<<X.nblk(L.N), X.nb, 0, X.s>>>(X.P, L); return fz == 2; });
+        k.push_back([&] { if (fz) k_ts_lap<1><<<X.nblk(L.N), X.nb, 0, X.s>>>(X.P, L); return fz != 0; });
+        k.push_back([&] { if (fz == 2) k_jflux_vgrad<1><<<X.nblk(L.N), X.nb, 0, X.s>>>(X.P, L); return fz == 2; });
         const int m = std::min<int>((int)k.size(), nmax);
         std::vector<cudaEvent_t> ev(m + 1);
         for (auto &e : ev) CK(cudaEventCreate(&e));

@@ -405,31 +405,39 @@ __device__ __forceinline__ void boundary_gcl(const Params &P, const LevelView &L
 }
 
 // Contributions g1 (to node 1) and g2 (to node 2) of boundary edge b
-// (def_par:2182-2511)
-__device__ __forceinline__ void boundary_flux(const Params &P, const LevelView &L, int b, double *g1, double *g2) {
+// (def_par:2182-2511); state(j) gives node j's state
+template <class State>
+__device__ __forceinline__ void boundary_flux(const Params &P, const LevelView &L, int b, State &&state, double *g1,
+                                              double *g2) {
     const int2 nd = L.bedge[b];
     const int ind = L.bind[b];
     const double wx = L.bwx[b], wy = L.bwy[b], wz = L.bwz[b];
     for (int k = 0; k < 5; ++k) { g1[k] = 0.0; g2[k] = 0.0; }
-    const NodeState s1 = load_state(L, nd.x), s2 = load_state(L, nd.y);
-    const bool fe = P.boundaryTerm == 1;
+    const bool fe = P.boundaryTerm == 1, wall = ind <= 2 || ind == 9, far = !wall && ind <= 4;
+    const double rnorm = sqrt((wx * wx + wy * wy) + wz * wz);
+    double rnx = 0.0, rny = 0.0, rnz = 0.0;
+    if (wall || far) {
+        if (!(rnorm > 1.0e-10)) return;
+        rnx = wx / rnorm; rny = wy / rnorm; rnz = wz / rnorm;
+    }
+    const double *inf = &P.inf[ind == 4 ? 6 : 0];
+    // one copy of the three fluxes, run for each end (both ends unrolled take
+    // twice the registers, which the node passes that inline this pay for)
     double F1[5], F2[5];
-    if (ind <= 2 || ind == 9) {
-        double rnorm = sqrt((wx * wx + wy * wy) + wz * wz);
-        if (!(rnorm > 1.0e-10)) return;
-        double rnx = wx / rnorm, rny = wy / rnorm, rnz = wz / rnorm;
-        wall_flux(s1, rnx, rny, rnz, F1);
-        wall_flux(s2, rnx, rny, rnz, F2);
-    } else if (ind <= 4) {
-        double rnorm = sqrt((wx * wx + wy * wy) + wz * wz);
-        if (!(rnorm > 1.0e-10)) return;
-        double rnx = wx / rnorm, rny = wy / rnorm, rnz = wz / rnorm;
-        const double *inf = &P.inf[(ind - 3) * 6];
-        farfield_flux(P, s1, rnx, rny, rnz, inf, F1);
-        farfield_flux(P, s2, rnx, rny, rnz, inf, F2);
-    } else {  // engine faces: the two fluxes' sum plus twice the node's own (def_par:2493-2505)
-        engine_flux(s1, wx, wy, wz, F1);
-        engine_flux(s2, wx, wy, wz, F2);
+#pragma unroll 1
+    for (int end = 0; end < 2; ++end) {
+        const NodeState s = state(end == 0 ? nd.x : nd.y);
+        double F[5];
+        if (wall) wall_flux(s, rnx, rny, rnz, F);
+        else if (far) farfield_flux(P, s, rnx, rny, rnz, inf, F);
+        else engine_flux(s, wx, wy, wz, F);
+#pragma unroll
+        for (int k = 0; k < 5; ++k) {
+            if (end == 0) F1[k] = F[k];
+            else F2[k] = F[k];
+        }
+    }
+    if (!wall && !far) {  // engine faces: the two fluxes' sum plus twice the node's own (def_par:2493-2505)
         for (int k = 0; k < 5; ++k) {
             const double fs = F1[k] + F2[k];
             g1[k] = fs + 2.0 * F1[k];
@@ -437,7 +445,6 @@ __device__ __forceinline__ void boundary_flux(const Params &P, const LevelView &
         }
         return;
     }
-    const double rnorm = sqrt((wx * wx + wy * wy) + wz * wz);
     for (int k = 0; k < 5; ++k) {
         if (fe) {
             g1[k] = rnorm * (3. * F1[k] + F2[k]);

@@ -96,17 +96,50 @@ __device__ __forceinline__ void group_sum(T *gs, int beg, int end, bool active, 
     T *gs = gslab_ + (U > 1 ? (threadIdx.x >> 5) * (K)*kSlabRow : 0)
 
 // ---- makePressureField (def_par:13612-13630) ------------------------------
-template <bool B>
-__global__ void k_pressure(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_) {
+// One pass over the state: the pressure, the node records, and on request the
+// (u, v, w, T) of the viscous routine (def_par:5260-5270; each edge of the
+// reference divides again, the quotients are the same numbers) and the start
+// of a relaxation step (def_par:983-987), which would each read the state
+// again in a launch of their own.  Bound by its bytes: 40 read, 56 written
+// per node, 40 more with the step's copy and 32 with the primitives.
+template <bool BND, bool B>
+__global__ void k_state_pass(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_, int what, const int *src) {
     FLITE_CASE_P(B, P, L);
     FLITE_CASE_L(B, L);
-    int i = tid();
-    if (i >= L.N) return;
+    const int i = tid();
     const int N = L.N;
+    if (i >= N) {
+        // a boundary edge; its nodes' pressures are formed here as the node
+        // threads form them
+        if (!BND || i - N >= L.B) return;
+        const auto state = [&](int j) {
+            NodeState s;
+            s.r = L.u[j]; s.ru = L.u[N + j]; s.rv = L.u[2 * N + j]; s.rw = L.u[3 * N + j]; s.E = L.u[4 * N + j];
+            s.p = pressure(P, s.r, s.ru, s.rv, s.rw, s.E);
+            return s;
+        };
+        double g1[5], g2[5];
+        boundary_flux(P, L, i - N, state, g1, g2);
+        double *o = L.bflux + (size_t)(i - N) * 10;
+        for (int k = 0; k < 5; ++k) { o[k] = g1[k]; o[5 + k] = g2[k]; }
+        return;
+    }
     const double r = L.u[i], ru = L.u[N + i], rv = L.u[2 * N + i], rw = L.u[3 * N + i], E = L.u[4 * N + i];
+    if (what & STATE_STEP) {
+        if (i == 0) *L.cyc = *src;
+        L.uprev[i] = r; L.uprev[N + i] = ru; L.uprev[2 * N + i] = rv; L.uprev[3 * N + i] = rw; L.uprev[4 * N + i] = E;
+        if (L.nvar == 6) L.uprev[5 * (size_t)N + i] = L.u[5 * (size_t)N + i];
+    }
     const double p = pressure(P, r, ru, rv, rw, E);
     L.p[i] = p;
-    store_node(L.q, i, r, ru, rv, rw, E, p);
+    if (what & STATE_REC) store_node(L.q, i, r, ru, rv, rw, E, p);
+    if (what & STATE_PRIM) {
+        const double gOg = P.gamma / (P.gamma - 1.0);
+        L.prim[i] = ru / r;
+        L.prim[N + i] = rv / r;
+        L.prim[2 * N + i] = rw / r;
+        L.prim[3 * N + i] = gOg * p / r;
+    }
 }
 
 // ---- makeTimeSteps (def_par:13335-13610) as a node gather -----------------
@@ -184,6 +217,35 @@ __device__ __forceinline__ void ts_finish(const Params &P, const LevelView &L, i
     ts_store(L, i, acc, h);
 }
 
+// node i's time step with U lanes (lane gl, the warp's slab gs of 8 terms)
+template <int U>
+__device__ __forceinline__ void ts_group(const Params &P, const LevelView &L, int i, bool active, int gl, double *gs,
+                                         double m1, double m2, double m3, double ro, double cc) {
+    const int N = L.N;
+    // sum 0: the convective and acoustic terms; sum 1: the viscous ones
+    double x[2] = {0.0, 0.0};
+    group_sum<U, 2, 2, double>(
+        gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl,
+        [&](int k, double *v) {
+            const int2 t = L.inc[k];
+            const int e = t.x >= 0 ? t.x : ~t.x;
+            const double wx = L.wx[e], wy = L.wy[e], wz = L.wz[e];
+            const double al = (wx * wx + wy * wy) + wz * wz;
+            const double vn = ((wx * m1 + wy * m2) + wz * m3) * ro;
+            v[0] = fabs(vn);
+            v[1] = sqrt(cc * al);
+            if (P.viscous) {
+                const int j = t.y;
+                const double vis = dmax(P.am, P.sa ? L.mu[j] + L.u[5 * N + j] / P.Re : L.mu[j]);
+                v[2] = 2.0 * vis * al / L.u[j];
+            }
+        },
+        x);
+    group_sum<U, 2, 4, double>(
+        gs, L.binc_ptr[i], L.binc_ptr[i + 1], active, gl, [&](int k, double *v) { ts_bterms(P, L, k, v); }, x);
+    if (active && gl == 0) ts_store(L, i, x[0], x[1]);
+}
+
 template <int U, bool B>
 __global__ void k_timestep(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_) {
     FLITE_CASE_P(B, P, L);
@@ -194,35 +256,12 @@ __global__ void k_timestep(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_) {
     const bool active = i_raw < L.N;
     const int i = active ? i_raw : L.N - 1;  // idle groups read a valid node
     const int N = L.N;
-    const double c1 = P.gamma;
-    const double ri = L.u[i], ro = 1. / ri;
+    const double ro = 1. / L.u[i];
     const double m1 = L.u[N + i], m2 = L.u[2 * N + i], m3 = L.u[3 * N + i];
-    const double cc = dmax(c1 * L.p[i] * ro, 0.001);
+    const double cc = dmax(P.gamma * L.p[i] * ro, 0.001);
     if constexpr (U > 1) {
         FLITE_GROUP_SLAB(double, 8);
-        // sum 0: the convective and acoustic terms; sum 1: the viscous ones
-        double x[2] = {0.0, 0.0};
-        group_sum<U, 2, 2, double>(
-            gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl,
-            [&](int k, double *v) {
-                const int2 t = L.inc[k];
-                const int e = t.x >= 0 ? t.x : ~t.x;
-                const double wx = L.wx[e], wy = L.wy[e], wz = L.wz[e];
-                const double al = (wx * wx + wy * wy) + wz * wz;
-                const double vn = ((wx * m1 + wy * m2) + wz * m3) * ro;
-                v[0] = fabs(vn);
-                v[1] = sqrt(cc * al);
-                if (P.viscous) {
-                    const int j = t.y;
-                    const double vis = dmax(P.am, P.sa ? L.mu[j] + L.u[5 * N + j] / P.Re : L.mu[j]);
-                    v[2] = 2.0 * vis * al / L.u[j];
-                }
-            },
-            x);
-        group_sum<U, 2, 4, double>(
-            gs, L.binc_ptr[i], L.binc_ptr[i + 1], active, gl, [&](int k, double *v) { ts_bterms(P, L, k, v); }, x);
-        if (!active || gl) return;
-        ts_store(L, i, x[0], x[1]);
+        ts_group<U>(P, L, i, active, gl, gs, m1, m2, m3, ro, cc);
     } else {
         double acc = 0.0, h = 0.0;
         FLITE_FOR_INC(L, i, t) ts_inc(P, L, t, m1, m2, m3, ro, cc, acc, h);
@@ -268,6 +307,42 @@ __device__ __forceinline__ void lap_store(const LevelView &L, int i, const LapAc
     for (int c = 0; c < 5; ++c) L.lap[c * N + i] = fact * a.l[c];
 }
 
+// node i's Laplacian and sensor with U lanes (a slab of 7 terms)
+template <int U>
+__device__ __forceinline__ void lap_group(const Params &P, const LevelView &L, int i, bool active, int gl, double *gs,
+                                          const double *ui, double pi) {
+    const int N = L.N;
+    double x[7] = {0, 0, 0, 0, 0, 0, 0};
+    group_sum<U, 7, 1, double>(
+        gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl,
+        [&](int k, double *v) {
+            const int2 t = L.inc[k];
+            const int j = t.y;
+            double df = 1.0;
+            if (P.useDissW) df = 1. / L.slen[t.x >= 0 ? t.x : ~t.x];
+            const double uj[5] = {L.u[j], L.u[N + j], L.u[2 * N + j], L.u[3 * N + j], L.u[4 * N + j]};
+            const double pj = L.p[j];
+            // x - y is x + (-y): the subtractions of the serial loop become
+            // additions of negated terms
+            if (t.x >= 0) {
+#pragma unroll
+                for (int c = 0; c < 4; ++c) v[c] = -((ui[c] - uj[c]) * df);
+                v[4] = -((((ui[4] - uj[4]) + pi) - pj) * df);
+                v[5] = -(pi - pj); v[6] = pi + pj;
+            } else {
+#pragma unroll
+                for (int c = 0; c < 4; ++c) v[c] = (uj[c] - ui[c]) * df;
+                v[4] = (((uj[4] - ui[4]) + pj) - pi) * df;
+                v[5] = pj - pi; v[6] = pj + pi;
+            }
+        },
+        x);
+    if (active && gl == 0) {
+        const LapAcc a = {{x[0], x[1], x[2], x[3], x[4]}, x[5], x[6]};
+        lap_store(L, i, a);
+    }
+}
+
 template <int U, bool B>
 __global__ void k_jst_lap(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_) {
     FLITE_CASE_P(B, P, L);
@@ -282,34 +357,7 @@ __global__ void k_jst_lap(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_) {
     const double pi = L.p[i];
     if constexpr (U > 1) {
         FLITE_GROUP_SLAB(double, 7);
-        double x[7] = {0, 0, 0, 0, 0, 0, 0};
-        group_sum<U, 7, 1, double>(
-            gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl,
-            [&](int k, double *v) {
-                const int2 t = L.inc[k];
-                const int j = t.y;
-                double df = 1.0;
-                if (P.useDissW) df = 1. / L.slen[t.x >= 0 ? t.x : ~t.x];
-                const double uj[5] = {L.u[j], L.u[N + j], L.u[2 * N + j], L.u[3 * N + j], L.u[4 * N + j]};
-                const double pj = L.p[j];
-                // x - y is x + (-y): the subtractions of the serial loop become
-                // additions of negated terms
-                if (t.x >= 0) {
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) v[c] = -((ui[c] - uj[c]) * df);
-                    v[4] = -((((ui[4] - uj[4]) + pi) - pj) * df);
-                    v[5] = -(pi - pj); v[6] = pi + pj;
-                } else {
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) v[c] = (uj[c] - ui[c]) * df;
-                    v[4] = (((uj[4] - ui[4]) + pj) - pi) * df;
-                    v[5] = pj - pi; v[6] = pj + pi;
-                }
-            },
-            x);
-        if (!active || gl) return;
-        const LapAcc a = {{x[0], x[1], x[2], x[3], x[4]}, x[5], x[6]};
-        lap_store(L, i, a);
+        lap_group<U>(P, L, i, active, gl, gs, ui, pi);
     } else {
         LapAcc a = {{0, 0, 0, 0, 0}, 0, 0};
         FLITE_FOR_INC(L, i, t) lap_inc(P, L, t, ui, pi, a);
@@ -346,26 +394,20 @@ __device__ __forceinline__ void jflux_inc(const Params &P, const LevelView &L, i
     }
 }
 
-template <int U, bool B>
-__global__ void __launch_bounds__(256, U == 1 ? 4 : 1) k_jst_flux(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_) {
-    FLITE_CASE_P(B, P, L);
-    FLITE_CASE_L(B, L);
-    const int gl = U > 1 ? (int)(threadIdx.x % U) : 0;  // lane in the node's group
-    const int i_raw = U > 1 ? tid() / U : tid();
-    if (U == 1 && i_raw >= L.N) return;
-    const bool active = i_raw < L.N;
-    const int i = active ? i_raw : L.N - 1;  // idle groups read a valid node
+// node i's scalar JST flux with U lanes (a slab of 10 terms) at the state u;
+// every lane gets the sums
+template <int U>
+__device__ __forceinline__ void jflux_group(const Params &P, const LevelView &L, const double *u, int i, bool active,
+                                            int gl, double *gs, double *acc) {
     const int N = L.N;
     const double k4 = L.grid == 1 ? P.k4 : P.cgdf;
-    double acc[5] = {0, 0, 0, 0, 0};
     double Li[5], Ui[5];
-    for (int c = 0; c < 5; ++c) { Li[c] = L.lap[c * N + i]; Ui[c] = L.u[c * N + i]; }
+#pragma unroll
+    for (int c = 0; c < 5; ++c) { acc[c] = 0.0; Li[c] = L.lap[c * N + i]; Ui[c] = u[c * N + i]; }
     const double vdi = L.vdt[i], coni = L.conn[i], si = L.sens[i];
-    if constexpr (U > 1) {
-        FLITE_GROUP_SLAB(double, 10);
-        group_sum<U, 5, 2, double>(
-            gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl,
-            [&](int k, double *v) {
+    group_sum<U, 5, 2, double>(
+        gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl,
+        [&](int k, double *v) {
             const int2 t = L.inc[k];
             const int j = t.y;
             const double vdj = L.vdt[j];
@@ -376,8 +418,9 @@ __global__ void __launch_bounds__(256, U == 1 ? 4 : 1) k_jst_flux(CaseArg<B, Par
             const double d2 = d0 * P.k2 * (first ? dmax(si, sj) : dmax(sj, si));
             double d4 = d0 * k4;
             d4 = d4 > d2 ? d4 - d2 : 0.0;
+#pragma unroll
             for (int c = 0; c < 5; ++c) {
-                const double Lj = L.lap[c * N + j], Uj = L.u[c * N + j];
+                const double Lj = L.lap[c * N + j], Uj = u[c * N + j];
                 if (first) {
                     v[2 * c] = -((Li[c] - Lj) * d4);
                     v[2 * c + 1] = (Ui[c] - Uj) * d2;
@@ -386,11 +429,32 @@ __global__ void __launch_bounds__(256, U == 1 ? 4 : 1) k_jst_flux(CaseArg<B, Par
                     v[2 * c + 1] = -((Uj - Ui[c]) * d2);
                 }
             }
-            },
-            acc);
+        },
+        acc);
+}
+
+template <int U, bool B>
+__global__ void __launch_bounds__(256, U == 1 ? 4 : 1) k_jst_flux(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_) {
+    FLITE_CASE_P(B, P, L);
+    FLITE_CASE_L(B, L);
+    const int gl = U > 1 ? (int)(threadIdx.x % U) : 0;  // lane in the node's group
+    const int i_raw = U > 1 ? tid() / U : tid();
+    if (U == 1 && i_raw >= L.N) return;
+    const bool active = i_raw < L.N;
+    const int i = active ? i_raw : L.N - 1;  // idle groups read a valid node
+    const int N = L.N;
+    double acc[5] = {0, 0, 0, 0, 0};
+    if constexpr (U > 1) {
+        FLITE_GROUP_SLAB(double, 10);
+        jflux_group<U>(P, L, L.u, i, active, gl, gs, acc);
         if (!active || gl) return;
-    } else
-    FLITE_FOR_INC(L, i, t) jflux_inc(P, L, t, k4, vdi, coni, si, Li, Ui, acc);
+    } else {
+        const double k4 = L.grid == 1 ? P.k4 : P.cgdf;
+        double Li[5], Ui[5];
+        for (int c = 0; c < 5; ++c) { Li[c] = L.lap[c * N + i]; Ui[c] = L.u[c * N + i]; }
+        const double vdi = L.vdt[i], coni = L.conn[i], si = L.sens[i];
+        FLITE_FOR_INC(L, i, t) jflux_inc(P, L, t, k4, vdi, coni, si, Li, Ui, acc);
+    }
     for (int c = 0; c < 5; ++c) L.diss[c * N + i] = acc[c];
 }
 
@@ -593,23 +657,6 @@ __global__ void k_first_order_diss(Params P, LevelView L) {
 // pass 1: Galerkin gradients of (u, v, w, T), then per node the Sutherland
 // viscosity (T^1.5 evaluated as T*sqrt(T)), the stress tensor and heat
 // flux, the adiabatic-wall projection and the wall stress (level 1)
-// per node (u, v, w, T) of the viscous routine (def_par:5260-5270): each
-// edge of the reference divides again; the quotients are the same numbers
-template <bool B>
-__global__ void k_visc_prim(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_) {
-    FLITE_CASE_P(B, P, L);
-    FLITE_CASE_L(B, L);
-    int i = tid();
-    if (i >= L.N) return;
-    const int N = L.N;
-    const double gOg = P.gamma / (P.gamma - 1.0);
-    const double r = L.u[i];
-    L.prim[i] = L.u[N + i] / r;
-    L.prim[N + i] = L.u[2 * N + i] / r;
-    L.prim[2 * N + i] = L.u[3 * N + i] / r;
-    L.prim[3 * N + i] = gOg * L.p[i] / r;
-}
-
 // the boundary-face terms of node i's Galerkin gradients of (u, v, w, T)
 // (def_par:5322-5409), added to g in boundary-edge order
 __device__ __forceinline__ void visc_grad_bterms(const LevelView &L, int k, double *d) {
@@ -707,6 +754,34 @@ __device__ __forceinline__ void visc_grad_boundary(const LevelView &L, int i, do
     }
 }
 
+// node i's 12 gradient sums with U lanes (a slab of 12 terms), boundary
+// edges included; every lane gets them
+template <int U>
+__device__ __forceinline__ void vgrad_group(const LevelView &L, int i, bool active, int gl, double *gs, double *g) {
+    const int N = L.N;
+    const double qi[4] = {L.prim[i], L.prim[N + i], L.prim[2 * N + i], L.prim[3 * N + i]};
+#pragma unroll
+    for (int c = 0; c < 12; ++c) g[c] = 0.0;
+    group_sum<U, 12, 1, double>(
+        gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl,
+        [&](int k, double *d) {
+            const int2 t = L.inc[k];
+            const int e = t.x >= 0 ? t.x : ~t.x, j = t.y;
+            const double qj[4] = {L.prim[j], L.prim[N + j], L.prim[2 * N + j], L.prim[3 * N + j]};
+            const double w[3] = {L.wx[e], L.wy[e], L.wz[e]};
+#pragma unroll
+            for (int a = 0; a < 3; ++a)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const double x = (t.x >= 0 ? qi[c] + qj[c] : qj[c] + qi[c]) * w[a];
+                    d[a * 4 + c] = t.x >= 0 ? x : -x;  // g - x is g + (-x)
+                }
+        },
+        g);
+    group_sum<U, 12, 1, double>(
+        gs, L.binc_ptr[i], L.binc_ptr[i + 1], active, gl, [&](int k, double *d) { visc_grad_bterms(L, k, d); }, g);
+}
+
 template <int U, bool B>
 __global__ void __launch_bounds__(256, U == 1 ? 3 : 1) k_visc_grad(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_) {
     FLITE_CASE_P(B, P, L);
@@ -718,34 +793,13 @@ __global__ void __launch_bounds__(256, U == 1 ? 3 : 1) k_visc_grad(CaseArg<B, Pa
     const int i = active ? i_raw : L.N - 1;  // idle groups read a valid node
     const int N = L.N;
     double g[12];
-    for (int c = 0; c < 12; ++c) g[c] = 0.0;
-    auto prim = [&](int j, double *q) {
-        q[0] = L.prim[j]; q[1] = L.prim[N + j]; q[2] = L.prim[2 * N + j]; q[3] = L.prim[3 * N + j];
-    };
-    double qi[4];
-    prim(i, qi);
-    auto iterms = [&](const int2 t, double *d) {
-        int e = t.x >= 0 ? t.x : ~t.x;
-        double qj[4];
-        prim(t.y, qj);
-        const double w[3] = {L.wx[e], L.wy[e], L.wz[e]};
-        for (int a = 0; a < 3; ++a)
-            for (int c = 0; c < 4; ++c) {
-                double x = (t.x >= 0 ? qi[c] + qj[c] : qj[c] + qi[c]) * w[a];
-                d[a * 4 + c] = t.x >= 0 ? x : -x;  // g - x is g + (-x)
-            }
-    };
-    auto bterms = [&](int k, double *d) { visc_grad_bterms(L, k, d); };
-    auto add = [&](const double *d) {
-        for (int c = 0; c < 12; ++c) g[c] = g[c] + d[c];
-    };
     if constexpr (U > 1) {
         FLITE_GROUP_SLAB(double, 12);
-        group_sum<U, 12, 1, double>(gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl,
-                                         [&](int k, double *v) { iterms(L.inc[k], v); }, g);
-        group_sum<U, 12, 1, double>(gs, L.binc_ptr[i], L.binc_ptr[i + 1], active, gl, bterms, g);
+        vgrad_group<U>(L, i, active, gl, gs, g);
         if (!active || gl) return;
     } else {
+        for (int c = 0; c < 12; ++c) g[c] = 0.0;
+        const double qi[4] = {L.prim[i], L.prim[N + i], L.prim[2 * N + i], L.prim[3 * N + i]};
         FLITE_FOR_INC(L, i, t) vgrad_inc(L, t, qi, g);
         visc_grad_boundary(L, i, g);
     }
@@ -815,6 +869,45 @@ __device__ __forceinline__ void visc_flux_boundary(const LevelView &L, int i, do
 
 // pass 2: viscous edge fluxes gathered per node and subtracted from the
 // dissipation vector (def_par:5662-5892)
+// interior edge t of node i (tensor ti, velocity ui): the edge flux with the
+// sign of this node (x - y is x + (-y))
+__device__ __forceinline__ void vflux_terms(const LevelView &L, const int2 t, const double *ti, const double *ui,
+                                            double *g) {
+    const int N = L.N, e = t.x >= 0 ? t.x : ~t.x, j = t.y;
+    double tj[9], uj[3];
+    for (int c = 0; c < 9; ++c) tj[c] = L.tau[c * N + j];
+    uj[0] = L.prim[j]; uj[1] = L.prim[N + j]; uj[2] = L.prim[2 * N + j];
+    const bool first = t.x >= 0;
+    double f[4];
+    visc_edge_flux(first ? ti : tj, first ? tj : ti, first ? ui : uj, first ? uj : ui, L.wx[e], L.wy[e], L.wz[e], f);
+    for (int c = 0; c < 4; ++c) g[c] = first ? f[c] : -f[c];
+}
+// node i's viscous fluxes with U lanes (a slab of 8 terms); every lane gets
+// the sums
+template <int U>
+__device__ __forceinline__ void vflux_group(const LevelView &L, int i, bool active, int gl, double *gs, double *acc) {
+    const int N = L.N;
+    double ti[9];
+    for (int c = 0; c < 9; ++c) ti[c] = L.tau[c * N + i];
+    const double ui[3] = {L.prim[i], L.prim[N + i], L.prim[2 * N + i]};
+#pragma unroll
+    for (int c = 0; c < 4; ++c) acc[c] = 0.0;
+    group_sum<U, 4, 1, double>(
+        gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl,
+        [&](int k, double *v) { vflux_terms(L, L.inc[k], ti, ui, v); }, acc);
+    // a face that does not count leaves zeros
+    group_sum<U, 4, 2, double>(
+        gs, L.binc_ptr[i], L.binc_ptr[i + 1], active, gl,
+        [&](int k, double *v) {
+            double t[9];
+            visc_flux_bterms(L, k, t);
+            if (t[8] == 0.0) return;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) { v[2 * c] = t[c]; v[2 * c + 1] = t[4 + c]; }
+        },
+        acc);
+}
+
 template <int U, bool B>
 __global__ void __launch_bounds__(256, U == 1 ? 3 : 1) k_visc_flux(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_) {
     FLITE_CASE_P(B, P, L);
@@ -825,63 +918,26 @@ __global__ void __launch_bounds__(256, U == 1 ? 3 : 1) k_visc_flux(CaseArg<B, Pa
     const bool active = i_raw < L.N;
     const int i = active ? i_raw : L.N - 1;  // idle groups read a valid node
     const int N = L.N;
-    double ti[9], ui[3];
-    for (int c = 0; c < 9; ++c) ti[c] = L.tau[c * N + i];
-    ui[0] = L.prim[i]; ui[1] = L.prim[N + i]; ui[2] = L.prim[2 * N + i];
     double acc[4] = {0, 0, 0, 0};
-    // interior edge: the edge flux with the sign of this node (x - y is x + (-y))
-    auto iterms = [&](const int2 t, double *g) {
-        int e = t.x >= 0 ? t.x : ~t.x, j = t.y;
-        double tj[9], uj[3];
-        for (int c = 0; c < 9; ++c) tj[c] = L.tau[c * N + j];
-        uj[0] = L.prim[j]; uj[1] = L.prim[N + j]; uj[2] = L.prim[2 * N + j];
-        const bool first = t.x >= 0;
-        double f[4];
-        visc_edge_flux(first ? ti : tj, first ? tj : ti, first ? ui : uj, first ? uj : ui, L.wx[e], L.wy[e], L.wz[e],
-                       f);
-        for (int c = 0; c < 4; ++c) g[c] = first ? f[c] : -f[c];
-    };
-    auto iadd = [&](const double *g) {
-        for (int c = 0; c < 4; ++c) acc[c] = acc[c] + g[c];
-    };
-    // boundary edge: the two terms of each component, g[8] = 1 if it counts
-    auto bterms = [&](int k, double *g) { visc_flux_bterms(L, k, g); };
-    auto badd = [&](const double *g) {
-        if (g[8] == 0.0) return;
-        for (int c = 0; c < 4; ++c) acc[c] = (acc[c] + g[c]) + g[4 + c];
-    };
     if constexpr (U > 1) {
         FLITE_GROUP_SLAB(double, 8);
-        group_sum<U, 4, 1, double>(gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl,
-                                        [&](int k, double *v) { iterms(L.inc[k], v); }, acc);
-        // a face that does not count leaves zeros
-        group_sum<U, 4, 2, double>(
-            gs, L.binc_ptr[i], L.binc_ptr[i + 1], active, gl,
-            [&](int k, double *v) {
-                double t[9];
-                bterms(k, t);
-                if (t[8] == 0.0) return;
-#pragma unroll
-                for (int c = 0; c < 4; ++c) { v[2 * c] = t[c]; v[2 * c + 1] = t[4 + c]; }
-            },
-            acc);
+        vflux_group<U>(L, i, active, gl, gs, acc);
         if (!active || gl) return;
     } else {
+        double ti[9];
+        for (int c = 0; c < 9; ++c) ti[c] = L.tau[c * N + i];
+        const double ui[3] = {L.prim[i], L.prim[N + i], L.prim[2 * N + i]};
         FLITE_FOR_INC(L, i, t) {
             double v[4];
-            iterms(t, v);
-            iadd(v);
+            vflux_terms(L, t, ti, ui, v);
+            for (int c = 0; c < 4; ++c) acc[c] = acc[c] + v[c];
         }
-        for (int k = L.binc_ptr[i]; k < L.binc_ptr[i + 1]; ++k) {
-            double v[9];
-            bterms(k, v);
-            badd(v);
-        }
+        visc_flux_boundary(L, i, acc);
     }
     for (int c = 0; c < 4; ++c) L.diss[(1 + c) * N + i] = L.diss[(1 + c) * N + i] - acc[c];
 }
 
-// ---- fused walks of one incidence list (thread per node) -------------------
+// ---- fused walks of one incidence list --------------------------------------
 // Gathers that read the same neighbours and write disjoint arrays share one
 // walk of the node's incidence list: the incidences, their edges and the
 // neighbours' state are read once for both.  Each sum keeps its own
@@ -891,52 +947,74 @@ __global__ void __launch_bounds__(256, U == 1 ? 3 : 1) k_visc_flux(CaseArg<B, Pa
 // makeTimeSteps with passes 1-2 of makeArtificialDissipation2: the time
 // step reads mu of the neighbours (the previous viscous pass) and writes dt
 // and V/dt; the Laplacian reads u and p and writes the Laplacian and sensor
-template <bool B>
-__global__ void __launch_bounds__(256, 3) k_ts_lap(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_) {
+template <int U, bool B>
+__global__ void __launch_bounds__(256, U == 1 ? 3 : 1) k_ts_lap(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_) {
     FLITE_CASE_P(B, P, L);
     FLITE_CASE_L(B, L);
-    const int i = tid();
-    if (i >= L.N) return;
+    const int gl = U > 1 ? (int)(threadIdx.x % U) : 0;
+    const int i_raw = U > 1 ? tid() / U : tid();
+    if (U == 1 && i_raw >= L.N) return;
+    const bool active = i_raw < L.N;
+    const int i = active ? i_raw : L.N - 1;
     const int N = L.N;
     const double ui[5] = {L.u[i], L.u[N + i], L.u[2 * N + i], L.u[3 * N + i], L.u[4 * N + i]};
     const double pi = L.p[i];
     const double ro = 1. / ui[0];
     const double cc = dmax(P.gamma * pi * ro, 0.001);
-    double acc = 0.0, h = 0.0;
-    LapAcc a = {{0, 0, 0, 0, 0}, 0, 0};
-    FLITE_FOR_INC(L, i, t) {
-        ts_inc(P, L, t, ui[1], ui[2], ui[3], ro, cc, acc, h);
-        lap_inc(P, L, t, ui, pi, a);
+    if constexpr (U > 1) {
+        FLITE_GROUP_SLAB(double, 8);
+        lap_group<U>(P, L, i, active, gl, gs, ui, pi);
+        ts_group<U>(P, L, i, active, gl, gs, ui[1], ui[2], ui[3], ro, cc);
+    } else {
+        double acc = 0.0, h = 0.0;
+        LapAcc a = {{0, 0, 0, 0, 0}, 0, 0};
+        FLITE_FOR_INC(L, i, t) {
+            ts_inc(P, L, t, ui[1], ui[2], ui[3], ro, cc, acc, h);
+            lap_inc(P, L, t, ui, pi, a);
+        }
+        lap_store(L, i, a);
+        ts_finish(P, L, i, acc, h);
     }
-    lap_store(L, i, a);
-    ts_finish(P, L, i, acc, h);
 }
 
 // pass 3 of makeArtificialDissipation2 (scalar) with pass 1 of
 // makeViscosityTerm: the JST terms read the Laplacian, sensor, V/dt and u of
 // the neighbours and write the dissipation; the gradients read u, v, w, T
 // and write mu, the stress tensor and the wall stress
-template <bool B>
-__global__ void __launch_bounds__(256, 2) k_jflux_vgrad(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_) {
+template <int U, bool B>
+__global__ void __launch_bounds__(256, U == 1 ? 2 : 1) k_jflux_vgrad(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_) {
     FLITE_CASE_P(B, P, L);
     FLITE_CASE_L(B, L);
-    const int i = tid();
-    if (i >= L.N) return;
+    const int gl = U > 1 ? (int)(threadIdx.x % U) : 0;
+    const int i_raw = U > 1 ? tid() / U : tid();
+    if (U == 1 && i_raw >= L.N) return;
+    const bool active = i_raw < L.N;
+    const int i = active ? i_raw : L.N - 1;
     const int N = L.N;
-    const double k4 = L.grid == 1 ? P.k4 : P.cgdf;
-    double acc[5] = {0, 0, 0, 0, 0};
-    double Li[5], Ui[5];
-    for (int c = 0; c < 5; ++c) { Li[c] = L.lap[c * N + i]; Ui[c] = L.u[c * N + i]; }
-    const double vdi = L.vdt[i], coni = L.conn[i], si = L.sens[i];
-    const double qi[4] = {L.prim[i], L.prim[N + i], L.prim[2 * N + i], L.prim[3 * N + i]};
     double g[12];
-    for (int c = 0; c < 12; ++c) g[c] = 0.0;
-    FLITE_FOR_INC(L, i, t) {
-        jflux_inc(P, L, t, k4, vdi, coni, si, Li, Ui, acc);
-        vgrad_inc(L, t, qi, g);
+    if constexpr (U > 1) {
+        FLITE_GROUP_SLAB(double, 12);
+        double acc[5];
+        jflux_group<U>(P, L, L.u, i, active, gl, gs, acc);
+        if (active && gl == 0)
+            for (int c = 0; c < 5; ++c) L.diss[c * N + i] = acc[c];
+        vgrad_group<U>(L, i, active, gl, gs, g);
+        if (!active || gl) return;
+    } else {
+        const double k4 = L.grid == 1 ? P.k4 : P.cgdf;
+        double acc[5] = {0, 0, 0, 0, 0};
+        double Li[5], Ui[5];
+        for (int c = 0; c < 5; ++c) { Li[c] = L.lap[c * N + i]; Ui[c] = L.u[c * N + i]; }
+        const double vdi = L.vdt[i], coni = L.conn[i], si = L.sens[i];
+        const double qi[4] = {L.prim[i], L.prim[N + i], L.prim[2 * N + i], L.prim[3 * N + i]};
+        for (int c = 0; c < 12; ++c) g[c] = 0.0;
+        FLITE_FOR_INC(L, i, t) {
+            jflux_inc(P, L, t, k4, vdi, coni, si, Li, Ui, acc);
+            vgrad_inc(L, t, qi, g);
+        }
+        for (int c = 0; c < 5; ++c) L.diss[c * N + i] = acc[c];
+        visc_grad_boundary(L, i, g);
     }
-    for (int c = 0; c < 5; ++c) L.diss[c * N + i] = acc[c];
-    visc_grad_boundary(L, i, g);
     visc_grad_finish(P, L, i, g);
 }
 
@@ -1434,7 +1512,7 @@ __global__ void k_bnd_flux(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_) {
     int b = tid();
     if (b >= L.B) return;
     double g1[5], g2[5];
-    boundary_flux(P, L, b, g1, g2);
+    boundary_flux(P, L, b, [&](int j) { return load_state(L, j); }, g1, g2);
     double *o = L.bflux + (size_t)b * 10;
     for (int k = 0; k < 5; ++k) { o[k] = g1[k]; o[5 + k] = g2[k]; }
     if (L.bgterm) {
@@ -1462,36 +1540,114 @@ __global__ void k_bnd_flux(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_) {
 
 // the node's record for the increments: anchor primitives and u - ua (FP64
 // difference, rounded once), p - pa
+__device__ __forceinline__ void store_delta(const LevelView &L, DeltaRec *dq, int i, const double *u, double p) {
+    const int N = L.N;
+    DeltaRec o;
+    o.ra = L.a32[i]; o.vax = L.a32[N + i]; o.vay = L.a32[2 * N + i]; o.vaz = L.a32[3 * N + i];
+    o.ha = L.a32[4 * N + i];
+    o.dr = (float)(u[0] - L.ua[i]);
+    o.dmx = (float)(u[1] - L.ua[N + i]);
+    o.dmy = (float)(u[2] - L.ua[2 * N + i]);
+    o.dmz = (float)(u[3] - L.ua[3 * N + i]);
+    o.dE = (float)(u[4] - L.ua[4 * N + i]);
+    o.dp = (float)(p - L.pa[i]);
+    o.pad = 0.f;
+    float4 *d = reinterpret_cast<float4 *>(dq + i);
+    const float4 *v = reinterpret_cast<const float4 *>(&o);
+    d[0] = v[0]; d[1] = v[1]; d[2] = v[2];
+}
 template <bool B>
 __global__ void k_delta_state(CaseArg<B, LevelView> L_) {
     FLITE_CASE_L(B, L);
     int i = tid();
     if (i >= L.N) return;
     const int N = L.N;
-    DeltaRec o;
-    o.ra = L.a32[i]; o.vax = L.a32[N + i]; o.vay = L.a32[2 * N + i]; o.vaz = L.a32[3 * N + i];
-    o.ha = L.a32[4 * N + i];
-    o.dr = (float)(L.u[i] - L.ua[i]);
-    o.dmx = (float)(L.u[N + i] - L.ua[N + i]);
-    o.dmy = (float)(L.u[2 * N + i] - L.ua[2 * N + i]);
-    o.dmz = (float)(L.u[3 * N + i] - L.ua[3 * N + i]);
-    o.dE = (float)(L.u[4 * N + i] - L.ua[4 * N + i]);
-    o.dp = (float)(L.p[i] - L.pa[i]);
-    o.pad = 0.f;
-    float4 *p = reinterpret_cast<float4 *>(L.dq + i);
-    const float4 *d = reinterpret_cast<const float4 *>(&o);
-    p[0] = d[0]; p[1] = d[1]; p[2] = d[2];
+    const double u[5] = {L.u[i], L.u[N + i], L.u[2 * N + i], L.u[3 * N + i], L.u[4 * N + i]};
+    store_delta(L, L.dq, i, u, L.p[i]);
 }
 
 // the rows of a level from its incidence lists; entries past a node's
-// degree are the node itself with edge 0 (never used)
+// degree (never used) are the node itself as second node of edge 0
 __global__ void k_make_rows(LevelView L, int nrows, int2 *rows) {
     const int i = tid();
     if (i >= L.N) return;
     const int beg = L.inc_ptr[i], deg = L.inc_ptr[i + 1] - beg, s = i / kRow;
     const int first = L.row_ptr[s], last = (s + 1) * kRow < L.N ? L.row_ptr[s + 1] : nrows;
     for (int k = 0; k < last - first; ++k)
-        rows[(size_t)(first + k) * kRow + i % kRow] = k < deg ? L.inc[beg + k] : make_int2(0, i);
+        rows[(size_t)(first + k) * kRow + i % kRow] = k < deg ? L.inc[beg + k] : make_int2(~0, i);
+}
+// the device's edge numbers by rows: the number of edges whose first node
+// holds them in each row (a warp per row: kRow is the warp size), the first
+// number of each row, and each edge's; then the numbers put into the
+// incidences and the edges moved
+static_assert(kRow == 32, "a row is a warp");
+__global__ void k_row_firsts(const int2 *rows, int nrows, int *first) {
+    const int t = tid(), r = t / kRow;
+    if (r >= nrows) return;
+    const unsigned m = __ballot_sync(0xffffffffu, rows[t].x >= 0);
+    if (t % kRow == 0) first[r] = __popc(m);
+}
+// exclusive sums in place, one block
+__global__ void __launch_bounds__(1024) k_scan_rows(int *first, int nrows) {
+    __shared__ int part[32];
+    __shared__ int carry;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) carry = 0;
+    for (int base = 0; base < nrows; base += 1024) {
+        const int k = base + threadIdx.x;
+        const int own = k < nrows ? first[k] : 0;
+        int v = own;
+        for (int o = 1; o < 32; o *= 2) {
+            const int x = __shfl_up_sync(0xffffffffu, v, o);
+            if (lane >= o) v += x;
+        }
+        if (lane == 31) part[warp] = v;
+        __syncthreads();
+        if (warp == 0) {
+            int w = part[lane];
+            for (int o = 1; o < 32; o *= 2) {
+                const int x = __shfl_up_sync(0xffffffffu, w, o);
+                if (lane >= o) w += x;
+            }
+            part[lane] = w;
+        }
+        __syncthreads();
+        const int before = carry + (warp ? part[warp - 1] : 0) + v - own;
+        if (k < nrows) first[k] = before;
+        __syncthreads();
+        if (threadIdx.x == 0) carry += part[31];
+        __syncthreads();
+    }
+}
+__global__ void k_edge_slots(const int2 *rows, int nrows, const int *first, int *slot) {
+    const int t = tid(), r = t / kRow;
+    if (r >= nrows) return;
+    const int e = rows[t].x;
+    const unsigned m = __ballot_sync(0xffffffffu, e >= 0);
+    if (e >= 0) slot[e] = first[r] + __popc(m & ((1u << (t % kRow)) - 1u));
+}
+__global__ void k_renumber_edges(int2 *inc, int n, const int *slot) {
+    const int k = tid();
+    if (k >= n) return;
+    const int x = inc[k].x;
+    inc[k].x = x >= 0 ? slot[x] : ~slot[~x];
+}
+__global__ void k_move_edges(int E, const int *slot, const int2 *in, int2 *out) {
+    const int e = tid();
+    if (e < E) out[slot[e]] = in[e];
+}
+// edge arrays from the caller's edge order (w: [3][E])
+__global__ void k_put_edges(int E, const int *slot, const double *w, double *wx, double *wy, double *wz, EdgeW *ew) {
+    const int e = tid();
+    if (e >= E) return;
+    const int q = slot ? slot[e] : e;
+    const double x = w[e], y = w[(size_t)E + e], z = w[2 * (size_t)E + e];
+    wx[q] = x; wy[q] = y; wz[q] = z;
+    ew[q] = EdgeW{x, y, z, 0.0};
+}
+__global__ void k_put_edge_values(int E, const int *slot, const double *in, double *out) {
+    const int e = tid();
+    if (e < E) out[slot ? slot[e] : e] = in[e];
 }
 
 // FP32 incidences of the increments (w rounded once; j is ~j when the node
@@ -1529,13 +1685,13 @@ __device__ __forceinline__ void delta_flux(const DeltaRec &n, float wx, float wy
 // interior residual of node i as the anchor's FP64 sum plus the FP32 sum of
 // the flux increments of its edges
 template <int U>
-__device__ __forceinline__ void gather_interior_delta(const LevelView &L, int i, double *r, bool active, int gl,
-                                                      double *gs) {
+__device__ __forceinline__ void gather_interior_delta(const LevelView &L, const DeltaRec *dqin, int i, double *r,
+                                                      bool active, int gl, double *gs) {
     float acc[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
-    const DeltaRec me = load_delta(L.dq, i);
+    const DeltaRec me = load_delta(dqin, i);
     auto terms = [&](const IncRec32 &t, float *s5, bool &first) {
         first = t.j >= 0;
-        const DeltaRec nb = load_delta(L.dq, first ? t.j : ~t.j);
+        const DeltaRec nb = load_delta(dqin, first ? t.j : ~t.j);
         float g1[5], g2[5];
         delta_flux(first ? me : nb, t.wx, t.wy, t.wz, g1);
         delta_flux(first ? nb : me, t.wx, t.wy, t.wz, g2);
@@ -1589,18 +1745,18 @@ __device__ __forceinline__ void copy_ahead8(void *d, const void *g) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(d)), "l"(g)
                  : "memory");
 }
-__device__ __forceinline__ void gather_central_ahead(const LevelView &L, int i, double *r) {
+__device__ __forceinline__ void gather_central_ahead(const LevelView &L, const NodeRec *qin, int i, double *r) {
     __shared__ double2 sq[kPipe][3][kPipeThreads];
     __shared__ double sw[kPipe][3][kPipeThreads];
     const int tx = threadIdx.x;
     r[0] = r[1] = r[2] = r[3] = r[4] = 0.0;
     const int deg = L.inc_ptr[i + 1] - L.inc_ptr[i];
     const int2 *row = L.rows + ((size_t)L.row_ptr[i / kRow] * kRow + i % kRow);
-    const NodeRec si = load_node(L.q, i);
+    const NodeRec si = load_node(qin, i);
     int side[kPipe];
     auto issue = [&](const int2 t, int d) {
         const int e = t.x >= 0 ? t.x : ~t.x;
-        const double2 *q = reinterpret_cast<const double2 *>(L.q + t.y);
+        const double2 *q = reinterpret_cast<const double2 *>(qin + t.y);
         copy_ahead16(&sq[d][0][tx], q);
         copy_ahead16(&sq[d][1][tx], q + 1);
         copy_ahead16(&sq[d][2][tx], q + 2);
@@ -1653,16 +1809,16 @@ __device__ __forceinline__ void prefetch_rows(const LevelView &L) {
 
 // the same sums with a group of lanes per node
 template <int U>
-__device__ __forceinline__ void gather_interior_central(const LevelView &L, int i, double *r, bool active, int gl,
-                                                        double *gs) {
+__device__ __forceinline__ void gather_interior_central(const LevelView &L, const NodeRec *qin, int i, double *r,
+                                                        bool active, int gl, double *gs) {
     r[0] = r[1] = r[2] = r[3] = r[4] = 0.0;
-    const NodeRec si = load_node(L.q, i);
+    const NodeRec si = load_node(qin, i);
     group_sum<U, 5, 1, double>(
         gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl,
         [&](int k, double *g) {
             const int2 t = L.inc[k];
             const EdgeW w = load_edgew(L.ew, t.x >= 0 ? t.x : ~t.x);
-            const NodeRec n = load_node(L.q, t.y);
+            const NodeRec n = load_node(qin, t.y);
             if (t.x >= 0) {
                 central_flux_rec(si, n, w.wx, w.wy, w.wz, g);
             } else {  // this node's sign: x - y is x + (-y)
@@ -1772,6 +1928,31 @@ __device__ __forceinline__ void gather_boundary(const LevelView &L, int i, doubl
     }
 }
 
+// boundary edges of node i evaluated by its group (a static mesh's): lane by
+// lane, the edge's flux to this node from the states in uin and the pressures
+// of the records, the numbers k_bnd_flux leaves in bflux
+template <int U>
+__device__ __forceinline__ void gather_boundary_inline(const Params &P, const LevelView &L, const double *uin,
+                                                       const NodeRec *qin, int i, double *r, bool active, int gl,
+                                                       double *gs) {
+    const int N = L.N;
+    auto state = [&](int j) {
+        NodeState s;
+        s.r = uin[j]; s.ru = uin[N + j]; s.rv = uin[2 * N + j]; s.rw = uin[3 * N + j]; s.E = uin[4 * N + j];
+        s.p = qin[j].p;
+        return s;
+    };
+    group_sum<U, 5, 1, double>(
+        gs, L.binc_ptr[i], L.binc_ptr[i + 1], active, gl,
+        [&](int k, double *v) {
+            const int b = L.binc[k];
+            double g1[5], g2[5];
+            boundary_flux(P, L, b >> 1, state, g1, g2);
+            for (int c = 0; c < 5; ++c) v[c] = (b & 1) ? g2[c] : g1[c];
+        },
+        r);
+}
+
 // the FP64 evaluation becomes the new anchor of node i
 __device__ __forceinline__ void store_anchor(const LevelView &L, int i, const double *rint) {
     const int N = L.N;
@@ -1797,6 +1978,10 @@ __device__ __forceinline__ void store_anchor(const LevelView &L, int i, const do
 // one-step forms (modes as in k_node_update)
 // LEAN: a run without engine conditions and without explicit time stepping
 // (the branches for those are left out of the code)
+// the state a node pass reads
+__device__ __forceinline__ const double *io_in(const LevelView &L, int io) {
+    return (io & IO_UIN) == 0 ? L.u : (io & IO_UIN) == 1 ? L.uprev : L.ub;
+}
 struct TailIn {  // what the tail reads of its node, loaded ahead by the group gathers
     double diss[5], up[5], dt, V, p;
     unsigned char cls;
@@ -1811,16 +1996,19 @@ __device__ __forceinline__ TailIn load_tail(const LevelView &L, int i) {
     for (int c = 0; c < 5; ++c) { t.diss[c] = L.diss[c * N + i]; t.up[c] = L.uprev[c * N + i]; }
     return t;
 }
-template <bool LEAN = false>
-__device__ __forceinline__ void node_tail(const Params &P, const LevelView &L, int i, double *r, int mode,
-                                          int stage, const TailIn *in = nullptr) {
+// PREC names the records an IO_EMIT pass leaves for the next stage (none for
+// the edge buffer's fluxes)
+template <int PREC>
+__device__ __forceinline__ void node_tail(const Params &P, const LevelView &L, int i, double *r, int mode, int stage,
+                                          int io, const TailIn *in) {
+    constexpr bool LEAN = PREC == GATHER_LEAN;
     const int N = L.N;
     if (mode == MODE_RESID) {
         for (int c = 0; c < 5; ++c) L.rhs[c * N + i] = r[c];
         return;
     }
     if (P.addts && mode == MODE_STAGE)  // addTimeDifferences (def_par:1184-1241)
-        for (int c = 0; c < 5; ++c) r[c] = r[c] + time_difference(P, L, i, c);
+        for (int c = 0; c < 5; ++c) r[c] = r[c] + time_difference(P, L, io_in(L, io), i, c);
     for (int c = 0; c < 5; ++c) r[c] = r[c] + (in ? in->diss[c] : L.diss[c * N + i]);
     double dt = in ? in->dt : L.dt[i];
     const double V = in ? in->V : L.V[i];
@@ -1841,7 +2029,9 @@ __device__ __forceinline__ void node_tail(const Params &P, const LevelView &L, i
     if (mode == MODE_RFINE) {
         // the density floor of updateSolutionVector acts on grp%u, which is
         // not the array being updated in this call (def_par:1398-1403)
-        if (L.u[i] < P.minRho) L.u[i] = P.minRho;
+        // (IO_LATER: other lanes of this launch still read it; k_restrict_incr
+        // floors it)
+        if (!(io & IO_LATER) && L.u[i] < P.minRho) L.u[i] = P.minRho;
     } else {
         if (un[0] < P.minRho) un[0] = P.minRho;
     }
@@ -1862,21 +2052,31 @@ __device__ __forceinline__ void node_tail(const Params &P, const LevelView &L, i
         for (int c = 0; c < 5; ++c) T[c * N + i] = un[c];
         return;
     }
+    const double p_in = in ? in->p : L.p[i];
     if (mode == MODE_STAGE) {
         if (L.grid > 1) {
             const double a = P.RK[stage - 1];
             for (int c = 0; c < 5; ++c) un[c] = un[c] - a * L.src[c * N + i];
         }
         un[0] = dmax(un[0], P.minRho);  // limitDensity
-        bc_outer(P, cls, n0, n1, n2, L.p[i], un);
-        for (int c = 0; c < 5; ++c) L.u[c * N + i] = un[c];
+        bc_outer(P, cls, n0, n1, n2, p_in, un);
+        double *uo = io & IO_UOUT_B ? L.ub : L.u;
+        for (int c = 0; c < 5; ++c) uo[c * N + i] = un[c];
+        if (io & IO_EMIT) {  // makePressureField of the next stage
+            const double p = pressure(P, un[0], un[1], un[2], un[3], un[4]);
+            L.p[i] = p;
+            if constexpr (PREC == GATHER_ANCHOR || PREC == GATHER_DELTA)
+                store_delta(L, io & IO_REC_B ? L.dq : L.dqb, i, un, p);
+            else if constexpr (PREC != GATHER_BUFFER)
+                store_node(io & IO_REC_B ? L.q : L.qb, i, un[0], un[1], un[2], un[3], un[4], p);
+        }
     } else if (mode == MODE_RCOARSE) {
-        bc_outer(P, cls, n0, n1, n2, L.p[i], un);
+        bc_outer(P, cls, n0, n1, n2, p_in, un);
         for (int c = 0; c < 5; ++c) L.src[c * N + i] = un[c] - up[c];
     } else {  // MODE_RFINE
         if (L.grid > 1)
             for (int c = 0; c < 5; ++c) un[c] = un[c] - L.src[c * N + i];
-        bc_outer(P, cls, n0, n1, n2, L.p[i], un);
+        bc_outer(P, cls, n0, n1, n2, p_in, un);
         for (int c = 0; c < 5; ++c) L.rhs[c * N + i] = un[c] - up[c];
     }
 }
@@ -1890,9 +2090,10 @@ __device__ __forceinline__ void node_tail(const Params &P, const LevelView &L, i
 // GATHER_CENTRAL (central fluxes computed in the gather), GATHER_ANCHOR (the
 // same, stored as the new mixed-precision anchor), GATHER_DELTA (anchor +
 // FP32 increments)
-template <int PREC, int U, bool B>
-__global__ void __launch_bounds__(node_threads(PREC, U), U > 1 ? 1 : (central_ahead(PREC) ? 5 : 3))
-    k_node_update(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_, int mode, int stage) {
+template <int PREC, int U, int PRE, bool B>
+__global__ void __launch_bounds__(node_threads(PREC, U), U > 1 ? 2 : (central_ahead(PREC) ? 5 : 3))
+    k_node_update(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_, int mode, int stage, int io) {
+    static_assert(PRE == PRE_NONE || U > 1, "the dissipation part takes lanes per node");
     FLITE_CASE_P(B, P, L);
     FLITE_CASE_L(B, L);
     const int gl = U > 1 ? (int)(threadIdx.x % U) : 0;  // lane in the node's group
@@ -1906,146 +2107,81 @@ __global__ void __launch_bounds__(node_threads(PREC, U), U > 1 ? 1 : (central_ah
     // a node's own operands are read before the chain of its gather starts
     TailIn in;
     if constexpr (U > 1) in = load_tail(L, i);
+    if constexpr (PRE == PRE_JST) {
+        jflux_group<U>(P, L, io_in(L, io), i, active, gl, gs, in.diss);
+    } else if constexpr (PRE == PRE_VISC) {
+        double v[4];
+        vflux_group<U>(L, i, active, gl, gs, v);
+        for (int c = 0; c < 4; ++c) in.diss[1 + c] = in.diss[1 + c] - v[c];
+    }
+    if constexpr (PRE != PRE_NONE)
+        if (active && gl == 0)
+            for (int c = 0; c < 5; ++c) L.diss[c * L.N + i] = in.diss[c];
+    const NodeRec *qin = io & IO_REC_B ? L.qb : L.q;
     if constexpr (PREC == GATHER_DELTA) {
-        gather_interior_delta<U>(L, i, r, active, gl, gs);
+        gather_interior_delta<U>(L, io & IO_REC_B ? L.dqb : L.dq, i, r, active, gl, gs);
     } else if constexpr (PREC == GATHER_BUFFER) {
         gather_interior<U>(L, i, r, active, gl, gs);
     } else if constexpr (U == 1) {
-        gather_central_ahead(L, i, r);
+        gather_central_ahead(L, qin, i, r);
     } else {
-        gather_interior_central<U>(L, i, r, active, gl, gs);
+        gather_interior_central<U>(L, qin, i, r, active, gl, gs);
     }
     double rint[5];
     if constexpr (PREC == GATHER_ANCHOR)
         for (int c = 0; c < 5; ++c) rint[c] = r[c];
-    gather_boundary<U>(L, i, r, active, gl, gs);
+    if constexpr (U > 1 && PREC == GATHER_CENTRAL) {
+        if (io & IO_BND) gather_boundary_inline<U>(P, L, io_in(L, io), qin, i, r, active, gl, gs);
+        else gather_boundary<U>(L, i, r, active, gl, gs);
+    } else {
+        gather_boundary<U>(L, i, r, active, gl, gs);
+    }
     // with a group per node every lane holds the same sums; one lane goes on
     if constexpr (U > 1)
         if (!active || gl) return;
     if constexpr (PREC == GATHER_ANCHOR) store_anchor(L, i, rint);
-    node_tail<PREC == GATHER_LEAN>(P, L, i, r, mode, stage, U > 1 ? &in : nullptr);
+    node_tail<PREC>(P, L, i, r, mode, stage, io, U > 1 ? &in : nullptr);
 }
-template __global__ void k_node_update<GATHER_BUFFER, 1, false>(Params, LevelView, int, int);
-template __global__ void k_node_update<GATHER_BUFFER, 1, true>(CaseTab<Params>, CaseTab<LevelView>, int, int);
-template __global__ void k_node_update<GATHER_BUFFER, 4, false>(Params, LevelView, int, int);
-template __global__ void k_node_update<GATHER_BUFFER, 4, true>(CaseTab<Params>, CaseTab<LevelView>, int, int);
-template __global__ void k_node_update<GATHER_BUFFER, 8, false>(Params, LevelView, int, int);
-template __global__ void k_node_update<GATHER_BUFFER, 8, true>(CaseTab<Params>, CaseTab<LevelView>, int, int);
-template __global__ void k_node_update<GATHER_BUFFER, 16, false>(Params, LevelView, int, int);
-template __global__ void k_node_update<GATHER_BUFFER, 16, true>(CaseTab<Params>, CaseTab<LevelView>, int, int);
-template __global__ void k_node_update<GATHER_BUFFER, 32, false>(Params, LevelView, int, int);
-template __global__ void k_node_update<GATHER_BUFFER, 32, true>(CaseTab<Params>, CaseTab<LevelView>, int, int);
-template __global__ void k_node_update<GATHER_LEAN, 1, false>(Params, LevelView, int, int);
-template __global__ void k_node_update<GATHER_LEAN, 1, true>(CaseTab<Params>, CaseTab<LevelView>, int, int);
-template __global__ void k_node_update<GATHER_CENTRAL, 1, false>(Params, LevelView, int, int);
-template __global__ void k_node_update<GATHER_CENTRAL, 1, true>(CaseTab<Params>, CaseTab<LevelView>, int, int);
-template __global__ void k_node_update<GATHER_CENTRAL, 4, false>(Params, LevelView, int, int);
-template __global__ void k_node_update<GATHER_CENTRAL, 4, true>(CaseTab<Params>, CaseTab<LevelView>, int, int);
-template __global__ void k_node_update<GATHER_CENTRAL, 8, false>(Params, LevelView, int, int);
-template __global__ void k_node_update<GATHER_CENTRAL, 8, true>(CaseTab<Params>, CaseTab<LevelView>, int, int);
-template __global__ void k_node_update<GATHER_CENTRAL, 16, false>(Params, LevelView, int, int);
-template __global__ void k_node_update<GATHER_CENTRAL, 16, true>(CaseTab<Params>, CaseTab<LevelView>, int, int);
-template __global__ void k_node_update<GATHER_CENTRAL, 32, false>(Params, LevelView, int, int);
-template __global__ void k_node_update<GATHER_CENTRAL, 32, true>(CaseTab<Params>, CaseTab<LevelView>, int, int);
-template __global__ void k_node_update<GATHER_ANCHOR, 1, false>(Params, LevelView, int, int);
-template __global__ void k_node_update<GATHER_ANCHOR, 1, true>(CaseTab<Params>, CaseTab<LevelView>, int, int);
-template __global__ void k_node_update<GATHER_ANCHOR, 4, false>(Params, LevelView, int, int);
-template __global__ void k_node_update<GATHER_ANCHOR, 4, true>(CaseTab<Params>, CaseTab<LevelView>, int, int);
-template __global__ void k_node_update<GATHER_ANCHOR, 8, false>(Params, LevelView, int, int);
-template __global__ void k_node_update<GATHER_ANCHOR, 8, true>(CaseTab<Params>, CaseTab<LevelView>, int, int);
-template __global__ void k_node_update<GATHER_ANCHOR, 16, false>(Params, LevelView, int, int);
-template __global__ void k_node_update<GATHER_ANCHOR, 16, true>(CaseTab<Params>, CaseTab<LevelView>, int, int);
-template __global__ void k_node_update<GATHER_ANCHOR, 32, false>(Params, LevelView, int, int);
-template __global__ void k_node_update<GATHER_ANCHOR, 32, true>(CaseTab<Params>, CaseTab<LevelView>, int, int);
-template __global__ void k_node_update<GATHER_DELTA, 1, false>(Params, LevelView, int, int);
-template __global__ void k_node_update<GATHER_DELTA, 1, true>(CaseTab<Params>, CaseTab<LevelView>, int, int);
-template __global__ void k_node_update<GATHER_DELTA, 4, false>(Params, LevelView, int, int);
-template __global__ void k_node_update<GATHER_DELTA, 4, true>(CaseTab<Params>, CaseTab<LevelView>, int, int);
-template __global__ void k_node_update<GATHER_DELTA, 8, false>(Params, LevelView, int, int);
-template __global__ void k_node_update<GATHER_DELTA, 8, true>(CaseTab<Params>, CaseTab<LevelView>, int, int);
-template __global__ void k_node_update<GATHER_DELTA, 16, false>(Params, LevelView, int, int);
-template __global__ void k_node_update<GATHER_DELTA, 16, true>(CaseTab<Params>, CaseTab<LevelView>, int, int);
-template __global__ void k_node_update<GATHER_DELTA, 32, false>(Params, LevelView, int, int);
-template __global__ void k_node_update<GATHER_DELTA, 32, true>(CaseTab<Params>, CaseTab<LevelView>, int, int);
-template __global__ void k_timestep<1, false>(Params, LevelView);
-template __global__ void k_timestep<1, true>(CaseTab<Params>, CaseTab<LevelView>);
-template __global__ void k_timestep<4, false>(Params, LevelView);
-template __global__ void k_timestep<4, true>(CaseTab<Params>, CaseTab<LevelView>);
-template __global__ void k_timestep<8, false>(Params, LevelView);
-template __global__ void k_timestep<8, true>(CaseTab<Params>, CaseTab<LevelView>);
-template __global__ void k_timestep<16, false>(Params, LevelView);
-template __global__ void k_timestep<16, true>(CaseTab<Params>, CaseTab<LevelView>);
-template __global__ void k_timestep<32, false>(Params, LevelView);
-template __global__ void k_timestep<32, true>(CaseTab<Params>, CaseTab<LevelView>);
-template __global__ void k_jst_lap<1, false>(Params, LevelView);
-template __global__ void k_jst_lap<1, true>(CaseTab<Params>, CaseTab<LevelView>);
-template __global__ void k_jst_lap<4, false>(Params, LevelView);
-template __global__ void k_jst_lap<4, true>(CaseTab<Params>, CaseTab<LevelView>);
-template __global__ void k_jst_lap<8, false>(Params, LevelView);
-template __global__ void k_jst_lap<8, true>(CaseTab<Params>, CaseTab<LevelView>);
-template __global__ void k_jst_lap<16, false>(Params, LevelView);
-template __global__ void k_jst_lap<16, true>(CaseTab<Params>, CaseTab<LevelView>);
-template __global__ void k_jst_lap<32, false>(Params, LevelView);
-template __global__ void k_jst_lap<32, true>(CaseTab<Params>, CaseTab<LevelView>);
-template __global__ void k_jst_flux<1, false>(Params, LevelView);
-template __global__ void k_jst_flux<1, true>(CaseTab<Params>, CaseTab<LevelView>);
-template __global__ void k_jst_flux<4, false>(Params, LevelView);
-template __global__ void k_jst_flux<4, true>(CaseTab<Params>, CaseTab<LevelView>);
-template __global__ void k_jst_flux<8, false>(Params, LevelView);
-template __global__ void k_jst_flux<8, true>(CaseTab<Params>, CaseTab<LevelView>);
-template __global__ void k_jst_flux<16, false>(Params, LevelView);
-template __global__ void k_jst_flux<16, true>(CaseTab<Params>, CaseTab<LevelView>);
-template __global__ void k_jst_flux<32, false>(Params, LevelView);
-template __global__ void k_jst_flux<32, true>(CaseTab<Params>, CaseTab<LevelView>);
-template __global__ void k_visc_grad<1, false>(Params, LevelView);
-template __global__ void k_visc_grad<1, true>(CaseTab<Params>, CaseTab<LevelView>);
-template __global__ void k_visc_grad<4, false>(Params, LevelView);
-template __global__ void k_visc_grad<4, true>(CaseTab<Params>, CaseTab<LevelView>);
-template __global__ void k_visc_grad<8, false>(Params, LevelView);
-template __global__ void k_visc_grad<8, true>(CaseTab<Params>, CaseTab<LevelView>);
-template __global__ void k_visc_grad<16, false>(Params, LevelView);
-template __global__ void k_visc_grad<16, true>(CaseTab<Params>, CaseTab<LevelView>);
-template __global__ void k_visc_grad<32, false>(Params, LevelView);
-template __global__ void k_visc_grad<32, true>(CaseTab<Params>, CaseTab<LevelView>);
-template __global__ void k_visc2_grad<1, false>(Params, LevelView);
-template __global__ void k_visc2_grad<1, true>(CaseTab<Params>, CaseTab<LevelView>);
-template __global__ void k_visc2_grad<4, false>(Params, LevelView);
-template __global__ void k_visc2_grad<4, true>(CaseTab<Params>, CaseTab<LevelView>);
-template __global__ void k_visc2_grad<8, false>(Params, LevelView);
-template __global__ void k_visc2_grad<8, true>(CaseTab<Params>, CaseTab<LevelView>);
-template __global__ void k_visc2_grad<16, false>(Params, LevelView);
-template __global__ void k_visc2_grad<16, true>(CaseTab<Params>, CaseTab<LevelView>);
-template __global__ void k_visc2_grad<32, false>(Params, LevelView);
-template __global__ void k_visc2_grad<32, true>(CaseTab<Params>, CaseTab<LevelView>);
-template __global__ void k_visc2_flux<1, false>(Params, LevelView);
-template __global__ void k_visc2_flux<1, true>(CaseTab<Params>, CaseTab<LevelView>);
-template __global__ void k_visc2_flux<4, false>(Params, LevelView);
-template __global__ void k_visc2_flux<4, true>(CaseTab<Params>, CaseTab<LevelView>);
-template __global__ void k_visc2_flux<8, false>(Params, LevelView);
-template __global__ void k_visc2_flux<8, true>(CaseTab<Params>, CaseTab<LevelView>);
-template __global__ void k_visc2_flux<16, false>(Params, LevelView);
-template __global__ void k_visc2_flux<16, true>(CaseTab<Params>, CaseTab<LevelView>);
-template __global__ void k_visc2_flux<32, false>(Params, LevelView);
-template __global__ void k_visc2_flux<32, true>(CaseTab<Params>, CaseTab<LevelView>);
-template __global__ void k_visc_flux<1, false>(Params, LevelView);
-template __global__ void k_visc_flux<1, true>(CaseTab<Params>, CaseTab<LevelView>);
-template __global__ void k_visc_flux<4, false>(Params, LevelView);
-template __global__ void k_visc_flux<4, true>(CaseTab<Params>, CaseTab<LevelView>);
-template __global__ void k_visc_flux<8, false>(Params, LevelView);
-template __global__ void k_visc_flux<8, true>(CaseTab<Params>, CaseTab<LevelView>);
-template __global__ void k_visc_flux<16, false>(Params, LevelView);
-template __global__ void k_visc_flux<16, true>(CaseTab<Params>, CaseTab<LevelView>);
-template __global__ void k_visc_flux<32, false>(Params, LevelView);
-template __global__ void k_visc_flux<32, true>(CaseTab<Params>, CaseTab<LevelView>);
+#define FLITE_BOTH(kern, targs, ...)                                               \
+    template __global__ void kern<FLITE_ARGS targs false> FLITE_SINGLE(__VA_ARGS__); \
+    template __global__ void kern<FLITE_ARGS targs true> FLITE_GROUPED(__VA_ARGS__);
+#define FLITE_ARGS(...) __VA_ARGS__
+#define FLITE_SINGLE(...) (Params, LevelView __VA_ARGS__)
+#define FLITE_GROUPED(...) (CaseTab<Params>, CaseTab<LevelView> __VA_ARGS__)
+#define FLITE_NODE_INST(PREC, U, PRE)                                                                          \
+    template __global__ void k_node_update<PREC, U, PRE, false>(Params, LevelView, int, int, int);              \
+    template __global__ void k_node_update<PREC, U, PRE, true>(CaseTab<Params>, CaseTab<LevelView>, int, int, int);
+#define FLITE_GATHER_INST(U)                                                                 \
+    FLITE_BOTH(k_timestep, (U, ))                                                            \
+    FLITE_BOTH(k_jst_lap, (U, ))                                                             \
+    FLITE_BOTH(k_jst_flux, (U, ))                                                            \
+    FLITE_BOTH(k_visc_grad, (U, ))                                                           \
+    FLITE_BOTH(k_visc_flux, (U, ))                                                           \
+    FLITE_BOTH(k_visc2_grad, (U, ))                                                          \
+    FLITE_BOTH(k_visc2_flux, (U, ))                                                          \
+    FLITE_BOTH(k_ts_lap, (U, ))                                                              \
+    FLITE_BOTH(k_jflux_vgrad, (U, ))                                                         \
+    FLITE_NODE_INST(GATHER_BUFFER, U, PRE_NONE)                                              \
+    FLITE_NODE_INST(GATHER_CENTRAL, U, PRE_NONE)                                             \
+    FLITE_NODE_INST(GATHER_ANCHOR, U, PRE_NONE)                                              \
+    FLITE_NODE_INST(GATHER_DELTA, U, PRE_NONE)
+#define FLITE_GROUP_INST(U)                          \
+    FLITE_GATHER_INST(U)                             \
+    FLITE_NODE_INST(GATHER_CENTRAL, U, PRE_JST)      \
+    FLITE_NODE_INST(GATHER_CENTRAL, U, PRE_VISC)
+FLITE_GATHER_INST(1)
+FLITE_NODE_INST(GATHER_LEAN, 1, PRE_NONE)
+FLITE_GROUP_INST(4)
+FLITE_GROUP_INST(8)
+FLITE_GROUP_INST(16)
+FLITE_GROUP_INST(32)
 template __global__ void k_first_order_diss<1>(Params, LevelView);
-template __global__ void k_pressure<false>(Params, LevelView);
-template __global__ void k_pressure<true>(CaseTab<Params>, CaseTab<LevelView>);
-template __global__ void k_visc_prim<false>(Params, LevelView);
-template __global__ void k_visc_prim<true>(CaseTab<Params>, CaseTab<LevelView>);
-template __global__ void k_ts_lap<false>(Params, LevelView);
-template __global__ void k_ts_lap<true>(CaseTab<Params>, CaseTab<LevelView>);
-template __global__ void k_jflux_vgrad<false>(Params, LevelView);
-template __global__ void k_jflux_vgrad<true>(CaseTab<Params>, CaseTab<LevelView>);
+template __global__ void k_state_pass<false, false>(Params, LevelView, int, const int *);
+template __global__ void k_state_pass<false, true>(CaseTab<Params>, CaseTab<LevelView>, int, const int *);
+template __global__ void k_state_pass<true, false>(Params, LevelView, int, const int *);
+template __global__ void k_state_pass<true, true>(CaseTab<Params>, CaseTab<LevelView>, int, const int *);
+template __global__ void k_prolong<false>(Params, LevelView, LevelView);
+template __global__ void k_prolong<true>(CaseTab<Params>, CaseTab<LevelView>, CaseTab<LevelView>);
 template __global__ void k_bnd_flux<false>(Params, LevelView);
 template __global__ void k_bnd_flux<true>(CaseTab<Params>, CaseTab<LevelView>);
 template __global__ void k_delta_state<false>(LevelView);
@@ -2054,8 +2190,8 @@ template __global__ void k_restrict_u<false>(LevelView, LevelView);
 template __global__ void k_restrict_u<true>(CaseTab<LevelView>, CaseTab<LevelView>);
 template __global__ void k_restrict_state<false>(Params, LevelView, LevelView);
 template __global__ void k_restrict_state<true>(CaseTab<Params>, CaseTab<LevelView>, CaseTab<LevelView>);
-template __global__ void k_restrict_incr<false>(Params, LevelView, LevelView);
-template __global__ void k_restrict_incr<true>(CaseTab<Params>, CaseTab<LevelView>, CaseTab<LevelView>);
+template __global__ void k_restrict_incr<false>(Params, LevelView, LevelView, int);
+template __global__ void k_restrict_incr<true>(CaseTab<Params>, CaseTab<LevelView>, CaseTab<LevelView>, int);
 template __global__ void k_prolong_coarse<false>(Params, LevelView, LevelView);
 template __global__ void k_prolong_coarse<true>(CaseTab<Params>, CaseTab<LevelView>, CaseTab<LevelView>);
 template __global__ void k_prolong_fine<false>(Params, LevelView, LevelView);
@@ -2071,36 +2207,62 @@ __global__ void k_copy(const double *a, double *b, size_t n) {
 
 // mapFineToCoarse (def_par:12572-12596) as a gather over each coarse node's
 // children in increasing fine order: the same additions in the same order as
-// the reference's scatter over fine nodes
-__device__ __forceinline__ void restrict_gather(const LevelView &C, const double *fine, int nf, int c, int ncomp,
-                                                double *out) {
-    for (int k = 0; k < ncomp; ++k) out[k] = 0.0;
-    for (int q = C.child_ptr[c]; q < C.child_ptr[c + 1]; ++q) {
-        int f = C.child[q];
-        double w = C.rweight[f];
-        for (int k = 0; k < ncomp; ++k) out[k] = out[k] + w * fine[(size_t)k * nf + f];
-    }
+// the reference's scatter over fine nodes.  kChildLanes lanes take a coarse
+// node's children (8 to 9 on the agglomerated levels) and add the sums'
+// terms as group_sum does: with a thread per coarse node the transfers of the
+// 203,401-node mesh take 15 to 23 us each, bound by one thread's chain of
+// child -> value loads.
+template <int M>
+__device__ __forceinline__ void restrict_group(const LevelView &C, int c, bool active, int gl, double *gs,
+                                               const double *const (&fine)[M], double *out) {
+#pragma unroll
+    for (int k = 0; k < M; ++k) out[k] = 0.0;
+    group_sum<kChildLanes, M, 1, double>(
+        gs, C.child_ptr[c], C.child_ptr[c + 1], active, gl,
+        [&](int q, double *v) {
+            const int f = C.child[q];
+            const double w = C.rweight[f];
+#pragma unroll
+            for (int k = 0; k < M; ++k) v[k] = w * fine[k][f];
+        },
+        out);
 }
+// the coarse node and lane of a transfer kernel's thread
+#define FLITE_CHILD_LANES(M)                                                          \
+    constexpr int U = kChildLanes;                                                     \
+    FLITE_GROUP_SLAB(double, M);                                                       \
+    const int gl = (int)(threadIdx.x % U), c_raw = tid() / U;                          \
+    const bool active = c_raw < C.N;                                                   \
+    const int c = active ? c_raw : C.N - 1
 
 // C.u = R(F.u) (plain mapFineToCoarse of the solution)
 template <bool B>
 __global__ void k_restrict_u(CaseArg<B, LevelView> C_, CaseArg<B, LevelView> F_) {
     FLITE_CASE_L(B, C);
     FLITE_CASE_L(B, F);
-    int c = tid();
-    if (c >= C.N) return;
+    FLITE_CHILD_LANES(6);
+    const size_t n = F.N;
+    // (without nu~ the sixth sum repeats the first and is dropped)
+    const double *const src[6] = {F.u, F.u + n, F.u + 2 * n, F.u + 3 * n, F.u + 4 * n, C.nvar == 6 ? F.u + 5 * n : F.u};
     double v[6];
-    restrict_gather(C, F.u, F.N, c, C.nvar, v);
-    for (int k = 0; k < C.nvar; ++k) C.u[k * C.N + c] = v[k];
+    restrict_group<6>(C, c, active, gl, gs, src, v);
+    if (!active || gl) return;
+    for (int k = 0; k < 5; ++k) C.u[k * C.N + c] = v[k];
+    if (C.nvar == 6) C.u[5 * C.N + c] = v[5];
 }
 
 // mapFineToCoarse of another array (def_par:12572-12679)
 __global__ void k_restrict_arr(LevelView C, LevelView F, const double *fsrc, double *cdst, int ncomp) {
     int c = tid();
     if (c >= C.N) return;
-    double v[6];
-    restrict_gather(C, fsrc, F.N, c, ncomp, v);
-    for (int k = 0; k < ncomp; ++k) cdst[k * C.N + c] = v[k];
+    for (int k = 0; k < ncomp; ++k) {
+        double v = 0.0;
+        for (int q = C.child_ptr[c]; q < C.child_ptr[c + 1]; ++q) {
+            const int f = C.child[q];
+            v = v + C.rweight[f] * fsrc[(size_t)k * F.N + f];
+        }
+        cdst[k * C.N + c] = v;
+    }
 }
 
 // the nu~ solution conditions: zero on walls (def_par:4416-4418, 4446-4448,
@@ -2126,13 +2288,14 @@ __global__ void k_restrict_state(CaseArg<B, Params> P_, CaseArg<B, LevelView> C_
     FLITE_CASE_P(B, P, C);
     FLITE_CASE_L(B, C);
     FLITE_CASE_L(B, F);
-    int c = tid();
-    if (c >= C.N) return;
+    FLITE_CHILD_LANES(7);
     const int N = C.N;
-    double v[5], m;
-    restrict_gather(C, F.u, F.N, c, 5, v);
-    restrict_gather(C, F.mu, F.N, c, 1, &m);
-    C.mu[c] = m;
+    const size_t n = F.N;
+    const double *const src[7] = {F.u, F.u + n, F.u + 2 * n, F.u + 3 * n, F.u + 4 * n, F.mu, P.sa ? F.u + 5 * n : F.u};
+    double v[7];
+    restrict_group<7>(C, c, active, gl, gs, src, v);
+    if (!active || gl) return;
+    C.mu[c] = v[5];
     double p0 = pressure(P, v[0], v[1], v[2], v[3], v[4]);
     const unsigned char cls = C.bc[c];
     double n0 = 0, n1 = 0, n2 = 0;
@@ -2143,28 +2306,44 @@ __global__ void k_restrict_state(CaseArg<B, Params> P_, CaseArg<B, LevelView> C_
     bc_outer(P, cls, n0, n1, n2, p0, v);
     for (int k = 0; k < 5; ++k) { C.u[k * N + c] = v[k]; C.uprev[k * N + c] = v[k]; }
     if (P.sa) {
-        double t;
-        restrict_gather(C, F.u + 5 * (size_t)F.N, F.N, c, 1, &t);
-        t = sa_bc_solution(P, cls, rp, t);
+        const double t = sa_bc_solution(P, cls, rp, v[6]);
         C.u[5 * N + c] = t;
         C.uprev[5 * N + c] = t;
     }
-    C.p[c] = fabs(pressure(P, v[0], v[1], v[2], v[3], v[4]));
-    store_node(C.q, c, v[0], v[1], v[2], v[3], v[4], C.p[c]);
+    const double p = fabs(pressure(P, v[0], v[1], v[2], v[3], v[4]));
+    C.p[c] = p;
+    store_node(C.q, c, v[0], v[1], v[2], v[3], v[4], p);
+    if (C.prim) {  // the viscous primitives (k_state_pass)
+        const double gOg = P.gamma / (P.gamma - 1.0);
+        C.prim[c] = v[1] / v[0];
+        C.prim[N + c] = v[2] / v[0];
+        C.prim[2 * N + c] = v[3] / v[0];
+        C.prim[3 * N + c] = gOg * p / v[0];
+    }
 }
 
 // restrictGrid tail (def_par:12385-12427): C.rhs = R(F.rhs), increment
 // conditions, src -= rhs, u += rhs
 template <bool B>
-__global__ void k_restrict_incr(CaseArg<B, Params> P_, CaseArg<B, LevelView> C_, CaseArg<B, LevelView> F_) {
+__global__ void k_restrict_incr(CaseArg<B, Params> P_, CaseArg<B, LevelView> C_, CaseArg<B, LevelView> F_,
+                                int floor_fine) {
     FLITE_CASE_P(B, P, C);
     FLITE_CASE_L(B, C);
     FLITE_CASE_L(B, F);
-    int c = tid();
-    if (c >= C.N) return;
+    FLITE_CHILD_LANES(6);
     const int N = C.N;
-    double r[5];
-    restrict_gather(C, F.rhs, F.N, c, 5, r);
+    // the density floor that the fine node pass left (IO_LATER)
+    if (floor_fine && active)
+        for (int q = C.child_ptr[c] + gl; q < C.child_ptr[c + 1]; q += U) {
+            const int f = C.child[q];
+            if (F.u[f] < P.minRho) F.u[f] = P.minRho;
+        }
+    const size_t n = F.N;
+    const double *const in[6] = {F.rhs,         F.rhs + n,     F.rhs + 2 * n,
+                                 F.rhs + 3 * n, F.rhs + 4 * n, P.sa ? F.rhs + 5 * n : F.rhs};
+    double r[6];
+    restrict_group<6>(C, c, active, gl, gs, in, r);
+    if (!active || gl) return;
     const unsigned char cls = C.bc[c];
     double n0 = 0, n1 = 0, n2 = 0;
     if (cls != BC_NONE) { n0 = C.nx[c]; n1 = C.ny[c]; n2 = C.nz[c]; }
@@ -2175,9 +2354,7 @@ __global__ void k_restrict_incr(CaseArg<B, Params> P_, CaseArg<B, LevelView> C_,
         C.u[k * N + c] = C.u[k * N + c] + r[k];
     }
     if (P.sa) {
-        double t;
-        restrict_gather(C, F.rhs + 5 * (size_t)F.N, F.N, c, 1, &t);
-        t = sa_bc_increment(P, cls, t);
+        const double t = sa_bc_increment(P, cls, r[5]);
         C.rhs[5 * N + c] = t;
         C.src[5 * N + c] = C.src[5 * N + c] - t;
         C.u[5 * N + c] = C.u[5 * N + c] + t;
@@ -2186,16 +2363,10 @@ __global__ void k_restrict_incr(CaseArg<B, Params> P_, CaseArg<B, LevelView> C_,
 
 // prolongateGrid coarse part (def_par:12445-12468): uprev = R(F.u) with the
 // solution conditions, rhs = u - uprev with the increment conditions
-template <bool B>
-__global__ void k_prolong_coarse(CaseArg<B, Params> P_, CaseArg<B, LevelView> C_, CaseArg<B, LevelView> F_) {
-    FLITE_CASE_P(B, P, C);
-    FLITE_CASE_L(B, C);
-    FLITE_CASE_L(B, F);
-    int c = tid();
-    if (c >= C.N) return;
+// v: the restricted solution (and nu~); r: the correction (and nu~'s)
+__device__ __forceinline__ void prolong_coarse(const Params &P, const LevelView &C, int c, double *v, double *r,
+                                               bool store) {
     const int N = C.N;
-    double v[5];
-    restrict_gather(C, F.u, F.N, c, 5, v);
     const unsigned char cls = C.bc[c];
     double n0 = 0, n1 = 0, n2 = 0;
     if (cls != BC_NONE) { n0 = C.nx[c]; n1 = C.ny[c]; n2 = C.nz[c]; }
@@ -2203,45 +2374,50 @@ __global__ void k_prolong_coarse(CaseArg<B, Params> P_, CaseArg<B, LevelView> C_
     const double rp = eo_relax(P, *C.cyc);
     if (is_exhaust(cls)) bc_exhaust(P, cls, rp, v);
     bc_outer(P, cls, n0, n1, n2, C.p[c], v);
-    double r[5];
     for (int k = 0; k < 5; ++k) {
-        C.uprev[k * N + c] = v[k];
+        if (store) C.uprev[k * N + c] = v[k];
         r[k] = C.u[k * N + c] - v[k];
     }
     double r6 = 0.0;
     if (P.sa) {
-        double t;
-        restrict_gather(C, F.u + 5 * (size_t)F.N, F.N, c, 1, &t);
-        t = sa_bc_solution(P, cls, rp, t);
-        C.uprev[5 * N + c] = t;
+        const double t = sa_bc_solution(P, cls, rp, v[5]);
+        if (store) C.uprev[5 * N + c] = t;
         r6 = C.u[5 * N + c] - t;
         // nullifyOuterBoundary, then the increment conditions
         if (cls == BC_FAR3 || is_engine(cls)) { r[0] = r[1] = r[2] = r[3] = r[4] = 0.0; r6 = 0.0; }
         r6 = sa_bc_increment(P, cls, r6);
     }
     bc_increment(P, cls, n0, n1, n2, r);
+    r[5] = r6;
+    if (!store) return;
     for (int k = 0; k < 5; ++k) C.rhs[k * N + c] = r[k];
     if (P.sa) C.rhs[5 * N + c] = r6;
+}
+template <bool B>
+__global__ void k_prolong_coarse(CaseArg<B, Params> P_, CaseArg<B, LevelView> C_, CaseArg<B, LevelView> F_) {
+    FLITE_CASE_P(B, P, C);
+    FLITE_CASE_L(B, C);
+    FLITE_CASE_L(B, F);
+    FLITE_CHILD_LANES(6);
+    const size_t n = F.N;
+    const double *const src[6] = {F.u, F.u + n, F.u + 2 * n, F.u + 3 * n, F.u + 4 * n, P.sa ? F.u + 5 * n : F.u};
+    double v[6], r[6];
+    restrict_group<6>(C, c, active, gl, gs, src, v);
+    if (active && gl == 0) prolong_coarse(P, C, c, v, r, true);
 }
 
 // prolongateGrid fine part (def_par:12470-12567): injection, relaxation,
 // u += correction, boundary conditions, floors
-template <bool B>
-__global__ void k_prolong_fine(CaseArg<B, Params> P_, CaseArg<B, LevelView> C_, CaseArg<B, LevelView> F_) {
-    FLITE_CASE_P(B, P, C);
-    FLITE_CASE_L(B, C);
-    FLITE_CASE_L(B, F);
-    int i = tid();
-    if (i >= F.N) return;
+// corr: the parent's correction (and nu~'s)
+__device__ __forceinline__ void prolong_fine(const Params &P, const LevelView &F, int i, const double *corr) {
     const int N = F.N;
-    int pc = C.parent[i];
     const unsigned char cls = F.bc[i];
     // nullifyOuterBoundary of the injected correction (SA runs only)
     const bool nul = P.sa && (cls == BC_FAR3 || is_engine(cls));
     double un[5];
     for (int k = 0; k < 5; ++k) un[k] = F.u[k * N + i];
     for (int k = 0; k < 5; ++k) {
-        double r = pc >= 0 ? C.rhs[k * C.N + pc] : F.rhs[k * N + i];
+        double r = corr[k];
         if (nul) r = 0.0;
         r = P.prolRelax * r;
         if (i < F.Nb) r = P.mgBCRelax * r;
@@ -2250,7 +2426,7 @@ __global__ void k_prolong_fine(CaseArg<B, Params> P_, CaseArg<B, LevelView> C_, 
     }
     double un6 = 0.0;
     if (P.sa) {
-        double r = pc >= 0 ? C.rhs[5 * C.N + pc] : F.rhs[5 * N + i];
+        double r = corr[5];
         if (nul) r = 0.0;
         r = P.turbProlRelax * r;
         F.rhs[5 * N + i] = r;
@@ -2278,6 +2454,36 @@ __global__ void k_prolong_fine(CaseArg<B, Params> P_, CaseArg<B, LevelView> C_, 
     bc_outer(P, cls, n0, n1, n2, F.p[i], un);
     un[0] = dmax(un[0], P.minRho);
     for (int k = 0; k < 5; ++k) F.u[k * N + i] = un[k];
+}
+template <bool B>
+__global__ void k_prolong_fine(CaseArg<B, Params> P_, CaseArg<B, LevelView> C_, CaseArg<B, LevelView> F_) {
+    FLITE_CASE_P(B, P, C);
+    FLITE_CASE_L(B, C);
+    FLITE_CASE_L(B, F);
+    const int i = tid();
+    if (i >= F.N) return;
+    const int pc = C.parent[i];
+    double corr[6] = {0, 0, 0, 0, 0, 0};
+    for (int k = 0; k < F.nvar; ++k) corr[k] = pc >= 0 ? C.rhs[k * C.N + pc] : F.rhs[k * F.N + i];
+    prolong_fine(P, F, i, corr);
+}
+// both parts in one launch where every fine node has a parent: a coarse
+// node's lanes gather its children for the coarse part, then correct them.
+// No other group reads or writes these children.
+template <bool B>
+__global__ void k_prolong(CaseArg<B, Params> P_, CaseArg<B, LevelView> C_, CaseArg<B, LevelView> F_) {
+    FLITE_CASE_P(B, P, C);
+    FLITE_CASE_L(B, C);
+    FLITE_CASE_L(B, F);
+    FLITE_CHILD_LANES(6);
+    const size_t n = F.N;
+    const double *const src[6] = {F.u, F.u + n, F.u + 2 * n, F.u + 3 * n, F.u + 4 * n, P.sa ? F.u + 5 * n : F.u};
+    double v[6], r[6];
+    restrict_group<6>(C, c, active, gl, gs, src, v);
+    if (!active) return;
+    // every lane forms the correction; one stores the coarse arrays
+    prolong_coarse(P, C, c, v, r, gl == 0);
+    for (int q = C.child_ptr[c] + gl; q < C.child_ptr[c + 1]; q += U) prolong_fine(P, F, C.child[q], r);
 }
 
 // mapCoarseToFine of the solution (injection, def_par:12694-12700)

@@ -9,8 +9,13 @@ namespace flite {
 // and the start-up conditions for the engine pass that follows them
 enum { MODE_STAGE = 0, MODE_RCOARSE = 1, MODE_RFINE = 2, MODE_RESID = 3, MODE_PROLONG = 4, MODE_START = 5 };
 
-template <bool B = false>
-__global__ void k_pressure(CaseArg<B, Params> P, CaseArg<B, LevelView> L);
+// the pass over a level's state before its gathers: pressure and node records
+// (STATE_REC), with STATE_PRIM the viscous primitives, with STATE_STEP the
+// start of a relaxation step (cycle number from src, uprev = u); BND adds the
+// boundary edges' fluxes (threads N.. of the grid, one edge each)
+enum { STATE_PRIM = 1, STATE_STEP = 2, STATE_REC = 4 };
+template <bool BND, bool B = false>
+__global__ void k_state_pass(CaseArg<B, Params> P, CaseArg<B, LevelView> L, int what, const int *src);
 template <int U, bool B = false>
 __global__ void k_timestep(CaseArg<B, Params> P, CaseArg<B, LevelView> L);
 template <int U, bool B = false>
@@ -19,15 +24,13 @@ template <int U, bool B = false>
 __global__ void k_jst_flux(CaseArg<B, Params> P, CaseArg<B, LevelView> L);
 template <int U>
 __global__ void k_first_order_diss(Params P, LevelView L);
-template <bool B = false>
-__global__ void k_visc_prim(CaseArg<B, Params> P, CaseArg<B, LevelView> L);
 template <int U, bool B = false>
 __global__ void k_visc_grad(CaseArg<B, Params> P, CaseArg<B, LevelView> L);
 template <int U, bool B = false>
 __global__ void k_visc_flux(CaseArg<B, Params> P, CaseArg<B, LevelView> L);
-template <bool B = false>
+template <int U, bool B = false>
 __global__ void k_ts_lap(CaseArg<B, Params> P, CaseArg<B, LevelView> L);
-template <bool B = false>
+template <int U, bool B = false>
 __global__ void k_jflux_vgrad(CaseArg<B, Params> P, CaseArg<B, LevelView> L);
 template <int U, bool B = false>
 __global__ void k_visc2_grad(CaseArg<B, Params> P, CaseArg<B, LevelView> L);
@@ -55,8 +58,32 @@ enum { GATHER_BUFFER = 0, GATHER_CENTRAL = 1, GATHER_ANCHOR = 2, GATHER_DELTA = 
 // 128 threads
 constexpr bool central_ahead(int prec) { return prec == GATHER_CENTRAL || prec == GATHER_ANCHOR || prec == GATHER_LEAN; }
 constexpr int node_threads(int prec, int u) { return u == 1 && central_ahead(prec) ? 128 : 256; }
-template <int PREC, int U, bool B = false>
-__global__ void k_node_update(CaseArg<B, Params> P, CaseArg<B, LevelView> L, int mode, int stage);
+// What a node pass computes of the dissipation before its residual (lanes per
+// node only): nothing, the scalar JST flux, or the viscous fluxes, both
+// otherwise their own launches
+enum { PRE_NONE = 0, PRE_JST = 1, PRE_VISC = 2 };
+// Which copies of the state a node pass reads and writes (a word of flags).
+// The stages of a step alternate them, so that a stage can write its node's
+// new state, pressure and records in the launch whose other nodes still read
+// the old ones: no pressure pass between the stages, and with lanes per node
+// (which evaluate the boundary edges themselves, IO_BND) one launch a stage.
+//   stage    1               2            3            (4 as 2, 5 as 3)
+//   u        uprev -> u      u -> ub      ub -> u      with IO_BND, else u -> u
+//   records  q -> qb         qb -> q      q            (none after the last)
+enum {
+    IO_UIN = 3,      // 0 u, 1 uprev, 2 ub
+    IO_UOUT_B = 4,   // the new state goes to ub, else to u
+    IO_REC_B = 8,    // records read from qb (dqb), else from q (dq)
+    IO_EMIT = 16,    // the new pressure, and the records to the other copy
+    IO_BND = 32,     // boundary edges evaluated in the pass, else from bflux
+    IO_LATER = 64    // restrictGrid's fine pass leaves the density floor to k_restrict_incr
+};
+constexpr int stage_io(int stage, int nstage, bool bnd, bool emit) {
+    return (bnd ? (stage == 1 ? 1 : stage % 2 ? 2 : 0) | (stage % 2 ? 0 : IO_UOUT_B) | IO_BND : 0) |
+           (emit ? (stage % 2 ? 0 : IO_REC_B) | (stage < nstage ? IO_EMIT : 0) : 0);
+}
+template <int PREC, int U, int PRE = PRE_NONE, bool B = false>
+__global__ void k_node_update(CaseArg<B, Params> P, CaseArg<B, LevelView> L, int mode, int stage, int io);
 // gathers: U lanes per node (1 = a thread per node); by default the widest
 // group with at most this many threads on the level (flite_ctx::lanes_of)
 constexpr size_t kLaneThreads = 98304;
@@ -69,7 +96,15 @@ __global__ void k_sa_grad(Params P, LevelView L);
 __global__ void k_sa_diff(Params P, LevelView L);
 __global__ void k_sa_conv(Params P, LevelView L, int td);
 __global__ void k_sa_stage(Params P, LevelView L, int mode, int stage, int turb);
+// set-up of a level's edges on the device (kernels.cu)
 __global__ void k_make_rows(LevelView L, int nrows, int2 *rows);
+__global__ void k_row_firsts(const int2 *rows, int nrows, int *first);
+__global__ void __launch_bounds__(1024) k_scan_rows(int *first, int nrows);
+__global__ void k_edge_slots(const int2 *rows, int nrows, const int *first, int *slot);
+__global__ void k_renumber_edges(int2 *inc, int n, const int *slot);
+__global__ void k_move_edges(int E, const int *slot, const int2 *in, int2 *out);
+__global__ void k_put_edges(int E, const int *slot, const double *w, double *wx, double *wy, double *wz, EdgeW *ew);
+__global__ void k_put_edge_values(int E, const int *slot, const double *in, double *out);
 __global__ void k_make_inc32(const int2 *inc, const EdgeW *ew, int n, IncRec32 *o);
 __global__ void k_copy(const double *a, double *b, size_t n);
 template <bool B = false>
@@ -78,7 +113,9 @@ __global__ void k_restrict_arr(LevelView C, LevelView F, const double *fsrc, dou
 template <bool B = false>
 __global__ void k_restrict_state(CaseArg<B, Params> P, CaseArg<B, LevelView> C, CaseArg<B, LevelView> F);
 template <bool B = false>
-__global__ void k_restrict_incr(CaseArg<B, Params> P, CaseArg<B, LevelView> C, CaseArg<B, LevelView> F);
+__global__ void k_restrict_incr(CaseArg<B, Params> P, CaseArg<B, LevelView> C, CaseArg<B, LevelView> F, int floor_fine);
+template <bool B = false>
+__global__ void k_prolong(CaseArg<B, Params> P, CaseArg<B, LevelView> C, CaseArg<B, LevelView> F);
 template <bool B = false>
 __global__ void k_prolong_coarse(CaseArg<B, Params> P, CaseArg<B, LevelView> C, CaseArg<B, LevelView> F);
 template <bool B = false>
@@ -95,6 +132,8 @@ __global__ void k_set_int(int *dst, const int *src);
 __global__ void k_min_dt_init(LevelView L);
 __global__ void k_min_dt(LevelView L);
 // steps of the cycle on a level view (group form: every case of a group)
+// lanes per coarse node of the transfers that gather its children
+constexpr int kChildLanes = 8;
 template <bool B = false>
 __global__ void k_case_cycle(CaseArg<B, LevelView> L, const int *src);
 template <bool B = false>

@@ -207,7 +207,7 @@ __global__ void na_bnd(Params P, LevelView L) {
     if (b >= L.B) return;
     if (L.bedge[b].x < 0) return;  // dropped by the index check
     double g1[5], g2[5];
-    boundary_flux(P, L, b, g1, g2);
+    boundary_flux(P, L, b, [&](int j) { return load_state(L, j); }, g1, g2);
     double *o = L.bflux + (size_t)b * 10;
     for (int k = 0; k < 5; ++k) { o[k] = g1[k]; o[5 + k] = g2[k]; }
 }

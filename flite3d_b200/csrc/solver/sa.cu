@@ -170,7 +170,7 @@ __global__ void k_sa_conv(Params P, LevelView L, int td) {
     double qi[4];
     prim(i, qi);
     // an unsteady stage's time difference comes first (def_par:1073)
-    double acc = td ? time_difference(P, L, i, 5) : 0.0;
+    double acc = td ? time_difference(P, L, L.u, i, 5) : 0.0;
     FLITE_FOR_INC(L, i, t) {
         const int e = t.x >= 0 ? t.x : ~t.x;
         double qj[4];
@@ -243,7 +243,7 @@ __global__ void k_sa_stage(Params P, LevelView L, int mode, int stage, int turb)
     const unsigned char cls = L.bc[i];
     // convection from k_sa_conv (after the time difference of an unsteady
     // stage, which is all of it when the turbulence is not recomputed)
-    double r = turb ? L.rhs[o6] : (P.addts && mode == MODE_STAGE ? time_difference(P, L, i, 5) : 0.0);
+    double r = turb ? L.rhs[o6] : (P.addts && mode == MODE_STAGE ? time_difference(P, L, L.u, i, 5) : 0.0);
     if (turb) r = sa_source(P, L, i, r);
     // restrictGrid adds the (last computed) diffusion term whether or not
     // the turbulence is recomputed (def_par:12238-12240, 12315-12317)

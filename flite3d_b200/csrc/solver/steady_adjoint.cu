@@ -1785,8 +1785,7 @@ extern "C" int flite_objective(flite_ctx *ctx, int objective, double *J) {
             // are put back)
             copy(X, L.mu, A.mu_keep, N);
             copy(X, L.wstress, A.ws_keep, 3 * N);
-            X.pressure(0);
-            k_visc_prim<<<X.nblk(N), X.nb, 0, X.s>>>(X.P, L);
+            X.state_pass(0, STATE_PRIM);
             X.visc_grad(0);
             copy(X, L.tau, A.tau, 9 * N);
             copy(X, A.mu_keep, L.mu, N);

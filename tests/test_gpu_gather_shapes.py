@@ -3,9 +3,12 @@ of 4, 8, 16 and 32 lanes (one node's terms added by one lane per sum), on a
 mesh whose node counts leave a partly filled last warp on each level, and the
 default choice on levels on both sides of its threshold.
 """
+import ctypes
+
 import numpy as np
 import pytest
 
+from conftest import oracle_backend
 from flite3d_b200 import Mesh, Solver, default_controls, initial_state
 
 pytestmark = pytest.mark.gpu
@@ -50,4 +53,53 @@ def test_group_shapes_match_a_thread_per_node(name):
 def test_default_shape_matches_a_thread_per_node(size):
     mesh = Mesh.bump_channel(*size, 0.05, nlevels=3)
     for a, b in zip(states(mesh, CASES["laminar"], 1, 1), states(mesh, CASES["laminar"], 0, 1)):
+        assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("ctl", [dict(rungeKuttaStages=5, CFLNumber=1.0), dict(multigridScheme=2), dict(multigridScheme=7),
+                                 dict(numberOfRelaxationSteps=3), dict(boundaryTerm=2), dict(flowType=1, physicalTimeStep=0.2),
+                                 dict(secondOrderDissipationFactor=0.0, fourthOrderDissipationFactor=0.0),
+                                 dict(minimumDensity=1.0)],
+                         ids=["five_stages", "w_cycle", "scheme7", "steps", "fv_boundary", "unsteady", "no_jst", "floored"])
+@pytest.mark.parametrize("model", ["euler", "laminar"])
+def test_passes_between_stages_match_the_restatement(model, ctl):
+    """Stages that alternate the copies of the state, folded dissipation,
+    boundary edges evaluated in the node pass, the floor left to the
+    restriction, the branch of the restriction: bit for bit on every level."""
+    mesh = Mesh.bump_channel(17, 7, 6, 0.05, nlevels=3)
+    c = default_controls(**{**dict(ReynoldsNumber=0.0, fluxType=1, CFLNumber=2.0, multigridScheme=3,
+                                   numberOfGridsToUse=3), **CASES[model], **ctl})
+    u0 = initial_state(c, mesh, perturb_seed=5, amplitude=0.03)
+    got = []
+    for be in (None, oracle_backend()):
+        s = Solver(c, mesh, backend=be)
+        s.set_state(u0)
+        s.start()
+        for it in range(1, 4):
+            s.cycle(it)
+        got.append([s.get_state(level) for level in (1, 2, 3)] + [s.get_pressure()])
+        s.close()
+    for a, b in zip(*got):
+        assert np.all(np.isfinite(b))
+        assert np.array_equal(a, b)
+
+
+def test_fine_nodes_without_a_parent_match_the_restatement():
+    """Transfers where some fine nodes have no parent (the two-launch
+    prolongation)."""
+    mesh = Mesh.bump_channel(17, 7, 6, 0.05, nlevels=2)
+    n = mesh.level(1).n_nodes
+    parent = np.ctypeslib.as_array(ctypes.cast(mesh.level(2).parent, ctypes.POINTER(ctypes.c_int32)), (n,))
+    parent[::37] = 0
+    c = default_controls(ReynoldsNumber=0.0, fluxType=1, CFLNumber=1.0, multigridScheme=3, numberOfGridsToUse=2)
+    got = []
+    for be in (None, oracle_backend()):
+        s = Solver(c, mesh, backend=be)
+        s.set_state(initial_state(c, mesh, perturb_seed=5))
+        s.start()
+        for it in range(1, 3):
+            s.cycle(it)
+        got.append([s.get_state(level) for level in (1, 2)])
+        s.close()
+    for a, b in zip(*got):
         assert np.array_equal(a, b)
