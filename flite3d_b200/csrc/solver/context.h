@@ -200,10 +200,6 @@ struct flite_ctx {
         allocs.push_back(p);
         return (T *)p;
     }
-    void release(void *p) {
-        allocs.erase(std::find(allocs.begin(), allocs.end(), p));
-        CK(cudaFree(p));
-    }
     template <class T>
     T *upload(const std::vector<T> &h) {
         T *d = alloc<T>(h.size());
@@ -268,6 +264,7 @@ struct flite_ctx {
     void state_pass(int l, int what, bool bnd = false) {
         const LevelView &L = V(l);
         if (fused()) what |= STATE_REC;  // only the central gathers read the records
+        if (L.hprim) what |= STATE_HPRIM;
         counted();
         if (bnd)
             FLITE_LAUNCH(k_state_pass, (true,), nblk((size_t)L.N + L.B), nb, 0, P, L, what, (const int *)d_cycle);
@@ -473,11 +470,15 @@ struct flite_ctx {
         } else if (c.fluxType == 4 && c.HLLCFluxOrder > 1 && L.grid == 1) {
             no_group("the HLLC order-2 gradients");
             counted();
-            if (c.GradientMethod == 1) k_gradient<<<nblk(L.N), nb, 0, s>>>(P, L);
-            else k_ls_gradient<<<nblk(L.N), nb, 0, s>>>(P, L);
-            if (c.Automaticlipping == 1) {
-                counted();
-                k_minmax<<<nblk(L.N), nb, 0, s>>>(P, L);
+            if (c.GradientMethod == 1) {
+                if (c.Automaticlipping == 1) k_gradient<true><<<nblk(L.N), nb, 0, s>>>(P, L);
+                else k_gradient<false><<<nblk(L.N), nb, 0, s>>>(P, L);
+            } else {
+                k_ls_gradient<<<nblk(L.N), nb, 0, s>>>(P, L);
+                if (c.Automaticlipping == 1) {
+                    counted();
+                    k_minmax<<<nblk(L.N), nb, 0, s>>>(P, L);
+                }
             }
         }
         if (L.E > 0) {
@@ -516,7 +517,10 @@ struct flite_ctx {
                 else k_edge_flux<3, false><<<ng, eb, 0, s>>>(P, L);
                 break;
             case 4:
-                if (c.HLLCFluxOrder > 1) k_edge_flux<4, true><<<ng, eb, 0, s>>>(P, L);
+                if (c.HLLCFluxOrder > 1) {
+                    const int nt = std::min(eb, edge_threads(4, true));
+                    k_edge_flux<4, true><<<(unsigned)((L.E + nt - 1) / nt), nt, 0, s>>>(P, L);
+                }
                 else k_edge_flux<4, false><<<ng, eb, 0, s>>>(P, L);
                 break;
             default: k_edge_flux<1, false><<<ng, eb, 0, s>>>(P, L);

@@ -93,15 +93,18 @@ struct __align__(16) DeltaRec {  // FP32 anchor primitives and increments (48 B)
     float dr, dmx, dmy, dmz, dE, dp, pad;  // u - ua and p - pa
 };
 
-// Level-1 records of the upwind extension (no reference counterpart): the
-// primitives of the Galerkin gradient with the node's coordinates (64 B, two
-// sectors), and that gradient, component-major (g[3c + a] = d q_c / d x_a,
-// 128 B), so that an edge end costs six sectors instead of twenty-four SoA
-// ones and no divisions.
-struct __align__(16) PrimRec {
+// Level-1 node data of the upwind extension (no reference counterpart): the
+// primitives of the Galerkin gradient with the node's coordinates, and that
+// gradient, component-major (g[3c + a] = d q_c / d x_a).  Kept as pairs of
+// values, [pair][N]: the edges of a warp have neighbouring first nodes and
+// neighbouring second nodes, so a pair is read with one 16-byte load of 4 to
+// 5 cache lines a warp; as records of 64 and 128 bytes side by side the same
+// loads take 16 and 32 lines each, and the edge kernel's L1 throughput was at
+// 87 % of its peak (129 us for 1.4 million edges).
+struct PrimRec {
     double r, u, v, w, E, x, y, z;  // rho, (rho u)/rho, ..., rho E, coordinates
 };
-struct __align__(16) GradRec {
+struct GradRec {
     double g[16];  // 15 used
 };
 
@@ -171,9 +174,10 @@ struct LevelView {
     double *vdt;                           // [N]  V/dt of the dissipation
     double *wstress;                       // [3][N] wall stress (level 1)
     double *grad;                          // [15][N] (level 1, HLLC order 2)
-    PrimRec *qp;                           // [N] (level 1, upwind extension)
-    GradRec *gq;                           // [N] (level 1, upwind extension)
-    double *bnd;                           // [10][N]
+    double2 *qp;                           // [4][N] PrimRec in pairs (level 1, upwind extension)
+    double2 *gq;                           // [8][N] GradRec in pairs (level 1, upwind extension)
+    double *bnd;                           // [10][N] LED bounds, 5 lower then 5 upper
+    double *hprim;                         // [3][N] u, v, w of the gradients (level 1, HLLC order 2)
     double *flux;                          // [E][5] edge flux buffer
     // mixed precision (FLITE_MIXED): interior central fluxes as FP32
     // increments over an FP64 anchor state
@@ -293,7 +297,27 @@ __device__ __forceinline__ void store_rec(R *base, int j, const R &o) {
     for (int k = 0; k < K; ++k) p[k] = d[k];
 }
 __device__ __forceinline__ NodeRec load_node(const NodeRec *q, int j) { return load_rec<NodeRec, 3>(q, j); }
-__device__ __forceinline__ PrimRec load_prim(const PrimRec *q, int j) { return load_rec<PrimRec, 4>(q, j); }
+// node data kept as K pairs [pair][n]
+template <class R, int K>
+__device__ __forceinline__ R load_pairs(const double2 *q, int n, int j) {
+    static_assert(sizeof(R) == 16 * K, "record size");
+    R o;
+    double *d = reinterpret_cast<double *>(&o);
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const double2 v = __ldg(q + (size_t)k * n + j);
+        d[2 * k] = v.x; d[2 * k + 1] = v.y;
+    }
+    return o;
+}
+template <class R, int K>
+__device__ __forceinline__ void store_pairs(double2 *q, int n, int j, const R &o) {
+    static_assert(sizeof(R) == 16 * K, "record size");
+    const double *d = reinterpret_cast<const double *>(&o);
+#pragma unroll
+    for (int k = 0; k < K; ++k) q[(size_t)k * n + j] = make_double2(d[2 * k], d[2 * k + 1]);
+}
+__device__ __forceinline__ PrimRec load_prim(const double2 *q, int n, int j) { return load_pairs<PrimRec, 4>(q, n, j); }
 // 1/rho and E + p are the operations the central flux performs per edge
 // end, done once per node
 __device__ __forceinline__ void store_node(NodeRec *q, int j, double r, double ru, double rv, double rw, double E,

@@ -112,10 +112,7 @@ void flite::put_geometry(flite_ctx &X, int l, const flite_level_desc &d, bool cr
     };
     // edge arrays: from the caller's own memory, put into the device's edge
     // order there
-    double *edges_in = nullptr;  // staging: side_w (3E), then the GCL weights
-    auto free_staging = [](double *p) { cudaFree(p); };
-    if (E > 0) CK(cudaMalloc(&edges_in, 3 * (size_t)E * sizeof(double)));
-    std::unique_ptr<double, decltype(free_staging)> staging(edges_in, free_staging);
+    double *edges_in = X.io_buffer(3 * (size_t)std::max(E, 1));  // staging
     const unsigned ge = (unsigned)((E + 255) / 256);
     if (create) {
         double *w = X.alloc<double>(3 * (size_t)E);
@@ -395,8 +392,6 @@ int flite::create_context(const flite_controls *c, int nlevels, const flite_leve
                 }
             }
             // upload
-            int2 *dedge = X.upload(edge);
-            L.edge = dedge;
             L.bedge = X.upload(bedge); L.bind = X.upload(bind);
             int2 *dinc = X.upload(inc);
             L.inc_ptr = X.upload(ip); L.inc = dinc;
@@ -413,7 +408,9 @@ int flite::create_context(const flite_controls *c, int nlevels, const flite_leve
             // the sums keep the caller's order
             L.eslot = nullptr;
             if (4 * (size_t)N > kLaneThreads && E > 0) {
-                int *slot = X.alloc<int>(E), *first = X.alloc<int>(D.nrows);
+                int2 *dedge = reinterpret_cast<int2 *>(X.io_buffer((size_t)E + D.nrows));
+                int *slot = X.alloc<int>(E), *first = reinterpret_cast<int *>(dedge + E);
+                CK(cudaMemcpy(dedge, edge.data(), (size_t)E * sizeof(int2), cudaMemcpyHostToDevice));
                 const unsigned gr = flite_ctx::blocks((size_t)D.nrows * kRow);
                 k_row_firsts<<<gr, kBlock>>>(rows, D.nrows, first);
                 k_scan_rows<<<1, 1024>>>(first, D.nrows);
@@ -423,10 +420,11 @@ int flite::create_context(const flite_controls *c, int nlevels, const flite_leve
                 int2 *moved = X.alloc<int2>(E);
                 k_move_edges<<<flite_ctx::blocks(E), kBlock>>>(E, slot, dedge, moved);
                 CK(cudaGetLastError());
+                CK(cudaStreamSynchronize(nullptr));  // the staging buffer is free again
                 L.edge = moved;
                 L.eslot = slot;
-                X.release(dedge);
-                X.release(first);
+            } else {
+                L.edge = X.upload(edge);
             }
             L.rows = rows;
             L.binc_ptr = X.upload(bp); L.binc = X.upload(binc);
@@ -548,8 +546,9 @@ int flite::create_context(const flite_controls *c, int nlevels, const flite_leve
             CK(cudaMemset(L.wstress, 0, 3 * (size_t)N * sizeof(double)));
             L.grad = hllc2 ? X.alloc<double>(15 * (size_t)N) : nullptr;
             L.bnd = hllc2 ? X.alloc<double>(10 * (size_t)N) : nullptr;
-            L.qp = muscl ? X.alloc<PrimRec>(N) : nullptr;
-            L.gq = muscl ? X.alloc<GradRec>(N) : nullptr;
+            L.hprim = hllc2 ? X.alloc<double>(3 * (size_t)N) : nullptr;
+            L.qp = muscl ? X.alloc<double2>(4 * (size_t)N) : nullptr;
+            L.gq = muscl ? X.alloc<double2>(8 * (size_t)N) : nullptr;
             // the edge buffer carries the upwind fluxes; the central flux is
             // computed inside the node gather
             L.flux = !X.fused() ? X.alloc<double>(5 * (size_t)std::max(E, 1)) : nullptr;
@@ -589,6 +588,11 @@ int flite::create_context(const flite_controls *c, int nlevels, const flite_leve
             L.nvar = X.nvar();
         }
         CK(cudaDeviceSynchronize());
+        if (X.d_io) {  // the set-up's staging buffer
+            CK(cudaFree(X.d_io));
+            X.d_io = nullptr;
+            X.io_n = 0;
+        }
         return FLITE_OK;
     });
     if (rc != FLITE_OK) {

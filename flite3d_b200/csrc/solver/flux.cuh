@@ -20,26 +20,24 @@ __device__ __forceinline__ NodeState load_state(const LevelView &L, int i) {
 }
 
 // LED limiter of the HLLC reconstruction (def_par:1856-1867); the root
-// (1+t^nsig)^(1/nsig) is sqrt(sqrt(.)) for nsig=4 and sqrt(.) for nsig=2
-__device__ __forceinline__ double led(double a, double bmin, double bmax, int nsig) {
-    double cc = a;
-    double a1 = 2.0 * a;
-    if (a1 > 0.0) {
-        double invmax = 0.0;
-        if (bmax > 0.0) invmax = 1.0 / bmax;
-        double t = a1 * invmax;
-        double tn = nsig == 4 ? (t * t) * (t * t) : t * t;
-        double root = nsig == 4 ? sqrt(sqrt(1. + tn)) : sqrt(1. + tn);
-        cc = 0.5 * bmax * t / root;
-    } else if (a1 < 0.0) {
-        double invmin = 0.0;
-        if (bmin < 0.0) invmin = 1.0 / bmin;
-        double t = a1 * invmin;
-        double tn = nsig == 4 ? (t * t) * (t * t) : t * t;
-        double root = nsig == 4 ? sqrt(sqrt(1. + tn)) : sqrt(1. + tn);
-        cc = 0.5 * bmin * t / root;
-    }
-    return cc;
+// (1+t^nsig)^(1/nsig) is sqrt(sqrt(.)) for nsig=4 and sqrt(.) for nsig=2.
+// bnd points at the component's lower bounds of a level, the upper ones are 5
+// arrays of n on.  The reference's two branches (a > 0 with the upper bound,
+// a < 0 with the lower) are the same expressions of one bound, so the bound is
+// selected and they run once: lanes of both signs meet in nearly every warp.
+// The bounds' reciprocals formed once per node and read here made a cycle 1 to
+// 3 % slower: the two more loads per end cost more than its division.
+__device__ __forceinline__ double led(double a, const double *bnd, size_t n, int i, int nsig) {
+    const double a1 = 2.0 * a;
+    if (!(a1 > 0.0) && !(a1 < 0.0)) return a;
+    const bool up = a1 > 0.0;
+    const double b = bnd[(up ? 5 * n : 0) + i];
+    double inv = 0.0;
+    if (up ? b > 0.0 : b < 0.0) inv = 1.0 / b;
+    const double t = a1 * inv;
+    const double tn = nsig == 4 ? (t * t) * (t * t) : t * t;
+    const double root = nsig == 4 ? sqrt(sqrt(1. + tn)) : sqrt(1. + tn);
+    return 0.5 * b * t / root;
 }
 
 // central flux of an edge from its two node states (def_par:1664-1669)
@@ -109,13 +107,10 @@ __device__ __forceinline__ void edge_flux(const Params &P, const LevelView &L, i
         f[0] = f[0] - (r1 + r2) * wgcl; f[1] = f[1] - (ru1 + ru2) * wgcl; f[2] = f[2] - (rv1 + rv2) * wgcl;
         f[3] = f[3] - (rw1 + rw2) * wgcl; f[4] = f[4] - (E1 + E2) * wgcl;
     };
-    if constexpr (FT == 1 || FT == 4) {
-        // central flux; HLLC starts from it too (def_par:1798)
+    if constexpr (FT == 1) {
         central_flux(a, b, wx, wy, wz, f);
-        if constexpr (FT == 1) {
-            gcl_sum();
-            return;
-        }
+        gcl_sum();
+        return;
     }
     if constexpr (FT == 2) {  // local Lax-Friedrichs (def_par:1670-1724)
         double rnorm = sqrt((wx * wx + wy * wy) + wz * wz);
@@ -199,8 +194,8 @@ __device__ __forceinline__ void edge_flux(const Params &P, const LevelView &L, i
                 double dpv1 = 0.5 * ((L.grad[j * N + i1] * dx + L.grad[(j + 5) * N + i1] * dy) + L.grad[(j + 10) * N + i1] * dz);
                 double dpv11 = 0.5 * ((L.grad[j * N + i2] * dx + L.grad[(j + 5) * N + i2] * dy) + L.grad[(j + 10) * N + i2] * dz);
                 if (P.autoClip == 1) {
-                    dpv1 = led(dpv1, L.bnd[j * N + i1], L.bnd[(j + 5) * N + i1], P.nsig);
-                    dpv11 = -led(-dpv11, L.bnd[j * N + i2], L.bnd[(j + 5) * N + i2], P.nsig);
+                    dpv1 = led(dpv1, L.bnd + (size_t)j * N, N, i1, P.nsig);
+                    dpv11 = -led(-dpv11, L.bnd + (size_t)j * N, N, i2, P.nsig);
                 }
                 double aa = dpv1, bb = dpv11, cc;
                 if (aa * bb <= 0.0) {
@@ -248,73 +243,57 @@ __device__ __forceinline__ void edge_flux(const Params &P, const LevelView &L, i
     double fact = roe2 * (sr - nv2) - roe1 * (sl - nv1);
     if (fact != 0.0) fact = 1.0 / fact;
     sm = fact * sm;
+    // the wave regions (def_par:1988-2045): left or right of the contact,
+    // inside or outside the star region.  Left and right are the same
+    // expressions of their side's state, so the side is selected and they run
+    // once whatever the regions of a warp's edges.
+    const bool out1 = sl > 0.0, in1 = !out1 && sl <= 0.0 && sm > 0.0;
+    const bool in2 = !out1 && !in1 && sm <= 0.0 && sr >= 0.0, out2 = !out1 && !in1 && !in2 && sr < 0.0;
     // the state of the GCL term: rho and E of the node with the
     // (reconstructed) momentum outside the star region, the star state
     // inside it (def_par:2046-2085)
     double q[5] = {r1, ru1, rv1, rw1, E1};
-    if (sl > 0.0) {
-        f[0] = ((rnx * ru1 + rny * rv1) + rnz * rw1) * rnorm1;
-        f[1] = ((rnx * (ru1 * u1 + pr1) + rny * (ru1 * v1)) + rnz * (ru1 * w1)) * rnorm1;
-        f[2] = ((rnx * (rv1 * u1) + rny * (rv1 * v1 + pr1)) + rnz * (rv1 * w1)) * rnorm1;
-        f[3] = ((rnx * (rw1 * u1) + rny * (rw1 * v1)) + rnz * (rw1 * w1 + pr1)) * rnorm1;
-        f[4] = ((rnx * (rh1 * u1) + rny * (rh1 * v1)) + rnz * (rh1 * w1)) * rnorm1;
-    } else if (sl <= 0.0 && sm > 0.0) {
-        double fl0 = (rnx * ru1 + rny * rv1) + rnz * rw1;
-        double fl1 = (rnx * (ru1 * u1 + pr1) + rny * (ru1 * v1)) + rnz * (ru1 * w1);
-        double fl2 = (rnx * (rv1 * u1) + rny * (rv1 * v1 + pr1)) + rnz * (rv1 * w1);
-        double fl3 = (rnx * (rw1 * u1) + rny * (rw1 * v1)) + rnz * (rw1 * w1 + pr1);
-        double fl4 = (rnx * (rh1 * u1) + rny * (rh1 * v1)) + rnz * (rh1 * w1);
-        double pls = roe1 * (nv1 - sl) * (nv1 - sm) + pr1;
-        double ls0, ls1, ls2, ls3, ls4;
-        double factl = sl - sm;
-        if (factl != 0.0) {
-            factl = 1.0 / factl;
-            ls0 = roe1 * (sl - nv1) * factl;
-            ls1 = ((sl - nv1) * roe1 * u1 + (pls - pr1) * rnx) * factl;
-            ls2 = ((sl - nv1) * roe1 * v1 + (pls - pr1) * rny) * factl;
-            ls3 = ((sl - nv1) * roe1 * w1 + (pls - pr1) * rnz) * factl;
-            ls4 = (((sl - nv1) * re1 - pr1 * nv1) + pls * sm) * factl;
+    if (out1 || in1 || in2 || out2) {
+        const bool left = out1 || in1;
+        const double ro = left ? roe1 : roe2, re = left ? re1 : re2, pr = left ? pr1 : pr2, rh = left ? rh1 : rh2;
+        const double ru = left ? ru1 : ru2, rv = left ? rv1 : rv2, rw = left ? rw1 : rw2;
+        const double uu = left ? u1 : u2, vv = left ? v1 : v2, ww = left ? w1 : w2;
+        const double nv = left ? nv1 : nv2, sw = left ? sl : sr;
+        const double fl0 = (rnx * ru + rny * rv) + rnz * rw;
+        const double fl1 = (rnx * (ru * uu + pr) + rny * (ru * vv)) + rnz * (ru * ww);
+        const double fl2 = (rnx * (rv * uu) + rny * (rv * vv + pr)) + rnz * (rv * ww);
+        const double fl3 = (rnx * (rw * uu) + rny * (rw * vv)) + rnz * (rw * ww + pr);
+        const double fl4 = (rnx * (rh * uu) + rny * (rh * vv)) + rnz * (rh * ww);
+        if (in1 || in2) {
+            const double ps = ro * (nv - sw) * (nv - sm) + pr;
+            double s0 = ro, s1 = ru, s2 = rv, s3 = rw, s4 = re;
+            double fs = sw - sm;
+            if (fs != 0.0) {
+                fs = 1.0 / fs;
+                s0 = ro * (sw - nv) * fs;
+                s1 = ((sw - nv) * ro * uu + (ps - pr) * rnx) * fs;
+                s2 = ((sw - nv) * ro * vv + (ps - pr) * rny) * fs;
+                s3 = ((sw - nv) * ro * ww + (ps - pr) * rnz) * fs;
+                s4 = (((sw - nv) * re - pr * nv) + ps * sm) * fs;
+            }
+            f[0] = (fl0 + sw * (s0 - ro)) * rnorm1;
+            f[1] = (fl1 + sw * (s1 - ru)) * rnorm1;
+            f[2] = (fl2 + sw * (s2 - rv)) * rnorm1;
+            f[3] = (fl3 + sw * (s3 - rw)) * rnorm1;
+            f[4] = (fl4 + sw * (s4 - re)) * rnorm1;
+            q[0] = s0; q[1] = s1; q[2] = s2; q[3] = s3; q[4] = s4;
         } else {
-            ls0 = roe1; ls1 = ru1; ls2 = rv1; ls3 = rw1; ls4 = re1;
+            f[0] = fl0 * rnorm1;
+            f[1] = fl1 * rnorm1;
+            f[2] = fl2 * rnorm1;
+            f[3] = fl3 * rnorm1;
+            f[4] = fl4 * rnorm1;
+            if (out2) { q[0] = r2; q[1] = ru2; q[2] = rv2; q[3] = rw2; q[4] = E2; }
         }
-        f[0] = (fl0 + sl * (ls0 - roe1)) * rnorm1;
-        f[1] = (fl1 + sl * (ls1 - ru1)) * rnorm1;
-        f[2] = (fl2 + sl * (ls2 - rv1)) * rnorm1;
-        f[3] = (fl3 + sl * (ls3 - rw1)) * rnorm1;
-        f[4] = (fl4 + sl * (ls4 - re1)) * rnorm1;
-        q[0] = ls0; q[1] = ls1; q[2] = ls2; q[3] = ls3; q[4] = ls4;
-    } else if (sm <= 0.0 && sr >= 0.0) {
-        double fr0 = (rnx * ru2 + rny * rv2) + rnz * rw2;
-        double fr1 = (rnx * (ru2 * u2 + pr2) + rny * (ru2 * v2)) + rnz * (ru2 * w2);
-        double fr2 = (rnx * (rv2 * u2) + rny * (rv2 * v2 + pr2)) + rnz * (rv2 * w2);
-        double fr3 = (rnx * (rw2 * u2) + rny * (rw2 * v2)) + rnz * (rw2 * w2 + pr2);
-        double fr4 = (rnx * (rh2 * u2) + rny * (rh2 * v2)) + rnz * (rh2 * w2);
-        double prs = roe2 * (nv2 - sr) * (nv2 - sm) + pr2;
-        double rs0, rs1, rs2, rs3, rs4;
-        double factr = sr - sm;
-        if (factr != 0.0) {
-            factr = 1.0 / factr;
-            rs0 = roe2 * (sr - nv2) * factr;
-            rs1 = ((sr - nv2) * roe2 * u2 + (prs - pr2) * rnx) * factr;
-            rs2 = ((sr - nv2) * roe2 * v2 + (prs - pr2) * rny) * factr;
-            rs3 = ((sr - nv2) * roe2 * w2 + (prs - pr2) * rnz) * factr;
-            rs4 = (((sr - nv2) * re2 - pr2 * nv2) + prs * sm) * factr;
-        } else {
-            rs0 = roe2; rs1 = ru2; rs2 = rv2; rs3 = rw2; rs4 = re2;
-        }
-        f[0] = (fr0 + sr * (rs0 - roe2)) * rnorm1;
-        f[1] = (fr1 + sr * (rs1 - ru2)) * rnorm1;
-        f[2] = (fr2 + sr * (rs2 - rv2)) * rnorm1;
-        f[3] = (fr3 + sr * (rs3 - rw2)) * rnorm1;
-        f[4] = (fr4 + sr * (rs4 - re2)) * rnorm1;
-        q[0] = rs0; q[1] = rs1; q[2] = rs2; q[3] = rs3; q[4] = rs4;
-    } else if (sr < 0.0) {
-        f[0] = ((rnx * ru2 + rny * rv2) + rnz * rw2) * rnorm1;
-        f[1] = ((rnx * (ru2 * u2 + pr2) + rny * (ru2 * v2)) + rnz * (ru2 * w2)) * rnorm1;
-        f[2] = ((rnx * (rv2 * u2) + rny * (rv2 * v2 + pr2)) + rnz * (rv2 * w2)) * rnorm1;
-        f[3] = ((rnx * (rw2 * u2) + rny * (rw2 * v2)) + rnz * (rw2 * w2 + pr2)) * rnorm1;
-        f[4] = ((rnx * (rh2 * u2) + rny * (rh2 * v2)) + rnz * (rh2 * w2)) * rnorm1;
-        q[0] = r2; q[1] = ru2; q[2] = rv2; q[3] = rw2; q[4] = E2;
+    } else {
+        // no region (a wave speed is not a number): the central flux that the
+        // reference starts from (def_par:1798)
+        central_flux(a, b, wx, wy, wz, f);
     }
     if (L.gclw)
         for (int k = 0; k < 5; ++k) f[k] = f[k] - q[k] * wgcl;
@@ -473,18 +452,18 @@ __device__ __forceinline__ double prim_pressure(double gam1, const double *q) {
 __device__ __forceinline__ void edge_flux_muscl(const Params &P, const LevelView &L, int e, int i1, int i2,
                                                 double *f) {
     const double gam1 = P.gm1;
-    const PrimRec A = load_prim(L.qp, i1), B = load_prim(L.qp, i2);
+    const PrimRec A = load_prim(L.qp, L.N, i1), B = load_prim(L.qp, L.N, i2);
     const double dx = B.x - A.x, dy = B.y - A.y, dz = B.z - A.z;
     const double q1[5] = {A.r, A.u, A.v, A.w, A.E}, q2[5] = {B.r, B.u, B.v, B.w, B.E};
-    // g.d at each end, one gradient record (eight 16-byte loads) at a time
+    // g.d at each end, one end (eight 16-byte loads) at a time
     double g1[5], g2[5];
     {
-        const GradRec G = load_rec<GradRec, 8>(L.gq, i1);
+        const GradRec G = load_pairs<GradRec, 8>(L.gq, L.N, i1);
 #pragma unroll
         for (int j = 0; j < 5; ++j) g1[j] = (G.g[3 * j] * dx + G.g[3 * j + 1] * dy) + G.g[3 * j + 2] * dz;
     }
     {
-        const GradRec G = load_rec<GradRec, 8>(L.gq, i2);
+        const GradRec G = load_pairs<GradRec, 8>(L.gq, L.N, i2);
 #pragma unroll
         for (int j = 0; j < 5; ++j) g2[j] = (G.g[3 * j] * dx + G.g[3 * j + 1] * dy) + G.g[3 * j + 2] * dz;
     }
@@ -503,7 +482,7 @@ __device__ __forceinline__ void edge_flux_muscl(const Params &P, const LevelView
         pb = prim_pressure(gam1, qb);
     }
     f[0] = f[1] = f[2] = f[3] = f[4] = 0.0;
-    const EdgeW w = load_edgew(L.ew, e);
+    const struct { double wx, wy, wz; } w = {L.wx[e], L.wy[e], L.wz[e]};
     const double rnorm = sqrt((w.wx * w.wx + w.wy * w.wy) + w.wz * w.wz);
     if (!(rnorm > 1.0e-10)) return;
     const double rn = 1.0 / rnorm;

@@ -133,6 +133,7 @@ __global__ void k_state_pass(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_, in
     const double p = pressure(P, r, ru, rv, rw, E);
     L.p[i] = p;
     if (what & STATE_REC) store_node(L.q, i, r, ru, rv, rw, E, p);
+    if (what & STATE_HPRIM) { L.hprim[i] = ru / r; L.hprim[N + i] = rv / r; L.hprim[2 * N + i] = rw / r; }
     if (what & STATE_PRIM) {
         const double gOg = P.gamma / (P.gamma - 1.0);
         L.prim[i] = ru / r;
@@ -1284,44 +1285,78 @@ __global__ void k_fill(double *a, size_t n, double v) {
     if (i < n) a[i] = v;
 }
 
-// ---- computeGradient, Galerkin (def_par:2923-3245) ------------------------
-__global__ void k_gradient(Params P, LevelView L) {
-    int i = tid();
+// ---- computeGradient, Galerkin (def_par:2923-3245), and LocalMinMax --------
+// (def_par:3248-3459) in one walk of the incidences (MINMAX; alone without
+// automatic clipping).  Both read (rho, u, v, w, rho E) of the other node,
+// with the quotients formed once per node (hprim) and not per incidence.
+__device__ __forceinline__ void hllc_prim(const LevelView &L, int j, double *q) {
+    const int N = L.N;
+    q[0] = L.u[j]; q[1] = L.hprim[j]; q[2] = L.hprim[N + j]; q[3] = L.hprim[2 * N + j]; q[4] = L.u[4 * N + j];
+}
+template <bool MINMAX>
+__global__ void __launch_bounds__(256, 2) k_gradient(Params P, LevelView L) {
+    const int i = tid();
     if (i >= L.N) return;
     const int N = L.N;
-    double g[15];
+    double g[15], mn[5], mx[5];
+#pragma unroll
     for (int c = 0; c < 15; ++c) g[c] = 0.0;
-    const double ri = L.u[i];
-    const double qi[5] = {ri, L.u[N + i] / ri, L.u[2 * N + i] / ri, L.u[3 * N + i] / ri, L.u[4 * N + i]};
+#pragma unroll
+    for (int c = 0; c < 5; ++c) { mn[c] = 1.0e15; mx[c] = 1.0e15; }
+    double qi[5];
+    hllc_prim(L, i, qi);
     FLITE_FOR_INC(L, i, t) {
-        int e = t.x >= 0 ? t.x : ~t.x, j = t.y;
-        const double rj = L.u[j];
-        const double qj[5] = {rj, L.u[N + j] / rj, L.u[2 * N + j] / rj, L.u[3 * N + j] / rj, L.u[4 * N + j]};
+        const int e = t.x >= 0 ? t.x : ~t.x;
+        double qj[5];
+        hllc_prim(L, t.y, qj);
         const double w[3] = {L.wx[e], L.wy[e], L.wz[e]};
+#pragma unroll
         for (int a = 0; a < 3; ++a)
+#pragma unroll
             for (int c = 0; c < 5; ++c) {
-                double s = t.x >= 0 ? qi[c] + qj[c] : qj[c] + qi[c];
-                double dq = s * w[a];
+                const double s = t.x >= 0 ? qi[c] + qj[c] : qj[c] + qi[c];
+                const double dq = s * w[a];
                 g[a * 5 + c] = t.x >= 0 ? g[a * 5 + c] + dq : g[a * 5 + c] - dq;
             }
+        if (MINMAX) {
+            // amin1(q(i1), q(i2)) with the edge's own node order
+#pragma unroll
+            for (int c = 0; c < 5; ++c) {
+                const double a = t.x >= 0 ? qi[c] : qj[c], b = t.x >= 0 ? qj[c] : qi[c];
+                mn[c] = dmin(mn[c], dmin(a, b));
+                mx[c] = dmin(mx[c], dmin(-a, -b));
+            }
+        }
     }
     for (int k = L.binc_ptr[i]; k < L.binc_ptr[i + 1]; ++k) {
-        int b = L.binc[k] >> 1, side = L.binc[k] & 1;
-        int2 nd = L.bedge[b];
-        const double r1 = L.u[nd.x], r2 = L.u[nd.y];
-        const double q1[5] = {r1, L.u[N + nd.x] / r1, L.u[2 * N + nd.x] / r1, L.u[3 * N + nd.x] / r1, L.u[4 * N + nd.x]};
-        const double q2[5] = {r2, L.u[N + nd.y] / r2, L.u[2 * N + nd.y] / r2, L.u[3 * N + nd.y] / r2, L.u[4 * N + nd.y]};
+        const int b = L.binc[k] >> 1, side = L.binc[k] & 1;
+        const int2 nd = L.bedge[b];
+        double q1[5], q2[5];
+        hllc_prim(L, nd.x, q1);
+        hllc_prim(L, nd.y, q2);
         const double w[3] = {L.bwx[b], L.bwy[b], L.bwz[b]};
+#pragma unroll
         for (int a = 0; a < 3; ++a)
+#pragma unroll
             for (int c = 0; c < 5; ++c) {
-                double s = q1[c] + q2[c];
-                double own = side == 0 ? q1[c] : q2[c];
+                const double s = q1[c] + q2[c];
+                const double own = side == 0 ? q1[c] : q2[c];
                 g[a * 5 + c] = g[a * 5 + c] + (2. * own + s) * w[a];
             }
     }
     const double vt = 1. / L.V[i];
+#pragma unroll
     for (int c = 0; c < 15; ++c) L.grad[c * N + i] = g[c] * vt;
+    if (MINMAX) {
+#pragma unroll
+        for (int c = 0; c < 5; ++c) {
+            L.bnd[c * N + i] = mn[c] - qi[c];
+            L.bnd[(c + 5) * N + i] = -mx[c] - qi[c];
+        }
+    }
 }
+template __global__ void k_gradient<false>(Params, LevelView);
+template __global__ void k_gradient<true>(Params, LevelView);
 
 // ---- the upwind extension's level-1 records (no reference counterpart) ----
 // primitives (rho, (rho u)/rho, ..., rho E) and coordinates of every node
@@ -1333,7 +1368,7 @@ __global__ void k_prim_rec(LevelView L) {
     PrimRec o;
     o.r = r; o.u = L.u[N + i] / r; o.v = L.u[2 * N + i] / r; o.w = L.u[3 * N + i] / r; o.E = L.u[4 * N + i];
     o.x = L.cx[i]; o.y = L.cy[i]; o.z = L.cz[i];
-    store_rec<PrimRec, 4>(L.qp, i, o);
+    store_pairs<PrimRec, 4>(L.qp, N, i, o);
 }
 // the Galerkin gradient of k_gradient (computeGradient, def_par:2923-3245),
 // in the same summation order, from the primitive records, stored as
@@ -1344,14 +1379,14 @@ __global__ void k_gradient_rec(LevelView L) {
     double g[15];
 #pragma unroll
     for (int c = 0; c < 15; ++c) g[c] = 0.0;
-    const PrimRec Qi = load_prim(L.qp, i);
+    const PrimRec Qi = load_prim(L.qp, L.N, i);
     const double qi[5] = {Qi.r, Qi.u, Qi.v, Qi.w, Qi.E};
     FLITE_FOR_INC(L, i, t) {
         const int e = t.x >= 0 ? t.x : ~t.x;
-        const PrimRec Qj = load_prim(L.qp, t.y);
-        const double qj[5] = {Qj.r, Qj.u, Qj.v, Qj.w, Qj.E};
-        const EdgeW ew = load_edgew(L.ew, e);
-        const double w[3] = {ew.wx, ew.wy, ew.wz};
+        // (the fifth pair of values is rho E and a coordinate)
+        const double2 a0 = __ldg(L.qp + t.y), a1 = __ldg(L.qp + L.N + t.y);
+        const double qj[5] = {a0.x, a0.y, a1.x, a1.y, __ldg(&(L.qp + 2 * (size_t)L.N + t.y)->x)};
+        const double w[3] = {L.wx[e], L.wy[e], L.wz[e]};
 #pragma unroll
         for (int a = 0; a < 3; ++a)
 #pragma unroll
@@ -1364,7 +1399,7 @@ __global__ void k_gradient_rec(LevelView L) {
     for (int k = L.binc_ptr[i]; k < L.binc_ptr[i + 1]; ++k) {
         const int b = L.binc[k] >> 1, side = L.binc[k] & 1;
         const int2 nd = L.bedge[b];
-        const PrimRec Q1 = load_prim(L.qp, nd.x), Q2 = load_prim(L.qp, nd.y);
+        const PrimRec Q1 = load_prim(L.qp, L.N, nd.x), Q2 = load_prim(L.qp, L.N, nd.y);
         const double q1[5] = {Q1.r, Q1.u, Q1.v, Q1.w, Q1.E}, q2[5] = {Q2.r, Q2.u, Q2.v, Q2.w, Q2.E};
         const double w[3] = {L.bwx[b], L.bwy[b], L.bwz[b]};
 #pragma unroll
@@ -1383,7 +1418,7 @@ __global__ void k_gradient_rec(LevelView L) {
 #pragma unroll
         for (int a = 0; a < 3; ++a) o.g[3 * c + a] = g[a * 5 + c] * vt;
     o.g[15] = 0.0;
-    store_rec<GradRec, 8>(L.gq, i, o);
+    store_pairs<GradRec, 8>(L.gq, L.N, i, o);
 }
 
 // ---- LSComputeGradient + computegradhat (def_par:2593-2920) ---------------
@@ -1430,19 +1465,18 @@ __global__ void k_ls_gradient(Params P, LevelView L) {
     }
 }
 
-// ---- LocalMinMax (def_par:3248-3459) ---------------------------------------
+// ---- LocalMinMax (def_par:3248-3459) beside least-squares gradients ---------------------------------------
 __global__ void k_minmax(Params P, LevelView L) {
     int i = tid();
     if (i >= L.N) return;
     const int N = L.N;
     double mn[5], mx[5];
     for (int c = 0; c < 5; ++c) { mn[c] = 1.0e15; mx[c] = 1.0e15; }
-    const double ri = L.u[i];
-    const double qi[5] = {ri, L.u[N + i] / ri, L.u[2 * N + i] / ri, L.u[3 * N + i] / ri, L.u[4 * N + i]};
+    double qi[5];
+    hllc_prim(L, i, qi);
     FLITE_FOR_INC(L, i, t) {
-        int j = t.y;
-        const double rj = L.u[j];
-        const double qj[5] = {rj, L.u[N + j] / rj, L.u[2 * N + j] / rj, L.u[3 * N + j] / rj, L.u[4 * N + j]};
+        double qj[5];
+        hllc_prim(L, t.y, qj);
         // amin1(q(i1), q(i2)) with the edge's own node order
         for (int c = 0; c < 5; ++c) {
             double a = t.x >= 0 ? qi[c] : qj[c], b = t.x >= 0 ? qj[c] : qi[c];
@@ -1457,6 +1491,13 @@ __global__ void k_minmax(Params P, LevelView L) {
 }
 
 // ---- interior edge flux into the edge buffer ------------------------------
+// What bounds the HLLC order-2 kernel: FP64 instructions (two limited, clipped
+// reconstructions, some twenty divisions and fifteen square roots an edge),
+// not memory (2.6 % of DRAM, 10 % of L1).  With the limiter's and the wave
+// regions' two-sided branches run once instead of per side, and 7 blocks of
+// 128 threads (72 registers; the spills cost less than 2 blocks of 256 at 128
+// registers), the RANS cycle on 738,100 nodes takes 9.8 ms (12.2 before; 10.5
+// with the 128 registers), the HLLC cycle on 80,640 nodes 1.17 ms (1.63).
 // The block's fluxes (at most 256 x 5) are staged in shared memory and
 // written as one contiguous run of 16-byte stores; the block size is even,
 // so the run starts on a 16-byte boundary.
@@ -1468,7 +1509,7 @@ __device__ __forceinline__ void store_block_fluxes(double *flux, const double *s
     if ((n & 1) && threadIdx.x == 0) flux[(size_t)e0 * 5 + n - 1] = sf[n - 1];
 }
 template <int FT, bool O2>
-__global__ void __launch_bounds__(256) k_edge_flux(Params P, LevelView L) {
+__global__ void __launch_bounds__(edge_threads(FT, O2), FT == 4 && O2 ? 7 : 3) k_edge_flux(Params P, LevelView L) {
     __shared__ __align__(16) double sf[256 * 5];
     const int e0 = blockIdx.x * blockDim.x, e = e0 + threadIdx.x;
     if (e < L.E) {
@@ -2065,6 +2106,10 @@ __device__ __forceinline__ void node_tail(const Params &P, const LevelView &L, i
         if (io & IO_EMIT) {  // makePressureField of the next stage
             const double p = pressure(P, un[0], un[1], un[2], un[3], un[4]);
             L.p[i] = p;
+            if constexpr (PREC == GATHER_BUFFER)
+                if (L.hprim) {
+                    L.hprim[i] = un[1] / un[0]; L.hprim[N + i] = un[2] / un[0]; L.hprim[2 * N + i] = un[3] / un[0];
+                }
             if constexpr (PREC == GATHER_ANCHOR || PREC == GATHER_DELTA)
                 store_delta(L, io & IO_REC_B ? L.dq : L.dqb, i, un, p);
             else if constexpr (PREC != GATHER_BUFFER)

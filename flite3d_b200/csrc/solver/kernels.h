@@ -10,10 +10,11 @@ namespace flite {
 enum { MODE_STAGE = 0, MODE_RCOARSE = 1, MODE_RFINE = 2, MODE_RESID = 3, MODE_PROLONG = 4, MODE_START = 5 };
 
 // the pass over a level's state before its gathers: pressure and node records
-// (STATE_REC), with STATE_PRIM the viscous primitives, with STATE_STEP the
+// (STATE_REC), the velocities of the HLLC gradients (STATE_HPRIM), with
+// STATE_PRIM the viscous primitives, with STATE_STEP the
 // start of a relaxation step (cycle number from src, uprev = u); BND adds the
 // boundary edges' fluxes (threads N.. of the grid, one edge each)
-enum { STATE_PRIM = 1, STATE_STEP = 2, STATE_REC = 4 };
+enum { STATE_PRIM = 1, STATE_STEP = 2, STATE_REC = 4, STATE_HPRIM = 8 };
 template <bool BND, bool B = false>
 __global__ void k_state_pass(CaseArg<B, Params> P, CaseArg<B, LevelView> L, int what, const int *src);
 template <int U, bool B = false>
@@ -37,6 +38,7 @@ __global__ void k_visc2_grad(CaseArg<B, Params> P, CaseArg<B, LevelView> L);
 template <int U, bool B = false>
 __global__ void k_visc2_flux(CaseArg<B, Params> P, CaseArg<B, LevelView> L);
 __global__ void k_fill(double *a, size_t n, double v);
+template <bool MINMAX>
 __global__ void k_gradient(Params P, LevelView L);
 __global__ void k_jst_flux_matrix(Params P, LevelView L);
 __global__ void k_lp_sums(Params P, LevelView L);
@@ -46,6 +48,7 @@ __global__ void k_gradient_rec(LevelView L);
 __global__ void k_edge_flux_muscl(Params P, LevelView L);
 __global__ void k_ls_gradient(Params P, LevelView L);
 __global__ void k_minmax(Params P, LevelView L);
+constexpr int edge_threads(int ft, bool o2) { return ft == 4 && o2 ? 128 : 256; }
 template <int FT, bool O2>
 __global__ void k_edge_flux(Params P, LevelView L);
 template <bool B = false>
