@@ -82,10 +82,29 @@ struct flite_ctx {
     std::vector<DevLevel> lv;
     std::vector<void *> allocs;
     cudaStream_t s = nullptr;
-    // a second stream for the part of restrictGrid that does not depend on the
-    // other (in a captured cycle: a branch of the graph)
-    cudaStream_t side = nullptr;
-    cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
+    // Launches that do not depend on each other go to further streams (in a
+    // captured cycle: branches of the graph): beside(k, f) runs f's launches
+    // on stream k after what s holds now, join(k) makes s wait for them.
+    // Streams: 0 restrictGrid's coarse part; 1 and 2 boundary fluxes and the
+    // nu~ part of a pass; 3 and 4 those of the coarse part.
+    static constexpr int kBranches = 5;
+    cudaStream_t branch[kBranches] = {};
+    cudaEvent_t forked[kBranches] = {}, done[kBranches] = {}, coarse_ready = nullptr;
+    int pass_branch = 1;  // 3 within the coarse part
+    template <class F>
+    void beside(int k, F &&f) {
+        struct On {  // s is the branch's stream in its scope
+            cudaStream_t &a, &b;
+            ~On() { std::swap(a, b); }
+        };
+        CK(cudaEventRecord(forked[k], s));
+        CK(cudaStreamWaitEvent(branch[k], forked[k], 0));
+        std::swap(s, branch[k]);
+        On on{s, branch[k]};
+        f();
+        CK(cudaEventRecord(done[k], s));
+    }
+    void join(int k) { CK(cudaStreamWaitEvent(s, done[k], 0)); }
     int *d_cycle = nullptr;
     int *d_cyc = nullptr;  // per-level cycle numbers
     double *d_part = nullptr, *d_out = nullptr;
@@ -213,9 +232,12 @@ struct flite_ctx {
         if (d_io) cudaFree(d_io);
         for (void *p : allocs) cudaFree(p);
         if (h_cycle) cudaFreeHost(h_cycle);
-        for (cudaEvent_t e : ev)
-            if (e) cudaEventDestroy(e);
-        if (side) cudaStreamDestroy(side);
+        for (int k = 0; k < kBranches; ++k) {
+            if (forked[k]) cudaEventDestroy(forked[k]);
+            if (done[k]) cudaEventDestroy(done[k]);
+            if (branch[k]) cudaStreamDestroy(branch[k]);
+        }
+        if (coarse_ready) cudaEventDestroy(coarse_ready);
         if (s) cudaStreamDestroy(s);
     }
 
@@ -428,17 +450,22 @@ struct flite_ctx {
         FLITE_GATHER(k_visc_flux, l, P, V(l));
     }
     // ---- Spalart-Allmaras ----------------------------------------------
-    void sa_timesteps(int l) {
+#define FLITE_SA(kern, l, ...)                                                           \
+    do {                                                                                 \
+        counted();                                                                       \
+        switch (lanes_of(l)) {                                                           \
+            case 4: kern<4><<<gblk(l, 4), nb, 0, s>>>(__VA_ARGS__); break;               \
+            case 8: kern<8><<<gblk(l, 8), nb, 0, s>>>(__VA_ARGS__); break;               \
+            case 16: kern<16><<<gblk(l, 16), nb, 0, s>>>(__VA_ARGS__); break;            \
+            case 32: kern<32><<<gblk(l, 32), nb, 0, s>>>(__VA_ARGS__); break;            \
+            default: kern<1><<<gblk(l, 1), nb, 0, s>>>(__VA_ARGS__);                     \
+        }                                                                                \
+    } while (0)
+    // the turbulent time steps (ts), and the diffusion
+    void sa_diffusion(int l, bool ts) {
         no_group("the Spalart-Allmaras model");
-        counted();
-        k_sa_timestep<<<nblk(V(l).N), nb, 0, s>>>(P, V(l));
-    }
-    void sa_diffusion(int l) {
-        no_group("the Spalart-Allmaras model");
-        counted();
-        k_sa_grad<<<nblk(V(l).N), nb, 0, s>>>(P, V(l));
-        counted();
-        k_sa_diff<<<nblk(V(l).N), nb, 0, s>>>(P, V(l));
+        FLITE_SA(k_sa_grad, l, P, V(l), ts ? 1 : 0);
+        FLITE_SA(k_sa_diff, l, P, V(l));
     }
     // the nu~ part of a stage or one-step update; before the mean-flow node
     // update, which overwrites the density the source term reads
@@ -446,8 +473,7 @@ struct flite_ctx {
         if (!sa()) return;
         no_group("the Spalart-Allmaras model");
         if (turb()) {
-            counted();
-            k_sa_conv<<<nblk(V(l).N), nb, 0, s>>>(P, V(l), P.addts && mode == MODE_STAGE ? 1 : 0);
+            FLITE_SA(k_sa_conv, l, P, V(l), P.addts && mode == MODE_STAGE ? 1 : 0);
         }
         counted();
         k_sa_stage<<<nblk(V(l).N), nb, 0, s>>>(P, V(l), mode, stage, turb() ? 1 : 0);
@@ -493,10 +519,41 @@ struct flite_ctx {
                 edge_flux_launch(L);
             }
         }
-        if (L.B > 0 && !bnd) {
-            counted();
-            FLITE_LAUNCH(k_bnd_flux, (), eblk(L.B), eb, 0, P, L);
-        }
+        if (!bnd) bnd_flux(l);
+    }
+    void bnd_flux(int l) {
+        const LevelView &L = V(l);
+        if (L.B <= 0) return;
+        counted();
+        FLITE_LAUNCH(k_bnd_flux, (), eblk(L.B), eb, 0, P, L);
+    }
+    // The residual's terms of a pass with their node update: the boundary
+    // fluxes (where the pass neither has nor evaluates them) beside the edge
+    // fluxes, and with Spalart-Allmaras the diffusion (`diff`: 0 none, 1, 2
+    // with the turbulent time steps) and the nu~ part beside both.  With
+    // `bnd_forked` the boundary fluxes are under way already.  The branches
+    // pay where launches are short: the RANS cycle's four coarse levels.
+    void residual_pass(int l, int mode, int stage, bool anchor, bool delta, bool bnd, bool bnd_forked, int diff, int pre,
+                       int io) {
+        const int kb = pass_branch, ks = pass_branch + 1;
+        const bool fork_bnd = !bnd && !bnd_forked && !fused() && V(l).B > 0;
+        if (fork_bnd) beside(kb, [&] { bnd_flux(l); });
+        if (sa())
+            beside(ks, [&] {
+                if (turb() && diff) sa_diffusion(l, diff == 2);
+                sa_stage(l, mode, stage);
+            });
+        rhs_terms(l, anchor, delta, bnd || bnd_forked || fork_bnd);
+        if (fork_bnd || bnd_forked) join(kb);
+        if (sa()) join(ks);
+        node_update(l, mode, stage, anchor, pre, io);
+        engine_pass(l, mode);
+    }
+    // the boundary fluxes beside the dissipation that precedes the pass
+    bool bnd_beside(int l, bool bnd) {
+        if (bnd || V(l).B <= 0) return false;
+        beside(pass_branch, [&] { bnd_flux(l); });
+        return true;
     }
     bool mixed() const { return c.precision == FLITE_MIXED; }
     // the central flux (and FLITE_MIXED, which only takes it) is computed
@@ -595,7 +652,10 @@ struct flite_ctx {
     // `bnd`, boundary fluxes of stage 1)
     void singleIteration(int l, bool calcDiss, bool bnd) {
         int pre = PRE_NONE;
+        const bool own = inline_bnd(l), emit = emits();
+        bool early = false;
         if (calcDiss) {
+            early = bnd_beside(l, own || bnd);
             if ((c.dissipationScheme == 1 && V(l).grid == 1) || c.dissipationScheme == 3) {
                 timesteps(l);
                 dissipation(l);
@@ -603,20 +663,14 @@ struct flite_ctx {
             } else {
                 pre = ts_jst_viscous(l, true, true, true);
             }
-            if (turb()) {
-                sa_timesteps(l);
-                sa_diffusion(l);
-            }
         }
-        const bool own = inline_bnd(l), emit = emits();
         for (int st = 1; st <= P.nstage; ++st) {
             // u == uprev at stage 1: the FP64 evaluation there is the anchor
             // of the mixed-precision increments of the later stages
-            if (st > 1 && !emit) pressure(l);
-            rhs_terms(l, st == 1, st > 1 && emit, own || (st == 1 && bnd));
-            sa_stage(l, MODE_STAGE, st);
-            node_update(l, MODE_STAGE, st, st == 1, st == 1 ? pre : PRE_NONE, stage_io(st, P.nstage, own, emit));
-            engine_pass(l, MODE_STAGE);
+            const bool one = st == 1;
+            if (!one && !emit) pressure(l);
+            residual_pass(l, MODE_STAGE, st, one, !one && emit, own || (one && bnd), one && early,
+                          one && calcDiss ? 2 : 0, one ? pre : PRE_NONE, stage_io(st, P.nstage, own, emit));
         }
     }
     // ---- doTimeIterations (def_par:966-1000) -----------------------------
@@ -640,13 +694,15 @@ struct flite_ctx {
     // stepping the fine part reads the coarse level's step: no branch.
     void restrictGrid(int fl) {
         const int cl = fl + 1;
-        const bool branch = !(P.explicit_ && P.unsteady);
+        const bool parallel = !(P.explicit_ && P.unsteady);
         auto coarse_state = [&] {
             counted();
             FLITE_LAUNCH(k_restrict_state, (), nblk(kChildLanes * (size_t)V(cl).N), nb, 0, P, V(cl), V(fl));
         };
         auto coarse = [&] {
             int pre = PRE_NONE;
+            const bool mine = inline_bnd(cl);
+            const bool early = bnd_beside(cl, mine);
             if (c.coarseGridDissipationScheme == 2) {
                 pre = ts_jst_viscous(cl, true, true, true);
             } else {
@@ -654,14 +710,7 @@ struct flite_ctx {
                 if (c.coarseGridDissipationScheme == 3) first_order_diss(cl);
                 viscous(cl, true);
             }
-            const bool own = inline_bnd(cl);
-            rhs_terms(cl, true, false, own);
-            if (turb()) {
-                sa_timesteps(cl);
-                sa_diffusion(cl);
-            }
-            sa_stage(cl, MODE_RCOARSE, 0);
-            node_update(cl, MODE_RCOARSE, 0, true, pre, own ? IO_BND : 0);
+            residual_pass(cl, MODE_RCOARSE, 0, true, false, mine, early, 2, pre, mine ? IO_BND : 0);
         };
         // with lanes per node the fine pass reads its neighbours' state (the
         // folded JST flux, the boundary edges), so the density floor it would
@@ -669,11 +718,10 @@ struct flite_ctx {
         // parent
         const bool own = inline_bnd(fl) && !lv[cl].orphans;
         const bool bnd = group_level(fl) && !own && c.flowType != 2;
-        auto fine_head = [&] {
-            state_pass(fl, visc() ? STATE_PRIM : 0, bnd);
-        };
+        auto fine_head = [&] { state_pass(fl, visc() ? STATE_PRIM : 0, bnd); };
         auto fine = [&] {
             int pre = PRE_NONE;
+            const bool early = bnd_beside(fl, bnd || own);
             // the fine part uses scheme 1 on level 1 under dissipationScheme 1,
             // scheme 2 otherwise (def_par:12269-12273)
             if (c.dissipationScheme == 1 && V(fl).grid == 1) {
@@ -682,31 +730,26 @@ struct flite_ctx {
             } else {
                 pre = ts_jst_viscous(fl, false, true, own);
             }
-            rhs_terms(fl, false, false, bnd || own);
-            if (turb()) sa_diffusion(fl);  // the fine level keeps its turbulent time steps
-            sa_stage(fl, MODE_RFINE, 0);
-            node_update(fl, MODE_RFINE, 0, false, pre, own ? IO_BND | IO_LATER : 0);
-            engine_pass(fl, MODE_RFINE);
+            // the fine level keeps its turbulent time steps
+            residual_pass(fl, MODE_RFINE, 0, false, false, bnd || own, early, 1, pre, own ? IO_BND | IO_LATER : 0);
         };
-        if (branch) {
-            struct Side {  // launches go to the side stream in its scope
-                flite_ctx &x;
-                explicit Side(flite_ctx &c) : x(c) { std::swap(x.s, x.side); }
-                ~Side() { std::swap(x.s, x.side); }
-            };
-            CK(cudaEventRecord(ev[0], s));
-            CK(cudaStreamWaitEvent(side, ev[0], 0));
-            {
-                Side on(*this);
+        if (parallel) {
+            beside(0, [&] {
                 coarse_state();
-                CK(cudaEventRecord(ev[1], s));
-                coarse();
-                CK(cudaEventRecord(ev[2], s));
-            }
+                CK(cudaEventRecord(coarse_ready, s));
+                pass_branch = 3;
+                try {
+                    coarse();
+                } catch (...) {
+                    pass_branch = 1;
+                    throw;
+                }
+                pass_branch = 1;
+            });
             fine_head();
-            CK(cudaStreamWaitEvent(s, ev[1], 0));
+            CK(cudaStreamWaitEvent(s, coarse_ready, 0));
             fine();
-            CK(cudaStreamWaitEvent(s, ev[2], 0));
+            join(0);
         } else {
             coarse_state();
             coarse();

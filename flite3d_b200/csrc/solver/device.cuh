@@ -171,6 +171,8 @@ struct LevelView {
     double *turbDiff, *dtT, *vort, *divg;  // [N] diffusion, turbulent dt, |curl u|, div u
     double *sag;                           // [3][N] Galerkin gradient of nu~
     double *sanh;                          // [N] the cb2 term of the diffusion
+    double *saprim;                        // [3][N] (1/rho) rho u, ... of the nu~ convection
+    double *savis;                         // [N] Re mu/rho + nu~ of the nu~ diffusion
     double *vdt;                           // [N]  V/dt of the dissipation
     double *wstress;                       // [3][N] wall stress (level 1)
     double *grad;                          // [15][N] (level 1, HLLC order 2)
@@ -325,6 +327,15 @@ __device__ __forceinline__ void store_node(NodeRec *q, int j, double r, double r
     NodeRec o;
     o.ru = ru; o.rv = rv; o.rw = rw; o.rinv = 1. / r; o.p = p; o.rh = E + p;
     store_rec<NodeRec, 3>(q, j, o);
+}
+
+// the velocities of the nu~ convection (def_par:6809-6950), once per node with
+// the operations of an edge end
+__device__ __forceinline__ void store_saprim(const LevelView &L, int i, double r, double ru, double rv, double rw) {
+    const double rinv = 1. / r;
+    L.saprim[i] = rinv * ru;
+    L.saprim[L.N + i] = rinv * rv;
+    L.saprim[2 * (size_t)L.N + i] = rinv * rw;
 }
 
 __device__ __forceinline__ double dmin(double a, double b) { return (b < a) ? b : a; }

@@ -288,8 +288,12 @@ int flite::create_context(const flite_controls *c, int nlevels, const flite_leve
                 }
         }
         CK(cudaStreamCreateWithFlags(&X.s, cudaStreamNonBlocking));
-        CK(cudaStreamCreateWithFlags(&X.side, cudaStreamNonBlocking));
-        for (cudaEvent_t &e : X.ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        for (int k = 0; k < flite_ctx::kBranches; ++k) {
+            CK(cudaStreamCreateWithFlags(&X.branch[k], cudaStreamNonBlocking));
+            CK(cudaEventCreateWithFlags(&X.forked[k], cudaEventDisableTiming));
+            CK(cudaEventCreateWithFlags(&X.done[k], cudaEventDisableTiming));
+        }
+        CK(cudaEventCreateWithFlags(&X.coarse_ready, cudaEventDisableTiming));
         CK(cudaMallocHost(&X.h_cycle, sizeof(int)));
         X.d_cycle = X.alloc<int>(1);
         X.d_cyc = X.alloc<int>(G);
@@ -518,10 +522,11 @@ int flite::create_context(const flite_controls *c, int nlevels, const flite_leve
                 L.turbDiff = X.alloc<double>(N); L.dtT = X.alloc<double>(N);
                 L.vort = X.alloc<double>(N); L.divg = X.alloc<double>(N);
                 L.sag = X.alloc<double>(3 * (size_t)N); L.sanh = X.alloc<double>(N);
+                L.saprim = X.alloc<double>(3 * (size_t)N); L.savis = X.alloc<double>(N);
                 for (double *a : {L.turbDiff, L.dtT, L.vort, L.divg, L.sanh})
                     CK(cudaMemset(a, 0, (size_t)N * sizeof(double)));
             } else {
-                L.turbDiff = L.dtT = L.vort = L.divg = L.sag = L.sanh = nullptr;
+                L.turbDiff = L.dtT = L.vort = L.divg = L.sag = L.sanh = L.saprim = L.savis = nullptr;
             }
             for (double *a : {L.p, L.dt, L.mu, L.hvis}) CK(cudaMemset(a, 0, (size_t)N * sizeof(double)));
             const bool hllc2 = c->fluxType == 4 && c->HLLCFluxOrder > 1 && l == 0;

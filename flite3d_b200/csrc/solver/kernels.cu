@@ -24,76 +24,13 @@
 #include <cuda_runtime.h>
 
 #include "flux.cuh"
+#include "gather.cuh"
 #include "kernels.h"
 #include "pinned_math.h"
 
 namespace flite {
 
 static __device__ __forceinline__ int tid() { return blockIdx.x * blockDim.x + threadIdx.x; }
-
-// Group-per-node gathers (small levels): U lanes (a power of two up to 32)
-// serve one node, M sums of the node take R terms each from every incidence.
-// Lane l of the group evaluates the M*R terms of incidence k0 + l and leaves
-// them in the warp's shared slab gs[term][lane] (rows of 33 values: the lanes
-// that read different terms of one incidence hit different banks); lane m of
-// the group then adds sum m's terms in incidence order, so the sums are those
-// of the serial loop bit for bit (lanes past the last incidence leave zeros,
-// and x + 0 is x).  `out` holds the sums so far on entry and the new ones, in
-// every lane, on return.  Groups past the last node stay in the loop (the
-// warp's barriers need every lane) but add nothing.
-// What bounds it: the latency of one node's chain.  The serial part is one
-// add per term on M lanes at once; broadcasting every term to every lane
-// instead takes 2 M R shuffles and M R adds per incidence of the warp.
-constexpr int kSlabRow = 33;
-template <int U, int M, int R, class T, class Terms>
-__device__ __forceinline__ void group_sum(T *gs, int beg, int end, bool active, int gl, Terms &&terms, T *out) {
-    constexpr int C = (M + U - 1) / U;  // sums per lane
-    constexpr int S = U < 8 ? U : 8;    // incidences added per step
-    const int lane = (int)(threadIdx.x & 31), g0 = lane - gl;
-    T acc[C];
-#pragma unroll
-    for (int c = 0; c < C; ++c) acc[c] = T(0);
-#pragma unroll
-    for (int m = 0; m < M; ++m)
-        if (m % U == gl) acc[m / U] = out[m];
-    const int span = active ? end - beg : 0;
-    const int longest = (int)__reduce_max_sync(0xffffffffu, (unsigned)span);
-    for (int t = 0; t < longest; t += U) {
-        T v[M * R];
-#pragma unroll
-        for (int c = 0; c < M * R; ++c) v[c] = T(0);
-        if (t + gl < span) terms(beg + t + gl, v);
-#pragma unroll
-        for (int c = 0; c < M * R; ++c) gs[c * kSlabRow + lane] = v[c];
-        __syncwarp();
-        const int n = min(U, longest - t);
-        for (int q = 0; q < n; q += S) {
-            T x[C][S][R];
-#pragma unroll
-            for (int c = 0; c < C; ++c) {
-                const int m = gl + c * U < M ? gl + c * U : 0;
-#pragma unroll
-                for (int k = 0; k < S; ++k)
-#pragma unroll
-                    for (int r = 0; r < R; ++r) x[c][k][r] = gs[(m * R + r) * kSlabRow + g0 + q + k];
-            }
-#pragma unroll
-            for (int k = 0; k < S; ++k)
-#pragma unroll
-                for (int r = 0; r < R; ++r)
-#pragma unroll
-                    for (int c = 0; c < C; ++c) acc[c] = acc[c] + x[c][k][r];
-        }
-        __syncwarp();
-    }
-#pragma unroll
-    for (int m = 0; m < M; ++m) out[m] = __shfl_sync(0xffffffffu, acc[m / U], m % U, U);
-}
-// the calling warp's slab of K terms out of the block's (blocks of at most
-// 256 threads)
-#define FLITE_GROUP_SLAB(T, K)                                   \
-    __shared__ T gslab_[U > 1 ? 8 * (K)*kSlabRow : 1];           \
-    T *gs = gslab_ + (U > 1 ? (threadIdx.x >> 5) * (K)*kSlabRow : 0)
 
 // ---- makePressureField (def_par:13612-13630) ------------------------------
 // One pass over the state: the pressure, the node records, and on request the
@@ -133,6 +70,7 @@ __global__ void k_state_pass(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_, in
     const double p = pressure(P, r, ru, rv, rw, E);
     L.p[i] = p;
     if (what & STATE_REC) store_node(L.q, i, r, ru, rv, rw, E, p);
+    if (L.saprim) store_saprim(L, i, r, ru, rv, rw);
     if (what & STATE_HPRIM) { L.hprim[i] = ru / r; L.hprim[N + i] = rv / r; L.hprim[2 * N + i] = rw / r; }
     if (what & STATE_PRIM) {
         const double gOg = P.gamma / (P.gamma - 1.0);
@@ -2106,6 +2044,7 @@ __device__ __forceinline__ void node_tail(const Params &P, const LevelView &L, i
         if (io & IO_EMIT) {  // makePressureField of the next stage
             const double p = pressure(P, un[0], un[1], un[2], un[3], un[4]);
             L.p[i] = p;
+            if (L.saprim) store_saprim(L, i, un[0], un[1], un[2], un[3]);
             if constexpr (PREC == GATHER_BUFFER)
                 if (L.hprim) {
                     L.hprim[i] = un[1] / un[0]; L.hprim[N + i] = un[2] / un[0]; L.hprim[2 * N + i] = un[3] / un[0];
@@ -2358,6 +2297,7 @@ __global__ void k_restrict_state(CaseArg<B, Params> P_, CaseArg<B, LevelView> C_
     const double p = fabs(pressure(P, v[0], v[1], v[2], v[3], v[4]));
     C.p[c] = p;
     store_node(C.q, c, v[0], v[1], v[2], v[3], v[4], p);
+    if (C.saprim) store_saprim(C, c, v[0], v[1], v[2], v[3]);
     if (C.prim) {  // the viscous primitives (k_state_pass)
         const double gOg = P.gamma / (P.gamma - 1.0);
         C.prim[c] = v[1] / v[0];

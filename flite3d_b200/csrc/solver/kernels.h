@@ -94,9 +94,12 @@ constexpr int kSharedWalkNodes = 220000;
 constexpr int kMaxLevels = 16;
 template <bool B = false>
 __global__ void k_delta_state(CaseArg<B, LevelView> L);
-__global__ void k_sa_timestep(Params P, LevelView L);
-__global__ void k_sa_grad(Params P, LevelView L);
+// the turbulent time step (ts) and the nu~ gradient in one walk
+template <int U>
+__global__ void k_sa_grad(Params P, LevelView L, int ts);
+template <int U>
 __global__ void k_sa_diff(Params P, LevelView L);
+template <int U>
 __global__ void k_sa_conv(Params P, LevelView L, int td);
 __global__ void k_sa_stage(Params P, LevelView L, int mode, int stage, int turb);
 // set-up of a level's edges on the device (kernels.cu)

@@ -5,8 +5,8 @@
 // edge order (then the boundary edges in their order), and every expression
 // keeps the reference's operation order, so the results equal the CPU
 // restatement bit for bit:
-//   k_sa_timestep  makeTurbulentTimeSteps  (def_par:12878-13100)
-//   k_sa_grad      makeSADiffusion pass 1  (def_par:7436-7560): Galerkin
+//   k_sa_grad      makeTurbulentTimeSteps  (def_par:12878-13100) and
+//                  makeSADiffusion pass 1  (def_par:7436-7560): Galerkin
 //                  gradient of nu~ and the cb2 term
 //   k_sa_diff      makeSADiffusion pass 2  (def_par:7560-7809)
 //   k_sa_conv      makeSARHS               (def_par:6809-6950)
@@ -20,7 +20,7 @@
 // reads the stage-start density, which that update overwrites.
 #include <cuda_runtime.h>
 
-#include "device.cuh"
+#include "gather.cuh"
 #include "kernels.h"
 #include "pinned_math.h"
 
@@ -35,149 +35,226 @@ __device__ __forceinline__ double rp_exhaust(const Params &P, const LevelView &L
 }
 }  // namespace
 
-__global__ void k_sa_timestep(Params P, LevelView L) {
-    int i = tid();
-    if (i >= L.N) return;
+// The gathers take a thread or a group of lanes per node (lanes_of): on the
+// coarse levels of a 738,100-node mesh (78,360 to 53 nodes) a thread per node
+// takes 10 to 30 us a launch, one thread's chain of loads and divisions.
+//
+// makeTurbulentTimeSteps (def_par:12878-13100, ts) and the Galerkin gradient of
+// nu~ with the cb2 term of makeSADiffusion (def_par:7436-7560), which read nu~ of
+// the same neighbours
+namespace {
+struct SaConst {
+    double oneOverSigma = 3.0 / 2.0, oneOverKappaSquared = 1.0 / (0.41 * 0.41);
+    double cb1 = 0.1355, cb2 = 0.622, ct3 = 1.1;
+};
+// the terms of incidence t: v[0] the convective term, v[1] the other node's
+// diffusion term (def_par:12930-12935)
+__device__ __forceinline__ void sa_ts_terms(const Params &P, const LevelView &L, const int2 t, const double *m,
+                                            double ro, double oRe, double *v) {
+    const SaConst k;
+    const int N = L.N, e = t.x >= 0 ? t.x : ~t.x, j = t.y;
+    const double wx = L.wx[e], wy = L.wy[e], wz = L.wz[e];
+    const double al = (wx * wx + wy * wy) + wz * wz;
+    const double vn = ((wx * m[0] + wy * m[1]) + wz * m[2]) * ro;
+    v[0] = P.turbK * sqrt(al) + fabs(vn);
+    const double vis = k.oneOverSigma * (L.mu[j] + 3.0 * k.cb2 * L.u[5 * (size_t)N + j] * oRe);
+    v[1] = 2.0 * vis * al;
+}
+// boundary entry q: the two terms of each of the two sums
+__device__ __forceinline__ void sa_ts_bterms(const Params &P, const LevelView &L, int q, double oRe, double *v) {
+    const SaConst k;
     const int N = L.N;
-    const double* __restrict__ nt = L.u + 5 * (size_t)N;
-    const double oneOverSigma = 3.0 / 2.0, oneOverKappaSquared = 1.0 / (0.41 * 0.41);
-    const double cb1 = 0.1355, cb2 = 0.622, ct3 = 1.1;
-    const double cw1 = cb1 * oneOverKappaSquared + (1.0 + cb2) * oneOverSigma;
-    const double oRe = 1.0 / P.Re;
-    const double ro = 1. / L.u[i];
-    const double m1 = L.u[N + i], m2 = L.u[2 * N + i], m3 = L.u[3 * N + i];
-    double acc = 0.0, h = 0.0;
-    FLITE_FOR_INC(L, i, t) {
-        const int e = t.x >= 0 ? t.x : ~t.x, j = t.y;
-        const double wx = L.wx[e], wy = L.wy[e], wz = L.wz[e];
-        const double al = (wx * wx + wy * wy) + wz * wz;
-        double vn = ((wx * m1 + wy * m2) + wz * m3) * ro;
-        vn = P.turbK * sqrt(al) + fabs(vn);
-        acc = acc + vn;
-        // the other node's diffusion term (def_par:12930-12935)
-        const double vis = oneOverSigma * (L.mu[j] + 3.0 * cb2 * nt[j] * oRe);
-        const double dv = 2.0 * vis * al;
-        h = h + dv;
-    }
-    for (int k = L.binc_ptr[i]; k < L.binc_ptr[i + 1]; ++k) {
-        const int b = L.binc[k] >> 1, side = L.binc[k] & 1;
-        const int2 nd = L.bedge[b];
-        const double wx = L.bwx[b], wy = L.bwy[b], wz = L.bwz[b];
-        const double al = (wx * wx + wy * wy) + wz * wz;
-        const int j1 = nd.x, j2 = nd.y;
-        const double ro1 = 1. / L.u[j1], ro2 = 1. / L.u[j2];
-        double vn1 = ((wx * L.u[N + j1] + wy * L.u[2 * N + j1]) + wz * L.u[3 * N + j1]) * ro1;
-        double vn2 = ((wx * L.u[N + j2] + wy * L.u[2 * N + j2]) + wz * L.u[3 * N + j2]) * ro2;
-        vn1 = P.turbK * sqrt(al) + fabs(vn1);
-        vn2 = P.turbK * sqrt(al) + fabs(vn2);
-        const double vnm = vn1 + vn2;
-        acc = side == 0 ? (acc + vn1) + vnm : (acc + vn2) + vnm;
-        const double vis1 = oneOverSigma * (L.mu[j1] + 3.0 * cb2 * nt[j1] * oRe);
-        const double vis2 = oneOverSigma * (L.mu[j2] + 3.0 * cb2 * nt[j2] * oRe);
-        const double dv1 = 2.0 * vis1 * al, dv2 = 2.0 * vis2 * al;
-        const double dvm = dv1 + dv2;
-        h = side == 0 ? (h + dv1) + dvm : (h + dv2) + dvm;
-    }
+    const double *nt = L.u + 5 * (size_t)N;
+    const int b = L.binc[q] >> 1, side = L.binc[q] & 1;
+    const int2 nd = L.bedge[b];
+    const double wx = L.bwx[b], wy = L.bwy[b], wz = L.bwz[b];
+    const double al = (wx * wx + wy * wy) + wz * wz;
+    const int j1 = nd.x, j2 = nd.y;
+    const double ro1 = 1. / L.u[j1], ro2 = 1. / L.u[j2];
+    double vn1 = ((wx * L.u[N + j1] + wy * L.u[2 * N + j1]) + wz * L.u[3 * N + j1]) * ro1;
+    double vn2 = ((wx * L.u[N + j2] + wy * L.u[2 * N + j2]) + wz * L.u[3 * N + j2]) * ro2;
+    vn1 = P.turbK * sqrt(al) + fabs(vn1);
+    vn2 = P.turbK * sqrt(al) + fabs(vn2);
+    v[0] = side == 0 ? vn1 : vn2;
+    v[1] = vn1 + vn2;
+    const double vis1 = k.oneOverSigma * (L.mu[j1] + 3.0 * k.cb2 * nt[j1] * oRe);
+    const double vis2 = k.oneOverSigma * (L.mu[j2] + 3.0 * k.cb2 * nt[j2] * oRe);
+    const double dv1 = 2.0 * vis1 * al, dv2 = 2.0 * vis2 * al;
+    v[2] = side == 0 ? dv1 : dv2;
+    v[3] = dv1 + dv2;
+}
+__device__ __forceinline__ void sa_ts_store(const LevelView &L, int i, double acc, double h, double oRe) {
+    const SaConst k;
+    const double cw1 = k.cb1 * k.oneOverKappaSquared + (1.0 + k.cb2) * k.oneOverSigma;
+    const double nti = L.u[5 * (size_t)L.N + i];
     const double V = L.V[i];
     const double dt = 0.5 / (acc / V + h / (V * V));
     double dInvSquared = L.wdist[i] > 1.0e-10 ? 1.0 / L.wdist[i] : 1.0e10;
     dInvSquared = dInvSquared * dInvSquared;
     const double S = (fabs(L.divg[i]) +
-                      cb1 * (L.vort[i] + (1.0 + ct3) * nt[i] * oneOverKappaSquared * dInvSquared * oRe)) +
-                     cw1 * nt[i] * dInvSquared * oRe;
+                      k.cb1 * (L.vort[i] + (1.0 + k.ct3) * nti * k.oneOverKappaSquared * dInvSquared * oRe)) +
+                     cw1 * nti * dInvSquared * oRe;
     L.dtT[i] = dt / (1.0 + 0.5 * S * dt);
 }
-
-__global__ void k_sa_grad(Params P, LevelView L) {
-    int i = tid();
-    if (i >= L.N) return;
-    const int N = L.N;
-    const double* __restrict__ nt = L.u + 5 * (size_t)N;
-    const double ti = nt[i];
-    double g0 = 0.0, g1 = 0.0, g2 = 0.0;
-    FLITE_FOR_INC(L, i, t) {
-        const int e = t.x >= 0 ? t.x : ~t.x;
-        const double tj = nt[t.y];
-        const double s = t.x >= 0 ? ti + tj : tj + ti;  // (nu1 + nu2) in the edge's order
-        const double f1 = L.wx[e] * s, f2 = L.wy[e] * s, f3 = L.wz[e] * s;
-        if (t.x >= 0) { g0 = g0 + f1; g1 = g1 + f2; g2 = g2 + f3; }
-        else { g0 = g0 - f1; g1 = g1 - f2; g2 = g2 - f3; }
+// the gradient terms of incidence t (ti: this node's nu~), with its sign
+__device__ __forceinline__ void sa_grad_terms(const LevelView &L, const int2 t, double ti, double *v) {
+    const int e = t.x >= 0 ? t.x : ~t.x;
+    const double tj = L.u[5 * (size_t)L.N + t.y];
+    const double s = t.x >= 0 ? ti + tj : tj + ti;  // (nu1 + nu2) in the edge's order
+    const double f[3] = {L.wx[e] * s, L.wy[e] * s, L.wz[e] * s};
+    for (int c = 0; c < 3; ++c) v[c] = t.x >= 0 ? f[c] : -f[c];
+}
+__device__ __forceinline__ void sa_grad_bterms(const Params &P, const LevelView &L, int q, double *v) {
+    const double *nt = L.u + 5 * (size_t)L.N;
+    const int b = L.binc[q] >> 1, side = L.binc[q] & 1;
+    const int2 nd = L.bedge[b];
+    const double w[3] = {L.bwx[b], L.bwy[b], L.bwz[b]};
+    const double t1 = nt[nd.x], t2 = nt[nd.y];
+    if (P.boundaryTerm == 1) {
+        const double a = side == 0 ? 3. * t1 + t2 : t1 + 3. * t2;
+        for (int c = 0; c < 3; ++c) v[c] = a * w[c];
+    } else {
+        const double a = side == 0 ? t1 : t2;
+        for (int c = 0; c < 3; ++c) v[c] = 4. * a * w[c];
     }
-    for (int k = L.binc_ptr[i]; k < L.binc_ptr[i + 1]; ++k) {
-        const int b = L.binc[k] >> 1, side = L.binc[k] & 1;
-        const int2 nd = L.bedge[b];
-        const double wx = L.bwx[b], wy = L.bwy[b], wz = L.bwz[b];
-        const double t1 = nt[nd.x], t2 = nt[nd.y];
-        if (P.boundaryTerm == 1) {
-            const double a = side == 0 ? 3. * t1 + t2 : t1 + 3. * t2;
-            g0 = g0 + a * wx; g1 = g1 + a * wy; g2 = g2 + a * wz;
-        } else {
-            const double a = side == 0 ? t1 : t2;
-            g0 = g0 + 4. * a * wx; g1 = g1 + 4. * a * wy; g2 = g2 + 4. * a * wz;
+}
+}  // namespace
+
+// the node, lane and idle groups of a gather kernel
+#define SA_NODE()                                                    \
+    const int gl = U > 1 ? (int)(threadIdx.x % U) : 0;               \
+    const int i_raw = U > 1 ? tid() / U : tid();                     \
+    if (U == 1 && i_raw >= L.N) return;                              \
+    const bool active = i_raw < L.N;                                 \
+    const int i = active ? i_raw : L.N - 1;                          \
+    const int N = L.N
+
+template <int U>
+__global__ void k_sa_grad(Params P, LevelView L, int ts) {
+    SA_NODE();
+    const double oRe = 1. / P.Re;
+    const double ti = L.u[5 * (size_t)N + i];
+    const double ri = L.u[i], ro = 1. / ri;
+    const double m[3] = {L.u[N + i], L.u[2 * N + i], L.u[3 * N + i]};
+    double g[3] = {0.0, 0.0, 0.0}, x[2] = {0.0, 0.0};
+    if constexpr (U > 1) {
+        FLITE_GROUP_SLAB(double, 4);
+        if (ts) {
+            group_sum<U, 2, 1, double>(
+                gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl,
+                [&](int q, double *v) { sa_ts_terms(P, L, L.inc[q], m, ro, oRe, v); }, x);
+            group_sum<U, 2, 2, double>(
+                gs, L.binc_ptr[i], L.binc_ptr[i + 1], active, gl,
+                [&](int q, double *v) { sa_ts_bterms(P, L, q, oRe, v); }, x);
+        }
+        group_sum<U, 3, 1, double>(
+            gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl,
+            [&](int q, double *v) { sa_grad_terms(L, L.inc[q], ti, v); }, g);
+        group_sum<U, 3, 1, double>(
+            gs, L.binc_ptr[i], L.binc_ptr[i + 1], active, gl,
+            [&](int q, double *v) { sa_grad_bterms(P, L, q, v); }, g);
+        if (!active || gl) return;
+    } else {
+        FLITE_FOR_INC(L, i, t) {
+            double v[3];
+            if (ts) {
+                sa_ts_terms(P, L, t, m, ro, oRe, v);
+                x[0] = x[0] + v[0];
+                x[1] = x[1] + v[1];
+            }
+            sa_grad_terms(L, t, ti, v);
+            for (int c = 0; c < 3; ++c) g[c] = g[c] + v[c];
+        }
+        for (int q = L.binc_ptr[i]; q < L.binc_ptr[i + 1]; ++q) {
+            double v[4];
+            if (ts) {
+                sa_ts_bterms(P, L, q, oRe, v);
+                x[0] = (x[0] + v[0]) + v[1];
+                x[1] = (x[1] + v[2]) + v[3];
+            }
+            sa_grad_bterms(P, L, q, v);
+            for (int c = 0; c < 3; ++c) g[c] = g[c] + v[c];
         }
     }
-    const double sigma = 2. / 3., cb2 = 0.622, oRe = 1. / P.Re;
+    if (ts) sa_ts_store(L, i, x[0], x[1], oRe);
+    const double sigma = 2. / 3., cb2 = 0.622;
     const double fact = oRe * cb2 / sigma;
     const double vt = 1. / L.V[i];
-    const double dx = g0 * vt, dy = g1 * vt, dz = g2 * vt;
+    const double dx = g[0] * vt, dy = g[1] * vt, dz = g[2] * vt;
     L.sag[i] = dx;
     L.sag[N + i] = dy;
     L.sag[2 * N + i] = dz;
-    const double vp = (g0 * dx + g1 * dy) + g2 * dz;
+    const double vp = (g[0] * dx + g[1] * dy) + g[2] * dz;
     L.sanh[i] = 0.0 - fact * vp;
+    L.savis[i] = P.Re * L.mu[i] / ri + ti;
 }
 
+// makeSADiffusion's edge terms (def_par:7560-7809): the viscosity of a node
+// (savis) and its gradient are this launch's input from k_sa_grad
+template <int U>
 __global__ void k_sa_diff(Params P, LevelView L) {
-    int i = tid();
-    if (i >= L.N) return;
-    const int N = L.N;
-    const double* __restrict__ nt = L.u + 5 * (size_t)N;
+    SA_NODE();
     const double sigma = 2. / 3., oRe = 1. / P.Re;
     const double fact = oRe / sigma;
-    auto visc = [&](int n) { return P.Re * L.mu[n] / L.u[n] + nt[n]; };
     auto fd = [&](int n, double wx, double wy, double wz) {
-        return visc(n) * ((wx * L.sag[n] + wy * L.sag[N + n]) + wz * L.sag[2 * N + n]);
+        return L.savis[n] * ((wx * L.sag[n] + wy * L.sag[N + n]) + wz * L.sag[2 * N + n]);
     };
-    double acc = 0.0;
-    FLITE_FOR_INC(L, i, t) {
+    const double vi = L.savis[i], gi[3] = {L.sag[i], L.sag[N + i], L.sag[2 * N + i]};
+    auto terms = [&](const int2 t, double *v) {
         const int e = t.x >= 0 ? t.x : ~t.x;
-        const int n1 = t.x >= 0 ? i : t.y, n2 = t.x >= 0 ? t.y : i;
         const double wx = L.wx[e], wy = L.wy[e], wz = L.wz[e];
-        const double fd1 = fd(n1, wx, wy, wz), fd2 = fd(n2, wx, wy, wz);
-        acc = t.x >= 0 ? acc - fact * (fd1 + fd2) : acc + fact * (fd1 + fd2);
-    }
-    for (int k = L.binc_ptr[i]; k < L.binc_ptr[i + 1]; ++k) {
-        const int b = L.binc[k] >> 1, side = L.binc[k] & 1;
+        const double fi = vi * ((wx * gi[0] + wy * gi[1]) + wz * gi[2]), fj = fd(t.y, wx, wy, wz);
+        const double f = fact * (t.x >= 0 ? fi + fj : fj + fi);
+        v[0] = t.x >= 0 ? -f : f;
+    };
+    auto bterms = [&](int q, double *v) {
+        const int b = L.binc[q] >> 1, side = L.binc[q] & 1;
         const int2 nd = L.bedge[b];
         const double wx = L.bwx[b], wy = L.bwy[b], wz = L.bwz[b];
         const double fd1 = fd(nd.x, wx, wy, wz), fd2 = fd(nd.y, wx, wy, wz);
-        if (P.boundaryTerm == 1) acc = acc - fact * (side == 0 ? 3. * fd1 + fd2 : fd1 + 3. * fd2);
-        else acc = acc - fact * 4. * (side == 0 ? fd1 : fd2);
+        if (P.boundaryTerm == 1) v[0] = -(fact * (side == 0 ? 3. * fd1 + fd2 : fd1 + 3. * fd2));
+        else v[0] = -(fact * 4. * (side == 0 ? fd1 : fd2));
+    };
+    double acc[1] = {0.0};
+    if constexpr (U > 1) {
+        FLITE_GROUP_SLAB(double, 1);
+        group_sum<U, 1, 1, double>(
+            gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl, [&](int q, double *v) { terms(L.inc[q], v); }, acc);
+        group_sum<U, 1, 1, double>(gs, L.binc_ptr[i], L.binc_ptr[i + 1], active, gl, bterms, acc);
+        if (!active || gl) return;
+    } else {
+        double v[1];
+        FLITE_FOR_INC(L, i, t) {
+            terms(t, v);
+            acc[0] = acc[0] + v[0];
+        }
+        for (int q = L.binc_ptr[i]; q < L.binc_ptr[i + 1]; ++q) {
+            bterms(q, v);
+            acc[0] = acc[0] + v[0];
+        }
     }
-    L.turbDiff[i] = acc + L.sanh[i];
+    L.turbDiff[i] = acc[0] + L.sanh[i];
 }
 
+// makeSARHS (def_par:6809-6950): the nu~ convection, velocities from saprim
+template <int U>
 __global__ void k_sa_conv(Params P, LevelView L, int td) {
-    int i = tid();
-    if (i >= L.N) return;
-    const int N = L.N;
+    SA_NODE();
     const double* __restrict__ nt = L.u + 5 * (size_t)N;
     auto prim = [&](int n, double *q) {
-        const double rinv = 1. / L.u[n];
-        q[0] = rinv * L.u[N + n]; q[1] = rinv * L.u[2 * N + n]; q[2] = rinv * L.u[3 * N + n];
+        q[0] = L.saprim[n]; q[1] = L.saprim[N + n]; q[2] = L.saprim[2 * (size_t)N + n];
         q[3] = nt[n];
     };
     double qi[4];
     prim(i, qi);
-    // an unsteady stage's time difference comes first (def_par:1073)
-    double acc = td ? time_difference(P, L, L.u, i, 5) : 0.0;
-    FLITE_FOR_INC(L, i, t) {
+    auto terms = [&](const int2 t, double *v) {
         const int e = t.x >= 0 ? t.x : ~t.x;
         double qj[4];
         prim(t.y, qj);
-        const double *a = t.x >= 0 ? qi : qj, *b = t.x >= 0 ? qj : qi;
-        const double u1 = a[0], v1 = a[1], w1 = a[2], t1 = a[3];
-        const double u2 = b[0], v2 = b[1], w2 = b[2], t2 = b[3];
+        const bool first = t.x >= 0;
+        const double u1 = first ? qi[0] : qj[0], v1 = first ? qi[1] : qj[1], w1 = first ? qi[2] : qj[2];
+        const double u2 = first ? qj[0] : qi[0], v2 = first ? qj[1] : qi[1], w2 = first ? qj[2] : qi[2];
+        const double t1 = first ? qi[3] : qj[3], t2 = first ? qj[3] : qi[3];
         const double wx = L.wx[e], wy = L.wy[e], wz = L.wz[e];
         double fconv = (wx * (u1 * t1 + u2 * t2) + wy * (v1 * t1 + v2 * t2)) + wz * (w1 * t1 + w2 * t2);
         if (fabs(t1 - t2) > 1.0e-20) {
@@ -186,10 +263,35 @@ __global__ void k_sa_conv(Params P, LevelView L, int td) {
             const double az = (w2 * t2 - w1 * t1) / (t1 - t2);
             fconv = fconv + fabs((wx * ax + wy * ay) + wz * az) * (t1 - t2);
         }
-        acc = t.x >= 0 ? acc + fconv : acc - fconv;
+        v[0] = first ? fconv : -fconv;
+    };
+    // an unsteady stage's time difference comes first (def_par:1073)
+    double acc[1] = {td ? time_difference(P, L, L.u, i, 5) : 0.0};
+    if constexpr (U > 1) {
+        FLITE_GROUP_SLAB(double, 1);
+        group_sum<U, 1, 1, double>(
+            gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl, [&](int q, double *v) { terms(L.inc[q], v); }, acc);
+        if (!active || gl) return;
+    } else {
+        FLITE_FOR_INC(L, i, t) {
+            double v[1];
+            terms(t, v);
+            acc[0] = acc[0] + v[0];
+        }
     }
-    L.rhs[5 * (size_t)N + i] = acc;
+    L.rhs[5 * (size_t)N + i] = acc[0];
 }
+#undef SA_NODE
+#define SA_INST(U)                                                  \
+    template __global__ void k_sa_grad<U>(Params, LevelView, int);  \
+    template __global__ void k_sa_diff<U>(Params, LevelView);       \
+    template __global__ void k_sa_conv<U>(Params, LevelView, int);
+SA_INST(1)
+SA_INST(4)
+SA_INST(8)
+SA_INST(16)
+SA_INST(32)
+#undef SA_INST
 
 // makeSASourceTerm at node i added to r; the laminar viscosity floor writes
 // 0.1*Re into the array, as the reference does (def_par:9321-9323)
