@@ -295,6 +295,7 @@ int flite::create_context(const flite_controls *c, int nlevels, const flite_leve
         }
         CK(cudaEventCreateWithFlags(&X.coarse_ready, cudaEventDisableTiming));
         CK(cudaMallocHost(&X.h_cycle, sizeof(int)));
+        CK(cudaMallocHost(&X.h_out, 32 * sizeof(double)));
         X.d_cycle = X.alloc<int>(1);
         X.d_cyc = X.alloc<int>(G);
         {
@@ -303,7 +304,6 @@ int flite::create_context(const flite_controls *c, int nlevels, const flite_leve
             CK(cudaMemcpy(X.d_cyc, cyc0.data(), G * sizeof(int), cudaMemcpyHostToDevice));
         }
         X.d_part = X.alloc<double>(kResidBlocks * 18);
-        X.d_out = X.alloc<double>(32);
         // ivd%physicalTimeStep, which explicit time stepping overwrites
         X.d_ptsg = X.alloc<double>(1);
         CK(cudaMemcpy(X.d_ptsg, &c->physicalTimeStep, sizeof(double), cudaMemcpyHostToDevice));
@@ -801,10 +801,10 @@ int flite_residuals(flite_ctx *ctx, double res[7], double maxres[7], int32_t max
     return guarded(ctx, [&] {
         flite_ctx &X = *ctx;
         const LevelView &L = X.c.multigridScheme > 0 ? X.V(0) : X.V((int)X.lv.size() - 1);
-        k_resid_partial<<<kResidBlocks, 256, 0, X.s>>>(L, X.d_part, kResidBlocks);
-        k_resid_final<<<1, 192, 0, X.s>>>(X.d_part, kResidBlocks, X.d_out);
-        double h[18];
-        CK(cudaMemcpyAsync(h, X.d_out, sizeof h, cudaMemcpyDeviceToHost, X.s));
+        k_resid_partial<<<kResidBlocks, 256, 0, X.s>>>(L, X.d_part);
+        k_resid_final<<<1, 192, 0, X.s>>>(X.d_part, X.h_out);
+        CK(cudaGetLastError());
+        const double *h = X.h_out;
         CK(cudaStreamSynchronize(X.s));
         for (int k = 0; k < 7; ++k) { res[k] = 0.0; maxres[k] = 0.0; maxind[k] = 1; }
         bool finite = true;
@@ -834,15 +834,15 @@ int flite_forces(flite_ctx *ctx, double out[9]) {
         double *part1 = X.d_part, *part3 = X.d_part + 6 * kForceBlocks;
         k_forces<<<kForceBlocks, 256, 0, X.s>>>(X.P, D.v, D.d_wall, (int)D.wall.size(), aR, bR, X.c.groundplane,
                                                X.c.datum[0], X.c.datum[1], X.c.datum[2], part1);
-        k_forces_final<<<1, 32, 0, X.s>>>(part1, kForceBlocks, 6, X.d_out);
+        k_forces_final<<<1, 32, 0, X.s>>>(part1, 6, X.h_out);
         if (calc3) {
             k_forces3<<<kForceBlocks, 256, 0, X.s>>>(X.P, D.v, D.d_wall, (int)D.wall.size(), aR, bR,
                                                     X.c.groundplane, X.c.datum[0], X.c.datum[1], X.c.datum[2],
                                                     part3);
-            k_forces_final<<<1, 32, 0, X.s>>>(part3, kForceBlocks, 7, X.d_out + 8);
+            k_forces_final<<<1, 32, 0, X.s>>>(part3, 7, X.h_out + 8);
         }
-        double h[15];
-        CK(cudaMemcpyAsync(h, X.d_out, sizeof h, cudaMemcpyDeviceToHost, X.s));
+        CK(cudaGetLastError());
+        const double *h = X.h_out;
         CK(cudaStreamSynchronize(X.s));
         const double A = X.c.referenceArea;
         // lift, drag, latF, frictionDrag as coefficients; latM, longM as sums

@@ -2561,9 +2561,24 @@ template __global__ void k_case_save_u<true>(CaseTab<LevelView>, size_t);
 template __global__ void k_case_zero<false>(LevelView, int, size_t);
 template __global__ void k_case_zero<true>(CaseTab<LevelView>, int, size_t);
 
+// ---- block sums -----------------------------------------------------------
+// The sum of v[0..255] by halving (v[t] += v[t + w], w = 128, 64, ..., 1), by
+// one warp: the pairs of the first three halvings are added from shared
+// memory, the rest by shuffles, with one barrier before instead of eight.
+__device__ __forceinline__ double sum256(const double *v, int lane) {
+    const double a = (v[lane] + v[lane + 128]) + (v[lane + 64] + v[lane + 192]);
+    const double b = (v[lane + 32] + v[lane + 160]) + (v[lane + 96] + v[lane + 224]);
+    double s = a + b;
+    for (int w = 16; w > 0; w >>= 1) s += __shfl_down_sync(0xffffffffu, s, w);
+    return s;  // lane 0's
+}
+
 // ---- residual norms (writeResiduals mg_par:1299-1443) ---------------------
-// per block: sum (u-uprev)^2 and max |u-uprev| with its first index
-__global__ void k_resid_partial(LevelView L, double *part, int nblk) {
+// per block: sum (u-uprev)^2 and max |u-uprev| with its first index; a batch
+// takes all its cases in one launch (the case in blockIdx.y)
+template <bool B>
+__global__ void __launch_bounds__(256) k_resid_partial(CaseArg<B, LevelView> L_, double *part) {
+    FLITE_CASE_L(B, L);
     __shared__ double ss[6][256];
     __shared__ double sm[6][256];
     __shared__ int si[6][256];
@@ -2573,44 +2588,56 @@ __global__ void k_resid_partial(LevelView L, double *part, int nblk) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
         // the first node in the caller's numbering wins a tie (mg_par:1387-1396)
         const int oi = L.perm ? L.perm[i] : i;
-        for (int k = 0; k < nv; ++k) {
-            double d = L.u[k * N + i] - L.uprev[k * N + i];
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+            if (k >= nv) break;
+            const double d = L.u[(size_t)k * N + i] - L.uprev[(size_t)k * N + i];
             s[k] = s[k] + d * d;
-            double a = fabs(d);
+            const double a = fabs(d);
             if (a > m[k] || (a == m[k] && a > 0.0 && oi < mi[k])) { m[k] = a; mi[k] = oi; }
         }
     }
+#pragma unroll
     for (int k = 0; k < 6; ++k) { ss[k][threadIdx.x] = s[k]; sm[k][threadIdx.x] = m[k]; si[k][threadIdx.x] = mi[k]; }
     __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w) {
-            for (int k = 0; k < 6; ++k) {
-                ss[k][threadIdx.x] += ss[k][threadIdx.x + w];
-                double a = sm[k][threadIdx.x], b = sm[k][threadIdx.x + w];
-                int ia = si[k][threadIdx.x], ib = si[k][threadIdx.x + w];
-                if (b > a || (b == a && ib < ia)) { sm[k][threadIdx.x] = b; si[k][threadIdx.x] = ib; }
-            }
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        for (int k = 0; k < 6; ++k) {
-            part[blockIdx.x * 18 + k] = ss[k][0];
-            part[blockIdx.x * 18 + 6 + k] = sm[k][0];
-            part[blockIdx.x * 18 + 12 + k] = (double)si[k][0];
-        }
-    }
-}
-
-// one warp per component (blockDim.x = 192); each lane folds the block
-// partials b = lane, lane+32, ... and the warp combines the lanes in a fixed
-// tree, so the result does not depend on timing
-__global__ void k_resid_final(const double *part, int nblk, double *out) {
+    // a warp per component
     const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (k >= 6) return;
+    const double sum = sum256(ss[k], lane);
+    double v = 0.0;
+    int iv = 0x7fffffff;
+#pragma unroll
+    for (int t = lane; t < 256; t += 32)
+        if (sm[k][t] > v || (sm[k][t] == v && si[k][t] < iv)) { v = sm[k][t]; iv = si[k][t]; }
+    for (int w = 16; w > 0; w >>= 1) {
+        const double b = __shfl_down_sync(0xffffffffu, v, w);
+        const int ib = __shfl_down_sync(0xffffffffu, iv, w);
+        if (b > v || (b == v && ib < iv)) { v = b; iv = ib; }
+    }
+    if (lane == 0) {
+        double *o = part + ((size_t)blockIdx.y * kResidBlocks + blockIdx.x) * 18;
+        o[k] = sum;
+        o[6 + k] = v;
+        o[12 + k] = (double)iv;
+    }
+}
+template __global__ void k_resid_partial<false>(LevelView, double *);
+template __global__ void k_resid_partial<true>(CaseTab<LevelView>, double *);
+
+// one warp per component (blockDim.x = 192), a block per case; each lane folds
+// the block partials b = lane, lane+32, ... and the warp combines the lanes in
+// a fixed tree, so the result does not depend on timing
+__global__ void k_resid_final(const double *part, double *out) {
+    const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (k >= 6) return;
+    part += (size_t)blockIdx.x * kResidBlocks * 18;
+    out += (size_t)blockIdx.x * 18;
     double s = 0, m = 0;
     int mi = 0x7fffffff;
-    for (int b = lane; b < nblk; b += 32) {
+#pragma unroll
+    for (int b0 = 0; b0 < kResidBlocks; b0 += 32) {
+        const int b = b0 + lane;
+        if (b >= kResidBlocks) break;
         s += part[b * 18 + k];
         double v = part[b * 18 + 6 + k];
         int iv = (int)part[b * 18 + 12 + k];
@@ -2669,13 +2696,10 @@ __global__ void k_forces(Params P, LevelView L, const int *wall, int nwall, doub
     }
     for (int k = 0; k < 6; ++k) red[k][threadIdx.x] = acc[k];
     __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w)
-            for (int k = 0; k < 6; ++k) red[k][threadIdx.x] += red[k][threadIdx.x + w];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0)
-        for (int k = 0; k < 6; ++k) part[6 * blockIdx.x + k] = red[k][0];
+    const int kw = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (kw >= 6) return;
+    const double sum = sum256(red[kw], lane);
+    if (lane == 0) part[6 * blockIdx.x + kw] = sum;
 }
 
 __global__ void k_permute_nodes(double *dst, const double *src, const int *map, int N, int ncomp) {
@@ -2734,21 +2758,19 @@ __global__ void k_forces3(Params P, LevelView L, const int *wall, int nwall, dou
     }
     for (int k = 0; k < 7; ++k) red[k][threadIdx.x] = acc[k];
     __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w)
-            for (int k = 0; k < 7; ++k) red[k][threadIdx.x] += red[k][threadIdx.x + w];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0)
-        for (int k = 0; k < 7; ++k) part[7 * blockIdx.x + k] = red[k][0];
+    const int kw = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (kw >= 7) return;
+    const double sum = sum256(red[kw], lane);
+    if (lane == 0) part[7 * blockIdx.x + kw] = sum;
 }
 
 // out[k] = sum over blocks of part[nval*block + k], in block order
-__global__ void k_forces_final(const double *part, int nblk, int nval, double *out) {
+__global__ void k_forces_final(const double *part, int nval, double *out) {
     if (threadIdx.x >= nval) return;
     const int k = threadIdx.x;
     double s = 0.0;
-    for (int b = 0; b < nblk; ++b) s += part[nval * b + k];
+#pragma unroll 16
+    for (int b = 0; b < kForceBlocks; ++b) s += part[nval * b + k];
     out[k] = s;
 }
 }  // namespace flite

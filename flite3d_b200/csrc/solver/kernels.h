@@ -146,8 +146,10 @@ template <bool B = false>
 __global__ void k_case_save_u(CaseArg<B, LevelView> L, size_t n);
 template <bool B = false>
 __global__ void k_case_zero(CaseArg<B, LevelView> L, int which, size_t n);
-__global__ void k_resid_partial(LevelView L, double *part, int nblk);
-__global__ void k_resid_final(const double *part, int nblk, double *out);
+constexpr int kResidBlocks = 296;  // 2 x 148 SMs, of 256 threads
+template <bool B = false>
+__global__ void k_resid_partial(CaseArg<B, LevelView> L, double *part);
+__global__ void k_resid_final(const double *part, double *out);
 __global__ void k_forces(Params P, LevelView L, const int *wall, int nwall, double alphaR, double betaR,
                          double ground, double d0, double d1, double d2, double *part);
 // dst[c*N + i] = src[c*N + map[i]] for c < ncomp (node arrays between the
@@ -155,7 +157,7 @@ __global__ void k_forces(Params P, LevelView L, const int *wall, int nwall, doub
 __global__ void k_permute_nodes(double *dst, const double *src, const int *map, int N, int ncomp);
 __global__ void k_forces3(Params P, LevelView L, const int *wall, int nwall, double alphaR, double betaR,
                           double ground, double d0, double d1, double d2, double *part);
-__global__ void k_forces_final(const double *part, int nblk, int nval, double *out);
+__global__ void k_forces_final(const double *part, int nval, double *out);
 constexpr int kForceBlocks = 64;
 // transposed residual Jacobian at the state x (adjoint.cu)
 __global__ void k_vjp_farfield(Params P, LevelView L, const double *x, const double *rbar, double *bvjp);

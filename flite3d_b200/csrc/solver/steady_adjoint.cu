@@ -1461,7 +1461,7 @@ static void download_geometry(flite_ctx &X, SteadyAdjoint &A, double *swb, doubl
             CK(cudaGetLastError());
             src = t;
         }
-        CK(cudaMemcpyAsync(swb, src, n * sizeof(double), cudaMemcpyDeviceToHost, X.s));
+        X.to_host(swb, src, n * sizeof(double));
     }
     if (bwb && L.B > 0)
         CK(cudaMemcpyAsync(bwb, A.bwbar, 3 * (size_t)L.B * sizeof(double), cudaMemcpyDeviceToHost, X.s));
