@@ -18,6 +18,7 @@
 #include <cuda_runtime.h>
 
 #include "adjoint.cuh"
+#include "gather.cuh"
 #include "context.h"
 #include "flux.cuh"
 
@@ -25,11 +26,14 @@ namespace flite {
 
 // far-field contributions per boundary edge: J(u_b1)^T |w|(3 rbar1 + rbar2)
 // and J(u_b2)^T |w|(rbar1 + 3 rbar2) (FV weighting: 4 rbar_own)
+// (a thread per edge, end and column: one dual evaluation each.  With a
+// thread per edge, which did ten one after the other, a launch over 10,752
+// edges took 29 us)
 __global__ void k_vjp_farfield(Params P, LevelView L, const double *x, const double *rbar, double *bvjp) {
-    int b = blockIdx.x * blockDim.x + threadIdx.x;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int b = t / 10, side = (t % 10) / 5, j = t % 5;
     if (b >= L.B) return;
-    double *o = bvjp + (size_t)b * 10;
-    for (int k = 0; k < 10; ++k) o[k] = 0.0;
+    bvjp[t] = 0.0;
     const int ind = L.bind[b];
     if (ind != 3 && ind != 4) return;
     const double wx = L.bwx[b], wy = L.bwy[b], wz = L.bwz[b];
@@ -40,72 +44,86 @@ __global__ void k_vjp_farfield(Params P, LevelView L, const double *x, const dou
     const int2 nd = L.bedge[b];
     const int N = L.N;
     const bool fe = P.boundaryTerm == 1;
-    for (int side = 0; side < 2; ++side) {
-        const int n = side == 0 ? nd.x : nd.y;
-        double a[5];
-        for (int k = 0; k < 5; ++k) {
-            double r1 = rbar[(size_t)k * N + nd.x], r2 = rbar[(size_t)k * N + nd.y];
-            a[k] = fe ? rnorm * (side == 0 ? 3. * r1 + r2 : r1 + 3. * r2) : rnorm * 4. * (side == 0 ? r1 : r2);
-        }
-        double u[5], p, dp[5];
-        for (int k = 0; k < 5; ++k) u[k] = x[(size_t)k * N + n];
-        pressure_grad(P, u, &p, dp);
-        for (int j = 0; j < 5; ++j) {  // column j of the Jacobian
-            Dual q[5];
-            for (int k = 0; k < 5; ++k) q[k] = Dual(u[k], k == j ? 1.0 : 0.0);
-            Dual F[5];
-            farfield_dual(P, q, Dual(p, dp[j]), rnx, rny, rnz, inf, F);
-            double s = 0.0;
-            for (int k = 0; k < 5; ++k) s += F[k].d * a[k];
-            o[side * 5 + j] = s;
-        }
+    const int n = side == 0 ? nd.x : nd.y;
+    double a[5];
+    for (int k = 0; k < 5; ++k) {
+        double r1 = rbar[(size_t)k * N + nd.x], r2 = rbar[(size_t)k * N + nd.y];
+        a[k] = fe ? rnorm * (side == 0 ? 3. * r1 + r2 : r1 + 3. * r2) : rnorm * 4. * (side == 0 ? r1 : r2);
     }
+    double u[5], p, dp[5];
+    for (int k = 0; k < 5; ++k) u[k] = x[(size_t)k * N + n];
+    pressure_grad(P, u, &p, dp);
+    Dual q[5];
+    double dpj = 0.0;
+    for (int k = 0; k < 5; ++k) {
+        q[k] = Dual(u[k], k == j ? 1.0 : 0.0);
+        if (k == j) dpj = dp[k];
+    }
+    Dual F[5];
+    farfield_dual(P, q, Dual(p, dpj), rnx, rny, rnz, inf, F);
+    double s = 0.0;
+    for (int k = 0; k < 5; ++k) s += F[k].d * a[k];
+    bvjp[t] = s;
 }
 
 // ubar = (dR/dx)^T rbar at the state x, plus pbar (dp/dx) when pbar is given
 // (a pressure read by the caller's own use of the state); add = 1 adds the
 // product to ubar instead of storing it
+template <int U>
 __global__ void k_vjp_node(Params P, LevelView L, const double *x, const double *rbar, const double *bvjp,
                            const double *pbar, double *ubar, int add) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= L.N) return;
+    FLITE_NODE_LANES(L);
     const int N = L.N;
-    double b[3][5];
-    for (int d = 0; d < 3; ++d)
-        for (int k = 0; k < 5; ++k) b[d][k] = 0.0;
+    FLITE_GROUP_SLAB(double, 20);
+    // 0..14: b[d][k]; 15..19: the far-field edges' parts
+    double acc[20];
+#pragma unroll
+    for (int k = 0; k < 20; ++k) acc[k] = 0.0;
     double ri[5];
     for (int k = 0; k < 5; ++k) ri[k] = rbar[(size_t)k * N + i];
-    FLITE_FOR_INC(L, i, t) {
-        int e = t.x >= 0 ? t.x : ~t.x, j = t.y;
-        const double w[3] = {L.wx[e], L.wy[e], L.wz[e]};
-        double a[5];
-        for (int k = 0; k < 5; ++k) {
-            double rj = rbar[(size_t)k * N + j];
-            a[k] = t.x >= 0 ? ri[k] - rj : rj - ri[k];  // rbar(i1) - rbar(i2)
-        }
-        for (int d = 0; d < 3; ++d)
-            for (int k = 0; k < 5; ++k) b[d][k] += w[d] * a[k];
-    }
-    double extra[5] = {0, 0, 0, 0, 0};
+    sum_incidences<U, 15>(
+        L, i, active, gl, gs,
+        [&](const int2 t, double *v) {
+            const int e = t.x >= 0 ? t.x : ~t.x, j = t.y;
+            const double w[3] = {L.wx[e], L.wy[e], L.wz[e]};
+#pragma unroll
+            for (int k = 0; k < 5; ++k) {
+                const double rj = rbar[(size_t)k * N + j];
+                const double a = t.x >= 0 ? ri[k] - rj : rj - ri[k];  // rbar(i1) - rbar(i2)
+#pragma unroll
+                for (int d = 0; d < 3; ++d) v[5 * d + k] = w[d] * a;
+            }
+        },
+        acc);
     const bool fe = P.boundaryTerm == 1;
-    for (int q = L.binc_ptr[i]; q < L.binc_ptr[i + 1]; ++q) {
-        int bb = L.binc[q] >> 1, side = L.binc[q] & 1;
-        int ind = L.bind[bb];
-        if (ind == 3 || ind == 4) {
-            for (int k = 0; k < 5; ++k) extra[k] += bvjp[(size_t)bb * 10 + side * 5 + k];
-            continue;
-        }
-        if (!(ind <= 2 || ind == 9)) continue;
-        const double w[3] = {L.bwx[bb], L.bwy[bb], L.bwz[bb]};
-        if (!(sqrt((w[0] * w[0] + w[1] * w[1]) + w[2] * w[2]) > 1.0e-10)) continue;
-        const int2 nd = L.bedge[bb];
-        double a[5];
-        for (int k = 0; k < 5; ++k) {
-            double r1 = rbar[(size_t)k * N + nd.x], r2 = rbar[(size_t)k * N + nd.y];
-            a[k] = fe ? (side == 0 ? 3. * r1 + r2 : r1 + 3. * r2) : 4. * (side == 0 ? r1 : r2);
-        }
-        for (int d = 0; d < 3; ++d)
-            for (int k = 0; k < 5; ++k) b[d][k] += w[d] * a[k];
+    sum_boundary<U, 20>(
+        L, i, active, gl, gs,
+        [&](int q, double *v) {
+            const int bb = L.binc[q] >> 1, side = L.binc[q] & 1;
+            const int ind = L.bind[bb];
+            if (ind == 3 || ind == 4) {
+#pragma unroll
+                for (int k = 0; k < 5; ++k) v[15 + k] = bvjp[(size_t)bb * 10 + side * 5 + k];
+                return;
+            }
+            if (!(ind <= 2 || ind == 9)) return;
+            const double w[3] = {L.bwx[bb], L.bwy[bb], L.bwz[bb]};
+            if (!(sqrt((w[0] * w[0] + w[1] * w[1]) + w[2] * w[2]) > 1.0e-10)) return;
+            const int2 nd = L.bedge[bb];
+#pragma unroll
+            for (int k = 0; k < 5; ++k) {
+                const double r1 = rbar[(size_t)k * N + nd.x], r2 = rbar[(size_t)k * N + nd.y];
+                const double a = fe ? (side == 0 ? 3. * r1 + r2 : r1 + 3. * r2) : 4. * (side == 0 ? r1 : r2);
+#pragma unroll
+                for (int d = 0; d < 3; ++d) v[5 * d + k] = w[d] * a;
+            }
+        },
+        acc);
+    if (U > 1 && (!active || gl)) return;
+    double b[3][5], extra[5];
+    for (int k = 0; k < 5; ++k) {
+        for (int d = 0; d < 3; ++d) b[d][k] = acc[5 * d + k];
+        extra[k] = acc[15 + k];
     }
     double u[5], ub[5];
     for (int k = 0; k < 5; ++k) u[k] = x[(size_t)k * N + i];
@@ -121,6 +139,11 @@ __global__ void k_vjp_node(Params P, LevelView L, const double *x, const double 
         ubar[(size_t)k * N + i] = add ? ubar[(size_t)k * N + i] + v : v;
     }
 }
+template __global__ void k_vjp_node<1>(Params, LevelView, const double *, const double *, const double *, const double *, double *, int);
+template __global__ void k_vjp_node<4>(Params, LevelView, const double *, const double *, const double *, const double *, double *, int);
+template __global__ void k_vjp_node<8>(Params, LevelView, const double *, const double *, const double *, const double *, double *, int);
+template __global__ void k_vjp_node<16>(Params, LevelView, const double *, const double *, const double *, const double *, double *, int);
+template __global__ void k_vjp_node<32>(Params, LevelView, const double *, const double *, const double *, const double *, double *, int);
 
 }  // namespace flite
 
@@ -158,8 +181,8 @@ extern "C" int flite_residual_vjp(flite_ctx *ctx, int level, const double *u, co
 
 void flite_ctx::vjp_kernels(int l) {
     LevelView &L = V(l);
-    if (L.B > 0) k_vjp_farfield<<<eblk(L.B), eb, 0, s>>>(P, L, L.u, adj_rbar, adj_b);
-    k_vjp_node<<<nblk(L.N), nb, 0, s>>>(P, L, L.u, adj_rbar, adj_b, nullptr, adj_ubar, 0);
+    if (L.B > 0) k_vjp_farfield<<<eblk(10 * (size_t)L.B), eb, 0, s>>>(P, L, L.u, adj_rbar, adj_b);
+    FLITE_ADJ_GATHER(k_vjp_node, (*this), l, P, L, L.u, adj_rbar, adj_b, nullptr, adj_ubar, 0);
 }
 
 extern "C" int flite_profile_adjoint(flite_ctx *ctx, int level, int reps, double *fwd_ms, double *vjp_ms) {

@@ -128,6 +128,21 @@ using namespace flite_detail;
         }                                                                                \
     } while (0)
 
+// an adjoint gather with the lanes per node of level l of context X (blocks of
+// at most 128 threads: its slabs hold up to 24 terms a lane)
+#define FLITE_ADJ_GATHER(kern, X, l, ...)                                                                        \
+    do {                                                                                                          \
+        const int u_ = X.lanes_of(l), t_ = std::min(X.nb, 128);                                                    \
+        const unsigned g_ = (unsigned)((u_ * (size_t)X.V(l).N + t_ - 1) / t_);                                     \
+        switch (u_) {                                                                                              \
+            case 4: kern<4><<<g_, t_, 0, X.s>>>(__VA_ARGS__); break;                                               \
+            case 8: kern<8><<<g_, t_, 0, X.s>>>(__VA_ARGS__); break;                                               \
+            case 16: kern<16><<<g_, t_, 0, X.s>>>(__VA_ARGS__); break;                                             \
+            case 32: kern<32><<<g_, t_, 0, X.s>>>(__VA_ARGS__); break;                                             \
+            default: kern<1><<<g_, t_, 0, X.s>>>(__VA_ARGS__);                                                     \
+        }                                                                                                          \
+    } while (0)
+
 struct flite_ctx {
     flite_controls c{};
     Params P{};
@@ -162,7 +177,8 @@ struct flite_ctx {
     double *d_part = nullptr;
     double *d_ptsg = nullptr;  // ivd%physicalTimeStep (explicit time stepping)
     int *h_cycle = nullptr;    // pinned
-    double *h_out = nullptr;  // pinned: the last kernel of residuals and forces writes here
+    double *h_out = nullptr;  // pinned: the last kernel of a reduction writes here (kOut values)
+    static constexpr int kOut = 2048;
     cudaGraphExec_t graph = nullptr;
     int64_t launches = 0;
     bool counting = false;

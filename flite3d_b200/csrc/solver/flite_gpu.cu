@@ -295,7 +295,7 @@ int flite::create_context(const flite_controls *c, int nlevels, const flite_leve
         }
         CK(cudaEventCreateWithFlags(&X.coarse_ready, cudaEventDisableTiming));
         CK(cudaMallocHost(&X.h_cycle, sizeof(int)));
-        CK(cudaMallocHost(&X.h_out, 32 * sizeof(double)));
+        CK(cudaMallocHost(&X.h_out, flite_ctx::kOut * sizeof(double)));
         X.d_cycle = X.alloc<int>(1);
         X.d_cyc = X.alloc<int>(G);
         {

@@ -64,9 +64,53 @@ __device__ __forceinline__ void group_sum(T *gs, int beg, int end, bool active, 
     for (int m = 0; m < M; ++m) out[m] = __shfl_sync(0xffffffffu, acc[m / U], m % U, U);
 }
 // the calling warp's slab of K terms out of the block's (blocks of at most
-// 256 threads)
-#define FLITE_GROUP_SLAB(T, K)                                   \
-    __shared__ T gslab_[U > 1 ? 8 * (K)*kSlabRow : 1];           \
+// 256 threads; 128 with more than 16 terms)
+#define FLITE_GROUP_SLAB(T, K)                                            \
+    __shared__ T gslab_[U > 1 ? ((K) > 16 ? 4 : 8) * (K)*kSlabRow : 1];   \
     T *gs = gslab_ + (U > 1 ? (threadIdx.x >> 5) * (K)*kSlabRow : 0)
+
+// the node i, lane gl and idle groups of a gather kernel templated on U
+#define FLITE_NODE_LANES(L)                                          \
+    const int gl = U > 1 ? (int)(threadIdx.x % U) : 0;               \
+    const int i_raw = (int)(blockIdx.x * blockDim.x + threadIdx.x) / U; \
+    if (U == 1 && i_raw >= L.N) return;                              \
+    const bool active = i_raw < L.N;                                 \
+    const int i = active ? i_raw : L.N - 1
+// M sums of node i over its incidences (terms(t, v): one term per sum) and
+// boundary entries (bterms(q, v)), with a thread or a group per node, both in
+// order.  gs: the group's slab of M terms (unused with a thread).
+template <int U, int M, class Terms>
+__device__ __forceinline__ void sum_incidences(const LevelView &L, int i, bool active, int gl, double *gs,
+                                               Terms &&terms, double *out) {
+    if constexpr (U > 1) {
+        group_sum<U, M, 1, double>(
+            gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl, [&](int q, double *v) { terms(L.inc[q], v); }, out);
+    } else {
+        FLITE_FOR_INC(L, i, t) {
+            double v[M];
+#pragma unroll
+            for (int m = 0; m < M; ++m) v[m] = 0.0;
+            terms(t, v);
+#pragma unroll
+            for (int m = 0; m < M; ++m) out[m] = out[m] + v[m];
+        }
+    }
+}
+template <int U, int M, class Terms>
+__device__ __forceinline__ void sum_boundary(const LevelView &L, int i, bool active, int gl, double *gs,
+                                             Terms &&terms, double *out) {
+    if constexpr (U > 1) {
+        group_sum<U, M, 1, double>(gs, L.binc_ptr[i], L.binc_ptr[i + 1], active, gl, terms, out);
+    } else {
+        for (int q = L.binc_ptr[i]; q < L.binc_ptr[i + 1]; ++q) {
+            double v[M];
+#pragma unroll
+            for (int m = 0; m < M; ++m) v[m] = 0.0;
+            terms(q, v);
+#pragma unroll
+            for (int m = 0; m < M; ++m) out[m] = out[m] + v[m];
+        }
+    }
+}
 
 }  // namespace flite

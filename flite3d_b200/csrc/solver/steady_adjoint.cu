@@ -38,6 +38,7 @@
 
 #include "adjoint.cuh"
 #include "context.h"
+#include "gather.cuh"
 
 namespace flite {
 
@@ -271,15 +272,18 @@ __global__ void k_adj_stage(Params P, LevelView L, int stage, const double *vbar
 // Edge part (pass 3) gathered per node: the adjoints of this node's undivided
 // Laplacian (scaled back to nodeHelpArray 1:5), of its sensor terms nh6/nh7
 // and of its V/dt; the direct u part goes to ubar.
+template <int U>
 __global__ void k_adj_jst_edges(Params P, LevelView L, const double *u0, const double *dt, const double *lap,
                                 const double *sens, const double *nh6, const double *nh7, const double *Dbar,
                                 double *ubar, double *dtbar, double *nhbar, double *nh6bar, double *nh7bar,
                                 double *Vbar) {
-    const int i = tidx();
-    if (i >= L.N) return;
+    FLITE_NODE_LANES(L);
     const int N = L.N;
+    FLITE_GROUP_SLAB(double, 12);
     const double k2 = P.k2, k4 = L.grid == 1 ? P.k4 : P.cgdf;
-    double lapb[5] = {0, 0, 0, 0, 0}, ubd[5] = {0, 0, 0, 0, 0}, sensb = 0.0, rb = 0.0;
+    // sums: the Laplacian's adjoint (5), the direct part of ubar (5), the
+    // sensor's adjoint, that of V/dt
+    double acc[12] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
     const double Vi = L.V[i], dti = dt[i], ri = Vi / dti, ci = L.conn[i], si = sens[i];
     double ui[5], li[5], Dbi[5];
     for (int c = 0; c < 5; ++c) {
@@ -287,7 +291,7 @@ __global__ void k_adj_jst_edges(Params P, LevelView L, const double *u0, const d
         li[c] = lap[(size_t)c * N + i];
         Dbi[c] = Dbar[(size_t)c * N + i];
     }
-    FLITE_FOR_INC(L, i, t) {
+    sum_incidences<U, 12>(L, i, active, gl, gs, [&](const int2 t, double *v) {
         const int j = t.y;
         const bool first = t.x >= 0;  // this node is the edge's i1
         const double rj = L.V[j] / dt[j], cj = L.conn[j], sj = sens[j];
@@ -312,8 +316,8 @@ __global__ void k_adj_jst_edges(Params P, LevelView L, const double *u0, const d
         const double sig = first ? 1.0 : -1.0;
         double d4b = 0.0, d2b = 0.0;
         for (int c = 0; c < 5; ++c) {
-            lapb[c] += -sig * d4 * db[c];
-            ubd[c] += sig * d2 * db[c];
+            v[c] = -sig * d4 * db[c];
+            v[5 + c] = sig * d2 * db[c];
             d4b -= d4v[c] * db[c];
             d2b += d2v[c] * db[c];
         }
@@ -325,9 +329,11 @@ __global__ void k_adj_jst_edges(Params P, LevelView L, const double *u0, const d
         d0b += k2 * smax * d2b;
         // max(s1, s2) = (s1 < s2) ? s2 : s1; min(r1, r2) = (r2 < r1) ? r2 : r1
         const bool max_is_2 = s1 < s2, min_is_2 = r2 < r1;
-        if (max_is_2 != first) sensb += d0 * k2 * d2b;
-        if (min_is_2 != first) rb += d0b / cs;
-    }
+        if (max_is_2 != first) v[10] = d0 * k2 * d2b;
+        if (min_is_2 != first) v[11] = d0b / cs;
+    }, acc);
+    if (U > 1 && (!active || gl)) return;
+    const double *lapb = acc, *ubd = acc + 5, sensb = acc[10], rb = acc[11];
     const double fact = 1. / ci;
     for (int c = 0; c < 5; ++c) {
         nhbar[(size_t)c * N + i] = fact * lapb[c];
@@ -345,24 +351,43 @@ __global__ void k_adj_jst_edges(Params P, LevelView L, const double *u0, const d
 
 // passes 1 and 2 in reverse: the undivided Laplacian and the sensor sums
 // gathered back to the state and the pressure of the iteration's start
+template <int U>
 __global__ void k_adj_jst_lap(LevelView L, const double *nhbar, const double *nh6bar, const double *nh7bar,
                               double *ubar, double *p0bar) {
-    const int i = tidx();
-    if (i >= L.N) return;
+    FLITE_NODE_LANES(L);
     const int N = L.N;
+    FLITE_GROUP_SLAB(double, 8);
     double nbi[5];
     for (int c = 0; c < 5; ++c) nbi[c] = nhbar[(size_t)c * N + i];
     const double b6i = nh6bar[i], b7i = nh7bar[i];
-    double ub[5] = {0, 0, 0, 0, 0}, pb = 0.0;
-    FLITE_FOR_INC(L, i, t) {
-        const int j = t.y;
-        for (int c = 0; c < 5; ++c) ub[c] += nhbar[(size_t)c * N + j] - nbi[c];
-        pb += nhbar[(size_t)4 * N + j] - nbi[4];
-        pb += nh6bar[j] - b6i;
-        pb += nh7bar[j] + b7i;
+    double ub[5] = {0, 0, 0, 0, 0}, pb[1] = {0.0};
+    // the pressure takes three terms from each incidence
+    auto pterms = [&](int j, double *v) {
+        v[0] = nhbar[(size_t)4 * N + j] - nbi[4];
+        v[1] = nh6bar[j] - b6i;
+        v[2] = nh7bar[j] + b7i;
+    };
+    if constexpr (U > 1) {
+        group_sum<U, 5, 1, double>(
+            gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl,
+            [&](int q, double *v) {
+                const int j = L.inc[q].y;
+                for (int c = 0; c < 5; ++c) v[c] = nhbar[(size_t)c * N + j] - nbi[c];
+            },
+            ub);
+        group_sum<U, 1, 3, double>(
+            gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl, [&](int q, double *v) { pterms(L.inc[q].y, v); }, pb);
+        if (!active || gl) return;
+    } else {
+        FLITE_FOR_INC(L, i, t) {
+            for (int c = 0; c < 5; ++c) ub[c] += nhbar[(size_t)c * N + t.y] - nbi[c];
+            double v[3];
+            pterms(t.y, v);
+            pb[0] = ((pb[0] + v[0]) + v[1]) + v[2];
+        }
     }
     for (int c = 0; c < 5; ++c) ubar[(size_t)c * N + i] += ub[c];
-    p0bar[i] += pb;
+    p0bar[i] += pb[0];
 }
 
 // ---- local time step (def_par:13335-13610), inviscid, reverse -------------
@@ -414,71 +439,78 @@ __device__ __forceinline__ double visc_ts_term(const Params &P, double mu, doubl
 // (Sbar, Hbar), this node's own terms in reverse, then the pressure of the
 // iteration's start back to the state.  mu: the viscosity the step read;
 // mubar its adjoint (laminar runs)
+template <int U>
 __global__ void k_adj_timestep(Params P, LevelView L, const double *u0, const double *p0, const double *dt,
                                const double *dtbar, const double *p0bar, const double *mu, double *ubar,
                                double *mubar, double *Sbar, double *Hbar, double *Vbar) {
-    const int i = tidx();
-    if (i >= L.N) return;
+    FLITE_NODE_LANES(L);
     const int N = L.N;
+    FLITE_GROUP_SLAB(double, 9);
     const double Vi = L.V[i], dti = dt[i];
     const double tt = 0.5 / dti;  // S/V + h/V^2
     const double tb = -0.5 * dtbar[i] / (tt * tt);
     const double sbi = tb / Vi, hbi = tb / (Vi * Vi);
-    Sbar[i] = sbi;
-    Hbar[i] = hbi;
+    if (gl == 0 && active) {
+        Sbar[i] = sbi;
+        Hbar[i] = hbi;
+    }
     auto hbar_of = [&](int j) {
         const double tj = 0.5 / dt[j];
         return (-0.5 * dtbar[j] / (tj * tj)) / (L.V[j] * L.V[j]);
     };
-    double h = 0.0, mb = 0.0, rvb = 0.0;  // viscous sum, and this node's rho / mu adjoints from it
     const bool visc = P.viscous;
     const double mui = visc ? mu[i] : 0.0;
     double ui[5];
     for (int c = 0; c < 5; ++c) ui[c] = u0[(size_t)c * N + i];
     const double pi = p0[i];
-    double ub[5] = {0, 0, 0, 0, 0}, pb = 0.0;
-    double fu[5], fp;
-    FLITE_FOR_INC(L, i, t) {
+    // sums: the state's adjoint (5), the pressure's, and with viscosity the
+    // viscous sum and this node's rho and mu adjoints from it
+    double acc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    sum_incidences<U, 9>(L, i, active, gl, gs, [&](const int2 t, double *v) {
         const int e = t.x >= 0 ? t.x : ~t.x;
         const double w[3] = {L.wx[e], L.wy[e], L.wz[e]};
+        double fu[5], fp;
         ts_term_grad(P, ui, pi, w, fu, &fp, nullptr);
-        for (int c = 0; c < 5; ++c) ub[c] += sbi * fu[c];
-        pb += sbi * fp;
+        for (int c = 0; c < 5; ++c) v[c] = sbi * fu[c];
+        v[5] = sbi * fp;
         if (visc) {
             const int j = t.y;
             const double al = (w[0] * w[0] + w[1] * w[1]) + w[2] * w[2];
             double dr, dm, da;
-            h += visc_ts_term(P, mu[j], u0[j], al, &dr, &dm, &da);  // the other end's term
-            visc_ts_term(P, mui, ui[0], al, &dr, &dm, &da);         // this end's, in the other's h
+            v[6] = visc_ts_term(P, mu[j], u0[j], al, &dr, &dm, &da);  // the other end's term
+            visc_ts_term(P, mui, ui[0], al, &dr, &dm, &da);           // this end's, in the other's h
             const double hj = hbar_of(j);
-            rvb += hj * dr;
-            mb += hj * dm;
+            v[7] = hj * dr;
+            v[8] = hj * dm;
         }
-    }
-    for (int k = L.binc_ptr[i]; k < L.binc_ptr[i + 1]; ++k) {
+    }, acc);
+    sum_boundary<U, 9>(L, i, active, gl, gs, [&](int k, double *v) {
         const int b = L.binc[k] >> 1, side = L.binc[k] & 1;
         const int2 nd = L.bedge[b];
         const int j = side == 0 ? nd.y : nd.x;
         const double w[3] = {L.bwx[b], L.bwy[b], L.bwz[b]};
-        // Sbar of the other node is read after this kernel's writes are not
-        // needed: it is recomputed from its own dtbar
+        // Sbar of the other node is recomputed from its own dtbar
         const double ttj = 0.5 / dt[j];
         const double sbj = (-0.5 * dtbar[j] / (ttj * ttj)) / L.V[j];
         const double wgt = 2.0 * sbi + sbj;
+        double fu[5], fp;
         ts_term_grad(P, ui, pi, w, fu, &fp, nullptr);
-        for (int c = 0; c < 5; ++c) ub[c] += wgt * fu[c];
-        pb += wgt * fp;
+        for (int c = 0; c < 5; ++c) v[c] = wgt * fu[c];
+        v[5] = wgt * fp;
         if (visc) {
             const double al = (w[0] * w[0] + w[1] * w[1]) + w[2] * w[2];
             double dr, dm, da;
             const double own = visc_ts_term(P, mui, ui[0], al, &dr, &dm, &da);
             double drj, dmj, daj;
-            h += 2.0 * own + visc_ts_term(P, mu[j], u0[j], al, &drj, &dmj, &daj);
+            v[6] = 2.0 * own + visc_ts_term(P, mu[j], u0[j], al, &drj, &dmj, &daj);
             const double hw = 2.0 * hbi + hbar_of(j);
-            rvb += hw * dr;
-            mb += hw * dm;
+            v[7] = hw * dr;
+            v[8] = hw * dm;
         }
-    }
+    }, acc);
+    if (U > 1 && (!active || gl)) return;
+    double *ub = acc, pb = acc[5];
+    const double h = acc[6], rvb = acc[7], mb = acc[8];
     ub[0] += rvb;
     if (visc && mubar) mubar[i] = mb;
     // V: t = S/V + h/V^2
@@ -655,28 +687,24 @@ __global__ void k_adj_visc_sums(LevelView L, const double *prim, double *G) {
 // adjoint of one viscous edge flux (f2..f5 of def_par:5700-5760) to one end:
 // W = the adjoints of f2..f5, w the coefficients, t (9) and v (3) that end's
 // tensor and velocity; adds to tb (9) and vb (3)
+// As the terms of 12 sums (tb, then vb), two each: x[2 m] and x[2 m + 1] (0
+// where a sum takes one).
 __device__ __forceinline__ void visc_flux_end_rev(const double *W, const double *w, const double *t,
-                                                  const double *v, double *tb, double *vb) {
+                                                  const double *v, double *x) {
     const double wx = w[0], wy = w[1], wz = w[2];
-    tb[0] += wx * W[0];
-    tb[1] += wy * W[0] + wx * W[1];
-    tb[2] += wz * W[0] + wx * W[2];
-    tb[3] += wy * W[1];
-    tb[4] += wz * W[1] + wy * W[2];
-    tb[5] += wz * W[2];
-    tb[6] += wx * W[3];
-    tb[7] += wy * W[3];
-    tb[8] += wz * W[3];
     const double D0 = wx * W[3], D1 = wy * W[3], D2 = wz * W[3];  // adjoints of dut1..dut3
-    tb[0] += v[0] * D0;
-    tb[1] += v[1] * D0 + v[0] * D1;
-    tb[2] += v[2] * D0 + v[0] * D2;
-    tb[3] += v[1] * D1;
-    tb[4] += v[2] * D1 + v[1] * D2;
-    tb[5] += v[2] * D2;
-    vb[0] += (t[0] * D0 + t[1] * D1) + t[2] * D2;
-    vb[1] += (t[1] * D0 + t[3] * D1) + t[4] * D2;
-    vb[2] += (t[2] * D0 + t[4] * D1) + t[5] * D2;
+    x[0] = wx * W[0];                  x[1] = v[0] * D0;
+    x[2] = wy * W[0] + wx * W[1];      x[3] = v[1] * D0 + v[0] * D1;
+    x[4] = wz * W[0] + wx * W[2];      x[5] = v[2] * D0 + v[0] * D2;
+    x[6] = wy * W[1];                  x[7] = v[1] * D1;
+    x[8] = wz * W[1] + wy * W[2];      x[9] = v[2] * D1 + v[1] * D2;
+    x[10] = wz * W[2];                 x[11] = v[2] * D2;
+    x[12] = wx * W[3];                 x[13] = 0.0;
+    x[14] = wy * W[3];                 x[15] = 0.0;
+    x[16] = wz * W[3];                 x[17] = 0.0;
+    x[18] = (t[0] * D0 + t[1] * D1) + t[2] * D2;  x[19] = 0.0;
+    x[20] = (t[1] * D0 + t[3] * D1) + t[4] * D2;  x[21] = 0.0;
+    x[22] = (t[2] * D0 + t[4] * D1) + t[5] * D2;  x[23] = 0.0;
 }
 // d f2..f5 / d w of the same terms (dt = the summed tensors, dut the summed
 // velocity products)
@@ -693,16 +721,17 @@ __device__ __forceinline__ void visc_dut(const double *t, const double *v, doubl
 
 // pass 2 in reverse, gathered per node: the adjoints of this node's tensor and
 // velocity from the adjoints of the viscous fluxes (diss(:,2:5) -= flux)
+template <int U>
 __global__ void k_adj_visc_flux(LevelView L, const double *Dbar, const double *tau, const double *prim,
                                 double *tbar, double *velbar) {
-    const int i = tidx();
-    if (i >= L.N) return;
+    FLITE_NODE_LANES(L);
     const int N = L.N;
-    double ti[9], vi[3], Wi[4], tb[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, vb[3] = {0, 0, 0};
+    FLITE_GROUP_SLAB(double, 24);
+    double ti[9], vi[3], Wi[4], acc[12] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
     for (int c = 0; c < 9; ++c) ti[c] = tau[(size_t)c * N + i];
     for (int c = 0; c < 3; ++c) vi[c] = prim[(size_t)c * N + i];
     for (int c = 0; c < 4; ++c) Wi[c] = -Dbar[(size_t)(1 + c) * N + i];
-    FLITE_FOR_INC(L, i, t) {
+    auto terms = [&](const int2 t, double *x) {
         const int e = t.x >= 0 ? t.x : ~t.x;
         const double w[3] = {L.wx[e], L.wy[e], L.wz[e]};
         double W[4];
@@ -710,22 +739,44 @@ __global__ void k_adj_visc_flux(LevelView L, const double *Dbar, const double *t
             const double Wj = -Dbar[(size_t)(1 + c) * N + t.y];
             W[c] = t.x >= 0 ? Wi[c] - Wj : Wj - Wi[c];  // +f to node 1, -f to node 2
         }
-        visc_flux_end_rev(W, w, ti, vi, tb, vb);
-    }
-    for (int k = L.binc_ptr[i]; k < L.binc_ptr[i + 1]; ++k) {
+        visc_flux_end_rev(W, w, ti, vi, x);
+    };
+    // a face that does not count leaves x as it is (zeros)
+    auto bterms = [&](int k, double *x) {
         const int b = L.binc[k] >> 1, side = L.binc[k] & 1;
         const int ind = L.bind[b];
-        if (ind == 2 || ind == 9) continue;
+        if (ind == 2 || ind == 9) return;
         const int2 nd = L.bedge[b];
         const int j = side == 0 ? nd.y : nd.x;
         const double w[3] = {L.bwx[b], L.bwy[b], L.bwz[b]};
         double W[4];
         // +f to both ends and 2 g(own) to each: f's weight W_i + W_j, g's 2 W_i
         for (int c = 0; c < 4; ++c) W[c] = 3. * Wi[c] - Dbar[(size_t)(1 + c) * N + j];
-        visc_flux_end_rev(W, w, ti, vi, tb, vb);
+        visc_flux_end_rev(W, w, ti, vi, x);
+    };
+    if constexpr (U > 1) {
+        group_sum<U, 12, 2, double>(
+            gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl, [&](int q, double *x) { terms(L.inc[q], x); }, acc);
+        group_sum<U, 12, 2, double>(gs, L.binc_ptr[i], L.binc_ptr[i + 1], active, gl, bterms, acc);
+        if (!active || gl) return;
+    } else {
+        FLITE_FOR_INC(L, i, t) {
+            double x[24];
+            terms(t, x);
+#pragma unroll
+            for (int m = 0; m < 12; ++m) acc[m] = (acc[m] + x[2 * m]) + x[2 * m + 1];
+        }
+        for (int q = L.binc_ptr[i]; q < L.binc_ptr[i + 1]; ++q) {
+            double x[24];
+#pragma unroll
+            for (int m = 0; m < 24; ++m) x[m] = 0.0;
+            bterms(q, x);
+#pragma unroll
+            for (int m = 0; m < 12; ++m) acc[m] = (acc[m] + x[2 * m]) + x[2 * m + 1];
+        }
     }
-    for (int c = 0; c < 9; ++c) tbar[(size_t)c * N + i] = tb[c];
-    for (int c = 0; c < 3; ++c) velbar[(size_t)c * N + i] = vb[c];
+    for (int c = 0; c < 9; ++c) tbar[(size_t)c * N + i] = acc[c];
+    for (int c = 0; c < 3; ++c) velbar[(size_t)c * N + i] = acc[9 + c];
 }
 
 // the node part in reverse (def_par:5500-5635): tensor and heat flux from the
@@ -803,30 +854,55 @@ __global__ void k_adj_visc_node(Params P, LevelView L, const double *u0, const d
 // sums' adjoints (interior edges: G(1) += (q1+q2) w, G(2) -= (q1+q2) w;
 // boundary edges: G(own) += (3 q_own + q_other) w), plus the velocities'
 // adjoints of the flux pass, to the state and the pressure
+template <int U>
 __global__ void k_adj_visc_prim(Params P, LevelView L, const double *u0, const double *p0, const double *Gbar,
                                 const double *velbar, double *ubar, double *p0bar) {
-    const int i = tidx();
-    if (i >= L.N) return;
+    FLITE_NODE_LANES(L);
     const int N = L.N;
+    FLITE_GROUP_SLAB(double, 12);
     double gi[12], qb[4] = {0, 0, 0, 0};
     for (int c = 0; c < 12; ++c) gi[c] = Gbar[(size_t)c * N + i];
-    FLITE_FOR_INC(L, i, t) {
+    // three terms (the directions) for each of the four sums
+    auto terms = [&](const int2 t, double *x) {
         const int e = t.x >= 0 ? t.x : ~t.x;
         const double w[3] = {L.wx[e], L.wy[e], L.wz[e]};
+#pragma unroll
         for (int c = 0; c < 4; ++c)
+#pragma unroll
             for (int a = 0; a < 3; ++a) {
                 const double gj = Gbar[(size_t)(a * 4 + c) * N + t.y];
-                qb[c] += w[a] * (t.x >= 0 ? gi[a * 4 + c] - gj : gj - gi[a * 4 + c]);
+                x[3 * c + a] = w[a] * (t.x >= 0 ? gi[a * 4 + c] - gj : gj - gi[a * 4 + c]);
             }
-    }
-    for (int k = L.binc_ptr[i]; k < L.binc_ptr[i + 1]; ++k) {
+    };
+    auto bterms = [&](int k, double *x) {
         const int b = L.binc[k] >> 1, side = L.binc[k] & 1;
         const int2 nd = L.bedge[b];
         const int j = side == 0 ? nd.y : nd.x;
         const double w[3] = {L.bwx[b], L.bwy[b], L.bwz[b]};
+#pragma unroll
         for (int c = 0; c < 4; ++c)
+#pragma unroll
             for (int a = 0; a < 3; ++a)
-                qb[c] += w[a] * (3. * gi[a * 4 + c] + Gbar[(size_t)(a * 4 + c) * N + j]);
+                x[3 * c + a] = w[a] * (3. * gi[a * 4 + c] + Gbar[(size_t)(a * 4 + c) * N + j]);
+    };
+    if constexpr (U > 1) {
+        group_sum<U, 4, 3, double>(
+            gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl, [&](int q, double *x) { terms(L.inc[q], x); }, qb);
+        group_sum<U, 4, 3, double>(gs, L.binc_ptr[i], L.binc_ptr[i + 1], active, gl, bterms, qb);
+        if (!active || gl) return;
+    } else {
+        FLITE_FOR_INC(L, i, t) {
+            double x[12];
+            terms(t, x);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) qb[c] = ((qb[c] + x[3 * c]) + x[3 * c + 1]) + x[3 * c + 2];
+        }
+        for (int q = L.binc_ptr[i]; q < L.binc_ptr[i + 1]; ++q) {
+            double x[12];
+            bterms(q, x);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) qb[c] = ((qb[c] + x[3 * c]) + x[3 * c + 1]) + x[3 * c + 2];
+        }
     }
     for (int c = 0; c < 3; ++c) qb[c] += velbar[(size_t)c * N + i];
     const double gOg = P.gamma / (P.gamma - 1.0);
@@ -1155,12 +1231,15 @@ __global__ void k_gm_dots(const double *V, size_t n, const double *w, double *pa
     }
     if (threadIdx.x == 0) part[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = red[0];
 }
-__global__ void k_gm_dots_final(const double *part, int nblk, int k, double *h) {
+// (host: a pinned copy, or NULL)
+__global__ void k_gm_dots_final(const double *part, int nblk, int k, double *h, double *host) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= k) return;
     double s = 0.0;
+#pragma unroll 16
     for (int b = 0; b < nblk; ++b) s += part[(size_t)j * nblk + b];
     h[j] = s;
+    if (host) host[j] = s;
 }
 // w += sgn sum_j c[j] V_j
 __global__ void k_gm_combine(const double *V, size_t n, int k, const double *c, double sgn, double *w) {
@@ -1169,6 +1248,14 @@ __global__ void k_gm_combine(const double *V, size_t n, int k, const double *c, 
         for (int j = 0; j < k; ++j) s += c[j] * V[(size_t)j * n + i];
         w[i] = w[i] + sgn * s;
     }
+}
+// w <- w / |w| with |w|^2 in h2 (unchanged when that is not positive)
+__global__ void k_gm_unit(double *w, size_t n, const double *h2) {
+    const double hn = sqrt(*h2);
+    if (!(hn > 0)) return;
+    const double a = 1.0 / hn;
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+        w[i] = a * w[i];
 }
 __global__ void k_gm_scale(double *w, size_t n, double a) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
@@ -1242,10 +1329,13 @@ static SteadyAdjoint &buffers(flite_ctx &X) {
         a->nc = X.P.viscous ? 6 : 5;
         const size_t n5 = 5 * (size_t)L.N, N = L.N, na = (size_t)a->nc * N;
         for (double **p : {&a->u0, &a->v1, &a->v2, &a->Q[0], &a->Q[1], &a->Q[2], &a->D, &a->lap, &a->vb[0],
-                           &a->vb[1], &a->Qbar, &a->Dbar, &a->nhbar})
+                           &a->vb[1], &a->Qbar, &a->nhbar})
             *p = X.alloc<double>(n5);
-        for (double **p : {&a->lam, &a->ubar, &a->Ju}) *p = X.alloc<double>(na);
-        for (double **p : {&a->p0, &a->dt, &a->sens, &a->nh6, &a->nh7, &a->dtbar, &a->pbar, &a->p0bar, &a->nh6bar,
+        for (double **p : {&a->lam, &a->Ju}) *p = X.alloc<double>(na);
+        // what a reverse sweep zeroes, side by side
+        a->ubar = X.alloc<double>(na + 7 * N);
+        a->Dbar = a->ubar + na; a->dtbar = a->Dbar + n5; a->p0bar = a->dtbar + N;
+        for (double **p : {&a->p0, &a->dt, &a->sens, &a->nh6, &a->nh7, &a->pbar, &a->nh6bar,
                            &a->nh7bar, &a->Sbar, &a->Hbar, &a->Vbar, &a->Abar})
             *p = X.alloc<double>(N);
         if (X.P.viscous) {
@@ -1296,7 +1386,7 @@ static void objective_terms(flite_ctx &X, SteadyAdjoint &A, int objective, const
         k_adj_objective_par<<<kObjBlocks, 256, 0, X.s>>>(X.P, L, D.d_wall, nw, X.c.groundplane, dir[0], dir[1],
                                                          dir[2], X.c.referenceArea, u, tau, A.part, A.Ju, A.Abar,
                                                          A.nbar);
-        k_gm_dots_final<<<1, 32, 0, X.s>>>(A.part, kObjBlocks, 1, A.out);
+        k_gm_dots_final<<<1, 32, 0, X.s>>>(A.part, kObjBlocks, 1, A.out, nullptr);
     } else {
         k_adj_objective<<<1, 1, 0, X.s>>>(X.P, L, D.d_wall, nw, X.c.groundplane, dir[0], dir[1], dir[2],
                                           X.c.referenceArea, u, tau, A.out, A.Ju, A.Abar, A.nbar);
@@ -1325,7 +1415,7 @@ static void viscous_reverse(flite_ctx &X, SteadyAdjoint &A, const double *lam_mu
     const size_t N = L.N;
     const unsigned nbk = X.nblk(N);
     if (from_fluxes) {
-        k_adj_visc_flux<<<nbk, X.nb, 0, X.s>>>(L, A.Dbar, A.tau, A.prim, A.tbar, A.velbar);
+        FLITE_ADJ_GATHER(k_adj_visc_flux, X, 0, L, A.Dbar, A.tau, A.prim, A.tbar, A.velbar);
     } else {
         zero(X, A.tbar, 9 * N);
         zero(X, A.velbar, 3 * N);
@@ -1333,7 +1423,7 @@ static void viscous_reverse(flite_ctx &X, SteadyAdjoint &A, const double *lam_mu
     if (tseed) k_adj_add<<<592, 256, 0, X.s>>>(tseed, 9 * N, A.tbar);
     k_adj_visc_node<<<nbk, X.nb, 0, X.s>>>(X.P, L, A.u0, A.p0, A.Gv, A.tbar, lam_mu, A.Gbar, A.ubar, A.p0bar,
                                            geom ? A.Vbar : nullptr, geom ? A.nbar : nullptr);
-    k_adj_visc_prim<<<nbk, X.nb, 0, X.s>>>(X.P, L, A.u0, A.p0, A.Gbar, A.velbar, A.ubar, A.p0bar);
+    FLITE_ADJ_GATHER(k_adj_visc_prim, X, 0, X.P, L, A.u0, A.p0, A.Gbar, A.velbar, A.ubar, A.p0bar);
     if (geom) {
         k_adj_visc_w<<<X.eblk(L.E), X.eb, 0, X.s>>>(L, A.Dbar, A.tau, A.prim, A.Gbar, A.swbar);
         if (L.B > 0) k_adj_visc_bw<<<X.eblk(L.B), X.eb, 0, X.s>>>(L, A.Dbar, A.tau, A.prim, A.Gbar, A.bwbar);
@@ -1402,10 +1492,7 @@ static void reverse(flite_ctx &X, SteadyAdjoint &A, const double *lam, bool geom
     LevelView &L = X.V(0);
     const size_t n5 = 5 * (size_t)L.N, N = L.N;
     const unsigned nbk = X.nblk(N);
-    zero(X, A.ubar, (size_t)A.nc * N);
-    zero(X, A.Dbar, n5);
-    zero(X, A.dtbar, N);
-    zero(X, A.p0bar, N);
+    zero(X, A.ubar, ((size_t)A.nc + 7) * N);  // ubar, Dbar, dtbar, p0bar
     double *Vb = geom ? A.Vbar : nullptr, *nb = geom ? A.nbar : nullptr;
     const double *in[3] = {A.u0, A.v1, A.v2};
     const double *vin = lam;
@@ -1413,10 +1500,10 @@ static void reverse(flite_ctx &X, SteadyAdjoint &A, const double *lam, bool geom
         const double *x = in[k - 1];
         k_adj_stage<<<nbk, X.nb, 0, X.s>>>(X.P, L, k, vin, A.u0, x, A.Q[k - 1], A.D, A.dt, A.ubar, A.Qbar, A.Dbar,
                                            A.dtbar, A.pbar, Vb, nb);
-        if (L.B > 0) k_vjp_farfield<<<X.eblk(L.B), X.eb, 0, X.s>>>(X.P, L, x, A.Qbar, A.bvjp);
+        if (L.B > 0) k_vjp_farfield<<<X.eblk(10 * (size_t)L.B), X.eb, 0, X.s>>>(X.P, L, x, A.Qbar, A.bvjp);
         double *vout = A.vb[k & 1];
-        if (k > 1) k_vjp_node<<<nbk, X.nb, 0, X.s>>>(X.P, L, x, A.Qbar, A.bvjp, A.pbar, vout, 0);
-        else k_vjp_node<<<nbk, X.nb, 0, X.s>>>(X.P, L, x, A.Qbar, A.bvjp, A.pbar, A.ubar, 1);
+        if (k > 1) FLITE_ADJ_GATHER(k_vjp_node, X, 0, X.P, L, x, A.Qbar, A.bvjp, A.pbar, vout, 0);
+        else FLITE_ADJ_GATHER(k_vjp_node, X, 0, X.P, L, x, A.Qbar, A.bvjp, A.pbar, A.ubar, 1);
         if (geom) {
             k_adj_flux_w<<<X.eblk(L.E), X.eb, 0, X.s>>>(X.P, L, x, A.Qbar, A.swbar);
             if (L.B > 0) k_adj_flux_bw<<<X.eblk(L.B), X.eb, 0, X.s>>>(X.P, L, x, A.Qbar, A.bwbar);
@@ -1426,11 +1513,11 @@ static void reverse(flite_ctx &X, SteadyAdjoint &A, const double *lam, bool geom
     if (X.P.viscous) viscous_reverse(X, A, lam + n5, geom ? tseed : nullptr, true, geom);
     const bool jst = !(X.c.fourthOrderDissipationFactor == 0 && X.c.secondOrderDissipationFactor == 0);
     if (jst) {
-        k_adj_jst_edges<<<nbk, X.nb, 0, X.s>>>(X.P, L, A.u0, A.dt, A.lap, A.sens, A.nh6, A.nh7, A.Dbar, A.ubar,
+        FLITE_ADJ_GATHER(k_adj_jst_edges, X, 0, X.P, L, A.u0, A.dt, A.lap, A.sens, A.nh6, A.nh7, A.Dbar, A.ubar,
                                                A.dtbar, A.nhbar, A.nh6bar, A.nh7bar, Vb);
-        k_adj_jst_lap<<<nbk, X.nb, 0, X.s>>>(L, A.nhbar, A.nh6bar, A.nh7bar, A.ubar, A.p0bar);
+        FLITE_ADJ_GATHER(k_adj_jst_lap, X, 0, L, A.nhbar, A.nh6bar, A.nh7bar, A.ubar, A.p0bar);
     }
-    k_adj_timestep<<<nbk, X.nb, 0, X.s>>>(X.P, L, A.u0, A.p0, A.dt, A.dtbar, A.p0bar, A.mu0, A.ubar,
+    FLITE_ADJ_GATHER(k_adj_timestep, X, 0, X.P, L, A.u0, A.p0, A.dt, A.dtbar, A.p0bar, A.mu0, A.ubar,
                                           X.P.viscous ? A.ubar + n5 : nullptr, A.Sbar, A.Hbar, Vb);
     if (geom) {
         k_adj_timestep_w<<<X.eblk(L.E), X.eb, 0, X.s>>>(X.P, L, A.u0, A.p0, A.Sbar, A.Hbar, A.mu0, A.swbar);
@@ -1523,29 +1610,26 @@ static int gmres_solve(flite_ctx &X, SteadyAdjoint &A, double bnorm, double tol,
         // the vectors of a smaller restart length stay allocated until the context goes
         A.kry = X.alloc<double>((size_t)(m + 1) * n);
         A.gpart = X.alloc<double>((size_t)kDotBlocks * (m + 1));
-        A.gh = X.alloc<double>(m + 1);
+        A.gh = X.alloc<double>(2 * (size_t)(m + 1) + 1);
         if (!A.rhs) A.rhs = X.alloc<double>(n);
         A.kry_m = m;
     }
     const unsigned eb = 592;
     k_gm_apply<<<eb, 256, 0, X.s>>>(X.P, L, A.nc, A.Ju, nullptr, nullptr, A.rhs, 2);  // b = P Ju
     auto Vj = [&](int j) { return A.kry + (size_t)j * n; };
-    // h[0..k) = V[0..k)^T w, copied to the host
-    auto dots = [&](int k, const double *w, double *h) {
-        k_gm_dots<<<dim3(kDotBlocks, k), 256, 0, X.s>>>(A.kry, n, w, A.gpart);
-        k_gm_dots_final<<<(k + 127) / 128, 128, 0, X.s>>>(A.gpart, kDotBlocks, k, A.gh);
-        CK(cudaMemcpyAsync(h, A.gh, k * sizeof(double), cudaMemcpyDeviceToHost, X.s));
-        CK(cudaStreamSynchronize(X.s));
+    // A.gh[at..at+k) = V[0..k)^T w, copied to pinned memory: the host needs them
+    // at the end of an iteration only (one wait there, where waiting after
+    // each of its three reductions left the GPU idle three times)
+    auto dots = [&](const double *V, int k, const double *w, int at) {
+        k_gm_dots<<<dim3(kDotBlocks, k), 256, 0, X.s>>>(V, n, w, A.gpart);
+        k_gm_dots_final<<<(k + 31) / 32, 32, 0, X.s>>>(A.gpart, kDotBlocks, k, A.gh + at, X.h_out + at);
     };
     auto norm = [&](const double *w) {
-        k_gm_dots<<<dim3(kDotBlocks, 1), 256, 0, X.s>>>(w, n, w, A.gpart);
-        k_gm_dots_final<<<1, 32, 0, X.s>>>(A.gpart, kDotBlocks, 1, A.gh);
-        double h;
-        CK(cudaMemcpyAsync(&h, A.gh, sizeof(double), cudaMemcpyDeviceToHost, X.s));
+        dots(w, 1, w, 0);
         CK(cudaStreamSynchronize(X.s));
-        return std::sqrt(h);
+        return std::sqrt(X.h_out[0]);
     };
-    std::vector<double> H((size_t)(m + 1) * m), cs(m), sn(m), g(m + 1), hv(m + 1), y(m);
+    std::vector<double> H((size_t)(m + 1) * m), cs(m), sn(m), g(m + 1), y(m);
     auto Hij = [&](int i, int j) -> double & { return H[(size_t)j * (m + 1) + i]; };
     int total = 0;
     double res = 1.0, prev = -1.0;
@@ -1585,16 +1669,17 @@ static int gmres_solve(flite_ctx &X, SteadyAdjoint &A, double bnorm, double tol,
             reverse(X, A, Vj(k), false);
             k_gm_apply<<<eb, 256, 0, X.s>>>(X.P, L, A.nc, Vj(k), A.ubar, nullptr, w, 0);
             ++total;
-            for (int i = 0; i <= k; ++i) Hij(i, k) = 0.0;
             for (int pass = 0; pass < 2; ++pass) {  // classical Gram-Schmidt, twice
-                dots(k + 1, w, hv.data());  // also left in A.gh
-                k_gm_combine<<<eb, 256, 0, X.s>>>(A.kry, n, k + 1, A.gh, -1.0, w);
-                for (int i = 0; i <= k; ++i) Hij(i, k) += hv[i];
+                dots(A.kry, k + 1, w, pass * (m + 1));
+                k_gm_combine<<<eb, 256, 0, X.s>>>(A.kry, n, k + 1, A.gh + pass * (m + 1), -1.0, w);
             }
-            const double hn = norm(w);
+            dots(w, 1, w, 2 * (m + 1));
+            k_gm_unit<<<eb, 256, 0, X.s>>>(w, n, A.gh + 2 * (m + 1));
+            CK(cudaStreamSynchronize(X.s));
+            for (int i = 0; i <= k; ++i) Hij(i, k) = (0.0 + X.h_out[i]) + X.h_out[m + 1 + i];
+            const double hn = std::sqrt(X.h_out[2 * (m + 1)]);
             if (!std::isfinite(hn)) return FLITE_ENAN;
             Hij(k + 1, k) = hn;
-            if (hn > 0) k_gm_scale<<<eb, 256, 0, X.s>>>(w, n, 1.0 / hn);
             for (int i = 0; i < k; ++i) {  // earlier rotations
                 const double a = Hij(i, k), b = Hij(i + 1, k);
                 Hij(i, k) = cs[i] * a + sn[i] * b;
