@@ -89,20 +89,24 @@ __global__ void k_state_pass(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_, in
 // 0.001)): the convective and acoustic terms, and with viscosity the other
 // node's viscous term (def_par:13432-13433; with SA the viscosity is
 // mu + nu~/Re)
-__device__ __forceinline__ void ts_inc(const Params &P, const LevelView &L, int2 t, double m1, double m2, double m3,
-                                       double ro, double cc, double &acc, double &h) {
+__device__ __forceinline__ void ts_terms(const Params &P, const LevelView &L, int2 t, double m1, double m2, double m3,
+                                         double ro, double cc, double *v) {
     const int N = L.N;
     const int e = t.x >= 0 ? t.x : ~t.x;
     const double wx = L.wx[e], wy = L.wy[e], wz = L.wz[e];
     const double al = (wx * wx + wy * wy) + wz * wz;
     const double vn = ((wx * m1 + wy * m2) + wz * m3) * ro;
-    acc = (acc + fabs(vn)) + sqrt(cc * al);
+    v[0] = fabs(vn);
+    v[1] = sqrt(cc * al);
     if (P.viscous) {
         const int j = t.y;
         const double vis = dmax(P.am, P.sa ? L.mu[j] + L.u[5 * N + j] / P.Re : L.mu[j]);
-        const double dv = 2.0 * vis * al / L.u[j];
-        h = h + dv;
+        v[2] = 2.0 * vis * al / L.u[j];
     }
+}
+__device__ __forceinline__ void ts_add(const Params &P, const double *v, double &acc, double &h) {
+    acc = (acc + v[0]) + v[1];
+    if (P.viscous) h = h + v[2];
 }
 // boundary edge binc[k]: v[0..3] the convective and acoustic terms of the
 // node's side and of both, v[4..5] the viscous ones
@@ -165,28 +169,14 @@ __device__ __forceinline__ void ts_group(const Params &P, const LevelView &L, in
     double x[2] = {0.0, 0.0};
     group_sum<U, 2, 2, double>(
         gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl,
-        [&](int k, double *v) {
-            const int2 t = L.inc[k];
-            const int e = t.x >= 0 ? t.x : ~t.x;
-            const double wx = L.wx[e], wy = L.wy[e], wz = L.wz[e];
-            const double al = (wx * wx + wy * wy) + wz * wz;
-            const double vn = ((wx * m1 + wy * m2) + wz * m3) * ro;
-            v[0] = fabs(vn);
-            v[1] = sqrt(cc * al);
-            if (P.viscous) {
-                const int j = t.y;
-                const double vis = dmax(P.am, P.sa ? L.mu[j] + L.u[5 * N + j] / P.Re : L.mu[j]);
-                v[2] = 2.0 * vis * al / L.u[j];
-            }
-        },
-        x);
+        [&](int k, double *v) { ts_terms(P, L, L.inc[k], m1, m2, m3, ro, cc, v); }, x);
     group_sum<U, 2, 4, double>(
         gs, L.binc_ptr[i], L.binc_ptr[i + 1], active, gl, [&](int k, double *v) { ts_bterms(P, L, k, v); }, x);
     if (active && gl == 0) ts_store(L, i, x[0], x[1]);
 }
 
 template <int U, bool B>
-__global__ void k_timestep(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_) {
+__global__ void __launch_bounds__(256, U == 1 ? 4 : 1) k_timestep(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_) {
     FLITE_CASE_P(B, P, L);
     FLITE_CASE_L(B, L);
     const int gl = U > 1 ? (int)(threadIdx.x % U) : 0;  // lane in the node's group
@@ -203,7 +193,9 @@ __global__ void k_timestep(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_) {
         ts_group<U>(P, L, i, active, gl, gs, m1, m2, m3, ro, cc);
     } else {
         double acc = 0.0, h = 0.0;
-        FLITE_FOR_INC(L, i, t) ts_inc(P, L, t, m1, m2, m3, ro, cc, acc, h);
+        walk<2, 3>(
+            L, i, [&](const int2 t, double *v) { ts_terms(P, L, t, m1, m2, m3, ro, cc, v); },
+            [&](const double *v) { ts_add(P, v, acc, h); });
         ts_finish(P, L, i, acc, h);
     }
 }
@@ -214,29 +206,27 @@ struct LapAcc {
     double l[5], s7, s8;
 };
 // interior edge t of node i (state ui, pressure pi)
-__device__ __forceinline__ void lap_inc(const Params &P, const LevelView &L, int2 t, const double *ui, double pi,
-                                        LapAcc &a) {
+__device__ __forceinline__ void lap_terms(const Params &P, const LevelView &L, int2 t, const double *ui, double pi,
+                                          double *v) {
     const int N = L.N;
     const int j = t.y;
     double df = 1.0;
     if (P.useDissW) df = 1. / L.slen[t.x >= 0 ? t.x : ~t.x];
     const double uj[5] = {L.u[j], L.u[N + j], L.u[2 * N + j], L.u[3 * N + j], L.u[4 * N + j]};
     const double pj = L.p[j];
-    if (t.x >= 0) {  // this node is i1: d = u(i) - u(j)
+    // The edge's first node subtracts its differences d(i, j), the second adds
+    // d(j, i): the same terms, as -(x - y) is y - x, up to the order of the
+    // pressures in the last one (a zero's sign is lost in the sums)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) a.l[c] = a.l[c] - (ui[c] - uj[c]) * df;
-        const double d4 = ((ui[4] - uj[4]) + pi) - pj;
-        a.l[4] = a.l[4] - d4 * df;
-        const double dp = pi - pj, sp = pi + pj;
-        a.s7 = a.s7 - dp; a.s8 = a.s8 + sp;
-    } else {         // i2: d = u(j) - u(i)
+    for (int c = 0; c < 4; ++c) v[c] = (uj[c] - ui[c]) * df;
+    const bool first = t.x >= 0;
+    v[4] = (((uj[4] - ui[4]) + (first ? -pi : pj)) + (first ? pj : -pi)) * df;
+    v[5] = pj - pi; v[6] = pj + pi;
+}
+__device__ __forceinline__ void lap_add(const double *v, LapAcc &a) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c) a.l[c] = a.l[c] + (uj[c] - ui[c]) * df;
-        const double d4 = ((uj[4] - ui[4]) + pj) - pi;
-        a.l[4] = a.l[4] + d4 * df;
-        const double dp = pj - pi, sp = pj + pi;
-        a.s7 = a.s7 + dp; a.s8 = a.s8 + sp;
-    }
+    for (int c = 0; c < 5; ++c) a.l[c] = a.l[c] + v[c];
+    a.s7 = a.s7 + v[5]; a.s8 = a.s8 + v[6];
 }
 __device__ __forceinline__ void lap_store(const LevelView &L, int i, const LapAcc &a) {
     const int N = L.N;
@@ -250,32 +240,10 @@ __device__ __forceinline__ void lap_store(const LevelView &L, int i, const LapAc
 template <int U>
 __device__ __forceinline__ void lap_group(const Params &P, const LevelView &L, int i, bool active, int gl, double *gs,
                                           const double *ui, double pi) {
-    const int N = L.N;
     double x[7] = {0, 0, 0, 0, 0, 0, 0};
     group_sum<U, 7, 1, double>(
         gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl,
-        [&](int k, double *v) {
-            const int2 t = L.inc[k];
-            const int j = t.y;
-            double df = 1.0;
-            if (P.useDissW) df = 1. / L.slen[t.x >= 0 ? t.x : ~t.x];
-            const double uj[5] = {L.u[j], L.u[N + j], L.u[2 * N + j], L.u[3 * N + j], L.u[4 * N + j]};
-            const double pj = L.p[j];
-            // x - y is x + (-y): the subtractions of the serial loop become
-            // additions of negated terms
-            if (t.x >= 0) {
-#pragma unroll
-                for (int c = 0; c < 4; ++c) v[c] = -((ui[c] - uj[c]) * df);
-                v[4] = -((((ui[4] - uj[4]) + pi) - pj) * df);
-                v[5] = -(pi - pj); v[6] = pi + pj;
-            } else {
-#pragma unroll
-                for (int c = 0; c < 4; ++c) v[c] = (uj[c] - ui[c]) * df;
-                v[4] = (((uj[4] - ui[4]) + pj) - pi) * df;
-                v[5] = pj - pi; v[6] = pj + pi;
-            }
-        },
-        x);
+        [&](int k, double *v) { lap_terms(P, L, L.inc[k], ui, pi, v); }, x);
     if (active && gl == 0) {
         const LapAcc a = {{x[0], x[1], x[2], x[3], x[4]}, x[5], x[6]};
         lap_store(L, i, a);
@@ -283,7 +251,7 @@ __device__ __forceinline__ void lap_group(const Params &P, const LevelView &L, i
 }
 
 template <int U, bool B>
-__global__ void k_jst_lap(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_) {
+__global__ void __launch_bounds__(256, U == 1 ? 3 : 1) k_jst_lap(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_) {
     FLITE_CASE_P(B, P, L);
     FLITE_CASE_L(B, L);
     const int gl = U > 1 ? (int)(threadIdx.x % U) : 0;  // lane in the node's group
@@ -299,7 +267,9 @@ __global__ void k_jst_lap(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_) {
         lap_group<U>(P, L, i, active, gl, gs, ui, pi);
     } else {
         LapAcc a = {{0, 0, 0, 0, 0}, 0, 0};
-        FLITE_FOR_INC(L, i, t) lap_inc(P, L, t, ui, pi, a);
+        walk<2, 7>(
+            L, i, [&](const int2 t, double *v) { lap_terms(P, L, t, ui, pi, v); },
+            [&](const double *v) { lap_add(v, a); });
         lap_store(L, i, a);
     }
 }
@@ -308,29 +278,30 @@ __global__ void k_jst_lap(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_) {
 // interior edge t of node i (Laplacian Li, state Ui, V/dt vdi, connectivity
 // coni, sensor si): the fourth- and second-order terms with the sign of
 // this node
-__device__ __forceinline__ void jflux_inc(const Params &P, const LevelView &L, int2 t, double k4, double vdi,
-                                          double coni, double si, const double *Li, const double *Ui, double *acc) {
+__device__ __forceinline__ void jflux_terms(const Params &P, const LevelView &L, const double *u, int2 t, double k4,
+                                            double vdi, double coni, double si, const double *Li, const double *Ui,
+                                            double *v) {
     const int N = L.N;
     const int j = t.y;
     const double vdj = L.vdt[j];
     const bool first = t.x >= 0;
     double d0 = first ? dmin(vdi, vdj) : dmin(vdj, vdi);
-    d0 = d0 / (first ? (coni + L.conn[j]) : (L.conn[j] + coni));
+    d0 = d0 / (coni + L.conn[j]);
     const double sj = L.sens[j];
     const double d2 = d0 * P.k2 * (first ? dmax(si, sj) : dmax(sj, si));
     double d4 = d0 * k4;
     d4 = d4 > d2 ? d4 - d2 : 0.0;
+    // acc - (Li - Lj) d4 + (Ui - Uj) d2 for the edge's first node, acc +
+    // (Lj - Li) d4 - (Uj - Ui) d2 for its second: the same terms
 #pragma unroll
     for (int c = 0; c < 5; ++c) {
-        const double Lj = L.lap[c * N + j], Uj = L.u[c * N + j];
-        if (first) {
-            const double d4v = Li[c] - Lj, d2v = Ui[c] - Uj;
-            acc[c] = (acc[c] - d4v * d4) + d2v * d2;
-        } else {
-            const double d4v = Lj - Li[c], d2v = Uj - Ui[c];
-            acc[c] = (acc[c] + d4v * d4) - d2v * d2;
-        }
+        v[2 * c] = (L.lap[c * N + j] - Li[c]) * d4;
+        v[2 * c + 1] = (Ui[c] - u[c * N + j]) * d2;
     }
+}
+__device__ __forceinline__ void jflux_add(const double *v, double *acc) {
+#pragma unroll
+    for (int c = 0; c < 5; ++c) acc[c] = (acc[c] + v[2 * c]) + v[2 * c + 1];
 }
 
 // node i's scalar JST flux with U lanes (a slab of 10 terms) at the state u;
@@ -346,34 +317,11 @@ __device__ __forceinline__ void jflux_group(const Params &P, const LevelView &L,
     const double vdi = L.vdt[i], coni = L.conn[i], si = L.sens[i];
     group_sum<U, 5, 2, double>(
         gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl,
-        [&](int k, double *v) {
-            const int2 t = L.inc[k];
-            const int j = t.y;
-            const double vdj = L.vdt[j];
-            const bool first = t.x >= 0;
-            double d0 = first ? dmin(vdi, vdj) : dmin(vdj, vdi);
-            d0 = d0 / (first ? (coni + L.conn[j]) : (L.conn[j] + coni));
-            const double sj = L.sens[j];
-            const double d2 = d0 * P.k2 * (first ? dmax(si, sj) : dmax(sj, si));
-            double d4 = d0 * k4;
-            d4 = d4 > d2 ? d4 - d2 : 0.0;
-#pragma unroll
-            for (int c = 0; c < 5; ++c) {
-                const double Lj = L.lap[c * N + j], Uj = u[c * N + j];
-                if (first) {
-                    v[2 * c] = -((Li[c] - Lj) * d4);
-                    v[2 * c + 1] = (Ui[c] - Uj) * d2;
-                } else {
-                    v[2 * c] = (Lj - Li[c]) * d4;
-                    v[2 * c + 1] = -((Uj - Ui[c]) * d2);
-                }
-            }
-        },
-        acc);
+        [&](int k, double *v) { jflux_terms(P, L, u, L.inc[k], k4, vdi, coni, si, Li, Ui, v); }, acc);
 }
 
 template <int U, bool B>
-__global__ void __launch_bounds__(256, U == 1 ? 4 : 1) k_jst_flux(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_) {
+__global__ void __launch_bounds__(256, U == 1 ? 2 : 1) k_jst_flux(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_) {
     FLITE_CASE_P(B, P, L);
     FLITE_CASE_L(B, L);
     const int gl = U > 1 ? (int)(threadIdx.x % U) : 0;  // lane in the node's group
@@ -392,7 +340,9 @@ __global__ void __launch_bounds__(256, U == 1 ? 4 : 1) k_jst_flux(CaseArg<B, Par
         double Li[5], Ui[5];
         for (int c = 0; c < 5; ++c) { Li[c] = L.lap[c * N + i]; Ui[c] = L.u[c * N + i]; }
         const double vdi = L.vdt[i], coni = L.conn[i], si = L.sens[i];
-        FLITE_FOR_INC(L, i, t) jflux_inc(P, L, t, k4, vdi, coni, si, Li, Ui, acc);
+        walk<2, 10>(
+            L, i, [&](const int2 t, double *v) { jflux_terms(P, L, L.u, t, k4, vdi, coni, si, Li, Ui, v); },
+            [&](const double *v) { jflux_add(v, acc); });
     }
     for (int c = 0; c < 5; ++c) L.diss[c * N + i] = acc[c];
 }
@@ -670,18 +620,20 @@ __device__ __forceinline__ void visc_grad_finish(const Params &P, const LevelVie
 
 // interior edge t of node i (u, v, w, T of the node qi): the edge's terms
 // of the 12 gradient sums, added with the sign of this node
-__device__ __forceinline__ void vgrad_inc(const LevelView &L, int2 t, const double *qi, double *g) {
-    const int N = L.N;
-    const int e = t.x >= 0 ? t.x : ~t.x, j = t.y;
+__device__ __forceinline__ void vgrad_terms(const LevelView &L, int2 t, const double *qi, double *v) {
+    const int N = L.N, e = t.x >= 0 ? t.x : ~t.x, j = t.y;
     const double qj[4] = {L.prim[j], L.prim[N + j], L.prim[2 * N + j], L.prim[3 * N + j]};
     const double w[3] = {L.wx[e], L.wy[e], L.wz[e]};
 #pragma unroll
-    for (int a = 0; a < 3; ++a)
+    for (int a = 0; a < 3; ++a) {
+        const double ws = t.x >= 0 ? w[a] : -w[a];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const double x = (t.x >= 0 ? qi[c] + qj[c] : qj[c] + qi[c]) * w[a];
-            g[a * 4 + c] = t.x >= 0 ? g[a * 4 + c] + x : g[a * 4 + c] - x;
-        }
+        for (int c = 0; c < 4; ++c) v[a * 4 + c] = (qi[c] + qj[c]) * ws;
+    }
+}
+__device__ __forceinline__ void vgrad_add(const double *v, double *g) {
+#pragma unroll
+    for (int c = 0; c < 12; ++c) g[c] = g[c] + v[c];
 }
 // the boundary edges of node i in order
 __device__ __forceinline__ void visc_grad_boundary(const LevelView &L, int i, double *g) {
@@ -703,26 +655,13 @@ __device__ __forceinline__ void vgrad_group(const LevelView &L, int i, bool acti
     for (int c = 0; c < 12; ++c) g[c] = 0.0;
     group_sum<U, 12, 1, double>(
         gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl,
-        [&](int k, double *d) {
-            const int2 t = L.inc[k];
-            const int e = t.x >= 0 ? t.x : ~t.x, j = t.y;
-            const double qj[4] = {L.prim[j], L.prim[N + j], L.prim[2 * N + j], L.prim[3 * N + j]};
-            const double w[3] = {L.wx[e], L.wy[e], L.wz[e]};
-#pragma unroll
-            for (int a = 0; a < 3; ++a)
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const double x = (t.x >= 0 ? qi[c] + qj[c] : qj[c] + qi[c]) * w[a];
-                    d[a * 4 + c] = t.x >= 0 ? x : -x;  // g - x is g + (-x)
-                }
-        },
-        g);
+        [&](int k, double *v) { vgrad_terms(L, L.inc[k], qi, v); }, g);
     group_sum<U, 12, 1, double>(
         gs, L.binc_ptr[i], L.binc_ptr[i + 1], active, gl, [&](int k, double *d) { visc_grad_bterms(L, k, d); }, g);
 }
 
 template <int U, bool B>
-__global__ void __launch_bounds__(256, U == 1 ? 3 : 1) k_visc_grad(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_) {
+__global__ void __launch_bounds__(256, U == 1 ? 2 : 1) k_visc_grad(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_) {
     FLITE_CASE_P(B, P, L);
     FLITE_CASE_L(B, L);
     const int gl = U > 1 ? (int)(threadIdx.x % U) : 0;  // lane in the node's group
@@ -739,7 +678,9 @@ __global__ void __launch_bounds__(256, U == 1 ? 3 : 1) k_visc_grad(CaseArg<B, Pa
     } else {
         for (int c = 0; c < 12; ++c) g[c] = 0.0;
         const double qi[4] = {L.prim[i], L.prim[N + i], L.prim[2 * N + i], L.prim[3 * N + i]};
-        FLITE_FOR_INC(L, i, t) vgrad_inc(L, t, qi, g);
+        walk<2, 12>(
+            L, i, [&](const int2 t, double *v) { vgrad_terms(L, t, qi, v); },
+            [&](const double *v) { vgrad_add(v, g); });
         visc_grad_boundary(L, i, g);
     }
     visc_grad_finish(P, L, i, g);
@@ -848,7 +789,7 @@ __device__ __forceinline__ void vflux_group(const LevelView &L, int i, bool acti
 }
 
 template <int U, bool B>
-__global__ void __launch_bounds__(256, U == 1 ? 3 : 1) k_visc_flux(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_) {
+__global__ void __launch_bounds__(256, U == 1 ? 2 : 1) k_visc_flux(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_) {
     FLITE_CASE_P(B, P, L);
     FLITE_CASE_L(B, L);
     const int gl = U > 1 ? (int)(threadIdx.x % U) : 0;  // lane in the node's group
@@ -866,11 +807,11 @@ __global__ void __launch_bounds__(256, U == 1 ? 3 : 1) k_visc_flux(CaseArg<B, Pa
         double ti[9];
         for (int c = 0; c < 9; ++c) ti[c] = L.tau[c * N + i];
         const double ui[3] = {L.prim[i], L.prim[N + i], L.prim[2 * N + i]};
-        FLITE_FOR_INC(L, i, t) {
-            double v[4];
-            vflux_terms(L, t, ti, ui, v);
-            for (int c = 0; c < 4; ++c) acc[c] = acc[c] + v[c];
-        }
+        walk<2, 4>(
+            L, i, [&](const int2 t, double *v) { vflux_terms(L, t, ti, ui, v); },
+            [&](const double *v) {
+                for (int c = 0; c < 4; ++c) acc[c] = acc[c] + v[c];
+            });
         visc_flux_boundary(L, i, acc);
     }
     for (int c = 0; c < 4; ++c) L.diss[(1 + c) * N + i] = L.diss[(1 + c) * N + i] - acc[c];
@@ -907,10 +848,16 @@ __global__ void __launch_bounds__(256, U == 1 ? 3 : 1) k_ts_lap(CaseArg<B, Param
     } else {
         double acc = 0.0, h = 0.0;
         LapAcc a = {{0, 0, 0, 0, 0}, 0, 0};
-        FLITE_FOR_INC(L, i, t) {
-            ts_inc(P, L, t, ui[1], ui[2], ui[3], ro, cc, acc, h);
-            lap_inc(P, L, t, ui, pi, a);
-        }
+        walk<1, 10>(
+            L, i,
+            [&](const int2 t, double *v) {
+                ts_terms(P, L, t, ui[1], ui[2], ui[3], ro, cc, v);
+                lap_terms(P, L, t, ui, pi, v + 3);
+            },
+            [&](const double *v) {
+                ts_add(P, v, acc, h);
+                lap_add(v + 3, a);
+            });
         lap_store(L, i, a);
         ts_finish(P, L, i, acc, h);
     }
@@ -947,10 +894,16 @@ __global__ void __launch_bounds__(256, U == 1 ? 2 : 1) k_jflux_vgrad(CaseArg<B, 
         const double vdi = L.vdt[i], coni = L.conn[i], si = L.sens[i];
         const double qi[4] = {L.prim[i], L.prim[N + i], L.prim[2 * N + i], L.prim[3 * N + i]};
         for (int c = 0; c < 12; ++c) g[c] = 0.0;
-        FLITE_FOR_INC(L, i, t) {
-            jflux_inc(P, L, t, k4, vdi, coni, si, Li, Ui, acc);
-            vgrad_inc(L, t, qi, g);
-        }
+        walk<1, 22>(
+            L, i,
+            [&](const int2 t, double *v) {
+                jflux_terms(P, L, L.u, t, k4, vdi, coni, si, Li, Ui, v);
+                vgrad_terms(L, t, qi, v + 10);
+            },
+            [&](const double *v) {
+                jflux_add(v, acc);
+                vgrad_add(v + 10, g);
+            });
         for (int c = 0; c < 5; ++c) L.diss[c * N + i] = acc[c];
         visc_grad_boundary(L, i, g);
     }
@@ -1232,7 +1185,7 @@ __device__ __forceinline__ void hllc_prim(const LevelView &L, int j, double *q) 
     q[0] = L.u[j]; q[1] = L.hprim[j]; q[2] = L.hprim[N + j]; q[3] = L.hprim[2 * N + j]; q[4] = L.u[4 * N + j];
 }
 template <bool MINMAX>
-__global__ void __launch_bounds__(256, 2) k_gradient(Params P, LevelView L) {
+__global__ void __launch_bounds__(256) k_gradient(Params P, LevelView L) {
     const int i = tid();
     if (i >= L.N) return;
     const int N = L.N;
@@ -1243,29 +1196,26 @@ __global__ void __launch_bounds__(256, 2) k_gradient(Params P, LevelView L) {
     for (int c = 0; c < 5; ++c) { mn[c] = 1.0e15; mx[c] = 1.0e15; }
     double qi[5];
     hllc_prim(L, i, qi);
-    FLITE_FOR_INC(L, i, t) {
+    walk<2, 9>(L, i, [&](const int2 t, double *v) {
         const int e = t.x >= 0 ? t.x : ~t.x;
-        double qj[5];
-        hllc_prim(L, t.y, qj);
+        hllc_prim(L, t.y, v);
         const double w[3] = {L.wx[e], L.wy[e], L.wz[e]};
+        for (int a = 0; a < 3; ++a) v[5 + a] = t.x >= 0 ? w[a] : -w[a];
+        v[8] = t.x >= 0 ? 1.0 : 0.0;
+    }, [&](const double *v) {
 #pragma unroll
         for (int a = 0; a < 3; ++a)
 #pragma unroll
-            for (int c = 0; c < 5; ++c) {
-                const double s = t.x >= 0 ? qi[c] + qj[c] : qj[c] + qi[c];
-                const double dq = s * w[a];
-                g[a * 5 + c] = t.x >= 0 ? g[a * 5 + c] + dq : g[a * 5 + c] - dq;
-            }
+            for (int c = 0; c < 5; ++c) g[a * 5 + c] = g[a * 5 + c] + (qi[c] + v[c]) * v[5 + a];
         if (MINMAX) {
-            // amin1(q(i1), q(i2)) with the edge's own node order
 #pragma unroll
             for (int c = 0; c < 5; ++c) {
-                const double a = t.x >= 0 ? qi[c] : qj[c], b = t.x >= 0 ? qj[c] : qi[c];
+                const double a = v[8] != 0.0 ? qi[c] : v[c], b = v[8] != 0.0 ? v[c] : qi[c];
                 mn[c] = dmin(mn[c], dmin(a, b));
                 mx[c] = dmin(mx[c], dmin(-a, -b));
             }
         }
-    }
+    });
     for (int k = L.binc_ptr[i]; k < L.binc_ptr[i + 1]; ++k) {
         const int b = L.binc[k] >> 1, side = L.binc[k] & 1;
         const int2 nd = L.bedge[b];
@@ -1311,7 +1261,7 @@ __global__ void k_prim_rec(LevelView L) {
 // the Galerkin gradient of k_gradient (computeGradient, def_par:2923-3245),
 // in the same summation order, from the primitive records, stored as
 // component-major records
-__global__ void k_gradient_rec(LevelView L) {
+__global__ void __launch_bounds__(256) k_gradient_rec(LevelView L) {
     int i = tid();
     if (i >= L.N) return;
     double g[15];
@@ -1319,21 +1269,18 @@ __global__ void k_gradient_rec(LevelView L) {
     for (int c = 0; c < 15; ++c) g[c] = 0.0;
     const PrimRec Qi = load_prim(L.qp, L.N, i);
     const double qi[5] = {Qi.r, Qi.u, Qi.v, Qi.w, Qi.E};
-    FLITE_FOR_INC(L, i, t) {
+    walk<3, 8>(L, i, [&](const int2 t, double *v) {
         const int e = t.x >= 0 ? t.x : ~t.x;
-        // (the fifth pair of values is rho E and a coordinate)
         const double2 a0 = __ldg(L.qp + t.y), a1 = __ldg(L.qp + L.N + t.y);
-        const double qj[5] = {a0.x, a0.y, a1.x, a1.y, __ldg(&(L.qp + 2 * (size_t)L.N + t.y)->x)};
+        v[0] = a0.x; v[1] = a0.y; v[2] = a1.x; v[3] = a1.y; v[4] = __ldg(&(L.qp + 2 * (size_t)L.N + t.y)->x);
         const double w[3] = {L.wx[e], L.wy[e], L.wz[e]};
+        for (int a = 0; a < 3; ++a) v[5 + a] = t.x >= 0 ? w[a] : -w[a];
+    }, [&](const double *v) {
 #pragma unroll
         for (int a = 0; a < 3; ++a)
 #pragma unroll
-            for (int c = 0; c < 5; ++c) {
-                const double sum = t.x >= 0 ? qi[c] + qj[c] : qj[c] + qi[c];
-                const double dq = sum * w[a];
-                g[a * 5 + c] = t.x >= 0 ? g[a * 5 + c] + dq : g[a * 5 + c] - dq;
-            }
-    }
+            for (int c = 0; c < 5; ++c) g[a * 5 + c] = g[a * 5 + c] + (qi[c] + v[c]) * v[5 + a];
+    });
     for (int k = L.binc_ptr[i]; k < L.binc_ptr[i + 1]; ++k) {
         const int b = L.binc[k] >> 1, side = L.binc[k] & 1;
         const int2 nd = L.bedge[b];
@@ -1689,15 +1636,31 @@ __device__ __forceinline__ void gather_interior_delta(const LevelView &L, const 
     } else {
         const int deg = L.inc_ptr[i + 1] - L.inc_ptr[i];
         const IncRec32 *row = L.rows32 + ((size_t)L.row_ptr[i / kRow] * kRow + i % kRow);
-        for (int k = 0; k < deg; ++k, row += kRow) {
+        // two incidences at a time, for the loads in flight
+        auto add = [&](const float *v, bool first) {
+            for (int c = 0; c < 5; ++c) acc[c] += first ? v[c] : -v[c];
+        };
+        int k = 0;
+        IncRec32 a, b;
+        if (deg > 0) a = load_inc32(row, 0);
+        if (deg > 1) b = load_inc32(row, kRow);
+        for (; k + 1 < deg; k += 2) {
+            const IncRec32 t0 = a, t1 = b;
+            row += 2 * kRow;
+            if (k + 2 < deg) a = load_inc32(row, 0);
+            if (k + 3 < deg) b = load_inc32(row, kRow);
+            float v[5], w[5];
+            bool f, g;
+            terms(t0, v, f);
+            terms(t1, w, g);
+            add(v, f);
+            add(w, g);
+        }
+        if (k < deg) {
             float v[5];
-            bool first;
-            terms(load_inc32(row, 0), v, first);
-            if (first) {
-                for (int c = 0; c < 5; ++c) acc[c] += v[c];
-            } else {
-                for (int c = 0; c < 5; ++c) acc[c] -= v[c];
-            }
+            bool f;
+            terms(a, v, f);
+            add(v, f);
         }
     }
     const int N = L.N;
@@ -1826,11 +1789,7 @@ __device__ __forceinline__ void gather_interior(const LevelView &L, int i, doubl
         group_sum<U, 5, 1, double>(gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl,
                                         [&](int k, double *v) { terms(L.inc[k], v); }, r);
     } else {
-        FLITE_FOR_INC(L, i, t) {
-            double v[5];
-            terms(t, v);
-            add(v);
-        }
+        walk<2, 5>(L, i, terms, add);
     }
 }
 
@@ -2075,7 +2034,7 @@ __device__ __forceinline__ void node_tail(const Params &P, const LevelView &L, i
 // same, stored as the new mixed-precision anchor), GATHER_DELTA (anchor +
 // FP32 increments)
 template <int PREC, int U, int PRE, bool B>
-__global__ void __launch_bounds__(node_threads(PREC, U), U > 1 ? 2 : (central_ahead(PREC) ? 5 : 3))
+__global__ void __launch_bounds__(node_threads(PREC, U), U > 1 ? 2 : (central_ahead(PREC) ? 5 : (PREC == GATHER_DELTA ? 4 : 3)))
     k_node_update(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_, int mode, int stage, int io) {
     static_assert(PRE == PRE_NONE || U > 1, "the dissipation part takes lanes per node");
     FLITE_CASE_P(B, P, L);
@@ -2577,7 +2536,7 @@ __device__ __forceinline__ double sum256(const double *v, int lane) {
 // per block: sum (u-uprev)^2 and max |u-uprev| with its first index; a batch
 // takes all its cases in one launch (the case in blockIdx.y)
 template <bool B>
-__global__ void __launch_bounds__(256) k_resid_partial(CaseArg<B, LevelView> L_, double *part) {
+__global__ void __launch_bounds__(256, 2) k_resid_partial(CaseArg<B, LevelView> L_, double *part) {
     FLITE_CASE_L(B, L);
     __shared__ double ss[6][256];
     __shared__ double sm[6][256];
@@ -2585,16 +2544,32 @@ __global__ void __launch_bounds__(256) k_resid_partial(CaseArg<B, LevelView> L_,
     const int N = L.N, nv = L.nvar;
     double s[6] = {0, 0, 0, 0, 0, 0}, m[6] = {0, 0, 0, 0, 0, 0};
     int mi[6] = {0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff};
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
-        // the first node in the caller's numbering wins a tie (mg_par:1387-1396)
-        const int oi = L.perm ? L.perm[i] : i;
+    // the loads of two nodes at a time, all before the first sum: with a node's
+    // components read one after another the pass took 97 us on 815,425 nodes,
+    // with the loads of two nodes together 32 us (2 to 4 nodes: the same)
+    const int step = gridDim.x * blockDim.x;
+    for (int i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < N; i0 += 2 * step) {
+        double d[2][6];
+        int oi[2];
 #pragma unroll
-        for (int k = 0; k < 6; ++k) {
-            if (k >= nv) break;
-            const double d = L.u[(size_t)k * N + i] - L.uprev[(size_t)k * N + i];
-            s[k] = s[k] + d * d;
-            const double a = fabs(d);
-            if (a > m[k] || (a == m[k] && a > 0.0 && oi < mi[k])) { m[k] = a; mi[k] = oi; }
+        for (int q = 0; q < 2; ++q) {
+            const int i = i0 + q * step;
+            if (i >= N) break;
+            // the first node in the caller's numbering wins a tie (mg_par:1387-1396)
+            oi[q] = L.perm ? L.perm[i] : i;
+#pragma unroll
+            for (int k = 0; k < 5; ++k) d[q][k] = L.u[(size_t)k * N + i] - L.uprev[(size_t)k * N + i];
+            d[q][5] = nv == 6 ? L.u[5 * (size_t)N + i] - L.uprev[5 * (size_t)N + i] : 0.0;
+        }
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            if (i0 + q * step >= N) break;
+#pragma unroll
+            for (int k = 0; k < 6; ++k) {
+                const double a = fabs(d[q][k]);
+                s[k] = s[k] + a * a;
+                if (a > m[k] || (a == m[k] && a > 0.0 && oi[q] < mi[k])) { m[k] = a; mi[k] = oi[q]; }
+            }
         }
     }
 #pragma unroll

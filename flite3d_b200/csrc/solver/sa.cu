@@ -155,16 +155,19 @@ __global__ void k_sa_grad(Params P, LevelView L, int ts) {
             [&](int q, double *v) { sa_grad_bterms(P, L, q, v); }, g);
         if (!active || gl) return;
     } else {
-        FLITE_FOR_INC(L, i, t) {
-            double v[3];
-            if (ts) {
-                sa_ts_terms(P, L, t, m, ro, oRe, v);
-                x[0] = x[0] + v[0];
-                x[1] = x[1] + v[1];
-            }
-            sa_grad_terms(L, t, ti, v);
-            for (int c = 0; c < 3; ++c) g[c] = g[c] + v[c];
-        }
+        walk<2, 5>(
+            L, i,
+            [&](const int2 t, double *v) {
+                if (ts) sa_ts_terms(P, L, t, m, ro, oRe, v);
+                sa_grad_terms(L, t, ti, v + 2);
+            },
+            [&](const double *v) {
+                if (ts) {
+                    x[0] = x[0] + v[0];
+                    x[1] = x[1] + v[1];
+                }
+                for (int c = 0; c < 3; ++c) g[c] = g[c] + v[2 + c];
+            });
         for (int q = L.binc_ptr[i]; q < L.binc_ptr[i + 1]; ++q) {
             double v[4];
             if (ts) {
@@ -223,12 +226,9 @@ __global__ void k_sa_diff(Params P, LevelView L) {
         group_sum<U, 1, 1, double>(gs, L.binc_ptr[i], L.binc_ptr[i + 1], active, gl, bterms, acc);
         if (!active || gl) return;
     } else {
-        double v[1];
-        FLITE_FOR_INC(L, i, t) {
-            terms(t, v);
-            acc[0] = acc[0] + v[0];
-        }
+        walk<2, 1>(L, i, terms, [&](const double *v) { acc[0] = acc[0] + v[0]; });
         for (int q = L.binc_ptr[i]; q < L.binc_ptr[i + 1]; ++q) {
+            double v[1];
             bterms(q, v);
             acc[0] = acc[0] + v[0];
         }
@@ -273,11 +273,7 @@ __global__ void k_sa_conv(Params P, LevelView L, int td) {
             gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl, [&](int q, double *v) { terms(L.inc[q], v); }, acc);
         if (!active || gl) return;
     } else {
-        FLITE_FOR_INC(L, i, t) {
-            double v[1];
-            terms(t, v);
-            acc[0] = acc[0] + v[0];
-        }
+        walk<2, 1>(L, i, terms, [&](const double *v) { acc[0] = acc[0] + v[0]; });
     }
     L.rhs[5 * (size_t)N + i] = acc[0];
 }

@@ -103,3 +103,26 @@ def test_fine_nodes_without_a_parent_match_the_restatement():
         s.close()
     for a, b in zip(*got):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("size", [(46, 39, 40), (59, 51, 50)])
+def test_residual_norms_of_large_levels_match_the_restatement(size):
+    """Levels with more nodes than one pass of the norm's threads holds (77,080:
+    a second node for some threads; 159,120: a second round).  Any order of a
+    sum of n squares is within n eps of another, its root within half of that."""
+    mesh = Mesh.bump_channel(*size, 0.05, nlevels=1)
+    n = mesh.level(1).n_nodes
+    assert n > 296 * 256
+    c = default_controls(ReynoldsNumber=0.0, fluxType=1, CFLNumber=1.0, numberOfGridsToUse=1)
+    got = []
+    for be in (None, oracle_backend()):
+        s = Solver(c, mesh, backend=be)
+        s.set_state(initial_state(c, mesh, perturb_seed=5))
+        s.start()
+        s.cycle(1)
+        got.append(s.residuals())
+        s.close()
+    (r, m, k), (r0, m0, k0) = got
+    assert np.all(r0 > 0) and np.all(m0 > 0)
+    np.testing.assert_allclose(r, r0, rtol=n * np.finfo(float).eps)
+    assert np.array_equal(m, m0) and np.array_equal(k, k0)
