@@ -26,14 +26,22 @@ namespace flite {
 
 // far-field contributions per boundary edge: J(u_b1)^T |w|(3 rbar1 + rbar2)
 // and J(u_b2)^T |w|(rbar1 + 3 rbar2) (FV weighting: 4 rbar_own)
-// (a thread per edge, end and column: one dual evaluation each.  With a
-// thread per edge, which did ten one after the other, a launch over 10,752
-// edges took 29 us)
+// A thread takes COLS of an edge's ten columns (five of each end): 1 on levels
+// of up to kFarfieldColumns boundary edges, which leave the chip short of
+// threads, 5 above, where the columns of an end share the evaluation of its
+// values.  Whole product with 1 and 5 columns a thread: 32.9 and 43.0 us at
+// 11 k boundary edges, 47.4 and 50.9 at 34 k, 98.9 and 83.7 at 66 k, 284 and
+// 245 at 172 k (ten columns a thread took 29 us for 11 k edges alone).
+constexpr int kFarfieldColumns = 40000;
+template <int COLS>
 __global__ void k_vjp_farfield(Params P, LevelView L, const double *x, const double *rbar, double *bvjp) {
+    static_assert(COLS == 1 || COLS == 5, "a thread's columns belong to one end");
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int b = t / 10, side = (t % 10) / 5, j = t % 5;
+    const int b = t / (10 / COLS), first = t % (10 / COLS) * COLS, side = first / 5;
     if (b >= L.B) return;
-    bvjp[t] = 0.0;
+    double *o = bvjp + (size_t)b * 10 + first;
+#pragma unroll
+    for (int c = 0; c < COLS; ++c) o[c] = 0.0;
     const int ind = L.bind[b];
     if (ind != 3 && ind != 4) return;
     const double wx = L.bwx[b], wy = L.bwy[b], wz = L.bwz[b];
@@ -53,24 +61,36 @@ __global__ void k_vjp_farfield(Params P, LevelView L, const double *x, const dou
     double u[5], p, dp[5];
     for (int k = 0; k < 5; ++k) u[k] = x[(size_t)k * N + n];
     pressure_grad(P, u, &p, dp);
-    Dual q[5];
-    double dpj = 0.0;
-    for (int k = 0; k < 5; ++k) {
-        q[k] = Dual(u[k], k == j ? 1.0 : 0.0);
-        if (k == j) dpj = dp[k];
+#pragma unroll
+    for (int c = 0; c < COLS; ++c) {
+        const int j = COLS == 5 ? c : first % 5;
+        Dual q[5];
+        double dpj = 0.0;
+#pragma unroll
+        for (int k = 0; k < 5; ++k) {
+            q[k] = Dual(u[k], k == j ? 1.0 : 0.0);
+            if (k == j) dpj = dp[k];
+        }
+        Dual F[5];
+        farfield_dual(P, q, Dual(p, dpj), rnx, rny, rnz, inf, F);
+        double s = 0.0;
+        for (int k = 0; k < 5; ++k) s += F[k].d * a[k];
+        o[c] = s;
     }
-    Dual F[5];
-    farfield_dual(P, q, Dual(p, dpj), rnx, rny, rnz, inf, F);
-    double s = 0.0;
-    for (int k = 0; k < 5; ++k) s += F[k].d * a[k];
-    bvjp[t] = s;
+}
+void vjp_farfield(flite_ctx &X, const LevelView &L, const double *x, const double *rbar, double *bvjp) {
+    if (L.B <= 0) return;
+    if (L.B <= kFarfieldColumns)
+        k_vjp_farfield<1><<<X.eblk(10 * (size_t)L.B), X.eb, 0, X.s>>>(X.P, L, x, rbar, bvjp);
+    else
+        k_vjp_farfield<5><<<X.eblk(2 * (size_t)L.B), X.eb, 0, X.s>>>(X.P, L, x, rbar, bvjp);
 }
 
 // ubar = (dR/dx)^T rbar at the state x, plus pbar (dp/dx) when pbar is given
 // (a pressure read by the caller's own use of the state); add = 1 adds the
 // product to ubar instead of storing it
 template <int U>
-__global__ void k_vjp_node(Params P, LevelView L, const double *x, const double *rbar, const double *bvjp,
+__global__ void __launch_bounds__(256, U == 1 ? 2 : 1) k_vjp_node(Params P, LevelView L, const double *x, const double *rbar, const double *bvjp,
                            const double *pbar, double *ubar, int add) {
     FLITE_NODE_LANES(L);
     const int N = L.N;
@@ -181,7 +201,7 @@ extern "C" int flite_residual_vjp(flite_ctx *ctx, int level, const double *u, co
 
 void flite_ctx::vjp_kernels(int l) {
     LevelView &L = V(l);
-    if (L.B > 0) k_vjp_farfield<<<eblk(10 * (size_t)L.B), eb, 0, s>>>(P, L, L.u, adj_rbar, adj_b);
+    vjp_farfield(*this, L, L.u, adj_rbar, adj_b);
     FLITE_ADJ_GATHER(k_vjp_node, (*this), l, P, L, L.u, adj_rbar, adj_b, nullptr, adj_ubar, 0);
 }
 

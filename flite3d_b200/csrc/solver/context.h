@@ -1066,6 +1066,8 @@ struct flite_ctx {
 namespace flite {
 int create_context(const flite_controls *c, int nlevels, const flite_level_desc *levels, const flite_ctx *donor,
                    flite_ctx **out);
+// far-field edges' part of the transposed Jacobian's product (adjoint.cu)
+void vjp_farfield(flite_ctx &X, const LevelView &L, const double *x, const double *rbar, double *bvjp);
 // the geometry arrays of level l from its descriptor (allocated when create)
 void put_geometry(flite_ctx &X, int l, const flite_level_desc &d, bool create);
 }  // namespace flite

@@ -125,14 +125,17 @@ __device__ __forceinline__ void sum_incidences(const LevelView &L, int i, bool a
         group_sum<U, M, 1, double>(
             gs, L.inc_ptr[i], L.inc_ptr[i + 1], active, gl, [&](int q, double *v) { terms(L.inc[q], v); }, out);
     } else {
-        FLITE_FOR_INC(L, i, t) {
-            double v[M];
+        walk<2, M>(
+            L, i,
+            [&](const int2 t, double *v) {
 #pragma unroll
-            for (int m = 0; m < M; ++m) v[m] = 0.0;
-            terms(t, v);
+                for (int m = 0; m < M; ++m) v[m] = 0.0;
+                terms(t, v);
+            },
+            [&](const double *v) {
 #pragma unroll
-            for (int m = 0; m < M; ++m) out[m] = out[m] + v[m];
-        }
+                for (int m = 0; m < M; ++m) out[m] = out[m] + v[m];
+            });
     }
 }
 template <int U, int M, class Terms>

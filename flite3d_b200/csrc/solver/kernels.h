@@ -160,7 +160,6 @@ __global__ void k_forces3(Params P, LevelView L, const int *wall, int nwall, dou
 __global__ void k_forces_final(const double *part, int nval, double *out);
 constexpr int kForceBlocks = 64;
 // transposed residual Jacobian at the state x (adjoint.cu)
-__global__ void k_vjp_farfield(Params P, LevelView L, const double *x, const double *rbar, double *bvjp);
 template <int U>
 __global__ void k_vjp_node(Params P, LevelView L, const double *x, const double *rbar, const double *bvjp,
                            const double *pbar, double *ubar, int add);

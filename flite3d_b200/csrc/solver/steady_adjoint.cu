@@ -1500,7 +1500,7 @@ static void reverse(flite_ctx &X, SteadyAdjoint &A, const double *lam, bool geom
         const double *x = in[k - 1];
         k_adj_stage<<<nbk, X.nb, 0, X.s>>>(X.P, L, k, vin, A.u0, x, A.Q[k - 1], A.D, A.dt, A.ubar, A.Qbar, A.Dbar,
                                            A.dtbar, A.pbar, Vb, nb);
-        if (L.B > 0) k_vjp_farfield<<<X.eblk(10 * (size_t)L.B), X.eb, 0, X.s>>>(X.P, L, x, A.Qbar, A.bvjp);
+        vjp_farfield(X, L, x, A.Qbar, A.bvjp);
         double *vout = A.vb[k & 1];
         if (k > 1) FLITE_ADJ_GATHER(k_vjp_node, X, 0, X.P, L, x, A.Qbar, A.bvjp, A.pbar, vout, 0);
         else FLITE_ADJ_GATHER(k_vjp_node, X, 0, X.P, L, x, A.Qbar, A.bvjp, A.pbar, A.ubar, 1);

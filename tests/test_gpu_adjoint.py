@@ -94,3 +94,20 @@ def test_adjoint_cost_ratio_is_measured():
     g.set_state(initial_state(c, mesh))
     fwd, vjp = g.profile_adjoint(level=1, reps=5)
     assert fwd > 0 and vjp > 0
+
+
+@pytest.mark.parametrize("size", [(30, 16, 16), (88, 44, 44)])
+@pytest.mark.parametrize("boundary_term", [0, 1])
+def test_vjp_dot_product_identity_on_both_sides_of_the_far_field_rule(size, boundary_term):
+    """One and five columns a thread (up to and above 40,000 boundary edges),
+    and levels with a thread and with several lanes per node."""
+    mesh = Mesh.bump_channel(*size, 0.05, nlevels=1)
+    assert (mesh.level(1).n_bsides > 40000) == (size[0] > 80)
+    c, g, o = pair(mesh, boundaryTerm=boundary_term, numberOfGridsToUse=1)
+    u = o.get_state(1)
+    rng = np.random.default_rng(17)
+    du, rbar = rng.standard_normal(u.shape), rng.standard_normal(u.shape)
+    jv = o.residual_jvp(u, du, level=1)
+    ub = g.residual_vjp(u, rbar, level=1)
+    lhs, rhs = float(np.dot(rbar.ravel(), jv.ravel())), float(np.dot(ub.ravel(), du.ravel()))
+    assert abs(lhs - rhs) <= 1e-11 * float(np.abs(rbar * jv).sum())
