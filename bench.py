@@ -147,11 +147,11 @@ def node_kernel_bytes(mesh):
     record (own and neighbours' reads of one array, counted once), uprev
     (40 B), dissipation (40 B), dt and volume (16 B), u(rho) (8 B), boundary
     class (1 B), two CSR offsets (8 B) and the result (40 B); per interior
-    edge its two 8-byte incidence entries and its 32-byte coefficient record;
-    per boundary edge two incidence entries and two 40-byte contributions; per
+    edge its two 8-byte incidence entries and its coefficients (24 B); per
+    boundary edge two incidence entries and two 40-byte contributions; per
     boundary node its normal (24 B)."""
     d = mesh.level(1)
-    return d.n_nodes * (48 + 40 + 40 + 16 + 8 + 1 + 8 + 40) + d.n_sides * 48 + d.n_bsides * 88 \
+    return d.n_nodes * (48 + 40 + 40 + 16 + 8 + 1 + 8 + 40) + d.n_sides * 40 + d.n_bsides * 88 \
         + d.n_bnodes * 24
 
 
@@ -224,10 +224,10 @@ def group_roofline(ms, nbytes, hbm):
 
 # DRAM traffic of the dominant kernel per algorithmic byte, from an ncu
 # capture (dram__bytes_read.sum + dram__bytes_write.sum) of one launch on the
-# 192x64x64 bump channel (453.8 MB measured against 448.8 MB algorithmic,
+# 192x64x64 bump channel (415.3 MB measured against 404.1 MB algorithmic,
 # the lean node tail); the bench mesh is too large to capture with --set
 # full, and the traffic scales with the nodes and edges processed
-NCU_TRAFFIC_PER_ALGORITHMIC_BYTE = (425.17888 + 28.584448) / 448.800825
+NCU_TRAFFIC_PER_ALGORITHMIC_BYTE = (387.363328 + 27.967488) / 404.069945
 
 
 def run_ours(args):

@@ -382,10 +382,11 @@ struct flite_ctx {
     // default the widest group that keeps the level's threads within
     // kLaneThreads: below that a thread per node leaves SMs idle and each
     // thread waits on a long chain of dependent loads, above it the extra
-    // lanes only add instructions.  Sums of one relaxation step's kernels on
-    // bump-channel levels (us, lanes 1/4/8/32): 788 nodes 192/118/98/84,
-    // 1,707 147/103/91/82, 8,731 199/137/110/129, 23,549 156/135/134/209,
-    // 80,640 144/202/245/527.  A case group's cases share the launch.
+    // lanes only add instructions.  Sums of one relaxation step's kernels on the
+    // bump channel's agglomerated levels (us, lanes 1/4/8/32): 1,908 nodes
+    // 179/123/97/91, 21,972 193/163/164/227, 237,662 325/619/823/1856; on
+    // generated level-1 meshes 4,225 nodes 97/93/86/94, 32,269 99/123/144/250.
+    // A case group's cases share the launch.
     int lanes[kMaxLevels] = {0};
     int lanes_of(int l) const {
         if (l < kMaxLevels && lanes[l] > 0) return lanes[l];
@@ -400,8 +401,8 @@ struct flite_ctx {
     // (flite_set_gather_fusion: 1 on; 0 off, held as -1).  By default up to
     // kSharedWalkNodes nodes: there the walks are short of work and one launch
     // less pays; above, the separate kernels' smaller register counts do (one
-    // step's kernels, shared/separate: 92,988 nodes 188/212 us, 203,401 nodes
-    // 253/258, 237,662 nodes 364/345, 2,099,065 nodes 1866/1736)
+    // step's kernels, shared/separate: 99,099 nodes 137/150 us, 206,400 nodes
+    // 233/241, 242,219 nodes 283/271, 2,099,065 nodes 1661/1633)
     int fuse_mode[kMaxLevels] = {0};
     bool fuse_walks(int l) const {
         if (lanes_of(l) != 1) return false;

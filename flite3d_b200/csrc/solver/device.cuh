@@ -159,13 +159,12 @@ struct LevelView {
     NodeRec *qb;                           // [N] (central flux)
     DeltaRec *dqb;                         // [N] (FLITE_MIXED)
     double *p, *dt, *mu;                   // [N]
-    double *hvis;                          // [N]  viscous time-step term
     double *lap;                           // [5][N] undivided Laplacian
     double *sens;                          // [N]  pressure sensor
     double *lpw;                           // [N]  edge-factor sums of dissipation scheme 1 (level 1)
     double *tau;                           // [9][N] stress tensor + heat flux
     double *prim;                          // [4][N] u, v, w, T of the viscous term
-    NodeRec *q;                            // [N] written with p by k_pressure (48 B: the level-1
+    NodeRec *q;                            // [N] written with p by k_state_pass (48 B: the level-1
                                            // records of the bench mesh fit the 126 MB L2)
     // Spalart-Allmaras: nu~ is component 6 of u, uprev, rhs, src ([6][N])
     double *turbDiff, *dtT, *vort, *divg;  // [N] diffusion, turbulent dt, |curl u|, div u

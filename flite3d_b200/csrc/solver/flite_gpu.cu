@@ -514,7 +514,6 @@ int flite::create_context(const flite_controls *c, int nlevels, const flite_leve
             L.rhs = X.alloc<double>(nv * N); L.src = X.alloc<double>(nv * N);
             L.diss = X.alloc<double>(5 * (size_t)N);
             L.p = X.alloc<double>(N); L.dt = X.alloc<double>(N); L.mu = X.alloc<double>(N);
-            L.hvis = X.alloc<double>(N);
             for (double *a : {L.u, L.uprev, L.rhs, L.src})
                 CK(cudaMemset(a, 0, nv * N * sizeof(double)));
             CK(cudaMemset(L.diss, 0, 5 * (size_t)N * sizeof(double)));
@@ -528,7 +527,7 @@ int flite::create_context(const flite_controls *c, int nlevels, const flite_leve
             } else {
                 L.turbDiff = L.dtT = L.vort = L.divg = L.sag = L.sanh = L.saprim = L.savis = nullptr;
             }
-            for (double *a : {L.p, L.dt, L.mu, L.hvis}) CK(cudaMemset(a, 0, (size_t)N * sizeof(double)));
+            for (double *a : {L.p, L.dt, L.mu}) CK(cudaMemset(a, 0, (size_t)N * sizeof(double)));
             const bool hllc2 = c->fluxType == 4 && c->HLLCFluxOrder > 1 && l == 0;
             const bool muscl = c->reconstruction == FLITE_RECON_VAN_ALBADA && l == 0;
             const bool visc = c->ReynoldsNumber > 0.0;

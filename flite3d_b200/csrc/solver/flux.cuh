@@ -59,7 +59,7 @@ __device__ __forceinline__ void central_flux(const NodeState &a, const NodeState
 }
 
 // the same central flux from two node records (1/rho and E + p formed once
-// per node by k_pressure with the same operations)
+// per node by k_state_pass with the same operations)
 __device__ __forceinline__ void central_flux_rec(const NodeRec &a, const NodeRec &b, double wx, double wy,
                                                  double wz, double *f) {
     const double pr1 = a.p, rinv1 = a.rinv, ru1 = a.ru, rv1 = a.rv, rw1 = a.rw, rh1 = a.rh;

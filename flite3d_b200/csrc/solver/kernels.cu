@@ -3,11 +3,13 @@
 // Layout and scheduling:
 //  * node state is SoA [component][node] so node kernels read and write each
 //    component coalesced;
-//  * the interior-edge flux is computed once per edge into an edge buffer
-//    [E][5]; a node kernel then sums it through a CSR list of incident
-//    edges kept in edge order.  Summing in edge order reproduces the
-//    reference's scatter loop (rhs(i1)+=f, rhs(i2)-=f in edge order) bit for
-//    bit, with no atomics;
+//  * the interior edges' central fluxes are computed by both endpoints inside
+//    the node kernel; the upwind fluxes once per edge into an edge buffer
+//    [E][5], which the node kernel reads.  Either way a node sums its
+//    incident edges in edge order, which reproduces the reference's scatter
+//    loop (rhs(i1)+=f, rhs(i2)-=f in edge order) bit for bit, with no atomics;
+//  * every gather has two shapes: a thread per node on large levels, several
+//    lanes per node on small ones (gather.cuh);
 //  * cheap edge terms (time step, JST Laplacian and sensor, JST flux,
 //    gradients, min/max) are recomputed by both endpoints inside a node
 //    gather, which replaces an edge buffer round trip by reads of the
