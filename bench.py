@@ -172,7 +172,7 @@ def group_bytes(mesh, dissipation_weighting=False):
                  (8), dissipation out (40), two offsets; per edge its two
                  incidences twice (and the edge length twice with dissipation
                  weighting);
-      visc_prim  u0..3 and p in (40), u, v, w, T out (32);
+      visc_prim  the state (40) in, p and u, v, w, T out (40);
       visc_grad  u, v, w, T (32), volume, p, rho (24), class (1), offsets (8),
                  mu (8) and tau (72) out; per edge two incidences and its
                  coefficients (40); per boundary edge as in timestep (40);
@@ -198,7 +198,7 @@ def group_bytes(mesh, dissipation_weighting=False):
         "timestep": N * (32 + 8 + 8 + 8 + 8 + 16) + E * (16 + 24) + B * (8 + 8 + 24),
         "dissipation": N * (40 + 8 + 8 + 8 + 8 + 40 + 40 + 8 + 40 + 8) + E * 32
         + (E * 16 if dissipation_weighting else 0),
-        "visc_prim": N * (40 + 32),
+        "visc_prim": N * (40 + 40),
         "visc_grad": N * (32 + 24 + 1 + 8 + 8 + 72) + E * 40 + B * 40 + Nb * 48,
         "visc_flux": N * (72 + 24 + 64 + 8) + E * 40 + B * 44,
         "node_update": node_kernel_bytes(mesh),

@@ -698,7 +698,7 @@ struct flite_ctx {
             case 3:
                 // the extension: MUSCL on level 1, upwind first order below
                 if (P.recon == FLITE_RECON_VAN_ALBADA && L.grid == 1)  // 256 threads: its store staging
-                    k_edge_flux_muscl<<<(unsigned)((L.E + 255) / 256), 256, 0, s>>>(P, L);
+                    k_edge_flux_muscl<<<(unsigned)((L.E + kMusclThreads - 1) / kMusclThreads), kMusclThreads, 0, s>>>(P, L);
                 else if (P.recon == FLITE_RECON_VAN_ALBADA) k_edge_flux<3, true><<<ng, eb, 0, s>>>(P, L);
                 else k_edge_flux<3, false><<<ng, eb, 0, s>>>(P, L);
                 break;

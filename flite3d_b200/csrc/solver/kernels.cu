@@ -1417,9 +1417,12 @@ template __global__ void k_edge_flux<4, false>(Params, LevelView);
 template __global__ void k_edge_flux<4, true>(Params, LevelView);
 
 // the upwind extension's level-1 edge flux into the edge buffer, stored as
-// k_edge_flux stores
-__global__ void __launch_bounds__(256) k_edge_flux_muscl(Params P, LevelView L) {
-    __shared__ __align__(16) double sf[256 * 5];
+// k_edge_flux stores.  Bound by L1 and FP64 latency, so by the warps in
+// flight; cycles of a mid-size case (ms) with 256 threads and 2, 3 blocks
+// 2.66, 2.44, with 128 threads and 4 to 8 blocks 2.62, 2.47, 2.42, 2.39
+// (7 blocks, 40 bytes of spills), 2.42.
+__global__ void __launch_bounds__(kMusclThreads, 7) k_edge_flux_muscl(Params P, LevelView L) {
+    __shared__ __align__(16) double sf[kMusclThreads * 5];
     const int e0 = blockIdx.x * blockDim.x, e = e0 + threadIdx.x;
     if (e < L.E) {
         const int2 nd = L.edge[e];

@@ -45,6 +45,7 @@ __global__ void k_lp_sums(Params P, LevelView L);
 __global__ void k_lp_flux(Params P, LevelView L);
 __global__ void k_prim_rec(LevelView L);
 __global__ void k_gradient_rec(LevelView L);
+constexpr int kMusclThreads = 128;
 __global__ void k_edge_flux_muscl(Params P, LevelView L);
 __global__ void k_ls_gradient(Params P, LevelView L);
 __global__ void k_minmax(Params P, LevelView L);
