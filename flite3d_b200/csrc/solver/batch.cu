@@ -29,6 +29,7 @@ struct flite_batch {
     std::vector<int> donor;  // index of the case owning the mesh copy
     std::vector<char> active;  // cases the batch graph advances
     std::vector<char> turb;    // calculateTurbulence each case's part of the graph was captured with
+    std::vector<unsigned> options;  // the launch options it was captured with (flite_ctx::options)
     std::vector<double> h_res;  // res1 of every case
     // the cases' residual norms: block partials, and the norms (pinned)
     double *d_part = nullptr, *h_out = nullptr;
@@ -57,11 +58,12 @@ struct flite_batch {
     }
 
     // calculateTurbulence of every case for cycle `cyc` (SA cases); a change
-    // drops the batch graph
+    // drops the batch graph, and so does a launch option set on a case since
+    // the graph was made
     void select_cycle(int cyc) {
         for (size_t i = 0; i < cases.size(); ++i) {
             cases[i]->select_cycle(cyc);
-            if (graph && turb[i] != (char)cases[i]->calcTurb) drop_graph();
+            if (graph && (turb[i] != (char)cases[i]->calcTurb || options[i] != cases[i]->options)) drop_graph();
         }
     }
     // cases whose cycles take the same launches (the controls that choose
@@ -110,7 +112,11 @@ struct flite_batch {
         if (graph) return;
         whole = std::find(active.begin(), active.end(), 0) == active.end();
         turb.resize(cases.size());
-        for (size_t i = 0; i < cases.size(); ++i) turb[i] = (char)cases[i]->calcTurb;
+        options.resize(cases.size());
+        for (size_t i = 0; i < cases.size(); ++i) {
+            turb[i] = (char)cases[i]->calcTurb;
+            options[i] = cases[i]->options;
+        }
         cudaGraph_t parent = nullptr;
         CK(cudaGraphCreate(&parent, 0));
         launches = 0;

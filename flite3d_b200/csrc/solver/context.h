@@ -1039,6 +1039,13 @@ struct flite_ctx {
         if (graph) cudaGraphExecDestroy(graph);
         graph = nullptr;
     }
+    // a launch option was set: the context's graph goes, and a batch that
+    // holds the context sees by the number that its own is out of date
+    unsigned options = 0;
+    void options_changed() {
+        ++options;
+        drop_graph();
+    }
 
     void ensure_graph() {
         if (graph) return;

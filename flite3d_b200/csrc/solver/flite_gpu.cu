@@ -960,9 +960,9 @@ int flite_set_kernel_options(flite_ctx *ctx, int32_t edge_block, int32_t node_bl
     if (!ctx || edge_block < 32 || edge_block > 256 || node_block < 32 || node_block > 256 || edge_block % 32 ||
         node_block % 32 || (gather_unroll != 1 && gather_unroll != 2))
         return FLITE_EINVAL;
-    ctx->drop_graph();
     ctx->eb = edge_block;
     ctx->nb = node_block;
+    ctx->options_changed();
     return FLITE_OK;
 }
 
@@ -976,15 +976,15 @@ int flite_set_tiled_gather(flite_ctx *ctx, int32_t level, int32_t on) {
 int flite_set_gather_fusion(flite_ctx *ctx, int32_t level, int32_t on) {
     if (bad_level(ctx, level) || (on != 0 && on != 1) || level > kMaxLevels) return FLITE_EINVAL;
     ctx->fuse_mode[level - 1] = on ? 1 : -1;
-    ctx->drop_graph();
+    ctx->options_changed();
     return FLITE_OK;
 }
 
 int flite_set_gather_lanes(flite_ctx *ctx, int32_t level, int32_t lanes) {
     if (bad_level(ctx, level) || level > kMaxLevels) return FLITE_EINVAL;
     if (!(lanes == 0 || lanes == 1 || lanes == 4 || lanes == 8 || lanes == 16 || lanes == 32)) return FLITE_EINVAL;
-    ctx->drop_graph();
     ctx->lanes[level - 1] = lanes;
+    ctx->options_changed();
     return FLITE_OK;
 }
 

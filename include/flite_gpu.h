@@ -403,7 +403,9 @@ int flite_profile_level(flite_ctx *ctx, int level, int reps, double *edge_ms,
 /* Launch options of a context (no effect on any result): threads per block
  * of the edge kernels and of the node kernels (32..256, multiples of 32; the
  * central gather with a thread per node takes at most 128).  gather_unroll is
- * 1 or 2 and changes nothing.  Drops the captured cycle graph.              */
+ * 1 or 2 and changes nothing.  Drops the captured cycle graph; the graph of a
+ * batch that holds the context is made anew by the batch's next cycle (so with
+ * the two calls below that set lanes and shared walks).                     */
 int flite_set_kernel_options(flite_ctx *ctx, int32_t edge_block, int32_t node_block, int32_t gather_unroll);
 /* Node numbering of the contexts created after this call (no effect on any
  * result; no reference counterpart): 1 renumbers the nodes of every level

@@ -144,3 +144,39 @@ def test_cases_without_a_group_form_run_alone(gpu):
             s.cycle(cyc)
         assert np.array_equal(s.get_state(1), bs.get_state(1))
         s.close()
+
+
+@pytest.mark.parametrize("member", [0, 1])
+def test_launch_options_of_a_case_reach_the_next_run(gpu, member):
+    # options set on a case after a run (on the case that leads the group, or
+    # on its own graph without groups) change the launches of the next
+    # cycles to those of a batch that had them from the start; no state changes
+    m = Mesh.bump_channel(12, 4, 4, 0.05, nlevels=3)
+    cases = [(default_controls(ReynoldsNumber=0.0, fluxType=1, CFLNumber=2.0, numberOfGridsToUse=3, multigridScheme=3,
+                               alpha=a), m) for a in (0.0, 2.0)]
+    grouping = member == 0
+
+    def make():
+        b = Batch(cases)
+        b.set_grouping(grouping)
+        for (c, mm), bs in zip(cases, b.cases):
+            bs.set_state(initial_state(c, mm, perturb_seed=7, amplitude=0.02))
+            bs.start()
+        return b
+
+    def one_lane(b):
+        for level in (1, 2, 3):
+            b.cases[member].set_gather_lanes(level, 1)
+
+    late, early = make(), make()
+    late.run(orders=50.0, max_cycles=2)
+    before = late.time_cycles(1, cycle_no=3)[1]
+    one_lane(late)
+    late.run(orders=50.0, max_cycles=2, first_cycle=4)
+    one_lane(early)
+    early.run(orders=50.0, max_cycles=5)
+    after = late.time_cycles(1, cycle_no=6)[1]
+    assert after == early.time_cycles(1, cycle_no=6)[1]
+    assert after > before
+    for a, b in zip(late.cases, early.cases):
+        assert np.array_equal(a.get_state(1), b.get_state(1))
