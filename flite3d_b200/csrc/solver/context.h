@@ -4,6 +4,9 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -251,13 +254,16 @@ struct flite_ctx {
         return d_io;
     }
     // ---- results to the caller's arrays ---------------------------------
-    // A pageable array of more than kStageMin bytes is filled from the two
-    // halves of a pinned buffer (StagePool), one emptied while the other is
-    // under way: 0.78 ms to a fresh 8.1 MB array where the driver's own path
-    // takes 1.07 (from pinned memory 0.16; the rest is the array's page
-    // faults).  More threads for the copy cost more to start than they save,
-    // and in the other direction the driver's path is the faster one (0.45
-    // against 0.54 ms).
+    // A pageable array of more than kStageMin bytes whose pages are not there
+    // yet is filled from the two halves of a pinned buffer (StagePool), one
+    // emptied while the other is under way: 2.1 ms to 8.1 MB of fresh pages
+    // where the driver's own path takes 3.5 (from pinned memory 0.16; the rest
+    // is the page faults).  An array written before keeps the driver's path
+    // where it is longer than a piece: 0.48 against 0.53 ms at 8.1 MB, 1.8
+    // against 2.0 at 33 MB, 134 against 152 us at 2 MB; but 81 against 70 us at
+    // 1 MB.  More threads for the copy cost more to start than they save, and
+    // in the other direction the driver's path is the faster one (0.45 against
+    // 0.54 ms).
     static constexpr size_t kStageMin = (size_t)1 << 18, kStagePiece = StagePool::kBytes / 2;
     cudaEvent_t staged[2] = {nullptr, nullptr};
     static bool pageable(const void *p, size_t n) {
@@ -269,8 +275,14 @@ struct flite_ctx {
         }
         return a.type == cudaMemoryTypeUnregistered;
     }
+    // whether the middle page of the n bytes at p (several pages) is there
+    static bool touched(const void *p, size_t n) {
+        const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+        unsigned char there = 1;
+        return mincore((void *)(((uintptr_t)p + n / 2) & ~(page - 1)), page, &there) != 0 || (there & 1);
+    }
     void to_host(void *dst, const void *src, size_t n) {
-        if (!pageable(dst, n)) {
+        if (!pageable(dst, n) || (n > kStagePiece && touched(dst, n))) {
             CK(cudaMemcpyAsync(dst, src, n, cudaMemcpyDeviceToHost, s));
             return;
         }

@@ -141,14 +141,14 @@ class Solver:
         self._ck(self.be.set_state(self._h, level, _ptr(u)), "set_state")
 
     def get_state(self, level=1, out=None):
-        u = np.zeros((self.nvar, self.nodes[level - 1])) if out is None else out
+        u = np.empty((self.nvar, self.nodes[level - 1])) if out is None else out
         assert u.shape == (self.nvar, self.nodes[level - 1]) and u.dtype == np.float64
         assert u.flags["C_CONTIGUOUS"]
         self._ck(self.be.get_state(self._h, level, _ptr(u)), "get_state")
         return u
 
     def get_pressure(self, level=1):
-        p = np.zeros(self.nodes[level - 1])
+        p = np.empty(self.nodes[level - 1])
         self._ck(self.be.get_pressure(self._h, level, _ptr(p)), "get_pressure")
         return p
 
@@ -207,10 +207,17 @@ class Solver:
         self._ck(self.be.forces(self._h, out), "forces")
         return np.array(out[:])
 
+    def _result(self, u, level, like=False):
+        # a result of 5 components per node, which the call writes whole (not
+        # zeroed first: each page would be written twice)
+        if u.shape == (5, self.nodes[level - 1]):
+            return np.empty(u.shape)
+        return np.zeros_like(u) if like else np.zeros((5, u.shape[1]))
+
     def residual_fwd(self, u, level=1):
         """makeRHS of the mean flow (5 components) at the state u of a level."""
         u = np.ascontiguousarray(u, dtype=np.float64)
-        r = np.zeros((5, u.shape[1]))
+        r = self._result(u, level)
         self._ck(self.be.residual_fwd(self._h, level, _ptr(u), _ptr(r)), "residual_fwd")
         return r
 
@@ -218,7 +225,7 @@ class Solver:
         """ubar = (dR/du)^T rbar of residual_fwd (GPU library only)."""
         u = np.ascontiguousarray(u, dtype=np.float64)
         rbar = np.ascontiguousarray(rbar, dtype=np.float64)
-        ub = np.zeros_like(u)
+        ub = self._result(u, level, like=True)
         self._ck(self.be.residual_vjp(self._h, level, _ptr(u), _ptr(rbar), _ptr(ub)), "residual_vjp")
         return ub
 
@@ -247,9 +254,9 @@ class Solver:
         with mu_bar."""
         u = np.ascontiguousarray(u, dtype=np.float64)
         lam = np.ascontiguousarray(lam, dtype=np.float64)
-        ub = np.zeros_like(u)
+        ub = self._result(u, 1, like=True)
         d = self.mesh.level(1)
-        g = [np.zeros((3, d.n_sides)), np.zeros((3, d.n_bsides)), np.zeros(d.n_nodes)] if geometry else None
+        g = [np.empty((3, d.n_sides)), np.empty((3, d.n_bsides)), np.empty(d.n_nodes)] if geometry else None
         gp = [_ptr(a) for a in g] if geometry else [None, None, None]
         m = None if mu is None else np.ascontiguousarray(mu, dtype=np.float64)
         lm = None if lam_mu is None else np.ascontiguousarray(lam_mu, dtype=np.float64)
@@ -305,7 +312,7 @@ class Solver:
         bnd_w_bar (3, B), volume_bar (N), iterations and residual.  The
         sensitivity to node coordinates is Mesh.geometry_vjp of the three."""
         d = self.mesh.level(1)
-        sw, bw, vol = np.zeros((3, d.n_sides)), np.zeros((3, d.n_bsides)), np.zeros(d.n_nodes)
+        sw, bw, vol = np.empty((3, d.n_sides)), np.empty((3, d.n_bsides)), np.empty(d.n_nodes)
         J, it, res = ctypes.c_double(), ctypes.c_int32(), ctypes.c_double()
         self._ck(self.be.adjoint_solve(self._h, self.OBJECTIVES[name], ctypes.c_double(tol), int(max_iter),
                                        ctypes.byref(J), _ptr(sw), _ptr(bw), _ptr(vol), ctypes.byref(it),

@@ -297,3 +297,20 @@ def test_node_order_changes_no_result():
     np.testing.assert_allclose(a[4][0], b[4][0], rtol=1e-12)
     assert np.array_equal(a[4][1], b[4][1]) and np.array_equal(a[4][2], b[4][2])
     np.testing.assert_allclose(a[5], b[5], rtol=1e-12, atol=1e-15)
+
+
+@pytest.mark.parametrize("size", [(24, 8, 8), (48, 16, 16), (83, 29, 31)])
+def test_states_reach_every_kind_of_host_array(size):
+    # below the staged size (81 KB), one piece (566 KB), three pieces and a bit
+    # (3.2 MB); arrays never written, written before, and pinned
+    import torch
+    mesh = Mesh.bump_channel(*size, 0.05, nlevels=1)
+    c = default_controls(ReynoldsNumber=0.0, fluxType=1, numberOfGridsToUse=1)
+    s = Solver(c, mesh)
+    u = np.random.default_rng(3).standard_normal((5, mesh.level(1).n_nodes))
+    s.set_state(u)
+    written = np.full_like(u, 7.0)
+    pinned = torch.empty(u.shape, dtype=torch.float64, pin_memory=True)
+    for out in (None, np.empty_like(u), written, written, pinned.numpy()):
+        assert np.array_equal(s.get_state(out=out), u)
+    s.close()
