@@ -320,7 +320,9 @@ class Solver:
         return dict(J=J.value, side_w_bar=sw, bnd_w_bar=bw, volume_bar=vol, iterations=it.value,
                     residual=res.value)
 
-    def set_kernel_options(self, edge_block=256, node_block=256, gather_unroll=1):
+    def set_kernel_options(self, edge_block=256, node_block=128, gather_unroll=1):
+        """Threads per block of the edge kernels and of the node kernels; the
+        defaults are a new context's own."""
         self._ck(self.be.set_kernel_options(self._h, edge_block, node_block, gather_unroll), "set_kernel_options")
 
     def set_tiled_gather(self, level, mode=1):

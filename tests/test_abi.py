@@ -81,3 +81,26 @@ def test_fortran_interface_module_matches_the_c_abi():
         base = typ._type_ if hasattr(typ, "_length_") else typ
         want.append((name, "double" if base is ctypes.c_double else "int", n))
     assert fields == want
+
+
+def test_kernel_option_defaults_are_the_contexts_own():
+    # set_kernel_options without arguments, or with the edge block alone, gives
+    # a context the blocks that it is created with
+    from flite3d_b200 import Solver
+    src = os.path.join(ROOT, "flite3d_b200", "csrc", "solver", "context.h")
+    with open(src) as f:
+        text = f.read()
+    eb = int(re.search(r"constexpr int kBlock = (\d+);", text).group(1))
+    nb = int(re.search(r"int eb = kBlock, nb = (\d+);", text).group(1))
+    seen = []
+
+    class Recorder:
+        def set_kernel_options(self, handle, *blocks):
+            seen.append(blocks)
+            return _abi.FLITE_OK
+
+    s = Solver.__new__(Solver)
+    s.be, s._h = Recorder(), None
+    s.set_kernel_options()
+    s.set_kernel_options(64)
+    assert seen == [(eb, nb, 1), (64, nb, 1)]
