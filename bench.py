@@ -162,7 +162,8 @@ def group_bytes(mesh, dissipation_weighting=False):
     and its neighbours' reads of an array are one read), an incidence entry
     is 8 bytes (two per interior edge), a boundary incidence 4 (two per
     boundary edge), a CSR offset 4 per node and list:
-      pressure   u (40) in, p (8) and the 48-byte central-flux record out;
+      pressure   the state pass: u (40) in, p (8), the 48-byte central-flux
+                 record and u, v, w, T (32) out;
       timestep   u0..3 (32), p, mu, volume (24), two offsets (8), dt and V/dt
                  out (16); per edge two incidences and wx, wy, wz (24); per
                  boundary edge its two incidences, node pair (8) and
@@ -172,7 +173,6 @@ def group_bytes(mesh, dissipation_weighting=False):
                  (8), dissipation out (40), two offsets; per edge its two
                  incidences twice (and the edge length twice with dissipation
                  weighting);
-      visc_prim  the state (40) in, p and u, v, w, T out (40);
       visc_grad  u, v, w, T (32), volume, p, rho (24), class (1), offsets (8),
                  mu (8) and tau (72) out; per edge two incidences and its
                  coefficients (40); per boundary edge as in timestep (40);
@@ -194,11 +194,10 @@ def group_bytes(mesh, dissipation_weighting=False):
     d = mesh.level(1)
     N, E, B, Nb = d.n_nodes, d.n_sides, d.n_bsides, d.n_bnodes
     return {
-        "pressure": N * (40 + 8 + 48),
+        "pressure": N * (40 + 8 + 48 + 32),
         "timestep": N * (32 + 8 + 8 + 8 + 8 + 16) + E * (16 + 24) + B * (8 + 8 + 24),
         "dissipation": N * (40 + 8 + 8 + 8 + 8 + 40 + 40 + 8 + 40 + 8) + E * 32
         + (E * 16 if dissipation_weighting else 0),
-        "visc_prim": N * (40 + 40),
         "visc_grad": N * (32 + 24 + 1 + 8 + 8 + 72) + E * 40 + B * 40 + Nb * 48,
         "visc_flux": N * (72 + 24 + 64 + 8) + E * 40 + B * 44,
         "node_update": node_kernel_bytes(mesh),

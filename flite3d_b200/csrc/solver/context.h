@@ -496,45 +496,61 @@ struct flite_ctx {
             FLITE_GATHER(k_jst_flux, l, P, V(l));
         }
     }
-    // the time step (ts), the JST dissipation (or its zero) and the viscous
-    // terms of a level, in the order of singleIteration and restrictGrid.
-    // Where a thread serves a node, the time step and the Laplacian share one
-    // walk of the incidence lists (k_ts_lap), and so do the JST flux and the
-    // viscous gradients (k_jflux_vgrad); the viscous primitives, which only
-    // these gradients read, go before the JST flux.
-    // the walks singleIteration's relaxation step shares on level l: 0 none;
-    // 1 k_ts_lap; 2 k_ts_lap and k_jflux_vgrad
-    int step_fusion(int l) {
-        if ((c.dissipationScheme == 1 && V(l).grid == 1) || c.dissipationScheme == 3) return 0;
-        if (!fuse_walks(l) || !jst_gathers(l)) return 0;
-        return (c.ReynoldsNumber > 0.0 && !P.matrixDiss && c.viscosityScheme == 1) ? 2 : 1;
+    // the walks that the scalar dissipation's passes of level l share: 0 none;
+    // 1 time step and Laplacian (k_ts_lap); 2 also JST flux and viscous
+    // gradients (k_jflux_vgrad).  With lanes per node they are always shared.
+    int shared_walks(int l) {
+        if (!(group_level(l) || fuse_walks(l)) || !jst_gathers(l)) return 0;
+        return visc() && !P.matrixDiss && c.viscosityScheme == 1 ? 2 : 1;
     }
-    // `prim`: the viscous primitives are there already.  With lanes per node
-    // the shared walks are always taken, and with `fold` the last part may be
+    // the part of the dissipation that is left to the node pass where it
+    // evaluates the boundary edges (and so does not write the state it reads)
+    int folded(int l, int walks) {
+        if (!inline_bnd(l)) return PRE_NONE;
+        return walks == 2 ? PRE_VISC : walks == 1 && !visc() && !P.matrixDiss ? PRE_JST : PRE_NONE;
+    }
+    void ts_lap(int l) {
+        counted();
+        FLITE_GATHER(k_ts_lap, l, P, V(l));
+    }
+    void jflux_vgrad(int l) {
+        counted();
+        FLITE_GATHER(k_jflux_vgrad, l, P, V(l));
+    }
+    // whether a relaxation step of level l takes its dissipation from
+    // ts_jst_viscous (else from the separate kernels of `dissipation`)
+    bool step_jst(int l) {
+        return !((c.dissipationScheme == 1 && V(l).grid == 1) || c.dissipationScheme == 3);
+    }
+    // whether the state pass at the head of a relaxation step leaves the
+    // boundary fluxes of its first stage
+    bool step_bnd(int l) const { return group_level(l) && !inline_bnd(l) && c.flowType != 2; }
+    // the time step (ts), the JST dissipation (or its zero) and the viscous
+    // terms of a level, in the order of singleIteration and restrictGrid; the
+    // viscous primitives, which only the gradients read, go before the JST
+    // flux.  `prim`: they are there already.  With `fold` the last part may be
     // left to the node pass that follows (the PRE_* returned).
     int ts_jst_viscous(int l, bool ts, bool prim, bool fold) {
-        const bool grp = group_level(l);
-        if ((!grp && !fuse_walks(l)) || !jst_gathers(l)) {
+        const int walks = shared_walks(l);
+        if (!walks) {
             if (ts) timesteps(l);
             jst(l);
             viscous(l, prim);
             return PRE_NONE;
         }
         if (ts) {
-            counted();
-            FLITE_GATHER(k_ts_lap, l, P, V(l));
+            ts_lap(l);
             explicit_step(l);
         } else {
             jst_lap(l);
         }
         if (visc() && !prim) viscous_prim(l);
-        fold = fold && inline_bnd(l);  // (the pass must not write the state it reads)
-        if (visc() && !P.matrixDiss && c.viscosityScheme == 1) {
-            counted();
-            FLITE_GATHER(k_jflux_vgrad, l, P, V(l));
-            if (fold) return PRE_VISC;
+        const int pre = fold ? folded(l, walks) : PRE_NONE;
+        if (walks == 2) {
+            jflux_vgrad(l);
+            if (pre) return pre;
         } else {
-            if (fold && !visc() && !P.matrixDiss) return PRE_JST;
+            if (pre) return pre;
             jst_flux(l);
             if (visc()) {
                 counted();
@@ -797,7 +813,7 @@ struct flite_ctx {
         bool early = false;
         if (calcDiss) {
             early = bnd_beside(l, own || bnd);
-            if ((c.dissipationScheme == 1 && V(l).grid == 1) || c.dissipationScheme == 3) {
+            if (!step_jst(l)) {
                 timesteps(l);
                 dissipation(l);
                 viscous(l, true);
@@ -821,7 +837,7 @@ struct flite_ctx {
             FLITE_LAUNCH(k_case_cycle, (), 1, 1, 0, V(l), d_cycle);
         }
         for (int i = 0; i < nsteps; ++i) {
-            const bool bnd = group_level(l) && !inline_bnd(l) && c.flowType != 2;
+            const bool bnd = step_bnd(l);
             state_pass(l, STATE_STEP | (calcDiss && visc() ? STATE_PRIM : 0), bnd);
             singleIteration(l, calcDiss, bnd);
         }

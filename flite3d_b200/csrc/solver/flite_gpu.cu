@@ -994,29 +994,29 @@ int flite_profile_kernels(flite_ctx *ctx, int level, int reps, double *ms, int32
         flite_ctx &X = *ctx;
         const int l = level - 1;
         LevelView &L = X.V(l);
-        // the kernels of one relaxation step of this level, in cycle order
-        // (with shared walks the time step and Laplacian are timed as
-        // ts_lap, the JST flux and viscous gradients as jflux_vgrad, and
-        // their separate groups hold what is left of them)
-        const int fz = X.step_fusion(l);
-        const bool visc = X.c.ReynoldsNumber > 0;
+        // the kernels that the cycle launches for one relaxation step of this
+        // level, by the same decisions: shared walks are timed as ts_lap and
+        // jflux_vgrad, with the separate groups holding what is left of them,
+        // and a folded part or boundary edges as part of the node update
+        const bool visc = X.visc(), own = X.inline_bnd(l), bnd = X.step_bnd(l);
+        const int fz = X.step_jst(l) ? X.shared_walks(l) : 0, pre = X.folded(l, fz);
         // each group launches its kernels and tells whether it had any (a
         // group without kernels reports 0 ms)
         std::vector<std::function<bool()>> k;
-        k.push_back([&] { X.pressure(l); return true; });
+        k.push_back([&] { X.state_pass(l, visc ? STATE_PRIM : 0, bnd); return true; });
         k.push_back([&] { if (!fz) X.timesteps(l); return !fz; });
         k.push_back([&] {
             if (!fz) X.dissipation(l);
-            else if (fz == 1) X.jst_flux(l);
-            return fz != 2;
+            else if (fz == 1 && !pre) X.jst_flux(l);
+            return !fz || (fz == 1 && !pre);
         });
-        k.push_back([&] { if (visc) X.viscous_prim(l); return visc; });
+        k.push_back([] { return false; });  // the viscous primitives: in the state pass
         k.push_back([&] { if (visc && fz != 2) X.visc_grad(l); return visc && fz != 2; });
-        k.push_back([&] { if (visc) X.visc_flux(l); return visc; });
-        k.push_back([&] { X.rhs_terms(l, true); return true; });
-        k.push_back([&] { X.launch_node_update(l, MODE_RFINE, 0, true); return true; });
-        k.push_back([&] { if (fz) k_ts_lap<1><<<X.nblk(L.N), X.nb, 0, X.s>>>(X.P, L); return fz != 0; });
-        k.push_back([&] { if (fz == 2) k_jflux_vgrad<1><<<X.nblk(L.N), X.nb, 0, X.s>>>(X.P, L); return fz == 2; });
+        k.push_back([&] { if (visc && pre != PRE_VISC) X.visc_flux(l); return visc && pre != PRE_VISC; });
+        k.push_back([&] { X.rhs_terms(l, true, false, bnd || own); return !X.fused() || !(bnd || own); });
+        k.push_back([&] { X.launch_node_update(l, MODE_RFINE, 0, true, pre, own ? IO_BND | IO_LATER : 0); return true; });
+        k.push_back([&] { if (fz) X.ts_lap(l); return fz != 0; });
+        k.push_back([&] { if (fz == 2) X.jflux_vgrad(l); return fz == 2; });
         const int m = std::min<int>((int)k.size(), nmax);
         std::vector<cudaEvent_t> ev(m + 1);
         for (auto &e : ev) CK(cudaEventCreate(&e));

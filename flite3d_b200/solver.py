@@ -345,7 +345,8 @@ class Solver:
                      "flux_terms", "node_update", "ts_lap", "jflux_vgrad")
 
     def profile_kernels(self, level=1, reps=10):
-        """{kernel group: average device ms} over one relaxation step of a level."""
+        """{kernel group: average device ms} of the kernels that the cycle runs
+        for one relaxation step of a level (0 for a group without kernels)."""
         ms = (ctypes.c_double * 16)()
         n = ctypes.c_int32()
         self._ck(self.be.profile_kernels(self._h, level, reps, ms, 16, ctypes.byref(n)), "profile_kernels")

@@ -428,14 +428,19 @@ int flite_set_tiled_gather(flite_ctx *ctx, int32_t level, int32_t on);
  * separate kernels; without this call levels of at most 220,000 nodes share.
  * No effect on any result.  Drops the captured cycle graph.                 */
 int flite_set_gather_fusion(flite_ctx *ctx, int32_t level, int32_t on);
-/* Average device ms of the kernel groups of one relaxation step of a level,
- * in order: pressure, time steps, dissipation, viscous primitives, viscous
- * gradients, viscous fluxes, flux terms (edge or boundary kernels), node
- * update (restrictGrid's fine-increment mode: the stage's read set), the
- * shared walk of time step and Laplacian, the shared walk of JST flux and
- * viscous gradients (where the walks are shared, the separate groups hold
- * what is left of them); *n is the number written (at most nmax).  The
- * level's rhs and dissipation are overwritten.                              */
+/* Average device ms of the kernel groups that the cycle runs for one
+ * relaxation step of the mean flow on a level, in order: the state pass
+ * (pressure, records, viscous primitives and, where the level's passes take
+ * them from there, boundary fluxes), time steps, dissipation, 0 (the viscous
+ * primitives' own pass of earlier versions), viscous gradients, viscous
+ * fluxes, flux terms (edge or boundary kernels), node update (restrictGrid's
+ * fine-increment mode: the stage's read set; with lanes per node the first
+ * stage's form, which holds the last part of the dissipation and the boundary
+ * edges), the shared walk of time step and Laplacian, the shared walk of JST
+ * flux and viscous gradients (where the walks are shared, the separate groups
+ * hold what is left of them).  A group that the level does not launch has 0;
+ * *n is the number written (at most nmax).  The level's rhs and dissipation
+ * are overwritten.                                                          */
 int flite_profile_kernels(flite_ctx *ctx, int level, int reps, double *ms, int32_t nmax, int32_t *n);
 
 #ifdef __cplusplus

@@ -314,3 +314,28 @@ def test_states_reach_every_kind_of_host_array(size):
     for out in (None, np.empty_like(u), written, written, pinned.numpy()):
         assert np.array_equal(s.get_state(out=out), u)
     s.close()
+
+
+# the groups of one relaxation step by the shape of the level's gathers: what
+# the cycle shares or folds is not timed as kernels that it does not launch
+STEP_GROUPS = {
+    ("central_jst", 8): {"pressure", "ts_lap", "node_update"},
+    ("central_jst", 1): {"pressure", "ts_lap", "dissipation", "flux_terms", "node_update"},
+    ("laminar_adiabatic", 8): {"pressure", "ts_lap", "jflux_vgrad", "node_update"},
+    ("laminar_adiabatic", 1): {"pressure", "ts_lap", "jflux_vgrad", "visc_flux", "flux_terms", "node_update"},
+    ("laminar_visc2_adiabatic", 8): {"pressure", "ts_lap", "dissipation", "visc_grad", "visc_flux", "node_update"},
+    ("matrix_dissipation", 8): {"pressure", "ts_lap", "dissipation", "node_update"},
+    ("first_order_diss", 8): {"pressure", "timestep", "dissipation", "node_update"},
+    ("hllc2_autoclip", 8): {"pressure", "timestep", "dissipation", "flux_terms", "node_update"},
+}
+
+
+@pytest.mark.parametrize("name,lanes", list(STEP_GROUPS))
+def test_profiled_groups_are_the_kernels_of_the_cycle(name, lanes):
+    mesh = Mesh.bump_channel(24, 8, 8, 0.05, nlevels=3)
+    c, g, o = make_pair(mesh, **CASES[name])
+    g.set_gather_lanes(1, lanes)
+    u = g.get_state(1)
+    ms = g.profile_kernels(1, reps=2)
+    assert {k for k, v in ms.items() if v > 0} == STEP_GROUPS[name, lanes]
+    assert np.array_equal(g.get_state(1), u)
