@@ -182,6 +182,9 @@ struct flite_ctx {
     int *h_cycle = nullptr;    // pinned
     double *h_out = nullptr;  // pinned: the last kernel of a reduction writes here (kOut values)
     static constexpr int kOut = 2048;
+    // a GMRES iteration leaves two passes of restart + 1 dot products and a norm there
+    static constexpr int kMaxRestart = 500;
+    static_assert(2 * (kMaxRestart + 1) + 1 <= kOut, "the GMRES results fit the pinned buffer");
     cudaGraphExec_t graph = nullptr;
     int64_t launches = 0;
     bool counting = false;

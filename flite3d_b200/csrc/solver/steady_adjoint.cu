@@ -1888,7 +1888,7 @@ extern "C" int flite_objective(flite_ctx *ctx, int objective, double *J) {
 }
 
 extern "C" int flite_set_adjoint_method(flite_ctx *ctx, int method, int restart) {
-    if (!ctx || method < 0 || method > 1 || (method == 1 && (restart < 1 || restart > 500))) return FLITE_EINVAL;
+    if (!ctx || method < 0 || method > 1 || (method == 1 && (restart < 1 || restart > flite_ctx::kMaxRestart))) return FLITE_EINVAL;
     ctx->adj_method = method;
     if (method == 1) ctx->adj_restart = restart;
     return FLITE_OK;

@@ -335,3 +335,13 @@ def test_mixed_precision_solution_has_the_fp64_sensitivities(lam):
     assert abs(r1["J"] - r0["J"]) <= 1e-10 * abs(r0["J"])
     for k in ("side_w_bar", "bnd_w_bar"):
         assert np.abs(r1[k] - r0[k]).max() <= 1e-8 * np.abs(r0[k]).max()
+
+
+def test_restart_lengths_within_the_result_buffer():
+    mesh = Mesh.bump_channel(6, 2, 2, 0.05, nlevels=1)
+    s = Solver(controls(numberOfGridsToUse=1), mesh)
+    for m in (1, 500):
+        s.set_adjoint_method("gmres", restart=m)
+    for m in (0, 501):
+        with pytest.raises(RuntimeError, match="status 1"):
+            s.set_adjoint_method("gmres", restart=m)
