@@ -345,3 +345,53 @@ def test_restart_lengths_within_the_result_buffer():
     for m in (0, 501):
         with pytest.raises(RuntimeError, match="status 1"):
             s.set_adjoint_method("gmres", restart=m)
+
+
+# ---- every gather shape of the reverse sweeps ------------------------------
+
+def generic_state(c, mesh):
+    u = initial_state(c, mesh, perturb_seed=3, amplitude=0.02)
+    return u + np.random.default_rng(7).standard_normal(u.shape) * 0.01
+
+
+@pytest.mark.parametrize("ctl", [dict(), dict(boundaryTerm=0), LAMINAR], ids=["euler", "fv_boundary", "laminar"])
+def test_every_gather_shape_gives_the_same_sweep(ctl):
+    """A thread and groups of 4 to 32 lanes per node add the same terms in the
+    same order: equal products.  Node counts leave a partly filled last group."""
+    mesh = Mesh.bump_channel(17, 7, 6, 0.05, nlevels=1)
+    c = controls(numberOfGridsToUse=1, **ctl)
+    g = Solver(c, mesh)
+    u = generic_state(c, mesh)
+    lam = np.random.default_rng(5).standard_normal(u.shape)
+    visc = {}
+    if ctl is LAMINAR:
+        mu = np.full(u.shape[1], 1.0 / 500.0) * (1 + 0.05 * np.random.default_rng(3).standard_normal(u.shape[1]))
+        visc = dict(mu=mu, lam_mu=np.random.default_rng(8).standard_normal(u.shape[1]) * 1e2)
+    want = None
+    for lanes in (1, 4, 8, 16, 32):
+        g.set_gather_lanes(1, lanes)
+        g.set_state(u)
+        g.start()
+        got = g.iteration_vjp(u, lam, geometry=True, **visc) + (g.residual_vjp(u, lam),)
+        assert all(np.all(np.isfinite(a)) for a in got)
+        want = want or got
+        for a, b in zip(want, got):
+            assert np.array_equal(a, b), lanes
+
+
+@pytest.mark.parametrize("ctl", [dict(), LAMINAR], ids=["euler", "laminar"])
+def test_sweep_of_a_level_with_a_thread_per_node(ctl):
+    """28,750 nodes: a thread per node by default, and edges that the device
+    numbers by rows (the sensitivities come back in the caller's order)."""
+    mesh = Mesh.bump_channel(45, 24, 24, 0.05, nlevels=1)
+    assert mesh.level(1).n_nodes > 24576
+    c = controls(numberOfGridsToUse=1, **ctl)
+    g, o = Solver(c, mesh), Solver(c, mesh, backend=oracle_backend())
+    u = generic_state(c, mesh)
+    for s in (g, o):
+        s.set_state(u)
+        s.start()
+    if ctl is LAMINAR:
+        laminar_dot_check(g, o, u, viscosity_of(o, u), 1)
+    else:
+        dot_check(g, o, u, 1)
