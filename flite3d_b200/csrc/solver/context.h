@@ -446,10 +446,12 @@ struct flite_ctx {
     // the node pass leaves the pressure (and records) of the next stage; with
     // engines the pass of the inlet nodes ends later (k_engine_finish)
     bool emits() const { return !P.engines; }
-    // the node pass evaluates the boundary edges: lanes per node, the FP64
-    // central flux of a static mesh without engines; the Spalart-Allmaras
-    // kernels between the stages read the state in u
-    bool inline_bnd(int l) const { return group_level(l) && fused() && !mixed() && !sa() && emits(); }
+    // runs whose levels with lanes per node alternate the copies of the state:
+    // the FP64 central flux of a static mesh without engines (the
+    // Spalart-Allmaras kernels between the stages read the state in u)
+    bool alternates() const { return fused() && !mixed() && !sa() && emits(); }
+    // the node pass evaluates the boundary edges
+    bool inline_bnd(int l) const { return group_level(l) && alternates(); }
     // makeTimeSteps's ivd%physicalTimeStep under explicit time stepping
     // (unsteady runs read it; steady ones never do)
     void explicit_step(int l) {

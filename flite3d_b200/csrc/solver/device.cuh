@@ -155,7 +155,7 @@ struct LevelView {
     double *u, *uprev, *rhs, *src, *diss;  // [5][N]
     // the state and records between the stages of a step: a stage that reads
     // its neighbours' values writes the other copy (StageIO, kernels.h)
-    double *ub;                            // [5][N] (levels with group gathers)
+    double *ub;                            // [5][N] (flite_ctx::alternates)
     NodeRec *qb;                           // [N] (central flux)
     DeltaRec *dqb;                         // [N] (FLITE_MIXED)
     double *p, *dt, *mu;                   // [N]

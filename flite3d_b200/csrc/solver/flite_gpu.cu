@@ -534,9 +534,10 @@ int flite::create_context(const flite_controls *c, int nlevels, const flite_leve
             L.q = X.alloc<NodeRec>(N);
             CK(cudaMemset(L.q, 0, (size_t)N * sizeof(NodeRec)));
             // the other copies of the records and of the state that the stages
-            // alternate (any level may be given lanes per node later)
+            // alternate (of the state on every level: any may be given lanes per
+            // node later, for its own run or as a member of a case group)
             L.qb = X.fused() && !X.mixed() ? X.alloc<NodeRec>(N) : nullptr;
-            L.ub = X.fused() && !X.mixed() ? X.alloc<double>(5 * (size_t)N) : nullptr;
+            L.ub = X.alternates() ? X.alloc<double>(5 * (size_t)N) : nullptr;
             L.dqb = nullptr;
             // stress and heat flux (scheme 1), or the scaled gradients with mu
             // and k (scheme 2)
