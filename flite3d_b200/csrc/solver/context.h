@@ -804,7 +804,9 @@ struct flite_ctx {
             }
             FLITE_NODE(GATHER_CENTRAL, PRE_NONE);
         } else {
-            FLITE_NODE(GATHER_BUFFER, PRE_NONE);
+            no_group("the edge buffer's fluxes");
+            const unsigned nt = blk(GATHER_BUFFER);
+            k_node_update<GATHER_BUFFER, U><<<grid(nt), nt, 0, s>>>(P, V(l), mode, stage, io);
         }
 #undef FLITE_NODE
     }

@@ -2109,7 +2109,7 @@ __global__ void __launch_bounds__(node_threads(PREC, U), U > 1 ? 2 : (central_ah
     FLITE_BOTH(k_visc2_flux, (U, ))                                                          \
     FLITE_BOTH(k_ts_lap, (U, ))                                                              \
     FLITE_BOTH(k_jflux_vgrad, (U, ))                                                         \
-    FLITE_NODE_INST(GATHER_BUFFER, U, PRE_NONE)                                              \
+    template __global__ void k_node_update<GATHER_BUFFER, U>(Params, LevelView, int, int, int); \
     FLITE_NODE_INST(GATHER_CENTRAL, U, PRE_NONE)                                             \
     FLITE_NODE_INST(GATHER_ANCHOR, U, PRE_NONE)                                              \
     FLITE_NODE_INST(GATHER_DELTA, U, PRE_NONE)
@@ -2146,12 +2146,6 @@ template __global__ void k_prolong_fine<false>(Params, LevelView, LevelView);
 template __global__ void k_prolong_fine<true>(CaseTab<Params>, CaseTab<LevelView>, CaseTab<LevelView>);
 template __global__ void k_inject_u<false>(LevelView, LevelView);
 template __global__ void k_inject_u<true>(CaseTab<LevelView>, CaseTab<LevelView>);
-
-// ---- copy u -> uprev (doTimeIterations def_par:983-987) -------------------
-__global__ void k_copy(const double *a, double *b, size_t n) {
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) b[i] = a[i];
-}
 
 // mapFineToCoarse (def_par:12572-12596) as a gather over each coarse node's
 // children in increasing fine order: the same additions in the same order as

@@ -113,7 +113,6 @@ __global__ void k_move_edges(int E, const int *slot, const int2 *in, int2 *out);
 __global__ void k_put_edges(int E, const int *slot, const double *w, double *wx, double *wy, double *wz, EdgeW *ew);
 __global__ void k_put_edge_values(int E, const int *slot, const double *in, double *out);
 __global__ void k_make_inc32(const int2 *inc, const EdgeW *ew, int n, IncRec32 *o);
-__global__ void k_copy(const double *a, double *b, size_t n);
 template <bool B = false>
 __global__ void k_restrict_u(CaseArg<B, LevelView> C, CaseArg<B, LevelView> F);
 __global__ void k_restrict_arr(LevelView C, LevelView F, const double *fsrc, double *cdst, int ncomp);
