@@ -397,10 +397,13 @@ struct flite_ctx {
     // default the widest group that keeps the level's threads within
     // kLaneThreads: below that a thread per node leaves SMs idle and each
     // thread waits on a long chain of dependent loads, above it the extra
-    // lanes only add instructions.  Sums of one relaxation step's kernels on the
-    // bump channel's agglomerated levels (us, lanes 1/4/8/32): 1,908 nodes
-    // 179/123/97/91, 21,972 193/163/164/227, 237,662 325/619/823/1856; on
-    // generated level-1 meshes 4,225 nodes 97/93/86/94, 32,269 99/123/144/250.
+    // lanes only add instructions.  Kernels of one relaxation step (laminar,
+    // flite_profile_kernels, us, lanes 1/4/8/16/32) on the bump channel's
+    // agglomerated levels: 1,908 nodes 170/94/66/56/54, 21,972
+    // 185/128/121/140/184, 237,662 313/555/738/1027/1623; on generated level-1
+    // meshes 4,225 nodes 88/61/53/53/59, 14,161 90/67/70/82/113, 33,327
+    // 92/94/108/143/214.  Whole cycles order them alike (four levels, 2,099,065
+    // nodes: 6.39/6.22/6.21/6.38/6.84 ms by the lanes of the 21,972-node level).
     // A case group's cases share the launch.
     int lanes[kMaxLevels] = {0};
     int lanes_of(int l) const {
@@ -694,7 +697,11 @@ struct flite_ctx {
     // fluxes, and with Spalart-Allmaras the diffusion (`diff`: 0 none, 1, 2
     // with the turbulent time steps) and the nu~ part beside both.  With
     // `bnd_forked` the boundary fluxes are under way already.  The branches
-    // pay where launches are short: the RANS cycle's four coarse levels.
+    // pay where launches are short, the RANS cycle's four coarse levels, and
+    // cost at the graph's instantiation: the boundary branches of the upwind
+    // cycle on 14,161 nodes take 0.096 ms off each cycle (0.576 -> 0.480) and
+    // put 1.15 ms on the first (1.32 -> 2.47), won back in twelve cycles; on
+    // 203,401 nodes (W-cycle) 0.123 and 1.87 ms, fifteen.
     void residual_pass(int l, int mode, int stage, bool anchor, bool delta, bool bnd, bool bnd_forked, int diff, int pre,
                        int io) {
         const int kb = pass_branch, ks = pass_branch + 1;
@@ -730,7 +737,7 @@ struct flite_ctx {
             case 2: k_edge_flux<2, false><<<ng, eb, 0, s>>>(P, L); break;
             case 3:
                 // the extension: MUSCL on level 1, upwind first order below
-                if (P.recon == FLITE_RECON_VAN_ALBADA && L.grid == 1)  // 256 threads: its store staging
+                if (P.recon == FLITE_RECON_VAN_ALBADA && L.grid == 1)
                     k_edge_flux_muscl<<<(unsigned)((L.E + kMusclThreads - 1) / kMusclThreads), kMusclThreads, 0, s>>>(P, L);
                 else if (P.recon == FLITE_RECON_VAN_ALBADA) k_edge_flux<3, true><<<ng, eb, 0, s>>>(P, L);
                 else k_edge_flux<3, false><<<ng, eb, 0, s>>>(P, L);

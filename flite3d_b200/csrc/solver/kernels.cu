@@ -84,8 +84,8 @@ __global__ void k_state_pass(CaseArg<B, Params> P_, CaseArg<B, LevelView> L_, in
 }
 
 // ---- makeTimeSteps (def_par:13335-13610) as a node gather -----------------
-// The pieces of a thread-per-node gather, shared by the separate kernel, its
-// incidence-row form and the fused walks below.
+// The pieces of the gather, shared by the separate kernel and the fused walks
+// below, with a thread or a group of lanes per node.
 //
 // interior edge t of node i (momentum m, 1/rho ro, cc = max(gamma p/rho,
 // 0.001)): the convective and acoustic terms, and with viscosity the other
@@ -1378,13 +1378,21 @@ __global__ void k_minmax(Params P, LevelView L) {
 }
 
 // ---- interior edge flux into the edge buffer ------------------------------
-// What bounds the HLLC order-2 kernel: FP64 instructions (two limited, clipped
-// reconstructions, some twenty divisions and fifteen square roots an edge),
-// not memory (2.6 % of DRAM, 10 % of L1).  With the limiter's and the wave
-// regions' two-sided branches run once instead of per side, and 7 blocks of
-// 128 threads (72 registers; the spills cost less than 2 blocks of 256 at 128
-// registers), the RANS cycle on 738,100 nodes takes 9.8 ms (12.2 before; 10.5
-// with the 128 registers), the HLLC cycle on 80,640 nodes 1.17 ms (1.63).
+// What bounds the HLLC order-2 kernel: the chains of dependent FP64
+// instructions (two limited, clipped reconstructions, some twenty divisions
+// and fifteen square roots an edge: 2,850 thread instructions) and the loads
+// between them, not a rate (on 5,094,100 edges 0.87 ms with 46 % of the issue
+// slots, 28 % of the FP64 pipe, 35 % of L1 and 10 % of DRAM in use at 43 % of
+// the warps; 1.25 ms and 3,800 instructions with two-sided branches).  The
+// limiter's and the wave regions' branches run once instead of per side, in 7
+// blocks of 128 threads (72 registers; the spills cost less than 2 blocks of
+// 256 at 128 registers): the RANS cycle on 738,100 nodes 12.2 -> 9.8 ms (10.5
+// with the 128 registers), the HLLC cycle on 80,640 nodes 1.63 -> 1.17 ms.
+// The other fluxes take three blocks of 256 (80 registers, 48 to 76 bytes of
+// spills in Roe and HLLC order 1) for the loads in flight: 815,425 nodes with
+// three blocks and without a bound (106 to 150 registers), us: central (moving
+// meshes) 126 and 164, LLF 140 and 140, Roe 173 and 222, HLLC order 1 215 and
+// 276; 14,161 nodes 8.7 and 9.0, 9.1 and 9.2, 9.6 and 11.0, 10.9 and 11.5.
 // The block's fluxes (at most 256 x 5) are staged in shared memory and
 // written as one contiguous run of 16-byte stores; the block size is even,
 // so the run starts on a 16-byte boundary.
@@ -1417,8 +1425,9 @@ template __global__ void k_edge_flux<4, false>(Params, LevelView);
 template __global__ void k_edge_flux<4, true>(Params, LevelView);
 
 // the upwind extension's level-1 edge flux into the edge buffer, stored as
-// k_edge_flux stores.  Bound by L1 and FP64 latency, so by the warps in
-// flight; cycles of a mid-size case (ms) with 256 threads and 2, 3 blocks
+// k_edge_flux stores.  Bound by FP64 latency, so by the warps in flight (283 us
+// for 5,591,360 edges: FP64 pipe 56 %, L1 49 %, DRAM 24 %, 42 % of the warps);
+// cycles of a mid-size case (ms) with 256 threads and 2, 3 blocks
 // 2.66, 2.44, with 128 threads and 4 to 8 blocks 2.62, 2.47, 2.42, 2.39
 // (7 blocks, 40 bytes of spills), 2.42.
 __global__ void __launch_bounds__(kMusclThreads, 7) k_edge_flux_muscl(Params P, LevelView L) {
